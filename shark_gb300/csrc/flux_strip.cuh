@@ -1,7 +1,7 @@
 // flux_strip.cuh -- K1 for 2D grids: barrier-free "column march" of one warp per strip.
 //
 // A warp owns 32 consecutive columns (lane = column) of one species and walks up a strip of
-// STRIP_H rows.  Each iteration loads one new row of conserved values (one coalesced 128-byte
+// p.strip_h rows.  Each iteration loads one new row of conserved values (one coalesced 128-byte
 // access per variable), converts it to primitives and keeps a sliding window of three rows in
 // registers.  The middle row is then predicted (limited slopes: y neighbours from the window,
 // x neighbours by warp shuffle), its x-face fluxes are solved between neighbouring lanes
@@ -11,14 +11,17 @@
 //
 // Same per-cell algorithm and expressions as flux_tile.cuh (ctoprim solve.f90:195-253, predictor
 // godunov.f90:7-629, add_delta_u godunov.f90:659-750, kick force_kicks.f90:2-41, polar sources
-// source_terms.f90:37-47); the FP64 instantiation keeps the oracle's operation order.
+// source_terms.f90:37-47).  The FP64 instantiation rounds as the oracle's operation order does; it
+// is bound by the number of FP64 instructions, so its quotients share reciprocals, its compares run
+// on the bit patterns and scalings by 1/2 are folded into constants (fp64.cuh; all exact): SI
+// 1024^2 x 8 15.0 -> 6.7 ms.
 #pragma once
 
 namespace shark {
 
 constexpr int STRIP_UX = 28;     // columns updated per warp
-constexpr int STRIP_H = 32;      // rows updated per warp
-constexpr int STRIP_WARPS = 4;   // warps per CTA (along y)
+constexpr int STRIP_H = 32;      // rows updated per warp on the mixed path (strip_heights on the FP64 path)
+constexpr int STRIP_WARPS = 4;   // warps per CTA (along y) on the mixed path, one on the FP64 path
 
 template <typename R>
 __device__ __forceinline__ R shfl_up1(R v) { return __shfl_up_sync(0xffffffffu, v, 1); }
@@ -34,9 +37,9 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
     const int lane = threadIdx.x & 31;
     const int ax0 = p.ng + bx * STRIP_UX;      // first active column updated by this warp
     const int gx = ax0 - 2 + lane;             // this lane's column (>= 0)
-    const int ay0 = p.ng + by * STRIP_H;       // first active row updated by this warp
+    const int ay0 = p.ng + by * p.strip_h;     // first active row updated by this warp
     if (ay0 >= p.ng + p.ny) return;            // whole warp beyond the domain (uniform)
-    const int ylast = min(ay0 + STRIP_H, p.ng + p.ny) - 1;
+    const int ylast = min(ay0 + p.strip_h, p.ng + p.ny) - 1;
     const int gxc = min(gx, p.nx_max - 1);
     const bool col_in = gx < p.nx_max;
     const bool col_pred = lane >= 1 && lane <= 30 && gx <= p.nx_max - 2;                 // slopes defined
@@ -60,7 +63,43 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
     const R vol = p.vol[gxc], rvol = p.rvol[gxc];
     const R cs_col = p.cs[gxc];
     const R dxl = dx1, dyl = (polar ? radc : R(1)) * dx2;
-    const R hdt = half * dt, hdx = half * dxl, hdy = half * dyl, dtv = dt * rvol;   // mixed path
+    // scaling by 1/2 is exact, so half * a * b rounds as a * (half * b) does
+    const R hdt = half * dt, hdx = half * dxl, hdy = half * dyl;
+    // FP64: the halved denominators of the x slopes (2 d / (dx + dx') = d / ((dx + dx') / 2) exactly;
+    // along y the half is dx2 itself), and the reciprocals of the grid's denominators for div64
+    const bool even_x = __all_sync(0xffffffffu, dx1l == dx1 && dx1r == dx1);
+    R bxl = R(0), bxr = R(0), yxl = R(0), yxr = R(0), yy = R(0), yr = R(0), yvol = R(0), yg1 = R(0), ff1 = R(0), ff2 = R(0);
+    if constexpr (!FAST) {
+        bxl = half * (dx1 + dx1l); bxr = half * (dx1r + dx1);
+        yxl = rcp64(bxl); yxr = rcp64(bxr); yy = rcp64(dx2); yvol = rcp64(vol);
+        yg1 = rcp64(gamma - R(1));
+        if (polar) yr = rcp64(radc);
+        // the force's parts that a row does not change (setup_force's terms, in its order)
+        if (p.setup == SHARK_SETUP_SI) {
+            ff1 = R(2) * p.si_q * sq(p.si_om) * (p.xpos[gxc] - half * p.box_l);
+            ff2 = R(2) * p.si_r0 * p.si_om * p.si_eta;
+        } else if (p.setup == SHARK_SETUP_DISK_POLAR) {
+            ff1 = p.fgrav[gxc];
+        }
+    }
+    auto over_vol = [&](R x) -> R { if constexpr (FAST) return x * rvol; else return div64(x, vol, yvol); };
+    // slopes at one row from the differences to both neighbours
+    auto slope_x = [&](R dl, R dr) -> R {
+        if constexpr (FAST) return slope_limit_t<ST>(dl * sfl, dr * sfr);
+        else {
+            // minmod takes one of the two quotients and division keeps their order
+            if (ST == 1 && even_x) return div64(limit_minmod_d(dl, dr), bxl, yxl);
+            return slope_limit_t<ST>(div64(dl, bxl, yxl), div64(dr, bxr, yxr));
+        }
+    };
+    auto slope_y = [&](R dl, R dr) -> R {
+        if constexpr (FAST) return slope_limit_t<ST>(dl * sfy, dr * sfy);
+        else {
+            const R s = ST == 1 ? div64(limit_minmod_d(dl, dr), dx2, yy)
+                                : slope_limit_t<ST>(div64(dl, dx2, yy), div64(dr, dx2, yy));
+            return polar ? div64(s, radc, yr) : s;
+        }
+    };
 
     R q0[NV], q1[NV], q2[NV];       // primitive rows P-1, P, P+1 (P = row being predicted)
     R c0 = R(0), c1 = R(0), c2 = R(0);
@@ -95,22 +134,33 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                 const R ir = R(1) / rho;
                 vx = px * ir; vy = py * ir; vz = pz * ir;
                 P = fmax2((gamma - R(1)) * (us[4] - half * (px * vx + py * vy + pz * vz)), smallP);
+                const R qrho = fmax2(rho, smallR);
+                if (!iso) c = sqrt(gamma * P / qrho);
+                else { c = cs_at(row); P = rho * sq(c); }
+                q[0] = qrho;
             } else {
-                vx = px / rho; vy = py / rho; vz = pz / rho;
-                const R ekin = half * rho * sq(px / rho) + half * rho * sq(py / rho) + half * rho * sq(pz / rho);
-                P = fmax2((gamma - R(1)) * (us[4] - ekin - R(0)), smallP);
+                const R y = rcp64(rho);
+                vx = div64(px, rho, y); vy = div64(py, rho, y); vz = div64(pz, rho, y);
+                q[0] = max64(rho, smallR);
+                if (iso) {
+                    c = cs_at(row);
+                    P = rho * sq(c);
+                } else {
+                    const R hr = half * rho;
+                    const R ekin = hr * sq(vx) + hr * sq(vy) + hr * sq(vz);
+                    P = max64((gamma - R(1)) * (us[4] - ekin), smallP);
+                    c = sqrt(div64(gamma * P, q[0], q[0] == rho ? y : rcp64(q[0])));
+                }
             }
-            const R qrho = fmax2(rho, smallR);
-            if (!iso) c = sqrt(gamma * P / qrho);
-            else { c = cs_at(row); P = rho * sq(c); }
-            q[0] = qrho; q[1] = vx; q[2] = vy; q[3] = vz; q[4] = P;
+            q[1] = vx; q[2] = vy; q[3] = vz; q[4] = P;
         } else {
             q[0] = us[0];
             if constexpr (FAST) {
                 const R ir = R(1) / us[0];
                 q[1] = us[1] * ir; q[2] = us[2] * ir; q[3] = us[3] * ir;
             } else {
-                q[1] = us[1] / us[0]; q[2] = us[2] / us[0]; q[3] = us[3] / us[0];
+                const R y = rcp64(us[0]);
+                q[1] = div64(us[1], us[0], y); q[2] = div64(us[2], us[0], y); q[3] = div64(us[3], us[0], y);
             }
         }
     };
@@ -146,14 +196,8 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
             if (IS_GAS && k == 4 && iso) continue;   // isothermal: the pressure slopes are rho's times cs^2
             const R ql = shfl_up1(q1[k]), qr = shfl_dn1(q1[k]);
             if constexpr (ST > 0) {
-                if constexpr (FAST) {
-                    dqx[k] = slope_limit_t<ST>((q1[k] - ql) * sfl, (qr - q1[k]) * sfr);
-                    dqy[k] = slope_limit_t<ST>((q1[k] - q0[k]) * sfy, (q2[k] - q1[k]) * sfy);
-                } else {
-                    dqx[k] = slope_limit_t<ST>(R(2) * (q1[k] - ql) / (dx1 + dx1l), R(2) * (qr - q1[k]) / (dx1r + dx1));
-                    dqy[k] = slope_limit_t<ST>(R(2) * (q1[k] - q0[k]) / (dx2 + dx2), R(2) * (q2[k] - q1[k]) / (dx2 + dx2)) /
-                             (polar ? radc : R(1));
-                }
+                dqx[k] = slope_x(q1[k] - ql, qr - q1[k]);
+                dqy[k] = slope_y(q1[k] - q0[k], q2[k] - q1[k]);
             }
         }
         R r_rho = q1[0], u = q1[1], v = q1[2], w = q1[3];
@@ -162,12 +206,34 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
         R f1 = R(0), f2 = R(0), f3 = R(0);   // force of row P; the kick of row P below reuses it
         if (fk) {
             const bool active = col_active && P >= p.ng && P < p.ng + p.ny;
-            if (active) setup_force(p, s, gxc, (long long)P * pitch + gxc, u, w, f1, f2, f3);   // ghost cells keep force = 0 (SI/setup.f90:339)
-            u = u + f1 * half * dt;
-            v = v + f2 * half * dt;
-            w = w + f3 * half * dt;
+            // ghost cells keep force = 0 (SI/setup.f90:339)
+            if constexpr (FAST) {
+                if (active) setup_force(p, s, gxc, (long long)P * pitch + gxc, u, w, f1, f2, f3);
+                u = u + f1 * half * dt;
+                v = v + f2 * half * dt;
+                w = w + f3 * half * dt;
+            } else {
+                // setup_force with the components a setup has
+                if (p.setup == SHARK_SETUP_SI) {
+                    const R om2 = R(2) * p.si_om;
+                    if (active) {
+                        f1 = ff1 - om2 * w;
+                        if (IS_GAS) f1 = f1 - ff2;
+                        f3 = om2 * u;
+                    }
+                    u = u + f1 * hdt;
+                    w = w + f3 * hdt;
+                } else if (p.setup == SHARK_SETUP_DISK_POLAR) {
+                    if (active) f1 = ff1;
+                    u = u + f1 * hdt;
+                } else if (p.setup == SHARK_SETUP_DISK_CART) {
+                    if (active) { f1 = p.cfx[(long long)P * pitch + gxc]; f2 = p.cfy[(long long)P * pitch + gxc]; }
+                    u = u + f1 * hdt;
+                    v = v + f2 * hdt;
+                }
+            }
         }
-        auto over_r = [&](R x) -> R { if constexpr (FAST) return x * irp; else return x / radc; };
+        auto over_r = [&](R x) -> R { if constexpr (FAST) return x * irp; else return div64(x, radc, yr); };
         R qmx[NV], qpx[NV], qmy[NV], qpy[NV];
         R sr0 = -u * drx - v * dry - (dux + dvy) * r_rho;
         if (IS_GAS) {
@@ -177,52 +243,33 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                 dpx = dqx[0] * sq(c1);
                 dpy = dqy[0] * sq(c1);
             }
-            R sp0 = -u * dpx - v * dpy - (dux + dvy) * gamma * pp;
             R dpx_r, dpy_r;
             if constexpr (FAST) { const R ir = R(1) / r_rho; dpx_r = dpx * ir; dpy_r = dpy * ir; }
-            else { dpx_r = (dpx) / r_rho; dpy_r = (dpy) / r_rho; }
+            else { const R y = rcp64(r_rho); dpx_r = div64(dpx, r_rho, y); dpy_r = div64(dpy, r_rho, y); }
             R su0 = -u * dux - v * duy - dpx_r;
             R sv0 = -u * dvx - v * dvy - dpy_r;
             R sw0 = -u * dwx - v * dwy;
             if (polar) {
                 sr0 = -u * drx - v * dry - (dux + dvy) * r_rho - over_r(r_rho * u);
-                sp0 = -u * dpx - v * dpy - (dux + dvy) * gamma * pp - over_r(gamma * pp * u);
                 su0 = -u * dux - v * duy - dpx_r + over_r(sq(v));
                 sv0 = -u * dvx - v * dvy - dpy_r - over_r(u * v);
             }
-            if constexpr (FAST) {
-                const R b0 = r_rho + hdt * sr0, b1 = u + hdt * su0, b2 = v + hdt * sv0, b3 = w + hdt * sw0, b4 = pp + hdt * sp0;
-                qmx[0] = b0 + hdx * drx; qpx[0] = b0 - hdx * drx;
-                qmx[1] = b1 + hdx * dux; qpx[1] = b1 - hdx * dux;
-                qmx[2] = b2 + hdx * dvx; qpx[2] = b2 - hdx * dvx;
-                qmx[3] = b3 + hdx * dwx; qpx[3] = b3 - hdx * dwx;
-                qmx[4] = fmaxf(b4 + hdx * dpx, smallP); qpx[4] = fmaxf(b4 - hdx * dpx, smallP);
-                qmy[0] = b0 + hdy * dry; qpy[0] = b0 - hdy * dry;
-                qmy[1] = b1 + hdy * duy; qpy[1] = b1 - hdy * duy;
-                qmy[2] = b2 + hdy * dvy; qpy[2] = b2 - hdy * dvy;
-                qmy[3] = b3 + hdy * dwy; qpy[3] = b3 - hdy * dwy;
-                qmy[4] = fmaxf(b4 + hdy * dpy, smallP); qpy[4] = fmaxf(b4 - hdy * dpy, smallP);
-            } else {
-                qmx[0] = r_rho + half * dt * sr0 + half * drx * dxl;
-                qmx[1] = u + half * dt * su0 + half * dux * dxl;
-                qmx[4] = fmax2(pp + half * dt * sp0 + half * dpx * dxl, smallP);
-                qmx[2] = v + half * dt * sv0 + half * dvx * dxl;
-                qmx[3] = w + half * dt * sw0 + half * dwx * dxl;
-                qpx[0] = r_rho + half * dt * sr0 - half * drx * dxl;
-                qpx[1] = u + half * dt * su0 - half * dux * dxl;
-                qpx[4] = fmax2(pp + half * dt * sp0 - half * dpx * dxl, smallP);
-                qpx[2] = v + half * dt * sv0 - half * dvx * dxl;
-                qpx[3] = w + half * dt * sw0 - half * dwx * dxl;
-                qmy[0] = r_rho + half * dt * sr0 + half * dry * dyl;
-                qmy[1] = u + half * dt * su0 + half * duy * dyl;
-                qmy[4] = fmax2(pp + half * dt * sp0 + half * dpy * dyl, smallP);
-                qmy[2] = v + half * dt * sv0 + half * dvy * dyl;
-                qmy[3] = w + half * dt * sw0 + half * dwy * dyl;
-                qpy[0] = r_rho + half * dt * sr0 - half * dry * dyl;
-                qpy[1] = u + half * dt * su0 - half * duy * dyl;
-                qpy[4] = fmax2(pp + half * dt * sp0 - half * dpy * dyl, smallP);
-                qpy[2] = v + half * dt * sv0 - half * dvy * dyl;
-                qpy[3] = w + half * dt * sw0 - half * dwy * dyl;
+            const R b0 = r_rho + hdt * sr0, b1 = u + hdt * su0, b2 = v + hdt * sv0, b3 = w + hdt * sw0;
+            qmx[0] = b0 + hdx * drx; qpx[0] = b0 - hdx * drx;
+            qmx[1] = b1 + hdx * dux; qpx[1] = b1 - hdx * dux;
+            qmx[2] = b2 + hdx * dvx; qpx[2] = b2 - hdx * dvx;
+            qmx[3] = b3 + hdx * dwx; qpx[3] = b3 - hdx * dwx;
+            qmy[0] = b0 + hdy * dry; qpy[0] = b0 - hdy * dry;
+            qmy[1] = b1 + hdy * duy; qpy[1] = b1 - hdy * duy;
+            qmy[2] = b2 + hdy * dvy; qpy[2] = b2 - hdy * dvy;
+            qmy[3] = b3 + hdy * dwy; qpy[3] = b3 - hdy * dwy;
+            if (FAST || !iso) {   // FP64: an isothermal gas takes its face pressures from the densities below
+                R sp0 = -u * dpx - v * dpy - (dux + dvy) * gamma * pp;
+                if (polar) sp0 = -u * dpx - v * dpy - (dux + dvy) * gamma * pp - over_r(gamma * pp * u);
+                const R b4 = pp + hdt * sp0;
+                auto floor_P = [&](R x) -> R { if constexpr (FAST) return fmaxf(x, smallP); else return max64(x, smallP); };
+                qmx[4] = floor_P(b4 + hdx * dpx); qpx[4] = floor_P(b4 - hdx * dpx);
+                qmy[4] = floor_P(b4 + hdy * dpy); qpy[4] = floor_P(b4 - hdy * dpy);
             }
             if (iso) {   // godunov.f90:606-611
                 qmx[4] = sq(c1) * qmx[0];
@@ -239,37 +286,22 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                 su0 = su0 + over_r(sq(v));
                 sv0 = sv0 - over_r(u * v);
             }
-            if constexpr (FAST) {
-                const R b0 = r_rho + hdt * sr0, b1 = u + hdt * su0, b2 = v + hdt * sv0, b3 = w + hdt * sw0;
-                qmx[0] = b0 + hdx * drx; qpx[0] = b0 - hdx * drx;
-                qmx[1] = b1 + hdx * dux; qpx[1] = b1 - hdx * dux;
-                qmx[2] = b2 + hdx * dvx; qpx[2] = b2 - hdx * dvx;
-                qmx[3] = b3 + hdx * dwx; qpx[3] = b3 - hdx * dwx;
-                qmy[0] = b0 + hdy * dry; qpy[0] = b0 - hdy * dry;
-                qmy[1] = b1 + hdy * duy; qpy[1] = b1 - hdy * duy;
-                qmy[2] = b2 + hdy * dvy; qpy[2] = b2 - hdy * dvy;
-                qmy[3] = b3 + hdy * dwy; qpy[3] = b3 - hdy * dwy;
-            } else {
-                qmx[0] = r_rho + half * dt * sr0 + half * drx * dxl;
-                qmx[1] = u + half * dt * su0 + half * dux * dxl;
-                qmx[2] = v + half * dt * sv0 + half * dvx * dxl;
-                qmx[3] = w + half * dt * sw0 + half * dwx * dxl;
-                qpx[0] = r_rho + half * dt * sr0 - half * drx * dxl;
-                qpx[1] = u + half * dt * su0 - half * dux * dxl;
-                qpx[2] = v + half * dt * sv0 - half * dvx * dxl;
-                qpx[3] = w + half * dt * sw0 - half * dwx * dxl;
-                qmy[0] = r_rho + half * dt * sr0 + half * dry * dyl;
-                qmy[1] = u + half * dt * su0 + half * duy * dyl;
-                qmy[2] = v + half * dt * sv0 + half * dvy * dyl;
-                qmy[3] = w + half * dt * sw0 + half * dwy * dyl;
-                qpy[0] = r_rho + half * dt * sr0 - half * dry * dyl;
-                qpy[1] = u + half * dt * su0 - half * duy * dyl;
-                qpy[2] = v + half * dt * sv0 - half * dvy * dyl;
-                qpy[3] = w + half * dt * sw0 - half * dwy * dyl;
-            }
+            const R b0 = r_rho + hdt * sr0, b1 = u + hdt * su0, b2 = v + hdt * sv0, b3 = w + hdt * sw0;
+            qmx[0] = b0 + hdx * drx; qpx[0] = b0 - hdx * drx;
+            qmx[1] = b1 + hdx * dux; qpx[1] = b1 - hdx * dux;
+            qmx[2] = b2 + hdx * dvx; qpx[2] = b2 - hdx * dvx;
+            qmx[3] = b3 + hdx * dwx; qpx[3] = b3 - hdx * dwx;
+            qmy[0] = b0 + hdy * dry; qpy[0] = b0 - hdy * dry;
+            qmy[1] = b1 + hdy * duy; qpy[1] = b1 - hdy * duy;
+            qmy[2] = b2 + hdy * dvy; qpy[2] = b2 - hdy * dvy;
+            qmy[3] = b3 + hdy * dwy; qpy[3] = b3 - hdy * dwy;
         }
         (void)col_pred;
 
+        auto face_cs = [&](R pf, R rf) -> R {
+            if constexpr (FAST) return sqrt(gamma * pf / rf);
+            else return sqrt(div64(gamma * pf, rf, rcp64(rf)));
+        };
         // ---- x faces of row P: left face of this lane = (qm_x of lane-1, qp_x of this lane) --------
         R fxl[NV];
         {
@@ -279,8 +311,8 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
             if (IS_GAS) {
                 R csl, csr;
                 if (iso) { csl = shfl_up1(c1); csr = c1; }
-                else { csl = sqrt(gamma * ql[4] / ql[0]); csr = sqrt(gamma * qpx[4] / qpx[0]); }
-                const GasFlux<R> g = gas_flux_t<SOLV>(gamma, inv_g1, ql[0], ql[1], ql[2], ql[3], ql[4],
+                else { csl = face_cs(ql[4], ql[0]); csr = face_cs(qpx[4], qpx[0]); }
+                const GasFlux<R> g = gas_flux_t<SOLV>(gamma, FAST ? inv_g1 : yg1, ql[0], ql[1], ql[2], ql[3], ql[4],
                                               qpx[0], qpx[1], qpx[2], qpx[3], qpx[4], csl, csr);
                 fxl[0] = g.rho; fxl[1] = g.mn; fxl[2] = g.mt; fxl[3] = g.mz; fxl[4] = g.e;
             } else {
@@ -289,6 +321,11 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                                                         shfl_up1(cs_col), cs_col);
                 fxl[0] = d.rho; fxl[1] = d.mn; fxl[2] = d.mt; fxl[3] = d.mz;
             }
+        }
+        // FP64: times the face's area, which the right neighbour's left face has alike
+        if constexpr (!FAST) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) fxl[k] = fxl[k] * s1l;
         }
         R fxr[NV];
 #pragma unroll
@@ -300,9 +337,9 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
             if (IS_GAS) {
                 R csl, csr;
                 if (iso) { csl = c_prev; csr = c1; }
-                else { csl = sqrt(gamma * qmy_prev[4] / qmy_prev[0]); csr = sqrt(gamma * qpy[4] / qpy[0]); }
+                else { csl = face_cs(qmy_prev[4], qmy_prev[0]); csr = face_cs(qpy[4], qpy[0]); }
                 // idim = 2: normal velocity vy, transverse vx (allocate_init.f90:249-252)
-                const GasFlux<R> g = gas_flux_t<SOLV>(gamma, inv_g1, qmy_prev[0], qmy_prev[2], qmy_prev[1], qmy_prev[3], qmy_prev[4],
+                const GasFlux<R> g = gas_flux_t<SOLV>(gamma, FAST ? inv_g1 : yg1, qmy_prev[0], qmy_prev[2], qmy_prev[1], qmy_prev[3], qmy_prev[4],
                                               qpy[0], qpy[2], qpy[1], qpy[3], qpy[4], csl, csr);
                 gb[0] = g.rho; gb[2] = g.mn; gb[1] = g.mt; gb[3] = g.mz; gb[4] = g.e;
             } else {
@@ -310,6 +347,10 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                                                 qpy[0], qpy[2], qpy[1], qpy[3], cs_col, cs_col);
                 gb[0] = d.rho; gb[2] = d.mn; gb[1] = d.mt; gb[3] = d.mz;
             }
+        }
+        if constexpr (!FAST) {   // times the face's area (carried to the row above with it)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) gb[k] = gb[k] * s2;
         }
         // radial neighbours of row P-1's old velocities for the viscous term (all lanes shuffle)
         R vxl = R(0), vxr = R(0), vyl = R(0), vyr = R(0);
@@ -323,7 +364,7 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
                 if constexpr (FAST) un[k] = t_prev[k] + (g_prev[k] - gb[k]) * s2 * (dt * rvol);
-                else un[k] = t_prev[k] + (g_prev[k] * s2 - gb[k] * s2) / vol * dt;
+                else un[k] = t_prev[k] + over_vol(g_prev[k] - gb[k]) * dt;
             }
             if (polar && IS_GAS && p.visc) {
                 // Source_terms GEOM==2 (source_terms.f90:37-47) plus the viscous term
@@ -340,8 +381,8 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                     S1 = S1 + qr * dt * eta * lu;
                     S2 = S2 + qr * dt * eta * lv;
                 } else {
-                    S1 = dt * (qr * sq(qvy) + q0[4]) / radc;
-                    S2 = R(0) - dt * (qr * qvy * qvx / radc);
+                    S1 = over_r(dt * (qr * sq(qvy) + q0[4]));
+                    S2 = R(0) - dt * over_r(qr * qvy * qvx);
                     const R lu = (vxr + vxl - R(2) * qvx) / (dx1 * dx1) + (vxr + vxl) / radc / dx1 / R(2) - qvx / radc / radc;
                     S1 = S1 + qr * dt * eta * lu;
                     const R lv = (vyr + vyl - R(2) * qvy) / (dx1 * dx1) - qvy / (radc * radc) + (vyr + vyl) / radc / dx1 / R(2);
@@ -372,9 +413,9 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                     else un[1] = un[1] + qr * sq(qvy) * dtr;
                     un[2] = un[2] - qr * qvy * qvx * dtr;
                 } else {
-                    if (IS_GAS) un[1] = un[1] + dt * (qr * sq(qvy) + q0[4]) / radc;
-                    else un[1] = un[1] + dt * (qr * sq(qvy) / radc);
-                    un[2] = un[2] + (R(0) - dt * (qr * qvy * qvx / radc));
+                    if (IS_GAS) un[1] = un[1] + over_r(dt * (qr * sq(qvy) + q0[4]));
+                    else un[1] = un[1] + dt * over_r(qr * sq(qvy));
+                    un[2] = un[2] - dt * over_r(qr * qvy * qvx);
                 }
             }
 #pragma unroll
@@ -394,23 +435,34 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                         uu[3] = uu[3] + rho * dt * f3;
                         en = half * (sq(uu[1]) + sq(uu[2]) + sq(uu[3])) * ir;
                     } else {
-                        eo = half * sq(uu[1]) / rho + half * sq(uu[2]) / rho + half * sq(uu[3]) / rho;
-                        uu[1] = uu[1] + rho * R(1) * dt * f1;
-                        uu[2] = uu[2] + rho * R(1) * dt * f2;
-                        uu[3] = uu[3] + rho * R(1) * dt * f3;
-                        en = half * sq(uu[1]) / rho + half * sq(uu[2]) / rho + half * sq(uu[3]) / rho;
+                        // a component without a force keeps its momentum and its energy
+                        const R y = rcp64(rho), rdt = rho * dt;
+                        const R e1 = div64(half * sq(uu[1]), rho, y), e2 = div64(half * sq(uu[2]), rho, y),
+                                e3 = div64(half * sq(uu[3]), rho, y);
+                        eo = e1 + e2 + e3;
+                        uu[1] = uu[1] + rdt * f1;
+                        R n2 = e2, n3 = e3;
+                        if (p.setup == SHARK_SETUP_DISK_CART) {
+                            uu[2] = uu[2] + rdt * f2;
+                            n2 = div64(half * sq(uu[2]), rho, y);
+                        } else if (p.setup == SHARK_SETUP_SI) {
+                            uu[3] = uu[3] + rdt * f3;
+                            n3 = div64(half * sq(uu[3]), rho, y);
+                        }
+                        en = div64(half * sq(uu[1]), rho, y) + n2 + n3;
                     }
                     uu[4] = uu[4] + (en - eo);
                 } else {
-                    uu[1] = uu[1] + rho * R(1) * dt * f1;
-                    uu[2] = uu[2] + rho * R(1) * dt * f2;
-                    uu[3] = uu[3] + rho * R(1) * dt * f3;
+                    const R rdt = rho * dt;
+                    uu[1] = uu[1] + rdt * f1;
+                    if (FAST || p.setup == SHARK_SETUP_DISK_CART) uu[2] = uu[2] + rdt * f2;
+                    if (FAST || p.setup == SHARK_SETUP_SI) uu[3] = uu[3] + rdt * f3;
                 }
             }
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
                 if constexpr (FAST) uu[k] = uu[k] + (fxl[k] * s1l - fxr[k] * s1r) * (dt * rvol);
-                else uu[k] = uu[k] + (fxl[k] * s1l - fxr[k] * s1r) / vol * dt;
+                else uu[k] = uu[k] + over_vol(fxl[k] - fxr[k]) * dt;
             }
         }
             // ---- slide the window ---------------------------------------------------------------
@@ -432,13 +484,15 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
 }
 
 // Gas and dust run as separate kernels so the dust warps (N of every N+1) are not held to the
-// register footprint of the 5-variable gas path with its HLLC solver.
+// register footprint of the 5-variable gas path with its HLLC solver.  FP64: 10 dust warps an SM
+// (192 registers); 12 at 168 registers measured the same (the FP64 pipe is the bound).
 template <typename R, bool IS_GAS, int ST, int SOLV>
-__global__ void __launch_bounds__(32 * STRIP_WARPS, (IS_GAS || !std::is_same<R, float>::value) ? 1 : 5)
+__global__ void __launch_bounds__(std::is_same<R, float>::value ? 32 * STRIP_WARPS : 32,
+                                  std::is_same<R, float>::value ? (IS_GAS ? 1 : 5) : (IS_GAS ? 8 : 10))
 k_flux_strip(KParams<R> p) {
     const int warp = threadIdx.x >> 5;
     const int bx = blockIdx.x;
-    const int by = blockIdx.y * STRIP_WARPS + warp;
+    const int by = blockIdx.y * (blockDim.x >> 5) + warp;
     const int s = IS_GAS ? 0 : blockIdx.z + 1;
     flux_strip<R, IS_GAS, ST, SOLV>(p, s, bx, by);
 }

@@ -169,9 +169,9 @@ __device__ __forceinline__ GasFlux<R> gas_flux_t(R gamma, R inv_g1, R rl, R ul, 
         else if constexpr (SOLVER == 1) return gas_hll_fast(inv_g1, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
         else return gas_llf(gamma, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
     } else {
-        if constexpr (SOLVER == 2) return gas_hllc(gamma, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
-        else if constexpr (SOLVER == 1) return gas_hll(gamma, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
-        else return gas_llf(gamma, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
+        if constexpr (SOLVER == 2) return gas_hllc_d(gamma, inv_g1, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
+        else if constexpr (SOLVER == 1) return gas_hll_d(gamma, inv_g1, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
+        else return gas_llf_d(gamma, inv_g1, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
     }
 }
 
@@ -179,7 +179,12 @@ __device__ __forceinline__ GasFlux<R> gas_flux_t(R gamma, R inv_g1, R rl, R ul, 
 template <int SOLVERDUST, typename R>
 __device__ __forceinline__ DustFlux<R> dust_flux_t(R rl, R ul, R vl, R wl, R rr, R ur, R vr, R wr, R csl, R csr) {
     if constexpr (SOLVERDUST == 0 && std::is_same<R, float>::value) return dust_hb_f(rl, ul, vl, wl, rr, ur, vr, wr);
-    else if constexpr (SOLVERDUST == 0) return dust_hb(rl, ul, vl, wl, rr, ur, vr, wr);
+    else if constexpr (std::is_same<R, double>::value) {
+        if constexpr (SOLVERDUST == 0) return dust_hb_d(rl, ul, vl, wl, rr, ur, vr, wr);
+        else if constexpr (SOLVERDUST == 1) return dust_llf_d(rl, ul, vl, wl, rr, ur, vr, wr);
+        else if constexpr (SOLVERDUST == 2) return dust_hll_d(rl, ul, vl, wl, rr, ur, vr, wr);
+        else return dust_hllc_d(rl, ul, vl, wl, rr, ur, vr, wr, csl, csr);
+    }
     else if constexpr (SOLVERDUST == 1) return dust_llf(rl, ul, vl, wl, rr, ur, vr, wr);
     else if constexpr (SOLVERDUST == 2) return dust_hll(rl, ul, vl, wl, rr, ur, vr, wr);
     else return dust_hllc(rl, ul, vl, wl, rr, ur, vr, wr, csl, csr);

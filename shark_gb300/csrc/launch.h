@@ -89,6 +89,7 @@ struct DeviceView {
     // (x, y, variable 0..4) and the dust planes (x, y, species, component)
     CUtensorMap k1_gas[3], k1_dust[3];
     int k1_warps;               // warps of one wave of the mixed 2D K1: SMs x resident blocks x warps per block
+    int nsm;                    // SMs of the device
     bool uniform;               // Cartesian grid with the same dx1, dx2, surf1, surf2, vol in every column
     bool cs_uniform;            // the same isothermal sound speed in every column
     // reference gas density of the mixed fused flux kernel: the mean active density of the first

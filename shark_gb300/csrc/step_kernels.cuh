@@ -27,6 +27,7 @@ struct KParams {
     long long plane;
     int ndust, nvar, ndim, geom, solver, solverdust, slope_type, iso, setup, flags;
     int sod_dir;
+    int strip_h;                      // rows a warp of the column-march flux kernel updates
     double gamma, cfl, smallr, smallp, dust_ratio_min, box_l, rhograin;
     double si_q, si_om, si_eta, si_r0;
     double sod_rho_l, sod_rho_r, sod_P_l, sod_P_r;
