@@ -8,8 +8,9 @@
 // forms it; per-pair constants that involve no state -- the collision cross-section factor, the
 // Brownian mass factor, and without fragmentation the target bins and their mass split -- are
 // tabulated on the host with the oracle's operations.  The FP64 path follows the oracle's
-// operations; the mixed path integrates in FP32 (growth_dv_f, growth_cell_f and the warp-per-cell
-// form in the mixed K2).  A cell needing more than 100000 sub-steps stops there and raises
+// operations (without fragmentation k_growth_d, a group of lanes per cell; with it growth_cell_d);
+// the mixed path integrates in FP32 (growth_dv_f, growth_cell_f and the warp-per-cell form in the
+// mixed K2).  A cell needing more than 100000 sub-steps stops there and raises
 // SHARK_STATUS_GROWTH.
 #pragma once
 
@@ -17,6 +18,7 @@
 #include <stdint.h>
 
 #include "../../include/shark_gpu.h"
+#include "fp64.cuh"
 
 namespace shark {
 
@@ -24,6 +26,13 @@ namespace shark {
 // per-cell pair tables in local memory in the FP64 path
 constexpr int GROWTH_MAX_DUST = 32;
 constexpr int GROWTH_MAX_PAIRS = GROWTH_MAX_DUST * (GROWTH_MAX_DUST + 1) / 2;
+
+// Lanes per cell of k_growth_d: a bin each up to 16 bins.  More lanes shorten a cell's sub-steps (the
+// longest cell bounds the small grids) and idle more: measured ms of K2 with 8 / 16 / 32 lanes, dusty
+// box 48^2 x 32 5.57 / 3.35 / 2.91, 256^2 x 32 12.3 / 12.5 / 13.6, disk 128 x 256 x 16 3.57 / 3.22 / 3.57,
+// 128 x 256 x 5 0.70 / 0.88 / 1.39.
+constexpr int growth_lanes(int ndust) { return ndust <= 8 ? 8 : 16; }
+constexpr int GROWTH_SLOTS = 2;
 
 struct GrowthDev {
     int on, kernel, mode, t_per_col;
@@ -37,6 +46,12 @@ struct GrowthDev {
     const float* gc;         //           and the net mass it moves into bin b per collision, in units of
                              //           mref (formed in FP64; 0 pads the short rows)
     int npair, gL;
+    // FP64 path without fragmentation (k_growth_d): per bin the mass changes of the pairs in the
+    // oracle's order, coefficient m of a change m dn/dt; the bins by falling list length in slots
+    // of G = growth_lanes(N), slot s's entry t of lane l at (sbase[s] + t) * G + l
+    const double* sc;        // coefficients (0 pads the shorter lists of a slot)
+    const int32_t* sq;       // pairs
+    int sbin[GROWTH_SLOTS * 16], sbase[GROWTH_SLOTS + 1];   // bin of (slot, lane), -1 none
     const double* pS;        // [N*N] m_k unit_m + m_j unit_m
     const double* pD;        // [N*N] m_k m_j unit_m^2
     const int32_t* pic;      // [N*N*2] target bins ic1, ic2 (1-based) without fragmentation
@@ -99,6 +114,62 @@ __device__ __forceinline__ double growth_dv_d(const GrowthDev& g, int N, int k, 
                                                 fabs(gam[j]) / sqrt(1.0 + gam[j] * gam[j]));
         const double vad = sqrt(d * d);
         dv = sqrt(dv * dv + vad * vad);
+    }
+    return dv;
+}
+
+// Constants of one cell (dust_growth.f90:60-87) in FP64.
+struct GrowthCellD {
+    double T, acs, t_L, t_eta, rm, vamb;   // acs = alpha_turb cs, vamb = vambi / unit_v
+};
+__device__ __forceinline__ GrowthCellD growth_cell_consts_d(const GrowthDev& g, int ix, double rho_q, double hs,
+                                                            double eta_a) {
+    const double* cc = g.col + (size_t)(g.t_per_col ? ix : 0) * 4;
+    GrowthCellD c;
+    c.T = cc[0];
+    const double cs_T = cc[1], cs_v = cc[2];
+    const double rho = rho_q / hs;
+    const double rho_cgs = rho * g.ud;
+    const double lambJ = sqrt(3. * grw::pi / (32. * grw::grav * rho_cgs)) * cs_T;
+    const double vambi = g.delta_vambi * (grw::clight * grw::clight) * eta_a / lambJ / (4.0 * grw::pi);
+    const double Re = 6.2e7 * sqrt(rho_cgs / (g.mu_gas * grw::mH) / 1e5) * sqrt(c.T / 10.0);
+    c.t_L = g.t_per_col ? cc[3] : sqrt(3. * grw::pi / (32. * grw::grav * rho_cgs)) / g.ut;
+    c.t_eta = c.t_L / sqrt(Re);
+    c.rm = pow(Re, -0.5);
+    c.acs = g.alpha_turb * cs_v;
+    c.vamb = vambi / g.uv;
+    return c;
+}
+
+// Relative velocity of species k and j <= k as growth_dv_d's, from per-species terms: stopping times
+// tk, tj; S = t/t_L, W = S^2/(S + rm), I = 1/(1 + S) of both; the drift (dx, dy, dz); the difference
+// dg of |gamma|/sqrt(1 + gamma^2); X the Brownian dv^2.  The square root of a square is the modulus
+// itself, and only the turbulent case that applies is formed.
+__device__ __forceinline__ double growth_dv_pair_d(const GrowthDev& g, const GrowthCellD& c, double tk, double tj,
+                                                   double Sk, double Sj, double Wk, double Wj, double Ik, double Ij,
+                                                   double X, double dx, double dy, double dz, double dg, bool ambi) {
+    double dv = 0.0;
+    if (g.mode & SHARK_GROWTH_TURB) {
+        if (is_less(c.t_L, tk)) dv = c.acs * sqrt(Ik + Ij);
+        else if (is_less(tk, c.t_eta)) dv = c.acs * sqrt((Sk - Sj) / (Sk + Sj)) * sqrt(Wk - Wj);
+        else {
+            const double x = div64(tj, tk, rcp64(tk)), b1 = 1. + x, b2 = (double)1.6f + x;
+            const double f = (double)3.2f - 1.0 - x +
+                             div64(2.0, b1, rcp64(b1)) * ((double)(1.0f / 2.6f) + div64(x * x * x, b2, rcp64(b2)));
+            dv = c.acs * sqrt(f * Sk);
+        }
+    }
+    if (g.mode & SHARK_GROWTH_BROWNIAN) {
+        const double v = sqrt(X);
+        dv = sqrt(dv * dv + v * v);
+    }
+    if (g.mode & SHARK_GROWTH_DRIFT) {
+        const double v = sqrt(dx * dx + dy * dy + dz * dz);
+        dv = sqrt(dv * dv + v * v);
+    }
+    if ((g.mode & SHARK_GROWTH_AMBIPOLAR) && ambi) {
+        const double d = c.vamb * dg;
+        dv = sqrt(dv * dv + d * d);
     }
     return dv;
 }
@@ -278,7 +349,8 @@ static __device__ __noinline__ bool growth_cell_f(const GrowthDev& g, int N, int
 // Sub-cycled growth of one cell: rd[N] in/out (dust densities after the drag), rho_gas the
 // conserved gas density, rho_q the floored gas density at the start of the step (q(irho)).
 // The pair velocities depend only on the start of the step, so they are formed once per cell
-// (the values the oracle re-forms every sub-step).  Returns false if the sub-step cap was reached.
+// (the values the oracle re-forms every sub-step).  With fragmentation; k_growth_d is the form
+// without.  Returns false if the sub-step cap was reached.
 static __device__ bool growth_cell_d(const GrowthDev& g, int N, int ix, double dt, double rho_gas, double rho_q, double hs,
                               double* rd, const double* ts, const double* vx, const double* vy, const double* vz,
                               const double* gam, double eta_a) {
@@ -293,7 +365,6 @@ static __device__ bool growth_cell_d(const GrowthDev& g, int N, int ix, double d
     const double t_L = g.t_per_col ? cc[3] : sqrt(3. * grw::pi / (32. * grw::grav * rho_cgs)) / g.ut;
     const double t_eta = t_L / sqrt(Re);
     const double rm = pow(Re, -0.5);
-    const bool frag = (g.mode & SHARK_GROWTH_FRAGMENTATION) != 0;
     double dvp[GROWTH_MAX_DUST * (GROWTH_MAX_DUST + 1) / 2];
     for (int k = 0, q = 0; k < N; ++k)
         for (int j = 0; j <= k; ++j, ++q)
@@ -310,7 +381,7 @@ static __device__ bool growth_cell_d(const GrowthDev& g, int N, int ix, double d
                 const double m2 = g.mk[j];
                 const double dv = dvp[q];
                 double f_frag = 0.0, p_coag = 1.0;
-                if (frag) {
+                {
                     const double Ecol = 0.5 * (m1 * m2) / (m1 + m2) * (dv * dv);
                     const double Ebr = (m1 + m2) / g.m_mono * g.Ebr_mono;
                     const double fr = (Ecol - 0.1 * Ebr) / (4.9 * Ebr);
@@ -354,7 +425,7 @@ static __device__ bool growth_cell_d(const GrowthDev& g, int N, int ix, double d
                         drhodt[ic2 - 1] = drhodt[ic2 - 1] + (1. - eps_m) * p_coag * (1.0 - f_frag) * (m1 + m2) * dndt * st;
                     }
                 }
-                if ((frag && f_frag > 0.0) && p_coag > 0.) {
+                if (f_frag > 0.0 && p_coag > 0.) {
                     const int b = (int)floor(log(0.1 * f_frag * (m1 + m2) / g.massmin) / log(g.eta) + 1);
                     const int ifrag2 = max(min(b, ic1), 1);
                     for (int kd = 0; kd < ifrag2; ++kd)

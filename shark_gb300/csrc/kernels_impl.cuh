@@ -86,10 +86,31 @@ static void finalize_launch(const KParams<R>& p, dim3 grid, cudaStream_t st) {
     else k_finalize<R, NS, MODE, GROW><<<grid, 256, 0, st>>>(p);
 }
 
+// FP64 growth without fragmentation: the drag, k_growth_d, the rest of K2.
+template <int GL>
+static void growth_kernel_d(const KParams<double>& p, cudaStream_t st) {
+    constexpr int cells = GROWTH_D_THREADS / GL;
+    const size_t smem = (size_t)cells * growth_d_stride(p.ndust, p.gw.npair) * sizeof(double);   // 35 kB at most
+    const long long nact = (long long)p.nx * (p.ndim == 2 ? p.ny : 1);
+    k_growth_d<GL><<<(unsigned)((nact + cells - 1) / cells), GROWTH_D_THREADS, smem, st>>>(p);
+}
+static void growth_launch_d(const KParams<double>& p, dim3 grid, cudaStream_t st) {
+    finalize_launch<double, -1, 2>(p, grid, st);
+    if (growth_lanes(p.ndust) == 8) growth_kernel_d<8>(p, st);
+    else growth_kernel_d<16>(p, st);
+    finalize_launch<double, -1, 3>(p, grid, st);
+}
+
 template <typename R, int MODE>
 static void finalize_dispatch(const KParams<R>& p, dim3 grid, cudaStream_t st) {
-    if (MODE == 0 && p.gw.on) {   // dust growth: run-time species count, growth in the epilogue
-        finalize_launch<R, -1, MODE, true>(p, grid, st);
+    if (MODE == 0 && p.gw.on) {   // dust growth: run-time species count
+        if constexpr (std::is_same<R, double>::value) {
+            if (!(p.gw.mode & SHARK_GROWTH_FRAGMENTATION)) {
+                growth_launch_d(p, grid, st);
+                return;
+            }
+        }
+        finalize_launch<R, -1, MODE, true>(p, grid, st);   // growth within K2
         return;
     }
     switch (p.ndust) {

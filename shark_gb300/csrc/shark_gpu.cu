@@ -616,7 +616,7 @@ void build_charge_tables(const shark_gpu_config& c, const Columns& col, int nx_m
 // ---- dust growth tables (src/dust/dust_growth.f90:3-256, dust_init.f90:11-45) --------------------
 // The operations follow the CPU oracle's growth_grid so the tables are bit-identical to it.
 void build_growth_tables(const shark_gpu_config& c, const Columns& col, int nx_max, std::vector<double>& hd,
-                         std::vector<int32_t>& hi, std::vector<float>& hf, shark::GrowthDev& g, size_t off[9]) {
+                         std::vector<int32_t>& hi, std::vector<float>& hf, shark::GrowthDev& g, size_t off[11]) {
     const int N = c.ndust;
     const double ul = unit1(c.unit_l), ud = unit1(c.unit_d), ut = unit1(c.unit_t);
     const double um = ul * ul * ul * ud, uv = ul / ut;
@@ -640,6 +640,7 @@ void build_growth_tables(const shark_gpu_config& c, const Columns& col, int nx_m
     std::vector<int32_t> pair(P);
     std::vector<float> pKf(P), pBf(P);
     std::vector<std::vector<std::pair<int32_t, float>>> gat(N);   // gather rows of the net transfers
+    std::vector<std::vector<std::pair<int32_t, double>>> seq(N);  // FP64: every change of a bin, in the oracle's order
     const double zeta = std::pow(c.grw_smax / c.grw_smin, 1.0 / N);
     const double eta = zeta * zeta * zeta;
     const double massmin = (c.grw_kernel == 0) ? f43 * kPi * rg_cgs * (c.grw_smin * c.grw_smin * c.grw_smin) / um
@@ -715,6 +716,11 @@ void build_growth_tables(const shark_gpu_config& c, const Columns& col, int nx_m
                 if (sh2 != 0.0) add(ic2 - 1, sh2);
             }
             const int pq = k * (k + 1) / 2 + j;
+            seq[k].emplace_back(pq, -mk[k]);
+            seq[j].emplace_back(pq, -mk[j]);
+            seq[ic1 - 1].emplace_back(pq, e * (mk[k] + mk[j]));
+            const double share2 = (1. - e) * (mk[k] + mk[j]);
+            if (share2 != 0.0) seq[ic2 - 1].emplace_back(pq, share2);
             pair[pq] = (k << 8) | j;
             pKf[pq] = (float)hd[off[8] + q];
             pBf[pq] = (float)((8.0 * kKB / kPi) * hd[off[1] + q] / hd[off[2] + q] / (uv * uv));
@@ -757,6 +763,32 @@ void build_growth_tables(const shark_gpu_config& c, const Columns& col, int nx_m
         }
     g.npair = P;
     g.gL = (int)L;
+    // k_growth_d's lists: the bins by falling list length, growth_lanes(N) to a slot
+    std::vector<int> order(N);
+    for (int b = 0; b < N; ++b) order[b] = b;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return seq[x].size() > seq[y].size(); });
+    const size_t sc0 = hd.size(), sq0 = hi.size();
+    const int G = shark::growth_lanes(N);
+    g.sbase[0] = 0;
+    for (int s = 0; s < shark::GROWTH_SLOTS; ++s) {
+        const int first = s * G;
+        const size_t len = first < N ? seq[order[first]].size() : 0;
+        g.sbase[s + 1] = g.sbase[s] + (int)len;
+        hd.resize(sc0 + (size_t)g.sbase[s + 1] * G, 0.0);
+        hi.resize(sq0 + (size_t)g.sbase[s + 1] * G, 0);
+        for (int l = 0; l < G; ++l) {
+            const int b = first + l < N ? order[first + l] : -1;
+            g.sbin[first + l] = b;
+            if (b < 0) continue;
+            for (size_t t = 0; t < seq[b].size(); ++t) {
+                const size_t at = (size_t)(g.sbase[s] + t) * G + l;
+                hi[sq0 + at] = seq[b][t].first;
+                hd[sc0 + at] = seq[b][t].second;
+            }
+        }
+    }
+    off[9] = sc0;
+    off[10] = sq0;
     const double a_mu = c.grw_size_mono / 2.0;
     g.Ebr_mono = c.grw_Abr * std::pow(c.grw_gamma_grains, 5.0 / 3.0) * std::pow(a_mu, 4.0 / 3.0) /
                  std::pow(c.grw_estar_grains, 2.0 / 3.0) / (uv * uv * um);
@@ -1296,7 +1328,7 @@ int32_t shark_gpu_init(const shark_gpu_config* cfg, shark_gpu_ctx** out) {
         std::vector<double> hd;
         std::vector<int32_t> hi;
         std::vector<float> hf;
-        size_t off[9];
+        size_t off[11];
         build_growth_tables(*cfg, col, v.nx_max, hd, hi, hf, v.gw, off);
         INIT_TRY(cudaMalloc(&c->grw_f, hf.size() * sizeof(float)));
         INIT_TRY(cudaMemcpy(c->grw_f, hf.data(), hf.size() * sizeof(float), cudaMemcpyHostToDevice));
@@ -1307,6 +1339,7 @@ int32_t shark_gpu_init(const shark_gpu_config* cfg, shark_gpu_ctx** out) {
         v.gw.pA = c->grw_d + off[0]; v.gw.pS = c->grw_d + off[1]; v.gw.pD = c->grw_d + off[2];
         v.gw.peps = c->grw_d + off[3]; v.gw.mk = c->grw_d + off[4]; v.gw.sk = c->grw_d + off[5];
         v.gw.redis = c->grw_d + off[6]; v.gw.col = c->grw_d + off[7]; v.gw.pic = c->grw_i;
+        v.gw.sc = c->grw_d + off[9]; v.gw.sq = c->grw_i + off[10];
         {
             const size_t NN = (size_t)cfg->ndust * cfg->ndust, P = (size_t)v.gw.npair;
             v.gw.pair = c->grw_i + NN * 2;

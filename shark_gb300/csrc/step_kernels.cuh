@@ -184,7 +184,8 @@ namespace shark {
 // ---------------------------------------------------------------------------------------------
 // K2: drag + floor + inloop + status + next-step CFL dt, one thread per active cell.
 // NS > 0: compile-time species count (register arrays); NS < 0: run-time count.
-// MODE 0: full finalize; MODE 1: dt only (first step after an upload).
+// MODE 0: full finalize; MODE 1: dt only (first step after an upload); MODES 2 and 3: the drag with
+// its floor and heating, and the rest, as two launches with k_growth_d between them (FP64).
 // ---------------------------------------------------------------------------------------------
 
 // Producer-side boundary fill: an active cell within nghost of a periodic or shear-periodic edge
@@ -644,6 +645,151 @@ static __device__ __noinline__ unsigned grow_block_warps(const KParams<float>& p
     return st;
 }
 
+// Dust growth of the FP64 path without fragmentation (dust_growth.f90:3-256) on the post-drag state
+// u_next: G = growth_lanes(N) lanes per cell, blocks of 128 threads.  Bit for bit the oracle's
+// sub-cycle: a sub-step's pair rates dn/dt are formed in the oracle's order of operations, the lanes
+// taking the pairs in turn, and exchanged through shared memory; then each lane sums its bins' mass
+// changes in the oracle's order, one list of (coefficient, pair) per bin.  What the sub-step does
+// not change is formed once per cell (the rate's factor A dv) or on the host (the coefficients).
+// The kernel is bound by the FP64 pipe: some 11 instructions for a pair's rate (its divisions by the
+// two masses share the masses' reciprocals) and two for each entry, against 80 for a pair in a
+// thread per cell; several lanes a cell spread the small grids over the chip and leave few cells that
+// wait for each other's sub-steps.  K2 with growth, in ms against a thread per cell: polar disk
+// 128 x 256 x 16 26.9 -> 3.2, 48 x 64 x 16 38.6 -> 1.4; dusty box 48^2 x 32 97 -> 3.4, 256^2 x 32 39 -> 12.5.
+constexpr int GROWTH_D_THREADS = 128;
+
+// doubles of shared memory per cell: densities, then the species' terms, reused by the pair rates;
+// a stride of 8 modulo 16 puts the cells of a warp in different banks
+__host__ __device__ __forceinline__ int growth_d_stride(int N, int P) {
+    const int n = N + (P > 8 * N ? P : 8 * N);
+    return n + ((8 - n % 16) + 16) % 16;
+}
+
+template <int GL>
+static __global__ void __launch_bounds__(GROWTH_D_THREADS) k_growth_d(KParams<double> p) {
+    extern __shared__ __align__(16) double sgrow[];
+    __shared__ double smk[GROWTH_MAX_DUST], symk[GROWTH_MAX_DUST];
+    const GrowthDev& g = p.gw;
+    const int N = p.ndust, P = g.npair;
+    if (threadIdx.x < N) {
+        smk[threadIdx.x] = g.mk[threadIdx.x];
+        symk[threadIdx.x] = rcp64(g.mk[threadIdx.x]);
+    }
+    __syncthreads();
+    constexpr int SLOTS = GL == 8 ? 1 : GROWTH_SLOTS;
+    const int l = threadIdx.x % GL, grp = threadIdx.x / GL;
+    const long long nact = (long long)p.nx * (p.ndim == 2 ? p.ny : 1);
+    const long long cell = blockIdx.x * (long long)(GROWTH_D_THREADS / GL) + grp;
+    const bool act = cell < nact;
+    // a group past the grid's end takes the last cell along and writes nothing
+    const long long ac = act ? cell : nact - 1;
+    const int gx = (int)(ac % p.nx) + p.ng, gy = p.ndim == 2 ? (int)(ac / p.nx) + p.ng : 0;
+    const unsigned mask = (0xffffffffu >> (32 - GL)) << (threadIdx.x & 31 & ~(GL - 1));
+    double* rd = sgrow + (size_t)grp * growth_d_stride(N, P);
+    double* w = rd + N;                       // pair rates
+    double *ts = w, *S = w + N, *W = w + 2 * N, *I = w + 3 * N, *vx = w + 4 * N, *vy = w + 5 * N, *vz = w + 6 * N, *G = w + 7 * N;
+    double* u = p.u_next;
+    const double dt = *p.dt;
+    const bool ambi = (g.mode & SHARK_GROWTH_AMBIPOLAR) && p.chg_gamma_d;
+    const long long e = (long long)gy * p.pitch + gx;
+    const double rho_old = p.u_cur[e], qrho_old = max64(rho_old, p.smallr);
+    const double hs = p.setup == SHARK_SETUP_DISK_POLAR ? p.hsd[gx] : 1.0, yhs = rcp64(hs);
+    const double rho_gas = u[e];
+    const GrowthCellD c = growth_cell_consts_d(g, gx, qrho_old, hs, ambi ? p.chg_eta[2 * p.plane + e] : 0.0);
+    // the species' terms
+    for (int k = l; k < N; k += GL) {
+        rd[k] = u[(5 + k) * p.plane + e];
+        const double t = tstop_cell(p, k, qrho_old, gx, gy), St = t / c.t_L;
+        ts[k] = t;
+        S[k] = St;
+        W[k] = St * St / (St + c.rm);
+        I[k] = 1.0 / (1.0 + St);
+        const double r0 = p.u_cur[(5 + k) * p.plane + e], y = rcp64(r0);
+        vx[k] = div64(p.u_cur[(5 + N + k) * p.plane + e], r0, y);
+        vy[k] = div64(p.u_cur[(5 + 2 * N + k) * p.plane + e], r0, y);
+        vz[k] = div64(p.u_cur[(5 + 3 * N + k) * p.plane + e], r0, y);
+        const double gm = ambi ? p.chg_gamma_d[(long long)k * p.plane + e] : 0.0;
+        G[k] = abs64(gm) / sqrt(1.0 + gm * gm);
+    }
+    __syncwarp(mask);
+    // A dv of this lane's pairs (the rate's first factor that a sub-step keeps)
+    double ka[(GL == 8 ? 36 : GROWTH_MAX_PAIRS) / GL + 1];
+    const double cB = 8.0 * grw::kB * c.T / grw::pi, yuv2 = rcp64(g.uv2);
+    for (int i = 0, q = l; q < P; ++i, q += GL) {
+        const int pr = g.pair[q], k = pr >> 8, j = pr & 255, kj = k * N + j;
+        double a = 1.0;
+        if (g.kernel == 0) {
+            const double pD = g.pD[kj], X = div64(div64(cB * g.pS[kj], pD, rcp64(pD)), g.uv2, yuv2);
+            a = g.pA[kj] * growth_dv_pair_d(g, c, ts[k], ts[j], S[k], S[j], W[k], W[j], I[k], I[j], X, vx[k] - vx[j],
+                                            vy[k] - vy[j], vz[k] - vz[j], G[k] - G[j], ambi);
+        } else if (g.kernel == 2) {
+            a = smk[k] + smk[j];
+        }
+        ka[i] = a;
+    }
+    __syncwarp(mask);                         // the terms are read; the rates may take their place
+    const double thr = g.eps_thr * rho_gas, fl = rho_gas * g.dust_ratio_min;
+    const bool thr_on = g.kernel == 0 && g.eps_thr > 0.0, hs_on = hs != 1.0, stick_on = g.sticking != 1.0;
+    int bin[SLOTS];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) bin[s] = g.sbin[s * GL + l];
+    double time = 0.0;
+    int niter = 0;
+    while (is_less(time, dt) && niter < grw::MAX_SUB) {
+        niter = niter + 1;
+        for (int i = 0, q = l; q < P; ++i, q += GL) {
+            const int pr = g.pair[q], k = pr >> 8, j = pr & 255;
+            const double rk = rd[k], rj = rd[j];
+            double d = (g.kernel == 1 ? rk : ka[i] * rk) * rj;
+            d = div64(div64(d, smk[k], symk[k]), smk[j], symk[j]);
+            if (hs_on) d = div64(d, hs, yhs);
+            if (k == j) d = 0.5 * d;
+            if (thr_on && (is_less(rk, thr) || is_less(rj, thr))) d = 0.0;
+            w[q] = d;
+        }
+        __syncwarp(mask);
+        double dr[SLOTS], cand = 1e32;
+#pragma unroll
+        for (int s = 0; s < SLOTS; ++s) {
+            dr[s] = 0.0;
+            if (s * GL >= N) continue;
+            double d = 0.0;
+            if (!stick_on) {
+                for (int t = g.sbase[s]; t < g.sbase[s + 1]; ++t)
+                    d = d + __ldg(g.sc + t * GL + l) * w[__ldg(g.sq + t * GL + l)];
+            } else {
+                for (int t = g.sbase[s]; t < g.sbase[s + 1]; ++t)
+                    d = d + __ldg(g.sc + t * GL + l) * w[__ldg(g.sq + t * GL + l)] * g.sticking;
+            }
+            dr[s] = d;
+            const int b = bin[s];
+            if (b >= 0 && !is_zero(d)) {
+                const double a = abs64(d), x = div64(rd[b], a, rcp64(a)) * g.cfl;
+                // positive numbers order as their bits, a result that is none never is the least
+                cand = abs_bits(x) < abs_bits(cand) ? x : cand;
+            }
+        }
+#pragma unroll
+        for (int o = GL / 2; o > 0; o >>= 1) {
+            const double x = __shfl_xor_sync(mask, cand, o);
+            cand = abs_bits(x) < abs_bits(cand) ? x : cand;
+        }
+        const double rest = dt - time;
+        double dtg = is_less(cand, rest) ? cand : rest;
+        if (g.dtctl > 0.0) dtg = g.dtctl < rest ? g.dtctl : rest;
+#pragma unroll
+        for (int s = 0; s < SLOTS; ++s) {
+            if (s * GL >= N) continue;
+            if (bin[s] >= 0) rd[bin[s]] = max64_pos(rd[bin[s]] + dr[s] * dtg, fl);
+        }
+        time = time + dtg;
+        __syncwarp(mask);
+    }
+    if (!act) return;
+    for (int k = l; k < N; k += GL) u[(5 + k) * p.plane + e] = rd[k];
+    if (l == 0 && is_less(time, dt)) atomicOr(p.status, (unsigned)SHARK_STATUS_GROWTH);
+}
+
 // Driven-turbulence kick of the dustyTurb box (turb.f90:227-324 in 2D): the gas momentum gains
 // rho a dt with the solenoidal Ornstein-Uhlenbeck acceleration of this step at the cell centre.
 // C = double follows the oracle's operations; C = float is the mixed-precision form.
@@ -670,6 +816,7 @@ __device__ __forceinline__ void turb_kick_cell(const KParams<R>& p, R* u, int gx
 template <typename R, int NS, int MODE, bool GROW = false>
 __global__ void __launch_bounds__(256) k_finalize(KParams<R> p) {
     constexpr int NMAX = NS > 0 ? NS : 1;
+    constexpr bool DRAG = MODE == 0 || MODE == 2, REST = MODE == 0 || MODE == 3;
     const int N = NS >= 0 ? NS : p.ndust;
     const int gx = blockIdx.x * blockDim.x + threadIdx.x + p.ng;
     const int gy = (p.ndim == 2) ? blockIdx.y + p.ng : 0;
@@ -680,7 +827,7 @@ __global__ void __launch_bounds__(256) k_finalize(KParams<R> p) {
         const double dt = *p.dt;
         double rho = (double)u[uidx(p, 0, gy, gx)];
         double px = (double)u[uidx(p, 1, gy, gx)], py = (double)u[uidx(p, 2, gy, gx)], pz = (double)u[uidx(p, 3, gy, gx)];
-        const bool drag = MODE == 0 && N > 0 && (p.flags & SHARK_FLAG_DRAG);
+        const bool drag = DRAG && N > 0 && (p.flags & SHARK_FLAG_DRAG);
         const bool br = (p.flags & SHARK_FLAG_BACK_REACTION) != 0;
         if (drag) {
             // dust_drag(1.0) (src/dust/dust_drag.f90:2-75), FP64 arithmetic
@@ -727,7 +874,7 @@ __global__ void __launch_bounds__(256) k_finalize(KParams<R> p) {
             py = (double)u[uidx(p, 2, gy, gx)];
             pz = (double)u[uidx(p, 3, gy, gx)];
         }
-        if (MODE == 0 && N > 0 && (p.flags & SHARK_FLAG_DRAG)) {
+        if (drag) {
             // regularisation floor (dust_drag.f90:63-73)
             for (int k = 0; k < N; ++k) {
                 const long long ir = uidx(p, 5 + k, gy, gx);
@@ -736,17 +883,17 @@ __global__ void __launch_bounds__(256) k_finalize(KParams<R> p) {
                 if (fl > rd) u[ir] = R(fl);
             }
         }
-        if (MODE == 0 && N > 0 && br && p.iso < 1) {   // drag heating, part of S_U (source_terms.f90:88-97)
+        if (DRAG && N > 0 && br && p.iso < 1) {   // drag heating, part of S_U (source_terms.f90:88-97)
             const long long ie = uidx(p, 4, gy, gx);
             u[ie] = R((double)u[ie] + drag_heating(p, gx, gy, dt));
         }
         if (GROW && MODE == 0) st |= grow_in_finalize(p, u, gx, gy, dt);   // dust_growth (solve.f90:113)
-        if (MODE == 0 && p.ou_nm > 0) {                                    // turbulence kick (solve.f90:129-146)
+        if (REST && p.ou_nm > 0) {                                    // turbulence kick (solve.f90:129-146)
             turb_kick_cell<double>(p, u, gx, gy, dt);
             px = (double)u[uidx(p, 1, gy, gx)];
             py = (double)u[uidx(p, 2, gy, gx)];
         }
-        if (MODE == 0 && p.setup == SHARK_SETUP_SI && !(p.flags & SHARK_FLAG_FORCE_KICK)) {
+        if (REST && p.setup == SHARK_SETUP_SI && !(p.flags & SHARK_FLAG_FORCE_KICK)) {
             // setup_inloop: Crank-Nicolson rotation (SI/setup.f90:299-332)
             const double om = p.si_om, qsh = p.si_q;
             const double Ohmdt = om * dt;
@@ -770,13 +917,14 @@ __global__ void __launch_bounds__(256) k_finalize(KParams<R> p) {
                 u[ixx] = R(d * (vx * (1. - Ohmdt * Ohmdt) - 2. * uz * Ohmdt + AA * Ohmdt) / (1. + Ohmdt * Ohmdt));
             }
         }
-        if (MODE == 0 && ((p.setup == SHARK_SETUP_DISK_POLAR && disk_inloop_cell<R, double>(p, u, gx, gy, dt)) ||
+        if (REST && ((p.setup == SHARK_SETUP_DISK_POLAR && disk_inloop_cell<R, double>(p, u, gx, gy, dt)) ||
                           (p.setup == SHARK_SETUP_DISK_CART && cdisk_inloop_cell<R>(p, u, gx, gy)))) {
             rho = (double)u[uidx(p, 0, gy, gx)];
             px = (double)u[uidx(p, 1, gy, gx)];
             py = (double)u[uidx(p, 2, gy, gx)];
             pz = (double)u[uidx(p, 3, gy, gx)];
         }
+        if (MODE == 2) return;   // k_growth_d and MODE 3 follow
         // ---- courant on the final state (src/solver/courant.f90:11-124) -----------------------
         const double cfl = p.cfl;
         const double qrho = rho > p.smallr ? rho : p.smallr;
@@ -842,8 +990,9 @@ __global__ void __launch_bounds__(256) k_finalize(KParams<R> p) {
         if (!isfinite(vx) || !isfinite(vy) || !isfinite(vz) || !isfinite(rho)) st |= SHARK_STATUS_NAN;
         if (!(dtc > 0.0) || !isfinite(dtc)) { st |= SHARK_STATUS_DT_UNDERFLOW; dtc = 2e44; }
     }
+    if (MODE == 2) return;
     block_reduce_dt(dtc, st, p.dt_next, p.status);
-    if (MODE == 0 && gx < p.ng + p.nx) fill_ghost_images(p, p.u_next, gx, gy);
+    if (REST && gx < p.ng + p.nx) fill_ghost_images(p, p.u_next, gx, gy);
 }
 
 // ---------------------------------------------------------------------------------------------
