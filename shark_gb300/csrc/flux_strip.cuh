@@ -141,14 +141,14 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
             } else {
                 const R y = rcp64(rho);
                 vx = div64(px, rho, y); vy = div64(py, rho, y); vz = div64(pz, rho, y);
-                q[0] = max64(rho, smallR);
+                q[0] = max64_pos(rho, smallR);
                 if (iso) {
                     c = cs_at(row);
                     P = rho * sq(c);
                 } else {
                     const R hr = half * rho;
                     const R ekin = hr * sq(vx) + hr * sq(vy) + hr * sq(vz);
-                    P = max64((gamma - R(1)) * (us[4] - ekin), smallP);
+                    P = max64_pos((gamma - R(1)) * (us[4] - ekin), smallP);
                     c = sqrt(div64(gamma * P, q[0], q[0] == rho ? y : rcp64(q[0])));
                 }
             }
@@ -267,7 +267,7 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                 R sp0 = -u * dpx - v * dpy - (dux + dvy) * gamma * pp;
                 if (polar) sp0 = -u * dpx - v * dpy - (dux + dvy) * gamma * pp - over_r(gamma * pp * u);
                 const R b4 = pp + hdt * sp0;
-                auto floor_P = [&](R x) -> R { if constexpr (FAST) return fmaxf(x, smallP); else return max64(x, smallP); };
+                auto floor_P = [&](R x) -> R { if constexpr (FAST) return fmaxf(x, smallP); else return max64_pos(x, smallP); };
                 qmx[4] = floor_P(b4 + hdx * dpx); qpx[4] = floor_P(b4 - hdx * dpx);
                 qmy[4] = floor_P(b4 + hdy * dpy); qpy[4] = floor_P(b4 - hdy * dpy);
             }

@@ -83,7 +83,11 @@ static void finalize_launch(const KParams<R>& p, dim3 grid, cudaStream_t st) {
             k_finalize_mixed<NS, MODE, GROW><<<g, K2M_THREADS, 0, st>>>(p);
         }
     }
-    else k_finalize<R, NS, MODE, GROW><<<grid, 256, 0, st>>>(p);
+    else {
+        dim3 g = grid;
+        g.x = (p.nx + K2D_THREADS - 1) / K2D_THREADS;
+        k_finalize<R, NS, MODE, GROW><<<g, K2D_THREADS, 0, st>>>(p);
+    }
 }
 
 // FP64 growth without fragmentation: the drag, k_growth_d, the rest of K2.

@@ -285,9 +285,9 @@ __device__ __forceinline__ void atomic_min_dt(unsigned long long* a, double v) {
 // Every thread of the block must call it (no early return before it).
 __device__ __forceinline__ void block_reduce_dt(double dtc, unsigned int st, unsigned long long* dt_next,
                                                 unsigned int* status) {
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = 16; o > 0; o >>= 1) {   // positive doubles order as their bits
         const double other = __shfl_xor_sync(0xffffffffu, dtc, o);
-        dtc = other < dtc ? other : dtc;
+        dtc = abs_less(other, dtc) ? other : dtc;
         st |= __shfl_xor_sync(0xffffffffu, st, o);
     }
     __shared__ double wmin[32];
@@ -301,7 +301,7 @@ __device__ __forceinline__ void block_reduce_dt(double dtc, unsigned int st, uns
         st = lane < nw ? wst[lane] : 0u;
         for (int o = 16; o > 0; o >>= 1) {
             const double other = __shfl_xor_sync(0xffffffffu, dtc, o);
-            dtc = other < dtc ? other : dtc;
+            dtc = abs_less(other, dtc) ? other : dtc;
             st |= __shfl_xor_sync(0xffffffffu, st, o);
         }
         if (lane == 0) {
@@ -345,54 +345,72 @@ template <typename R>
 __device__ __forceinline__ double cs_start(const KParams<R>& p, int gx, int gy) {
     if (p.iso == 1) return p.ccsd ? p.ccsd[(long long)gy * p.pitch + gx] : p.csd[gx];
     const double rho = (double)p.u_cur[uidx(p, 0, gy, gx)];
-    const double vx = (double)p.u_cur[uidx(p, 1, gy, gx)] / rho, vy = (double)p.u_cur[uidx(p, 2, gy, gx)] / rho;
-    const double vz = (double)p.u_cur[uidx(p, 3, gy, gx)] / rho;
-    const double ekin = 0.5 * rho * (vx * vx) + 0.5 * rho * (vy * vy) + 0.5 * rho * (vz * vz);
-    double P = (p.gamma - 1.0) * ((double)p.u_cur[uidx(p, 4, gy, gx)] - ekin - 0.0);
-    P = P > p.smallp ? P : p.smallp;
-    const double qr = rho > p.smallr ? rho : p.smallr;
-    return sqrt(p.gamma * P / qr);
+    const Over<double> by_rho(rho);
+    const double vx = by_rho((double)p.u_cur[uidx(p, 1, gy, gx)]), vy = by_rho((double)p.u_cur[uidx(p, 2, gy, gx)]);
+    const double vz = by_rho((double)p.u_cur[uidx(p, 3, gy, gx)]);
+    const double hr = 0.5 * rho;
+    const double ekin = hr * (vx * vx) + hr * (vy * vy) + hr * (vz * vz);
+    double P = (p.gamma - 1.0) * ((double)p.u_cur[uidx(p, 4, gy, gx)] - ekin);
+    P = max64_pos(P, p.smallp);
+    const Over<double> by_q(max64_pos(rho, p.smallr));
+    return sqrt(by_q(p.gamma * P));
 }
 
-// Stopping time of species k at cell (gx, gy) from the state at the start of the step
-// (compute_tstop runs before the update, solve.f90:34-35); qrho_old = max(rho_old, smallr).
+// Stopping times of a cell's species from the state at the start of the step (compute_tstop runs
+// before the update, solve.f90:34-35); qrho_old = max(rho_old, smallr).  What the species share (the
+// sound speed, the reciprocals) is formed once per cell.
 template <typename R>
-__device__ __forceinline__ double tstop_cell(const KParams<R>& p, int k, double qrho_old, int gx, int gy) {
-    constexpr double pi = 3.141592653589793238462643383279;
-    if (p.setup == SHARK_SETUP_SI) return p.dtstop[k];                       // SI/setup.f90:389-397
-    if (p.setup == SHARK_SETUP_DUSTYWAVE) {                                  // DUSTYWAVE/setup.f90:217
-        const double rd_old = (double)p.u_cur[uidx(p, 5 + k, gy, gx)];
-        return rd_old * qrho_old / p.dK[k] / (qrho_old);
+struct TStop {
+    const KParams<R>& p;
+    long long cell;
+    double c0;
+    Over<double> by_q, by_d;   // qrho_old; the sound speed (dustyTurb) or Epstein's rho cs
+    __device__ __forceinline__ TStop(const KParams<R>& p_, double qrho_old, int gx, int gy)
+        : p(p_), cell((long long)gy * p_.pitch + gx), c0(0.0),
+          by_q(p_.setup == SHARK_SETUP_DUSTYWAVE || p_.setup == SHARK_SETUP_DUSTYTURB ? qrho_old : 1.0),
+          by_d(denominator(p_, qrho_old, gx, gy)) {
+        constexpr double pi = 3.141592653589793238462643383279;
+        if (p.setup == SHARK_SETUP_DUSTYTURB) c0 = p.turb_rho0;
+        else if (p.setup != SHARK_SETUP_SI && p.setup != SHARK_SETUP_DUSTYWAVE) c0 = sqrt(pi * p.gamma / 8.0) * (p.rhograin);
     }
-    if (p.setup == SHARK_SETUP_DUSTYTURB)    // dustyTurb/setup.f90:456
-        return p.dstokes[k] * p.box_l * p.turb_rho0 / p.csd[gx] / qrho_old;
-    if (p.setup == SHARK_SETUP_DISK_POLAR)   // Epstein on the midplane density Sigma/(sqrt(2 pi) H)
-        return sqrt(pi * p.gamma / 8.0) * (p.rhograin) * p.dsize[k] / (qrho_old / p.hsd[gx] * p.csd[gx]);
-    if (p.setup == SHARK_SETUP_DISK_CART) {  // disk/setup.f90 compute_tstop: Sigma/sqrt(2 pi H)
-        const long long e = (long long)gy * p.pitch + gx;
-        return sqrt(pi * p.gamma / 8.0) * (p.rhograin) * p.dsize[k] / (qrho_old / p.chsd[e] * p.ccsd[e]);
+    static __device__ __forceinline__ double denominator(const KParams<R>& p, double qrho_old, int gx, int gy) {
+        if (p.setup == SHARK_SETUP_SI || p.setup == SHARK_SETUP_DUSTYWAVE) return 1.0;
+        if (p.setup == SHARK_SETUP_DUSTYTURB) return p.csd[gx];
+        if (p.setup == SHARK_SETUP_DISK_POLAR)   // Epstein on the midplane density Sigma/(sqrt(2 pi) H)
+            return Over<double>(p.hsd[gx])(qrho_old) * p.csd[gx];
+        if (p.setup == SHARK_SETUP_DISK_CART) {  // disk/setup.f90 compute_tstop: Sigma/sqrt(2 pi H)
+            const long long e = (long long)gy * p.pitch + gx;
+            return Over<double>(p.chsd[e])(qrho_old) * p.ccsd[e];
+        }
+        // Epstein (SOD/setup.f90:179-185) with the cell's sound speed
+        return qrho_old * cs_start(p, gx, gy);
     }
-    // Epstein (SOD/setup.f90:179-185) with the cell's sound speed
-    return sqrt(pi * p.gamma / 8.0) * (p.rhograin) * p.dsize[k] / (qrho_old * cs_start(p, gx, gy));
-}
+    __device__ __forceinline__ double operator()(int k) const {
+        if (p.setup == SHARK_SETUP_SI) return p.dtstop[k];                       // SI/setup.f90:389-397
+        if (p.setup == SHARK_SETUP_DUSTYWAVE)                                    // DUSTYWAVE/setup.f90:217
+            return by_q(Over<double>(p.dK[k])((double)p.u_cur[(5 + k) * p.plane + cell] * by_q.b));
+        if (p.setup == SHARK_SETUP_DUSTYTURB)                                    // dustyTurb/setup.f90:456
+            return by_q(by_d(p.dstokes[k] * p.box_l * c0));
+        return by_d(c0 * p.dsize[k]);
+    }
+};
 
 // Drag heating of an adiabatic gas with back reaction (source_terms.f90:88-97): the energy
 // gains sum_k dt v.(v - v_k)/t_k with the velocities and stopping times at the start of the step.
 template <typename R>
-__device__ __forceinline__ double drag_heating(const KParams<R>& p, int gx, int gy, double dt) {
+__device__ __forceinline__ double drag_heating(const KParams<R>& p, const TStop<R>& tstop, int gx, int gy, double dt) {
     const int N = p.ndust;
     const double rho = (double)p.u_cur[uidx(p, 0, gy, gx)];
-    const double qrho = rho > p.smallr ? rho : p.smallr;
-    const double vx = (double)p.u_cur[uidx(p, 1, gy, gx)] / rho, vy = (double)p.u_cur[uidx(p, 2, gy, gx)] / rho;
-    const double vz = (double)p.u_cur[uidx(p, 3, gy, gx)] / rho;
+    const Over<double> by_rho(rho);
+    const double vx = by_rho((double)p.u_cur[uidx(p, 1, gy, gx)]), vy = by_rho((double)p.u_cur[uidx(p, 2, gy, gx)]);
+    const double vz = by_rho((double)p.u_cur[uidx(p, 3, gy, gx)]);
     double S = 0.0;
     for (int k = 0; k < N; ++k) {
-        const double ts = tstop_cell(p, k, qrho, gx, gy);
-        const double rd = (double)p.u_cur[uidx(p, 5 + k, gy, gx)];
-        const double vdx = (double)p.u_cur[uidx(p, 5 + N + k, gy, gx)] / rd;
-        const double vdy = (double)p.u_cur[uidx(p, 5 + 2 * N + k, gy, gx)] / rd;
-        const double vdz = (double)p.u_cur[uidx(p, 5 + 3 * N + k, gy, gx)] / rd;
-        S = S + dt * (vx * (vx - vdx)) / ts + dt * (vy * (vy - vdy)) / ts + dt * (vz * (vz - vdz)) / ts;
+        const Over<double> by_ts(tstop(k)), by_rd((double)p.u_cur[uidx(p, 5 + k, gy, gx)]);
+        const double vdx = by_rd((double)p.u_cur[uidx(p, 5 + N + k, gy, gx)]);
+        const double vdy = by_rd((double)p.u_cur[uidx(p, 5 + 2 * N + k, gy, gx)]);
+        const double vdz = by_rd((double)p.u_cur[uidx(p, 5 + 3 * N + k, gy, gx)]);
+        S = S + by_ts(dt * (vx * (vx - vdx))) + by_ts(dt * (vy * (vy - vdy))) + by_ts(dt * (vz * (vz - vdz)));
     }
     return S;
 }
@@ -414,11 +432,13 @@ __device__ __forceinline__ bool disk_inloop_cell(const KParams<R>& p, R* u, int 
     for (int s = 0; s <= N; ++s) {
         const int ir = svar(s, 0, N), ivx = svar(s, 1, N), ivy = svar(s, 2, N);
         const C rho_init = C(p.u_init[uidx(p, ir, gy, gx)]);
-        const C vx_init = C(p.u_init[uidx(p, ivx, gy, gx)]) / rho_init;
-        const C vy_init = C(p.u_init[uidx(p, ivy, gy, gx)]) / rho_init;
+        const Over<C> by_init(rho_init);
+        const C vx_init = by_init(C(p.u_init[uidx(p, ivx, gy, gx)]));
+        const C vy_init = by_init(C(p.u_init[uidx(p, ivy, gy, gx)]));
         const C rho_old = C(u[uidx(p, ir, gy, gx)]);
-        const C vx_old = C(u[uidx(p, ivx, gy, gx)]) / rho_old;
-        const C vy_old = C(u[uidx(p, ivy, gy, gx)]) / rho_old;
+        const Over<C> by_old(rho_old);
+        const C vx_old = by_old(C(u[uidx(p, ivx, gy, gx)]));
+        const C vy_old = by_old(C(u[uidx(p, ivy, gy, gx)]));
         const C rho_new = (rho_init) * (C(1) - e) + rho_old * e;
         const C vx_new = (vx_init) * (C(1) - e) + vx_old * e;
         const C vy_new = (vy_init) * (C(1) - e) + vy_old * e;
@@ -462,9 +482,10 @@ __device__ __noinline__ unsigned grow_in_finalize(const KParams<R>& p, R* u, int
     const double qrho_old = rho_old > p.smallr ? rho_old : p.smallr;
     const bool ambi = (p.gw.mode & SHARK_GROWTH_AMBIPOLAR) && p.chg_gamma_d;
     const long long c = (long long)gy * p.pitch + gx;
+    const TStop<R> tstop(p, qrho_old, gx, gy);
     for (int k = 0; k < N; ++k) {
         rd[k] = (double)u[uidx(p, 5 + k, gy, gx)];
-        ts[k] = tstop_cell(p, k, qrho_old, gx, gy);
+        ts[k] = tstop(k);
         const double r0 = (double)p.u_cur[uidx(p, 5 + k, gy, gx)];
         vx[k] = (double)p.u_cur[uidx(p, 5 + N + k, gy, gx)] / r0;
         vy[k] = (double)p.u_cur[uidx(p, 5 + 2 * N + k, gy, gx)] / r0;
@@ -538,8 +559,7 @@ static __device__ __noinline__ unsigned grow_block_warps(const KParams<float>& p
     const float stick = (float)g.sticking, cflg = (float)g.cfl;
     const float eps_thr = (float)g.eps_thr, rmin = (float)g.dust_ratio_min, smallr = (float)p.smallr;
     // stopping times for the pair velocities (FP32): t_k = C_k / F_cell with the tabulated 1/C_k
-    // (dustyTurb F = c_s rho, polar disk F = rho/hs c_s); other setups through tstop_cell
-    const bool ts_tab = p.setup == SHARK_SETUP_DUSTYTURB || p.setup == SHARK_SETUP_DISK_POLAR;
+    // (dustyTurb F = c_s rho, polar disk F = rho/hs c_s: the setups with growth)
     const float invc = p.dinvts_f[b];
     const GrowthRunF rf = growth_run_consts_f(g);
     const float4 row0 = growth_row_f(g, 0);        // the one temperature row (dustyTurb)
@@ -550,13 +570,8 @@ static __device__ __noinline__ unsigned grow_block_warps(const KParams<float>& p
         const float rho_old = p.u_cur[uidx(p, 0, gy, gx)];
         const float qrho_old = rho_old > smallr ? rho_old : smallr;
         float rd = u[uidx(p, 5 + b, gy, gx)];
-        float ts;
-        if (ts_tab) {
-            const float F = p.setup == SHARK_SETUP_DUSTYTURB ? p.cs[gx] * qrho_old : qrho_old / (float)p.hsd[gx] * p.cs[gx];
-            ts = 1.f / (invc * F);
-        } else {
-            ts = (float)tstop_cell(p, b, (double)qrho_old, gx, gy);
-        }
+        const float F = p.setup == SHARK_SETUP_DUSTYTURB ? p.cs[gx] * qrho_old : qrho_old / (float)p.hsd[gx] * p.cs[gx];
+        const float ts = 1.f / (invc * F);
         const float r0 = p.u_cur[uidx(p, 5 + b, gy, gx)];
         const float vx = p.u_cur[uidx(p, 5 + N + b, gy, gx)] / r0;
         const float vy = p.u_cur[uidx(p, 5 + 2 * N + b, gy, gx)] / r0;
@@ -692,18 +707,20 @@ static __global__ void __launch_bounds__(GROWTH_D_THREADS) k_growth_d(KParams<do
     const double dt = *p.dt;
     const bool ambi = (g.mode & SHARK_GROWTH_AMBIPOLAR) && p.chg_gamma_d;
     const long long e = (long long)gy * p.pitch + gx;
-    const double rho_old = p.u_cur[e], qrho_old = max64(rho_old, p.smallr);
+    const double rho_old = p.u_cur[e], qrho_old = max64_pos(rho_old, p.smallr);
     const double hs = p.setup == SHARK_SETUP_DISK_POLAR ? p.hsd[gx] : 1.0, yhs = rcp64(hs);
     const double rho_gas = u[e];
     const GrowthCellD c = growth_cell_consts_d(g, gx, qrho_old, hs, ambi ? p.chg_eta[2 * p.plane + e] : 0.0);
     // the species' terms
+    const TStop<double> tstop(p, qrho_old, gx, gy);
+    const Over<double> by_tL(c.t_L);
     for (int k = l; k < N; k += GL) {
         rd[k] = u[(5 + k) * p.plane + e];
-        const double t = tstop_cell(p, k, qrho_old, gx, gy), St = t / c.t_L;
+        const double t = tstop(k), St = by_tL(t);
         ts[k] = t;
         S[k] = St;
-        W[k] = St * St / (St + c.rm);
-        I[k] = 1.0 / (1.0 + St);
+        W[k] = Over<double>(St + c.rm)(St * St);
+        I[k] = Over<double>(1.0 + St)(1.0);
         const double r0 = p.u_cur[(5 + k) * p.plane + e], y = rcp64(r0);
         vx[k] = div64(p.u_cur[(5 + N + k) * p.plane + e], r0, y);
         vy[k] = div64(p.u_cur[(5 + 2 * N + k) * p.plane + e], r0, y);
@@ -813,8 +830,15 @@ __device__ __forceinline__ void turb_kick_cell(const KParams<R>& p, R* u, int gx
     u[uidx(p, 2, gy, gx)] = R(C(u[uidx(p, 2, gy, gx)]) + rho * ay * C(dt));
 }
 
+// Bound by the FP64 pipe (64 clocks of an SM partition for a warp's instruction): quotients share
+// reciprocals, compares and finiteness checks run on the bits, one square root takes the largest of
+// the force limiter's sums; all exact.  SI boxes of 8 species: 1024^2 2.36 -> 1.38 ms, 256^2 0.183 ->
+// 0.116 ms; dusty wave of 2048 x 4 0.075 -> 0.026 ms.  Blocks of 128: the warps of one or two
+// thousand cells then each have a partition of their own.
+constexpr int K2D_THREADS = 128;
+
 template <typename R, int NS, int MODE, bool GROW = false>
-__global__ void __launch_bounds__(256) k_finalize(KParams<R> p) {
+__global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
     constexpr int NMAX = NS > 0 ? NS : 1;
     constexpr bool DRAG = MODE == 0 || MODE == 2, REST = MODE == 0 || MODE == 3;
     const int N = NS >= 0 ? NS : p.ndust;
@@ -829,66 +853,57 @@ __global__ void __launch_bounds__(256) k_finalize(KParams<R> p) {
         double px = (double)u[uidx(p, 1, gy, gx)], py = (double)u[uidx(p, 2, gy, gx)], pz = (double)u[uidx(p, 3, gy, gx)];
         const bool drag = DRAG && N > 0 && (p.flags & SHARK_FLAG_DRAG);
         const bool br = (p.flags & SHARK_FLAG_BACK_REACTION) != 0;
-        if (drag) {
-            // dust_drag(1.0) (src/dust/dust_drag.f90:2-75), FP64 arithmetic
-            double alpha[NMAX];
-            double rhon = rho, pnx = px, pny = py, pnz = pz;
-            // stopping time from the state at the start of the step (compute_tstop runs before
-            // the update in solve.f90:34-35)
+        const bool heat = DRAG && N > 0 && br && p.iso < 1;
+        if (drag || heat) {
+            // stopping times from the state at the start of the step (compute_tstop runs before the
+            // update in solve.f90:34-35)
             const double rho_old = (double)p.u_cur[uidx(p, 0, gy, gx)];
-            const double qrho_old = rho_old > p.smallr ? rho_old : p.smallr;
-            for (int k = 0; k < N; ++k) {
-                const double ts = tstop_cell(p, k, qrho_old, gx, gy);
-                const double a = 1.0 * dt / ts;
-                const double pdx = (double)u[uidx(p, 5 + N + k, gy, gx)];
-                const double pdy = (double)u[uidx(p, 5 + 2 * N + k, gy, gx)];
-                const double pdz = (double)u[uidx(p, 5 + 3 * N + k, gy, gx)];
-                const double rd = (double)u[uidx(p, 5 + k, gy, gx)];
-                pnx = pnx + a / (1.0 + a) * pdx;
-                pny = pny + a / (1.0 + a) * pdy;
-                pnz = pnz + a / (1.0 + a) * pdz;
-                rhon = rhon + a / (1.0 + a) * rd;
-                if (NS > 0) alpha[k < NMAX ? k : 0] = a;
+            const TStop<R> tstop(p, max64_pos(rho_old, p.smallr), gx, gy);
+            if (drag) {
+                // dust_drag(1.0) (src/dust/dust_drag.f90:2-75), FP64 arithmetic
+                double alpha[NMAX];
+                double rhon = rho, pnx = px, pny = py, pnz = pz;
+                for (int k = 0; k < N; ++k) {
+                    const double a = Over<double>(tstop(k))(dt);
+                    const double w = Over<double>(1.0 + a)(a);
+                    pnx = pnx + w * (double)u[uidx(p, 5 + N + k, gy, gx)];
+                    pny = pny + w * (double)u[uidx(p, 5 + 2 * N + k, gy, gx)];
+                    pnz = pnz + w * (double)u[uidx(p, 5 + 3 * N + k, gy, gx)];
+                    rhon = rhon + w * (double)u[uidx(p, 5 + k, gy, gx)];
+                    if (NS > 0) alpha[k < NMAX ? k : 0] = a;
+                }
+                const Over<double> by_rhon(rhon);
+                const double fl = rho * p.dust_ratio_min;   // regularisation floor (dust_drag.f90:63-73)
+                for (int k = 0; k < N; ++k) {
+                    double a;
+                    if (NS > 0) a = alpha[k < NMAX ? k : 0];
+                    else a = Over<double>(tstop(k))(dt);    // run-time species count
+                    const Over<double> by_a(1.0 + a);
+                    const double w = by_a(a);
+                    const long long ir = uidx(p, 5 + k, gy, gx), ix_ = uidx(p, 5 + N + k, gy, gx),
+                                    iy_ = uidx(p, 5 + 2 * N + k, gy, gx), iz_ = uidx(p, 5 + 3 * N + k, gy, gx);
+                    const double rd = (double)u[ir];
+                    u[ix_] = R(by_a((double)u[ix_]) + by_rhon(w * pnx) * rd);
+                    u[iy_] = R(by_a((double)u[iy_]) + by_rhon(w * pny) * rd);
+                    u[iz_] = R(by_a((double)u[iz_]) + by_rhon(w * pnz) * rd);
+                    if (less_num(rd, fl)) u[ir] = R(fl);
+                }
+                if (br) {
+                    px = by_rhon(pnx) * rho;
+                    py = by_rhon(pny) * rho;
+                    pz = by_rhon(pnz) * rho;
+                    u[uidx(p, 1, gy, gx)] = R(px);
+                    u[uidx(p, 2, gy, gx)] = R(py);
+                    u[uidx(p, 3, gy, gx)] = R(pz);
+                }
             }
-            for (int k = 0; k < N; ++k) {
-                double a;
-                if (NS > 0) a = alpha[k < NMAX ? k : 0];
-                else a = 1.0 * dt / tstop_cell(p, k, qrho_old, gx, gy);   // run-time species count
-                const long long ix_ = uidx(p, 5 + N + k, gy, gx), iy_ = uidx(p, 5 + 2 * N + k, gy, gx),
-                                iz_ = uidx(p, 5 + 3 * N + k, gy, gx);
-                const double rd = (double)u[uidx(p, 5 + k, gy, gx)];
-                u[ix_] = R((double)u[ix_] / (1.0 + a) + (a / (1.0 + a)) * pnx / rhon * rd);
-                u[iy_] = R((double)u[iy_] / (1.0 + a) + (a / (1.0 + a)) * pny / rhon * rd);
-                u[iz_] = R((double)u[iz_] / (1.0 + a) + (a / (1.0 + a)) * pnz / rhon * rd);
+            if (heat) {   // drag heating, part of S_U (source_terms.f90:88-97)
+                const long long ie = uidx(p, 4, gy, gx);
+                u[ie] = R((double)u[ie] + drag_heating(p, tstop, gx, gy, dt));
             }
-            if (br) {
-                px = pnx / rhon * rho;
-                py = pny / rhon * rho;
-                pz = pnz / rhon * rho;
-                u[uidx(p, 1, gy, gx)] = R(px);
-                u[uidx(p, 2, gy, gx)] = R(py);
-                u[uidx(p, 3, gy, gx)] = R(pz);
-            }
-            // re-read the stored (rounded) values so the dt below sees exactly the stored state
-            px = (double)u[uidx(p, 1, gy, gx)];
-            py = (double)u[uidx(p, 2, gy, gx)];
-            pz = (double)u[uidx(p, 3, gy, gx)];
-        }
-        if (drag) {
-            // regularisation floor (dust_drag.f90:63-73)
-            for (int k = 0; k < N; ++k) {
-                const long long ir = uidx(p, 5 + k, gy, gx);
-                const double rd = (double)u[ir];
-                const double fl = rho * p.dust_ratio_min;
-                if (fl > rd) u[ir] = R(fl);
-            }
-        }
-        if (DRAG && N > 0 && br && p.iso < 1) {   // drag heating, part of S_U (source_terms.f90:88-97)
-            const long long ie = uidx(p, 4, gy, gx);
-            u[ie] = R((double)u[ie] + drag_heating(p, gx, gy, dt));
         }
         if (GROW && MODE == 0) st |= grow_in_finalize(p, u, gx, gy, dt);   // dust_growth (solve.f90:113)
-        if (REST && p.ou_nm > 0) {                                    // turbulence kick (solve.f90:129-146)
+        if (REST && p.ou_nm > 0) {                                         // turbulence kick (solve.f90:129-146)
             turb_kick_cell<double>(p, u, gx, gy, dt);
             px = (double)u[uidx(p, 1, gy, gx)];
             py = (double)u[uidx(p, 2, gy, gx)];
@@ -898,27 +913,28 @@ __global__ void __launch_bounds__(256) k_finalize(KParams<R> p) {
             const double om = p.si_om, qsh = p.si_q;
             const double Ohmdt = om * dt;
             const double xc = p.xposd[gx] - 0.5 * p.box_l;
+            const Over<double> by_rot(1. + Ohmdt * Ohmdt);
             double AA = 2.0 * qsh * om * xc - 2.0 * p.si_r0 * p.si_eta;
             {
-                const double uz = pz / rho, vx = px / rho, d = rho;
-                pz = d * (uz * (1. - Ohmdt * Ohmdt) + 2. * vx * Ohmdt + AA * (Ohmdt * Ohmdt)) / (1. + Ohmdt * Ohmdt);
-                px = d * (vx * (1. - Ohmdt * Ohmdt) - 2. * uz * Ohmdt + AA * Ohmdt) / (1. + Ohmdt * Ohmdt);
+                const Over<double> by_rho(rho);
+                const double uz = by_rho(pz), vx = by_rho(px), d = rho;
+                pz = by_rot(d * (uz * (1. - Ohmdt * Ohmdt) + 2. * vx * Ohmdt + AA * (Ohmdt * Ohmdt)));
+                px = by_rot(d * (vx * (1. - Ohmdt * Ohmdt) - 2. * uz * Ohmdt + AA * Ohmdt));
                 u[uidx(p, 3, gy, gx)] = R(pz);
                 u[uidx(p, 1, gy, gx)] = R(px);
-                pz = (double)u[uidx(p, 3, gy, gx)];
-                px = (double)u[uidx(p, 1, gy, gx)];
             }
             AA = 2.0 * qsh * om * xc;
             for (int k = 0; k < N; ++k) {
                 const long long iz = uidx(p, 5 + 3 * N + k, gy, gx), ixx = uidx(p, 5 + N + k, gy, gx);
                 const double d = (double)u[uidx(p, 5 + k, gy, gx)];
-                const double uz = (double)u[iz] / d, vx = (double)u[ixx] / d;
-                u[iz] = R(d * (uz * (1. - Ohmdt * Ohmdt) + 2. * vx * Ohmdt + AA * (Ohmdt * Ohmdt)) / (1. + Ohmdt * Ohmdt));
-                u[ixx] = R(d * (vx * (1. - Ohmdt * Ohmdt) - 2. * uz * Ohmdt + AA * Ohmdt) / (1. + Ohmdt * Ohmdt));
+                const Over<double> by_d(d);
+                const double uz = by_d((double)u[iz]), vx = by_d((double)u[ixx]);
+                u[iz] = R(by_rot(d * (uz * (1. - Ohmdt * Ohmdt) + 2. * vx * Ohmdt + AA * (Ohmdt * Ohmdt))));
+                u[ixx] = R(by_rot(d * (vx * (1. - Ohmdt * Ohmdt) - 2. * uz * Ohmdt + AA * Ohmdt)));
             }
         }
         if (REST && ((p.setup == SHARK_SETUP_DISK_POLAR && disk_inloop_cell<R, double>(p, u, gx, gy, dt)) ||
-                          (p.setup == SHARK_SETUP_DISK_CART && cdisk_inloop_cell<R>(p, u, gx, gy)))) {
+                     (p.setup == SHARK_SETUP_DISK_CART && cdisk_inloop_cell<R>(p, u, gx, gy)))) {
             rho = (double)u[uidx(p, 0, gy, gx)];
             px = (double)u[uidx(p, 1, gy, gx)];
             py = (double)u[uidx(p, 2, gy, gx)];
@@ -927,68 +943,76 @@ __global__ void __launch_bounds__(256) k_finalize(KParams<R> p) {
         if (MODE == 2) return;   // k_growth_d and MODE 3 follow
         // ---- courant on the final state (src/solver/courant.f90:11-124) -----------------------
         const double cfl = p.cfl;
-        const double qrho = rho > p.smallr ? rho : p.smallr;
-        const double vx = px / rho, vy = py / rho, vz = pz / rho;
+        const Over<double> by_rho(rho);
+        const double vx = by_rho(px), vy = by_rho(py), vz = by_rho(pz);
         double cs;
         if (p.iso == 1) cs = p.ccsd ? p.ccsd[(long long)gy * p.pitch + gx] : p.csd[gx];
         else {
+            const double qrho = max64_pos(rho, p.smallr);
             const double E = (double)u[uidx(p, 4, gy, gx)];
-            const double ekin = 0.5 * rho * (vx * vx) + 0.5 * rho * (vy * vy) + 0.5 * rho * (vz * vz);
-            double P = (p.gamma - 1.0) * (E - ekin - 0.0);
-            P = P > p.smallp ? P : p.smallp;
-            cs = sqrt(p.gamma * P / qrho);
-            if (!(E == E)) st |= SHARK_STATUS_NAN;
+            const double hr = 0.5 * rho;
+            const double ekin = hr * (vx * vx) + hr * (vy * vy) + hr * (vz * vz);
+            const double P = max64_pos((p.gamma - 1.0) * (E - ekin), p.smallp);
+            cs = sqrt(Over<double>(qrho)(p.gamma * P));
+            if (abs_bits(E) > 0x7ff0000000000000ull) st |= SHARK_STATUS_NAN;
         }
         double dxx;
         if (p.ndim == 1) dxx = p.dx1d[gx];
-        else if (p.geom == 2) { const double a = p.dx1d[gx], b = p.radcd[gx] * p.dx2d[gx]; dxx = a < b ? a : b; }
-        else { const double a = p.dx1d[gx], b = p.dx2d[gx]; dxx = a < b ? a : b; }
-        double vv = fabs(vx) + fabs(vy) + fabs(vz);
+        else if (p.geom == 2) dxx = min64(p.dx1d[gx], p.radcd[gx] * p.dx2d[gx]);
+        else dxx = min64(p.dx1d[gx], p.dx2d[gx]);
+        double vv = abs64(vx) + abs64(vy) + abs64(vz);
         double vmax = cs + vv;
-        double fmax_d = 0.0;
+        double fmax_d = 0.0;     // SI: the largest square of a force until its root is taken below
         const bool fk = (p.flags & SHARK_FLAG_FORCE_KICK) != 0;
-        if (fk && p.setup == SHARK_SETUP_SI) {
+        const bool fk_si = fk && p.setup == SHARK_SETUP_SI;
+        double tide = 0.0, om2 = 0.0;
+        if (fk_si) {
             const double xc = p.xposd[gx] - 0.5 * p.box_l, om = p.si_om, qsh = p.si_q;
-            const double f1 = 2.0 * qsh * (om * om) * xc - 2.0 * om * vz - 2.0 * p.si_r0 * om * p.si_eta;
-            const double f3 = 2.0 * om * vx;
-            fmax_d = sqrt(f1 * f1 + 0.0 * 0.0 + f3 * f3);
+            tide = 2.0 * qsh * (om * om) * xc;
+            om2 = 2.0 * om;
+            const double f1 = tide - om2 * vz - 2.0 * p.si_r0 * om * p.si_eta;
+            const double f3 = om2 * vx;
+            fmax_d = f1 * f1 + f3 * f3;
         } else if (fk && p.setup == SHARK_SETUP_DISK_POLAR) {
             // the same point-mass force acts on gas and every dust species
             const double g = p.fgravd[gx];
-            fmax_d = sqrt(g * g + 0.0 * 0.0 + 0.0 * 0.0);
+            fmax_d = sqrt(g * g);
         } else if (fk && p.setup == SHARK_SETUP_DISK_CART) {   // the star's softened force, gas and dust
             const long long e = (long long)gy * p.pitch + gx;
             const double fx = (double)p.cfx[e], fy = (double)p.cfy[e];
-            fmax_d = sqrt(fx * fx + fy * fy + 0.0 * 0.0);
+            fmax_d = sqrt(fx * fx + fy * fy);
         }
         for (int k = 0; k < N; ++k) {
             const double rd = (double)u[uidx(p, 5 + k, gy, gx)];
-            const double vdx = (double)u[uidx(p, 5 + N + k, gy, gx)] / rd;
-            const double vdy = (double)u[uidx(p, 5 + 2 * N + k, gy, gx)] / rd;
-            const double vdz = (double)u[uidx(p, 5 + 3 * N + k, gy, gx)] / rd;
-            vv = fabs(vdx) + fabs(vdy) + fabs(vdz);
-            vmax = vmax > (0.0 + vv) ? vmax : (0.0 + vv);
-            if (fk && p.setup == SHARK_SETUP_SI) {
-                const double xc = p.xposd[gx] - 0.5 * p.box_l, om = p.si_om, qsh = p.si_q;
-                const double f1 = 2.0 * qsh * (om * om) * xc - 2.0 * om * vdz;
-                const double f3 = 2.0 * om * vdx;
-                const double fm = sqrt(f1 * f1 + 0.0 * 0.0 + f3 * f3);
-                fmax_d = fmax_d > fm ? fmax_d : fm;
+            const Over<double> by_rd(rd);
+            const double vdx = by_rd((double)u[uidx(p, 5 + N + k, gy, gx)]);
+            const double vdy = by_rd((double)u[uidx(p, 5 + 2 * N + k, gy, gx)]);
+            const double vdz = by_rd((double)u[uidx(p, 5 + 3 * N + k, gy, gx)]);
+            vv = abs64(vdx) + abs64(vdy) + abs64(vdz);
+            vmax = less_num(vv, vmax) ? vmax : vv;
+            if (fk_si) {
+                const double f1 = tide - om2 * vdz;
+                const double f3 = om2 * vdx;
+                const double fm = f1 * f1 + f3 * f3;
+                fmax_d = less_num(fm, fmax_d) ? fmax_d : fm;
             }
-            if (!(rd > 0.0)) st |= SHARK_STATUS_NEG_DENSITY;
-            if (!isfinite(vdx) || !isfinite(vdy) || !isfinite(vdz)) st |= SHARK_STATUS_NAN;
+            if (!is_pos_num(rd)) st |= SHARK_STATUS_NEG_DENSITY;
+            if (!is_finite(vdx) || !is_finite(vdy) || !is_finite(vdz)) st |= SHARK_STATUS_NAN;
         }
-        const double c1 = cfl * dxx / fabs(vmax);
-        dtc = dtc < c1 ? dtc : c1;
-        if (fk && vv != 0.0) {
+        if (fk_si) fmax_d = sqrt(fmax_d);
+        const double cd = cfl * dxx;
+        // plain divisions where a wave speed may be zero or its square underflow
+        const double c1 = cd / abs64(vmax);
+        dtc = less_num(2e44, c1) ? 2e44 : c1;
+        if (fk && !is_zero(vv)) {
             double fratio = fmax_d * dxx / (vv * vv);
-            fratio = fratio > 1e-3 ? fratio : 1e-3;
-            const double c2 = cfl * dxx / vv * (sqrt(1.0 + 2.0 * cfl * fratio) - 1.0) / fratio;
-            dtc = dtc < c2 ? dtc : c2;
+            fratio = max64_pos(fratio, 1e-3);
+            const double c2 = Over<double>(fratio)(cd / vv * (sqrt(1.0 + 2.0 * cfl * fratio) - 1.0));
+            dtc = less_num(dtc, c2) ? dtc : c2;
         }
-        if (!(rho > 0.0)) st |= SHARK_STATUS_NEG_DENSITY;
-        if (!isfinite(vx) || !isfinite(vy) || !isfinite(vz) || !isfinite(rho)) st |= SHARK_STATUS_NAN;
-        if (!(dtc > 0.0) || !isfinite(dtc)) { st |= SHARK_STATUS_DT_UNDERFLOW; dtc = 2e44; }
+        if (!is_pos_num(rho)) st |= SHARK_STATUS_NEG_DENSITY;
+        if (!is_finite(vx) || !is_finite(vy) || !is_finite(vz) || !is_finite(rho)) st |= SHARK_STATUS_NAN;
+        if (!is_pos_num(dtc) || !is_finite(dtc)) { st |= SHARK_STATUS_DT_UNDERFLOW; dtc = 2e44; }
     }
     if (MODE == 2) return;
     block_reduce_dt(dtc, st, p.dt_next, p.status);
@@ -1009,17 +1033,55 @@ __device__ __forceinline__ void drag_coeffs(double a, float& r, float& w) {
 }
 
 // a_k = dt/t_k of the mixed path where the per-cell stopping time factors as t_k = C_k / F_cell
-// (dustyTurb C_k = St_0,k L rho_0, F = c_s rho; the disks' Epstein F = rho/hs c_s): dt F_cell times
-// the tabulated 1/C_k, and the coefficients with a refined reciprocal (FP64 throughout; the
-// divisions cost most of K2's FP64 work at 32 species).  Other setups divide directly.
+// (dustyTurb C_k = St_0,k L rho_0, F = c_s rho; the disks' Epstein F = rho/hs c_s, Epstein of an
+// adiabatic gas F = rho c_s): dt F_cell times the tabulated 1/C_k.  The dusty wave's t_k = rho_k/K_k
+// divides per species.
 __device__ __forceinline__ double drag_cell_factor(const KParams<float>& p, double dt, double qrho_old, int gx, int gy) {
     if (p.setup == SHARK_SETUP_DUSTYTURB) return dt * (p.csd[gx] * qrho_old);
     if (p.setup == SHARK_SETUP_DISK_CART) {
         const long long e = (long long)gy * p.pitch + gx;
         return dt * (qrho_old / p.chsd[e] * p.ccsd[e]);
     }
-    return dt * (qrho_old / p.hsd[gx] * p.csd[gx]);
+    if (p.setup == SHARK_SETUP_DISK_POLAR) return dt * (qrho_old / p.hsd[gx] * p.csd[gx]);
+    return dt * (qrho_old * cs_start(p, gx, gy));
 }
+
+// Drag coefficients and drag heating (source_terms.f90:88-97) of one cell in FP64 for the setups
+// whose sound speed or stopping times need the state at the start of the step.  Bound by the FP64
+// pipe: the cell's sound speed is formed once and 1/t_k = F_cell / C_k multiplied out, for the
+// coefficients and the heating alike (adiabatic KH box 500 x 301 x 4: K2 0.289 -> 0.076 ms).
+struct DragCell {
+    const KParams<float>& p;
+    int cc;
+    double dt, dtF, heat, vx, vy, vz;   // heat: sum of dt v.(v - v_k)/t_k
+    bool wave, heats;
+    __device__ __forceinline__ DragCell(const KParams<float>& p_, double dt_, double qrho_old, int gx, int gy, bool heats_,
+                                        bool used = true)
+        : p(p_), cc(gy * p_.pitch + gx), dt(dt_), dtF(0.0), heat(0.0), vx(0.0), vy(0.0), vz(0.0),
+          wave(p_.setup == SHARK_SETUP_DUSTYWAVE), heats(heats_) {
+        if (used && !wave) dtF = drag_cell_factor(p, dt, qrho_old, gx, gy);
+        if (heats) {
+            const Over<double> by_rho((double)p.u_cur[cc]);
+            vx = by_rho((double)p.u_cur[cc + p.plane]);
+            vy = by_rho((double)p.u_cur[cc + 2 * p.plane]);
+            vz = by_rho((double)p.u_cur[cc + 3 * p.plane]);
+        }
+    }
+    // a_k = dt/t_k of species k, its heating added
+    __device__ __forceinline__ double operator()(int k) {
+        const int N = p.ndust;
+        const double rd = (wave || heats) ? (double)p.u_cur[cc + (5 + k) * p.plane] : 1.0;
+        const Over<double> by_rd(rd);
+        const double a = wave ? by_rd(dt * p.dK[k]) : dtF * p.dinvts[k];
+        if (heats) {
+            const double ux = by_rd((double)p.u_cur[cc + (5 + N + k) * p.plane]);
+            const double uy = by_rd((double)p.u_cur[cc + (5 + 2 * N + k) * p.plane]);
+            const double uz = by_rd((double)p.u_cur[cc + (5 + 3 * N + k) * p.plane]);
+            heat += a * (vx * (vx - ux) + vy * (vy - uy) + vz * (vz - uz));
+        }
+        return a;
+    }
+};
 
 // The same coefficients in FP32 from a = dt F_cell / C_k formed in FP32 (dt F_cell once per cell
 // in FP64, then per species one product): r = 1/(1+a) and w = a r are well conditioned for every
@@ -1090,7 +1152,12 @@ k_finalize_mixed(KParams<float> p) {
     const float xc = act ? p.xpos[gx] - p.f_half_box_l : 0.f;
     // part 1: drag, floor, drag heating; part 2: kick, setup_inloop, CFL.  With growth in between
     // (a block-wide phase) the two parts are separate; otherwise they form one block of code.
+    const bool heats = MODE == 0 && N > 0 && (p.flags & SHARK_FLAG_BACK_REACTION) && p.iso < 1;
+    const bool direct = !const_ts && p.setup != SHARK_SETUP_DUSTYTURB && p.setup != SHARK_SETUP_DISK_POLAR &&
+                        p.setup != SHARK_SETUP_DISK_CART;
     auto part1 = [&]() {
+        bool heated = false;
+        double gain = 0.0;
         // the loads take their offsets from an opaque copy of the cell offset, so that the
         // compiler forms the stores' offsets anew instead of keeping every load offset live
         int cl = cc;
@@ -1113,13 +1180,16 @@ k_finalize_mixed(KParams<float> p) {
                 } else {
                     const float rho_old = ucur[cc + (0) * pl];
                     const double qrho_old = (double)fmaxf(rho_old, p.f_smallr);
-                    const bool direct = p.setup != SHARK_SETUP_DUSTYTURB && p.setup != SHARK_SETUP_DISK_POLAR &&
-                                          p.setup != SHARK_SETUP_DISK_CART;
-                    const float Fcf = direct ? 0.f : (float)drag_cell_factor(p, dt, qrho_old, gx, gy);
+                    if (direct) {
+                        DragCell dc(p, dt, qrho_old, gx, gy, heats);
 #pragma unroll
-                    for (int k = 0; k < NS; ++k) {
-                        if (direct) drag_coeffs_mix(1.0 * dt / tstop_cell(p, k, qrho_old, gx, gy), rk[k], wk[k]);
-                        else drag_coeffs_f(Fcf * p.dinvts_f[k], rk[k], wk[k]);
+                        for (int k = 0; k < NS; ++k) drag_coeffs_mix(dc(k), rk[k], wk[k]);
+                        gain = dc.heat;
+                        heated = heats;
+                    } else {
+                        const float Fcf = (float)drag_cell_factor(p, dt, qrho_old, gx, gy);
+#pragma unroll
+                        for (int k = 0; k < NS; ++k) drag_coeffs_f(Fcf * p.dinvts_f[k], rk[k], wk[k]);
                     }
                 }
                 float rhon = rho, pnx = px, pny = py, pnz = pz;
@@ -1173,16 +1243,15 @@ k_finalize_mixed(KParams<float> p) {
             float rhon = rho, pnx = px, pny = py, pnz = pz;
             const float rho_old = ucur[cc + (0) * pl];
             const double qrho_old = (double)fmaxf(rho_old, p.f_smallr);
-            const bool direct = p.setup != SHARK_SETUP_DUSTYTURB && p.setup != SHARK_SETUP_DISK_POLAR &&
-                                          p.setup != SHARK_SETUP_DISK_CART;
             const float Fcf = (const_ts || direct) ? 0.f : (float)drag_cell_factor(p, dt, qrho_old, gx, gy);
+            DragCell dc(p, dt, qrho_old, gx, gy, direct && heats, direct);
             // run-time species count: the cell's coefficients are kept (thread-local memory) for
             // the update loop instead of being formed a second time
             float2 rw_local[NS < 0 ? SHARK_MAX_DUST : 1];
             for (int k = 0; k < N; ++k) {
                 float r, w;
                 if (const_ts) { r = cr[k]; w = cw[k]; }
-                else if (direct) drag_coeffs_mix(1.0 * dt / tstop_cell(p, k, qrho_old, gx, gy), r, w);
+                else if (direct) drag_coeffs_mix(dc(k), r, w);
                 else drag_coeffs_f(Fcf * p.dinvts_f[k], r, w);
                 if (NS > 0) { rk[k < NMAX ? k : 0] = r; wk[k < NMAX ? k : 0] = w; }
                 else if (!const_ts) rw_local[k] = make_float2(r, w);
@@ -1191,6 +1260,8 @@ k_finalize_mixed(KParams<float> p) {
                 pnz += w * u[cc + (5 + 3 * N + k) * pl];
                 rhon += w * u[cc + (5 + k) * pl];
             }
+            gain = dc.heat;
+            heated = direct && heats;
             const float irhon = 1.0f / rhon;
             const float vbx = pnx * irhon, vby = pny * irhon, vbz = pnz * irhon;
             for (int k = 0; k < N; ++k) {
@@ -1218,9 +1289,13 @@ k_finalize_mixed(KParams<float> p) {
                 if (fl > u[ir]) u[ir] = fl;
             }
         }
-        if (MODE == 0 && N > 0 && (p.flags & SHARK_FLAG_BACK_REACTION) && p.iso < 1) {   // drag heating
+        if (heats) {   // drag heating; without the drag, or with a setup's own stopping times, by itself
             const long long ie = uidx(p, 4, gy, gx);
-            u[ie] = (float)((double)u[ie] + drag_heating(p, gx, gy, dt));
+            if (!heated) {
+                const double rho_old = (double)ucur[cc];
+                gain = drag_heating(p, TStop<float>(p, max64_pos(rho_old, p.smallr), gx, gy), gx, gy, dt);
+            }
+            u[ie] = (float)((double)u[ie] + gain);
         }
     };
     auto part2 = [&]() {
