@@ -9,7 +9,7 @@
 // the row below is updated with the four fluxes now known.  No shared memory, no __syncthreads.
 // Lanes 0,1,30,31 are the x halo: 28 columns per warp are updated.
 //
-// Same per-cell algorithm and expressions as flux_tile.cuh (ctoprim solve.f90:195-253, predictor
+// Same per-cell algorithm as flux_line.cuh in 1D (ctoprim solve.f90:195-253, predictor
 // godunov.f90:7-629, add_delta_u godunov.f90:659-750, kick force_kicks.f90:2-41, polar sources
 // source_terms.f90:37-47).  The FP64 instantiation rounds as the oracle's operation order does; it
 // is bound by the number of FP64 instructions, so its quotients share reciprocals, its compares run

@@ -17,7 +17,7 @@ __device__ __forceinline__ float2 sel2(bool cx, bool cy, float2 a, float2 b) {
     return make_float2(cx ? a.x : b.x, cy ? a.y : b.y);
 }
 
-// The three gas solvers of gas_flux_t (flux_tile.cuh) on two faces.  f = (mass, normal momentum,
+// The three gas solvers of gas_flux_t (flux_line.cuh) on two faces.  f = (mass, normal momentum,
 // transverse momentum, second transverse momentum, energy).  The face pressures L[4], R[4] are
 // given as P - p0 for a constant p0: the momentum flux carries P - p0 (a constant added to it
 // cancels in the flux difference of a cell whose opposite faces have the same area) and the

@@ -174,14 +174,16 @@ cudaError_t launch_boundaries(const DeviceView& v) {
     return cudaGetLastError();
 }
 
-template <typename R, int NDIM>
-static cudaError_t flux_launch(const KParams<R>& p, cudaStream_t st) {
-    using T = Tile<R, NDIM>;
-    const size_t smem = TileSmem<R, NDIM>::bytes;
-    cudaError_t e = cudaFuncSetAttribute(k_flux<R, NDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    dim3 grid((p.nx + T::TX - 1) / T::TX, NDIM == 2 ? (p.ny + T::TY - 1) / T::TY : 1, p.ndust + 1);
-    k_flux<R, NDIM><<<grid, T::NT, smem, st>>>(p);
+// 1D K1: gas and dust in one launch.
+template <typename R>
+static cudaError_t line_launch(const KParams<R>& p, cudaStream_t st) {
+    const dim3 grid((p.nx + LINE_UX - 1) / LINE_UX, p.ndust + 1, 1);
+    switch (p.slope_type) {
+        case 0: k_flux_line<R, 0><<<grid, 32, 0, st>>>(p); break;
+        case 1: k_flux_line<R, 1><<<grid, 32, 0, st>>>(p); break;
+        case 2: k_flux_line<R, 2><<<grid, 32, 0, st>>>(p); break;
+        default: k_flux_line<R, 3><<<grid, 32, 0, st>>>(p); break;
+    }
     return cudaGetLastError();
 }
 
@@ -338,7 +340,7 @@ cudaError_t launch_step(const DeviceView& v, int slot) {
     if (v.ou_nm > 0)   // this step's forcing coefficients, from the dt on the device
         k_ou_update<<<1, 2 * v.ou_nm, 0, v.stream>>>(v.ou, v.ou_nm, p.dt, v.ou_sigma, v.ou_tcorr, v.ou_seed, v.step);
     if (v.time_kernels) cudaEventRecord(v.ev[1], v.stream);
-    e = (v.ndim == 2) ? strip_launch<R>(v, p) : flux_launch<R, 1>(p, v.stream);
+    e = (v.ndim == 2) ? strip_launch<R>(v, p) : line_launch<R>(p, v.stream);
     if (e != cudaSuccess) return e;
     if (v.nbuf == 3) {   // fargo_scheme after source_terms (solve.f90:105), into the third buffer
         R* dst = (R*)v.u[(v.cur + 2) % 3];

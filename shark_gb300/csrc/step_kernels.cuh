@@ -175,7 +175,7 @@ __global__ void k_boundaries(KParams<R> p, R* u) {
 
 }  // namespace shark
 
-#include "flux_tile.cuh"
+#include "flux_line.cuh"
 #include "flux_strip.cuh"
 #include "flux_strip2.cuh"
 
