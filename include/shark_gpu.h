@@ -284,7 +284,7 @@ int32_t shark_gpu_totals(shark_gpu_ctx* ctx, double* out);
 
 /* Device time of the last `step` in milliseconds: ms_out[0] work before the flux kernel (the dt
  * slot reset), ms_out[1] flux/update kernels (K1), ms_out[2] drag + dt + ghost-fill kernel (K2)
- * (CUDA events on the context's stream; waits for the step). */
+ * (stamps of the device clock that the step's kernels leave; waits for the step). */
 int32_t shark_gpu_last_step_ms(shark_gpu_ctx* ctx, float* ms_out);
 
 /* Benchmark helper: synchronize, record a CUDA event on the context's stream, queue nsteps steps

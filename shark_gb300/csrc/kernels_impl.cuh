@@ -44,6 +44,7 @@ static KParams<R> make_params(const DeviceView& v) {
     p.chg_gamma_d = (const R*)v.chg.gamma_d;
     p.dK = v.dK; p.dtstop = v.dtstop; p.dsize = v.dsize; p.dstokes = v.dstokes; p.dinvts = v.dinvts;
     p.turb_rho0 = c.turb_rho0;
+    p.stamps = v.stamps;
     p.dt = nullptr; p.dt_next = nullptr; p.status = v.status; p.coef = v.coef;
     p.dtf = v.coef + 2 * SHARK_MAX_DUST;
     p.dinvts_f = v.coef + SHARK_COEF_INVTS;
@@ -335,10 +336,11 @@ cudaError_t launch_step(const DeviceView& v, int slot) {
     if (v.time_kernels) cudaEventRecord(v.ev[0], v.stream);
     k_prepare_step<<<1, SHARK_MAX_DUST, 0, v.stream>>>(p.dt_next, p.dt, p.dtstop, p.ndust,
                                                       (p.setup == SHARK_SETUP_SI && std::is_same<R, float>::value) ? 1 : 0,
-                                                      p.coef, v.dt_log);
+                                                      p.coef, v.dt_log, v.post, v.status, v.post_step,
+                                                      v.stamps);
     if (v.chg.on && (e = launch_charge<R>(v)) != cudaSuccess) return e;   // charge: solve.f90:36-42
     if (v.ou_nm > 0)   // this step's forcing coefficients, from the dt on the device
-        k_ou_update<<<1, 2 * v.ou_nm, 0, v.stream>>>(v.ou, v.ou_nm, p.dt, v.ou_sigma, v.ou_tcorr, v.ou_seed, v.step);
+        k_ou_update<<<1, 2 * v.ou_nm, 0, v.stream>>>(v.ou, v.ou_nm, p.dt, v.ou_sigma, v.ou_tcorr, v.ou_seed, v.step, v.stamps);
     if (v.time_kernels) cudaEventRecord(v.ev[1], v.stream);
     e = (v.ndim == 2) ? strip_launch<R>(v, p) : line_launch<R>(p, v.stream);
     if (e != cudaSuccess) return e;
@@ -362,7 +364,7 @@ cudaError_t launch_courant(const DeviceView& v, int slot) {
     p.u_cur = (const R*)v.u[v.cur];
     p.dt = v.dt_slots + slot;   // unused in MODE 1 except by the drag (disabled)
     p.dt_next = reinterpret_cast<unsigned long long*>(v.dt_slots + slot);
-    k_prepare_step<<<1, 1, 0, v.stream>>>(p.dt_next, p.dt, p.dtstop, 0, 0, p.coef, nullptr);
+    k_prepare_step<<<1, 32, 0, v.stream>>>(p.dt_next, p.dt, p.dtstop, 0, 0, p.coef, nullptr, nullptr, nullptr, 0, v.stamps);
     dim3 g2((v.nx + 255) / 256, v.ndim == 2 ? v.ny : 1, 1);
     finalize_dispatch<R, 1>(p, g2, v.stream);
     return cudaGetLastError();
@@ -418,6 +420,7 @@ static ChargeParams<R> charge_params(const DeviceView& v) {
     q.psi_old = c.psi_old; q.zd = (R*)c.zd; q.ni = (R*)c.ni; q.ne = (R*)c.ne; q.eta = (R*)c.eta;
     q.gamma_d = (R*)c.gamma_d; q.seed = c.seed; q.hist = c.hist; q.iters = c.iters;
     q.status = v.status;
+    q.stamps = v.stamps;
     return q;
 }
 

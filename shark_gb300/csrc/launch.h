@@ -45,6 +45,14 @@ struct ChargeView {
     unsigned long long* hist;               // [CHARGE_HIST + 2]
 };
 
+// What a step tells the host, in pinned host memory: its preparation kernel stores the step's dt and
+// the status word, then the step's number.
+struct StepPost {
+    double dt;
+    unsigned int status, pad;
+    long long step;
+};
+
 // Device-side view of a context, shared by both precisions.  Metric arrays come in two copies:
 // `m` in the state precision (flux/update) and `md` in FP64 (drag, courant).
 struct DeviceView {
@@ -67,15 +75,19 @@ struct DeviceView {
     const double* dstokes;
     const double* dinvts;       // 1/C_k with t_k = C_k / (cell factor) for the per-cell stopping times
     double* dt_slots;           // [2] dt of step n lives in slot n % 2
-    double* dt_log = nullptr;   // when set, the step's preparation kernel stores the step's dt there
-                                // (pinned host memory of a timed run: no copy per step)
+    StepPost* post = nullptr;   // where the step's preparation kernel tells the host (device address)
+    long long post_step = 0;    // the number it carries
+    double* dt_log = nullptr;   // when set, it stores the step's dt there too (a timed run's log in
+                                // pinned host memory)
     unsigned int* status;       // OR of SHARK_STATUS_* bits
     float* coef;                // [SHARK_COEF_FLOATS] per-step drag coefficients (mixed path), float dt
     cudaStream_t stream;
     cudaStream_t stream2;       // side stream for the gas flux kernel (forked/joined per step)
     cudaEvent_t fork, join;
-    cudaEvent_t ev[4];          // timing: before boundaries, before flux, before finalize, end
-    bool time_kernels;
+    unsigned long long* stamps; // [4] device clock (ns) of the last step: its start, the end of what
+                                // precedes the flux kernel, the start and the end of K2
+    cudaEvent_t ev[4];          // kernel timing: before boundaries, before flux, before finalize, end
+    bool time_kernels;          // record them
     ChargeView chg;
     GrowthDev gw;               // dust growth (gw.on = 0: off)
     // dustyTurb Ornstein-Uhlenbeck forcing (ou_nm = 0: off)

@@ -9,6 +9,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -89,9 +90,9 @@ struct shark_gpu_ctx {
     double* staging = nullptr;       // ncells*nvar FP64 (Fortran order) for uploads/downloads
     double* part = nullptr;          // totals partials
     double* tot_out = nullptr;
-    double* host_ring = nullptr;     // pinned: [2] dt + [2] status (as doubles)
-    cudaEvent_t ev_read[2] = {nullptr, nullptr};
-    cudaEvent_t ev_time[4] = {nullptr, nullptr, nullptr, nullptr};
+    shark::StepPost* post = nullptr; // pinned: the last started step's dt, status and number
+    long long posts = 0;             // steps launched since init: the numbers the posts carry
+    unsigned long long* stamps = nullptr;   // [4] DeviceView::stamps
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -134,7 +135,6 @@ struct shark_gpu_ctx {
     long long nstep = 0;             // steps launched since upload
     bool uploaded = false;
     bool rho_ref_set = false;        // the mixed flux kernel's reference density is fixed at the first upload
-    bool pending_read[2] = {false, false};
     int totals_blocks = 0;
     unsigned int status_seen = 0;
 };
@@ -858,9 +858,8 @@ int32_t release(shark_gpu_ctx* c) {
     for (double* p : {c->metrics_d, c->species, c->dt_slots, c->staging, c->part, c->tot_out}) if (p) cudaFree(p);
     if (c->status) cudaFree(c->status);
     if (c->coef) cudaFree(c->coef);
-    if (c->host_ring) cudaFreeHost(c->host_ring);
-    for (auto& e : c->ev_read) if (e) cudaEventDestroy(e);
-    for (auto& e : c->ev_time) if (e) cudaEventDestroy(e);
+    if (c->post) cudaFreeHost(c->post);
+    if (c->stamps) cudaFree(c->stamps);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->stream2) cudaStreamDestroy(c->stream2);
@@ -943,22 +942,31 @@ cudaError_t do_step(shark_gpu_ctx* c, int slot) {
     return is_mixed(c) ? shark::launch_step<float>(c->v, slot) : shark::launch_step<double>(c->v, slot);
 }
 
-// queue the readback of dt slot `slot` and of the status word into the pinned ring
-int32_t queue_readback(shark_gpu_ctx* c, int slot) {
-    CUDA_TRY(cudaMemcpyAsync(c->host_ring + slot, c->dt_slots + slot, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<unsigned int*>(c->host_ring + 2 + slot), c->status, sizeof(unsigned int),
-                             cudaMemcpyDeviceToHost, c->stream));
-    CUDA_TRY(cudaEventRecord(c->ev_read[slot], c->stream));
-    c->pending_read[slot] = true;
+// Wait until the GPU has started the step with number `step`; its dt and the status word up to it.
+// The host spins on the pinned post (a few hundred ns after the store, against some 10 us for two
+// small copies and an event a step).  The stream is looked at now and then, so that an error, or an
+// idle stream without the post, ends the wait.
+int32_t wait_post(shark_gpu_ctx* c, long long step, double* dt, unsigned int* st) {
+    const volatile long long* posted = &c->post->step;
+    for (unsigned n = 1; *posted < step; ++n) {
+        if ((n & 0xffffu) != 0) continue;
+        const cudaError_t e = cudaStreamQuery(c->stream);
+        if (e == cudaErrorNotReady) continue;
+        if (e != cudaSuccess) return fail(SHARK_ERR_CUDA, "step: %s", cudaGetErrorString(e));
+        if (*posted < step) return fail(SHARK_ERR_STATE, "step %lld ended without its dt", step);
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    *dt = c->post->dt;
+    *st = c->post->status;
+    c->status_seen |= *st;
     return SHARK_OK;
 }
 
-int32_t wait_readback(shark_gpu_ctx* c, int slot, double* dt, unsigned int* st) {
-    if (!c->pending_read[slot]) return fail(SHARK_ERR_STATE, "no dt readback queued for slot %d", slot);
-    CUDA_TRY(cudaEventSynchronize(c->ev_read[slot]));
-    c->pending_read[slot] = false;
-    *dt = c->host_ring[slot];
-    *st = *reinterpret_cast<unsigned int*>(c->host_ring + 2 + slot);
+// dt slot `slot` and the status word as they are
+int32_t read_slot(shark_gpu_ctx* c, int slot, double* dt, unsigned int* st) {
+    CUDA_TRY(cudaMemcpyAsync(dt, c->dt_slots + slot, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(cudaMemcpyAsync(st, c->status, sizeof(unsigned int), cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->status_seen |= *st;
     return SHARK_OK;
 }
@@ -1173,8 +1181,9 @@ int32_t shark_gpu_init(const shark_gpu_config* cfg, shark_gpu_ctx** out) {
     v.stream2 = c->stream2;
     v.fork = c->ev_fork;
     v.join = c->ev_join;
-    for (auto& e : c->ev_read) INIT_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    for (auto& e : c->ev_time) INIT_TRY(cudaEventCreate(&e));
+    INIT_TRY(cudaMalloc(&c->stamps, 4 * sizeof(unsigned long long)));
+    INIT_TRY(cudaMemsetAsync(c->stamps, 0, 4 * sizeof(unsigned long long), c->stream));
+    v.stamps = c->stamps;
     v.nbuf = (cfg->flags & SHARK_FLAG_FARGO) ? 3 : 2;
     for (int b = 0; b < v.nbuf; ++b) {
         INIT_TRY(cudaMalloc(&c->ubuf[b], c->state_bytes));
@@ -1379,14 +1388,15 @@ int32_t shark_gpu_init(const shark_gpu_config* cfg, shark_gpu_ctx** out) {
         v.cdisk.gs = c->cdisk_gs;
         v.cdisk.on = true;
     }
-    INIT_TRY(cudaHostAlloc(&c->host_ring, 4 * sizeof(double), cudaHostAllocDefault));
-    std::memset(c->host_ring, 0, 4 * sizeof(double));
+    INIT_TRY(cudaHostAlloc(&c->post, sizeof(shark::StepPost), cudaHostAllocMapped));
+    *c->post = shark::StepPost{};
+    INIT_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&v.post), c->post, 0));
     const long long nact = (long long)v.nx * (v.ndim == 2 ? v.ny : 1);
     c->totals_blocks = (int)std::min<long long>(1024, std::max<long long>(1, nact / 256));
     INIT_TRY(cudaMalloc(&c->part, (size_t)c->totals_blocks * 4 * (v.ndust + 1) * 2 * sizeof(double)));
     INIT_TRY(cudaMalloc(&c->tot_out, 4 * (v.ndust + 1) * sizeof(double)));
-    for (int a = 0; a < 4; ++a) v.ev[a] = c->ev_time[a];
-    v.time_kernels = true;
+    for (auto& e : v.ev) e = nullptr;
+    v.time_kernels = false;
     INIT_TRY(cudaStreamSynchronize(c->stream));
 #undef INIT_TRY
     *out = c;
@@ -1425,8 +1435,6 @@ int32_t shark_gpu_upload(shark_gpu_ctx* c, const double* u_prim, int64_t ncells,
             c->v.rho_ref = std::isfinite(mean) && mean > 0.0 ? mean : 0.0;
         }
     }
-    // drain any readbacks still in flight: the new state starts a new dt sequence
-    for (int s = 0; s < 2; ++s) if (c->pending_read[s]) { cudaEventSynchronize(c->ev_read[s]); c->pending_read[s] = false; }
     const size_t bytes = (size_t)ncells * nvar * sizeof(double);
     const double* src = static_cast<const double*>(pinned_device_alias(u_prim));
     if (!src) {
@@ -1463,8 +1471,6 @@ int32_t shark_gpu_upload(shark_gpu_ctx* c, const double* u_prim, int64_t ncells,
     // first courant (src/solver/solve.f90:74) on the uploaded state -> dt slot 0
     cudaError_t e = is_mixed(c) ? shark::launch_courant<float>(c->v, 0) : shark::launch_courant<double>(c->v, 0);
     if (e != cudaSuccess) return fail(SHARK_ERR_CUDA, "courant: %s", cudaGetErrorString(e));
-    int32_t rc = queue_readback(c, 0);
-    if (rc) return rc;
     c->nstep = 0;
     c->uploaded = true;
     return SHARK_OK;
@@ -1477,9 +1483,8 @@ int32_t shark_gpu_step(shark_gpu_ctx* c, double* dt_out, int32_t* status_out) {
     if (c->cfg.flags & SHARK_FLAG_STATIC) {
         // static: solve returns before doing anything; dt keeps its value
         double dt; unsigned st;
-        int32_t rc = wait_readback(c, slot, &dt, &st);
+        int32_t rc = read_slot(c, slot, &dt, &st);
         if (rc) return rc;
-        if ((rc = queue_readback(c, slot))) return rc;
         if (dt_out) *dt_out = dt;
         if (status_out) *status_out = (int32_t)c->status_seen;
         return SHARK_OK;
@@ -1489,16 +1494,16 @@ int32_t shark_gpu_step(shark_gpu_ctx* c, double* dt_out, int32_t* status_out) {
         if (rs) return rs;
     }
     c->v.step = c->nstep + 1;
+    c->v.post_step = ++c->posts;
     cudaError_t e = do_step(c, slot);
     if (e != cudaSuccess) return fail(SHARK_ERR_CUDA, "step launch: %s", cudaGetErrorString(e));
     c->chg_cold = false;
     c->v.cur = shark::next_cur(c->v);
     c->nstep++;
-    int32_t rc = queue_readback(c, 1 - slot);   // dt of the next step, written by k_finalize
-    if (rc) return rc;
     double dt;
     unsigned st;
-    if ((rc = wait_readback(c, slot, &dt, &st))) return rc;   // dt this step used (ready one step earlier)
+    int32_t rc = wait_post(c, c->posts, &dt, &st);   // dt of this step, posted as it starts
+    if (rc) return rc;
     if (dt_out) *dt_out = dt;
     if (status_out) *status_out = (int32_t)c->status_seen;
     return SHARK_OK;
@@ -1805,10 +1810,10 @@ int32_t shark_gpu_totals(shark_gpu_ctx* c, double* out) {
 int32_t shark_gpu_last_step_ms(shark_gpu_ctx* c, float* ms_out) {
     if (!c || !ms_out) return fail(SHARK_ERR_INVALID_ARG, "NULL argument");
     if (c->nstep == 0) return fail(SHARK_ERR_STATE, "no step run yet");
-    CUDA_TRY(cudaEventSynchronize(c->ev_time[3]));
-    CUDA_TRY(cudaEventElapsedTime(&ms_out[0], c->ev_time[0], c->ev_time[1]));   // dt slot reset
-    CUDA_TRY(cudaEventElapsedTime(&ms_out[1], c->ev_time[1], c->ev_time[2]));   // flux/update
-    CUDA_TRY(cudaEventElapsedTime(&ms_out[2], c->ev_time[2], c->ev_time[3]));   // drag + dt
+    unsigned long long t[4];   // what precedes the flux kernel, flux/update, drag + dt
+    CUDA_TRY(cudaMemcpyAsync(t, c->stamps, sizeof t, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(cudaStreamSynchronize(c->stream));
+    for (int a = 0; a < 3; ++a) ms_out[a] = (float)((double)(long long)(t[a + 1] - t[a]) * 1e-6);
     return SHARK_OK;
 }
 
@@ -1834,23 +1839,16 @@ int32_t shark_gpu_timed_run(shark_gpu_ctx* c, int64_t nsteps, double* time_io, f
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     if (e != cudaSuccess) rc = fail(SHARK_ERR_CUDA, "timed run: %s", cudaGetErrorString(e));
     double time = *time_io;
-    const int slot0 = (int)(c->nstep & 1);
-    double dt_first = 0.0;
-    if (rc == SHARK_OK) {
-        unsigned st0;
-        rc = wait_readback(c, slot0, &dt_first, &st0);   // the readback the next step would wait on
-    }
     if (rc == SHARK_OK && c->v.chg.on) rc = seed_charges(c);
     if (rc == SHARK_OK) {
         if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) rc = fail(SHARK_ERR_CUDA, "timed run: %s", cudaGetErrorString(e));
     }
-    const bool tk = c->v.time_kernels;
-    c->v.time_kernels = false;
     if (rc == SHARK_OK) cudaEventRecord(e0, c->stream);
     for (int64_t n = 0; n < nsteps && rc == SHARK_OK; ++n) {
         const int slot = (int)(c->nstep & 1);
         if (!is_static) {
             c->v.step = c->nstep + 1;
+            c->v.post_step = ++c->posts;
             c->v.dt_log = dts_dev + n;
             e = do_step(c, slot);
             c->v.dt_log = nullptr;
@@ -1864,12 +1862,8 @@ int32_t shark_gpu_timed_run(shark_gpu_ctx* c, int64_t nsteps, double* time_io, f
         }
         if (!is_static) c->nstep++;   // a static step keeps its dt slot, as shark_gpu_step does
     }
-    c->v.time_kernels = tk;
     if (rc == SHARK_OK) {
         cudaEventRecord(e1, c->stream);
-        rc = queue_readback(c, (int)(c->nstep & 1));   // what the next step waits on
-    }
-    if (rc == SHARK_OK) {
         e = cudaEventSynchronize(e1);
         if (e == cudaSuccess) e = cudaEventElapsedTime(ms_out, e0, e1);
         if (e != cudaSuccess) rc = fail(SHARK_ERR_CUDA, "timed run: %s", cudaGetErrorString(e));
@@ -1881,7 +1875,6 @@ int32_t shark_gpu_timed_run(shark_gpu_ctx* c, int64_t nsteps, double* time_io, f
             rc = fail(SHARK_ERR_CUDA, "timed run: %s", cudaGetErrorString(e));
         c->status_seen |= st;
     }
-    (void)dt_first;
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     cudaFreeHost(dts);
@@ -1894,15 +1887,13 @@ int32_t shark_gpu_kernel_times(shark_gpu_ctx* c, int64_t nsteps, float* avg_ms) 
     if (!c->uploaded) return fail(SHARK_ERR_STATE, "kernel timing before upload");
     std::vector<cudaEvent_t> ev((size_t)nsteps * 4, nullptr);
     for (auto& e : ev) CUDA_TRY(cudaEventCreate(&e));
-    const bool tk = c->v.time_kernels;
     int32_t rc = SHARK_OK;
     for (int64_t n = 0; n < nsteps && rc == SHARK_OK; ++n) {
         for (int a = 0; a < 4; ++a) c->v.ev[a] = ev[(size_t)n * 4 + a];
         c->v.time_kernels = true;
         rc = shark_gpu_step(c, nullptr, nullptr);
     }
-    for (int a = 0; a < 4; ++a) c->v.ev[a] = c->ev_time[a];
-    c->v.time_kernels = tk;
+    c->v.time_kernels = false;
     double sum[4] = {0, 0, 0, 0};
     if (rc == SHARK_OK) {
         cudaError_t e = cudaStreamSynchronize(c->stream);

@@ -16,6 +16,7 @@
 
 #include "physics.cuh"
 #include "growth.cuh"
+#include "launch.h"
 #include "../../include/shark_gpu.h"
 
 namespace shark {
@@ -56,6 +57,7 @@ struct KParams {
     double turb_rho0;
     // time step bookkeeping
     const double* dt;                 // dt of the current step
+    unsigned long long* stamps;       // device clock at the step's phases (DeviceView)
     unsigned long long* dt_next;      // bit image of the next dt (positive doubles order as u64)
     unsigned int* status;             // SHARK_STATUS_* bits
     float* coef;                      // [2*SHARK_MAX_DUST] per-step drag coefficients 1/(1+a_k), a_k/(1+a_k)
@@ -77,6 +79,22 @@ struct KParams {
     const R* u_cur;                   // state at the start of the step (read only)
     R* u_next;                        // state after the step
 };
+
+// The device clock in ns.
+__device__ __forceinline__ unsigned long long clock_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+// K2's start (its first block) and end (the latest of its blocks, of its last row of blocks without
+// growth): one store and one reduction that nothing waits for, in place of two timing events a step
+// (some 2 us each).
+__device__ __forceinline__ void stamp_start(unsigned long long* stamps) {
+    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) stamps[2] = clock_ns();
+}
+__device__ __forceinline__ void stamp_end(unsigned long long* stamps, bool every_block) {
+    if (threadIdx.x == 0 && (every_block || blockIdx.y == gridDim.y - 1)) atomicMax(stamps + 3, clock_ns());
+}
 
 // A scalar parameter in the kernel's precision: the double itself, or its float copy.
 template <typename R>
@@ -846,6 +864,7 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
     const int gy = (p.ndim == 2) ? blockIdx.y + p.ng : 0;
     double dtc = 2e44;
     unsigned int st = 0;
+    if (DRAG) stamp_start(p.stamps);
     if (gx < p.ng + p.nx) {
         R* u = p.u_next;
         const double dt = *p.dt;
@@ -1017,6 +1036,7 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
     if (MODE == 2) return;
     block_reduce_dt(dtc, st, p.dt_next, p.status);
     if (REST && gx < p.ng + p.nx) fill_ghost_images(p, p.u_next, gx, gy);
+    if (REST) stamp_end(p.stamps, GROW);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1122,6 +1142,7 @@ k_finalize_mixed(KParams<float> p) {
     const bool const_ts = p.setup == SHARK_SETUP_SI;
     const float* __restrict__ cr = p.coef;
     const float* __restrict__ cw = p.coef + SHARK_MAX_DUST;
+    if (MODE == 0) stamp_start(p.stamps);
     const double dt = *p.dt;
     const int gx = blockIdx.x * blockDim.x + threadIdx.x + p.ng;
     const int gy = (p.ndim == 2) ? blockIdx.y + p.ng : 0;
@@ -1425,6 +1446,7 @@ k_finalize_mixed(KParams<float> p) {
     }
     block_reduce_dt_f(dtc, st, p.dt_next, p.status);
     if (MODE == 0 && gx < p.ng + p.nx) fill_ghost_images(p, p.u_next, gx, gy);
+    if (MODE == 0) stamp_end(p.stamps, GROW);
 }
 
 // Per-step preparation, one small block before the flux kernels: reset the next-dt slot and,
@@ -1441,8 +1463,9 @@ __device__ __forceinline__ double hash_uniform_d(unsigned long long seed, unsign
 // Ornstein-Uhlenbeck update of the forcing coefficients for step `step` (one thread each):
 // c <- f c + sigma sqrt(1 - f^2) xi with f = exp(-dt/tcorr) and a Box-Muller normal deviate.
 static __global__ void k_ou_update(double* ou, int nm, const double* dt, double sigma, double tcorr,
-                                   unsigned long long seed, long long step) {
+                                   unsigned long long seed, long long step, unsigned long long* stamps) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q == 0) stamps[1] = clock_ns();
     if (q >= 2 * nm) return;
     const double f = exp(-(*dt) / tcorr);
     const double sg = sigma * sqrt(1.0 - f * f);
@@ -1452,13 +1475,26 @@ static __global__ void k_ou_update(double* ou, int nm, const double* dt, double 
     ou[q] = f * ou[q] + sg * xi;
 }
 
+// It also posts the step's dt, the status word so far and then the step's number to pinned host
+// memory, where the host waits for them: no copy and no event per step.
 static __global__ void k_prepare_step(unsigned long long* dt_next, const double* dt, const double* dtstop, int ndust,
-                                      int const_ts, float* coef, double* dt_log) {
+                                      int const_ts, float* coef, double* dt_log, StepPost* post, const unsigned int* status,
+                                      long long step, unsigned long long* stamps) {
     const int k = threadIdx.x;
+    if (k == 1) {
+        stamps[0] = stamps[1] = clock_ns();
+        stamps[3] = 0;
+    }
     if (k == 0) {
         *dt_next = (unsigned long long)__double_as_longlong(2e44);
         coef[2 * SHARK_MAX_DUST] = (float)*dt;
         if (dt_log) *dt_log = *dt;
+    }
+    if (post && k == SHARK_MAX_DUST - 1) {
+        post->dt = *dt;
+        post->status = *status;
+        __threadfence_system();
+        *(volatile long long*)&post->step = step;
     }
     if (const_ts && k < ndust) {
         float r, w;
