@@ -9,8 +9,8 @@
 // Brownian mass factor, and without fragmentation the target bins and their mass split -- are
 // tabulated on the host with the oracle's operations.  The FP64 path follows the oracle's
 // operations (without fragmentation k_growth_d, a group of lanes per cell; with it growth_cell_d);
-// the mixed path integrates in FP32 (growth_dv_f, growth_cell_f and the warp-per-cell form in the
-// mixed K2).  A cell needing more than 100000 sub-steps stops there and raises
+// the mixed path integrates in FP32 (growth_dv_f; k_growth_f, a warp per cell, and with fragmentation
+// growth_cell_f).  A cell needing more than 100000 sub-steps stops there and raises
 // SHARK_STATUS_GROWTH.
 #pragma once
 
@@ -216,31 +216,34 @@ __device__ __forceinline__ GrowthCellF growth_cell_consts_f(const GrowthDev& g, 
     return c;
 }
 
-// FP32 relative velocity of a pair k >= j (dust_growth.f90:88-114): stopping times tk, tj, the
-// Brownian term X = T pBf, the drift (dx, dy, dz) = v_k - v_j and dg = |G_k| - |G_j| of the
-// ambipolar term, G = gamma / sqrt(1 + gamma^2).
+// FP32 relative velocity of a pair k >= j (dust_growth.f90:88-114): stopping times tk, tj and
+// St = t/t_L of both, the Brownian term T pB, the drift (dx, dy, dz) = v_k - v_j and
+// dg = |G_k| - |G_j| of the ambipolar term, G = gamma / sqrt(1 + gamma^2).  The turbulent term has
+// three cases; only the one that applies is formed.
 __device__ __forceinline__ float growth_dv_f(const GrowthDev& g, const GrowthRunF& r, const GrowthCellF& c, float tk,
-                                             float tj, float X, float dx, float dy, float dz, float dg, bool ambi) {
+                                             float tj, float St1, float St2, float pB, float dx, float dy, float dz,
+                                             float dg, bool ambi) {
     float dv = 0.f;
     if (g.mode & SHARK_GROWTH_TURB) {
         const float a = r.alpha;
-        const float x = tj / tk;
-        const float fS = 3.2f - 1.f - x + 2.f / (1.f + x) * (1.f / 2.6f + x * x * x / (1.6f + x));
-        const float St1 = tk / c.t_L, St2 = tj / c.t_L;
-        float vt = a * c.cs_v * sqrtf(fS * St1);
-        if (tk < c.t_eta) {
+        if (tk > c.t_L) {
+            dv = a * c.cs_v * sqrtf(1.f / (1.f + St1) + 1.f / (1.f + St2));
+        } else if (tk < c.t_eta) {
             // both radicands are >= 0 in exact arithmetic and 0 for k == j; with contracted,
             // reciprocal-based division the second can round to -1 ulp, whose square root (NaN)
             // would floor every bin the pair touches
             const float r1 = fmaxf((St1 - St2) / (St1 + St2), 0.f);
             const float r2 = fmaxf(St1 * St1 / (St1 + c.rm) - St2 * St2 / (St2 + c.rm), 0.f);
-            vt = a * c.cs_v * sqrtf(r1) * sqrtf(r2);
+            dv = a * c.cs_v * sqrtf(r1) * sqrtf(r2);
+        } else {
+            const float x = tj / tk;
+            const float fS = 3.2f - 1.f - x + 2.f / (1.f + x) * (1.f / 2.6f + x * x * x / (1.6f + x));
+            dv = a * c.cs_v * sqrtf(fS * St1);
         }
-        if (tk > c.t_L) vt = a * c.cs_v * sqrtf(1.f / (1.f + St1) + 1.f / (1.f + St2));
-        dv = vt;
     }
-    if (g.mode & SHARK_GROWTH_BROWNIAN) dv = sqrtf(dv * dv + X);
-    if (g.mode & SHARK_GROWTH_DRIFT) dv = sqrtf(dv * dv + dx * dx + dy * dy + dz * dz);
+    // the sums' contraction is written out: it is part of the result, which the sub-cycle amplifies
+    if (g.mode & SHARK_GROWTH_BROWNIAN) dv = sqrtf(fmaf(c.T, pB, __fmul_rn(dv, dv)));
+    if (g.mode & SHARK_GROWTH_DRIFT) dv = sqrtf(fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, __fmul_rn(dv, dv)))));
     if ((g.mode & SHARK_GROWTH_AMBIPOLAR) && ambi) {
         const float d = c.vambi * dg;                 // vambi carries 1/unit_v
         dv = sqrtf(dv * dv + d * d);
@@ -272,7 +275,7 @@ static __device__ __noinline__ bool growth_cell_f(const GrowthDev& g, int N, int
         for (int j = 0; j <= k; ++j, ++q) {
             float dv = 1.f;
             if (g.kernel == 0)
-                dv = growth_dv_f(g, rf, cc, ts[k], ts[j], cc.T * g.pBf[q], (float)(vxd[k] - vxd[j]), (float)(vyd[k] - vyd[j]),
+                dv = growth_dv_f(g, rf, cc, ts[k], ts[j], ts[k] / cc.t_L, ts[j] / cc.t_L, g.pBf[q], (float)(vxd[k] - vxd[j]), (float)(vyd[k] - vyd[j]),
                                  (float)(vzd[k] - vzd[j]), gm[k] - gm[j], gamd != nullptr);
             float ff = 0.f;
             if (frag) {

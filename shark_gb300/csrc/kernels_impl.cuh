@@ -91,7 +91,6 @@ static void finalize_launch(const KParams<R>& p, dim3 grid, cudaStream_t st) {
     }
 }
 
-// FP64 growth without fragmentation: the drag, k_growth_d, the rest of K2.
 template <int GL>
 static void growth_kernel_d(const KParams<double>& p, cudaStream_t st) {
     constexpr int cells = GROWTH_D_THREADS / GL;
@@ -99,21 +98,33 @@ static void growth_kernel_d(const KParams<double>& p, cudaStream_t st) {
     const long long nact = (long long)p.nx * (p.ndim == 2 ? p.ny : 1);
     k_growth_d<GL><<<(unsigned)((nact + cells - 1) / cells), GROWTH_D_THREADS, smem, st>>>(p);
 }
-static void growth_launch_d(const KParams<double>& p, dim3 grid, cudaStream_t st) {
-    finalize_launch<double, -1, 2>(p, grid, st);
-    if (growth_lanes(p.ndust) == 8) growth_kernel_d<8>(p, st);
-    else growth_kernel_d<16>(p, st);
-    finalize_launch<double, -1, 3>(p, grid, st);
+// one wave of blocks, each through chunks of cells
+static void growth_kernel_f(const KParams<float>& p, int nsm, cudaStream_t st) {
+    const GrowthSmemF smem(p.ndust, p.gw.npair, p.gw.gL);
+    const void* kernel = p.ndust <= 16 ? (const void*)k_growth_f<5> : (const void*)k_growth_f<GROWTH_PAIR_SLOTS>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem.total);
+    int resident = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, 32 * GROWTH_F_WARPS, smem.total);
+    const long long chunks = (long long)((p.ng + p.nx + GROWTH_F_CELLS - 1) / GROWTH_F_CELLS) * (p.ndim == 2 ? p.ny : 1);
+    const unsigned blocks = (unsigned)std::min<long long>((long long)nsm * std::max(resident, 1), (chunks + GROWTH_F_WARPS - 1) / GROWTH_F_WARPS);
+    if (p.ndust <= 16) k_growth_f<5><<<blocks, 32 * GROWTH_F_WARPS, smem.total, st>>>(p);
+    else k_growth_f<GROWTH_PAIR_SLOTS><<<blocks, 32 * GROWTH_F_WARPS, smem.total, st>>>(p);
 }
 
 template <typename R, int MODE>
-static void finalize_dispatch(const KParams<R>& p, dim3 grid, cudaStream_t st) {
+static void finalize_dispatch(const KParams<R>& p, dim3 grid, int nsm, cudaStream_t st) {
     if (MODE == 0 && p.gw.on) {   // dust growth: run-time species count
-        if constexpr (std::is_same<R, double>::value) {
-            if (!(p.gw.mode & SHARK_GROWTH_FRAGMENTATION)) {
-                growth_launch_d(p, grid, st);
-                return;
+        if (!(p.gw.mode & SHARK_GROWTH_FRAGMENTATION)) {
+            // the drag, the growth kernel, the rest of K2
+            finalize_launch<R, -1, 2>(p, grid, st);
+            if constexpr (std::is_same<R, double>::value) {
+                if (growth_lanes(p.ndust) == 8) growth_kernel_d<8>(p, st);
+                else growth_kernel_d<16>(p, st);
+            } else {
+                growth_kernel_f(p, nsm, st);
             }
+            finalize_launch<R, -1, 3>(p, grid, st);
+            return;
         }
         finalize_launch<R, -1, MODE, true>(p, grid, st);   // growth within K2
         return;
@@ -351,7 +362,7 @@ cudaError_t launch_step(const DeviceView& v, int slot) {
     }
     if (v.time_kernels) cudaEventRecord(v.ev[2], v.stream);
     dim3 g2((v.nx + 255) / 256, v.ndim == 2 ? v.ny : 1, 1);
-    finalize_dispatch<R, 0>(p, g2, v.stream);
+    finalize_dispatch<R, 0>(p, g2, v.nsm, v.stream);
     if (v.time_kernels) cudaEventRecord(v.ev[3], v.stream);
     return cudaGetLastError();
 }
@@ -366,7 +377,7 @@ cudaError_t launch_courant(const DeviceView& v, int slot) {
     p.dt_next = reinterpret_cast<unsigned long long*>(v.dt_slots + slot);
     k_prepare_step<<<1, 32, 0, v.stream>>>(p.dt_next, p.dt, p.dtstop, 0, 0, p.coef, nullptr, nullptr, nullptr, 0, v.stamps);
     dim3 g2((v.nx + 255) / 256, v.ndim == 2 ? v.ny : 1, 1);
-    finalize_dispatch<R, 1>(p, g2, v.stream);
+    finalize_dispatch<R, 1>(p, g2, v.nsm, v.stream);
     return cudaGetLastError();
 }
 

@@ -523,31 +523,65 @@ __device__ __noinline__ unsigned grow_in_finalize(const KParams<R>& p, R* u, int
     return ok ? 0u : (unsigned)SHARK_STATUS_GROWTH;
 }
 
-// Dust growth of the mixed path without fragmentation (dust_growth.f90:3-256), one warp per cell
-// for the 256 cells of a K2 block (warp w takes cells 32 w .. 32 w + 31 in turn).  Lane b holds
-// bin b's density.  Once per cell the lanes form the pair rates pK dv / hs of pairs
-// q = lane, lane + 32, ... from the start-of-step stopping times and velocities (exchanged by
-// shuffles).  Every sub-step each lane writes the collision rate w_q = rate_q rho_k rho_j (times
-// the sticking efficiency) of its pairs to shared memory, and lane b gathers
-// drho_b/dt = sum_t gc[t][b] w[gq[t][b]] from the host-built table of net transfers (staged in
-// shared memory as four rows' coefficients per 128-bit entry and two rows' pair indices, 16 bits
-// each, per 32-bit word, the four partial sums of rows t mod 4 as two packed FMAs); the sub-step is the warp minimum of CFL_growth rho_b/|drho_b/dt| (one redux.sync on the
-// candidates' bit patterns), and the part of dt still to integrate is kept as an FP32 fraction
-// (the last sub-step takes all of it).  The lanes of a warp take the same sub-steps, so a warp
-// costs the sub-steps of its own cell rather than those of the slowest of 32 cells.  Called by
-// every thread of the block.
+// Dust growth of the mixed path without fragmentation (dust_growth.f90:3-256) on the post-drag state
+// u_next, one warp per cell, a lane per bin.  Most cells take a single sub-step (on average 1.0-2.3
+// on the disk and the driven box), so a cell costs its setup: the relative velocities of its
+// N (N + 1)/2 pairs.  A warp takes chunks of 4 cells of a row:
+//  1. its lanes read the chunk's densities and momenta, 8 bins x 4 cells at a time, and leave the
+//     species' terms of the cells in shared memory (velocities, stopping times, t/t_L);
+//  2. two cells at a time (the pair's indices, factors and addresses serve both), the lanes form the
+//     rate factors pK dv / hs of pairs q = lane, lane + 32, ... from those terms, only the turbulent
+//     case that applies, and the rates of the first sub-step with them; lane b gathers drho_b/dt =
+//     sum_t gc[t][b] w[gq[t][b]] from the host-built table of net transfers (in shared memory as
+//     four rows' coefficients per 128-bit entry and two rows' pair indices, 16 bits each, per 32-bit
+//     word; four partial sums of rows t mod 4, both cells in one packed FMA); the sub-step is the
+//     warp minimum of CFL_growth rho_b/|drho_b/dt| (one redux.sync on the candidates' bit patterns),
+//     and the part of dt still to integrate is kept as an FP32 fraction (the last sub-step takes all
+//     of it).  A cell that needs more sub-steps goes on by itself;
+//  3. the cells' densities are written back together.
+// Bound by instruction issue (71 % of the slots).  The loops over pairs are not unrolled: unrolled
+// they overflowed the instruction cache (the largest stall).  As a phase of K2 with each cell's
+// inputs read by lane = bin and every turbulent case formed for every pair, K2 took 2.09 ms on the
+// disk 512 x 1024 x 16 and 5.20 ms on the driven box 768^2 x 32; unrolled per-cell warps 1.06 and
+// 3.98 ms, not unrolled 0.99 and 2.72 ms, two cells at a time 0.90 and 2.57 ms; bit for bit the same.
 constexpr int GROWTH_PAIR_SLOTS = (GROWTH_MAX_PAIRS + 31) / 32;
+// cells of a chunk, warps of a block: two blocks fill an SM's shared memory at 32 species
+constexpr int GROWTH_F_CELLS = 4, GROWTH_F_WARPS = 12;
 constexpr int GROWTH_SMEM_ROWS = 80;        // gather rows staged in shared memory (64 at 32 species)
 
-static __device__ __noinline__ unsigned grow_block_warps(const KParams<float>& p, int gx_block, int gy, double dt) {
-    __shared__ float sw[8][GROWTH_MAX_PAIRS];
-    // gather table: coefficient of row t, lane l at sgc[128 (t >> 2) + 4 l + (t & 3)]; pair
-    // indices of rows 4 u + 2 h, 4 u + 2 h + 1 (low, high 16 bits) at sgi[64 u + 2 l + h]
-    __shared__ __align__(16) float sgc[GROWTH_SMEM_ROWS * 32];
-    __shared__ __align__(8) unsigned sgi[GROWTH_SMEM_ROWS / 2 * 32];
-    __shared__ int spair[GROWTH_PAIR_SLOTS * 32];   // pair (k << 8 | j) of slot i, lane l at [32 i + l]
+// bins a cell's terms are laid out for
+__host__ __device__ constexpr int growth_f_bins(int N) { return N <= 16 ? 16 : 32; }
+
+// shared memory of a block in bytes: the tables, then per warp the species' terms of a chunk's cells,
+// their constants and two cells' pair rates
+struct GrowthSmemF {
+    int gc, gi, pair, pk, warp0, per_warp, total;
+    __host__ __device__ GrowthSmemF(int N, int P, int L) {
+        const int rows = L <= GROWTH_SMEM_ROWS ? (L + 3) & ~3 : 0, slots = (P + 31) / 32 * 32;
+        gc = 0;
+        gi = gc + rows * 32 * 4;
+        pk = gi + rows / 2 * 32 * 4;   // multiples of 256 bytes so far
+        pair = pk + slots * 8;
+        warp0 = (pair + slots * 4 + 15) & ~15;
+        per_warp = ((GROWTH_F_CELLS * growth_f_bins(N) * (16 + 8 + 4) + GROWTH_F_CELLS * 16 * 2 + slots * 8) + 15) & ~15;
+        total = warp0 + GROWTH_F_WARPS * per_warp;
+    }
+};
+
+// SLOTS: the most pairs per lane, 5 up to 16 bins.
+template <int SLOTS>
+static __global__ void __launch_bounds__(32 * GROWTH_F_WARPS, 2) k_growth_f(KParams<float> p) {
+    extern __shared__ __align__(16) unsigned char sgf[];
     const GrowthDev& g = p.gw;
     const int N = p.ndust, P = g.npair, L = g.gL;
+    const GrowthSmemF off(N, P, L);
+    // gather table: coefficient of row t, lane l at sgc[128 (t >> 2) + 4 l + (t & 3)]; pair
+    // indices of rows 4 u + 2 h, 4 u + 2 h + 1 (low, high 16 bits) at sgi[64 u + 2 l + h]
+    float* sgc = reinterpret_cast<float*>(sgf + off.gc);
+    unsigned* sgi = reinterpret_cast<unsigned*>(sgf + off.gi);
+    float2* spk = reinterpret_cast<float2*>(sgf + off.pk);         // rate factor (halved for k == j), Brownian factor
+    unsigned* spair = reinterpret_cast<unsigned*>(sgf + off.pair);   // k << 16 | j
+    const int slots = (P + 31) / 32;
     const bool staged = L <= GROWTH_SMEM_ROWS;
     if (staged) {   // rows past L are zero (coefficient 0, pair 0)
         const int L4 = (L + 3) & ~3;
@@ -562,13 +596,27 @@ static __device__ __noinline__ unsigned grow_block_warps(const KParams<float>& p
             sgi[64 * (t0 >> 2) + 2 * l + ((t0 >> 1) & 1)] = i0 | (i1 << 16);
         }
     }
-    for (int e = threadIdx.x; e < GROWTH_PAIR_SLOTS * 32; e += blockDim.x) spair[e] = e < P ? __ldg(g.pair + e) : 0;
+    for (int e = threadIdx.x; e < (P + 31) / 32 * 32; e += blockDim.x) {
+        const int pr = e < P ? __ldg(g.pair + e) : 0, k = pr >> 8, j = pr & 255;
+        spair[e] = (unsigned)k << 16 | (unsigned)j;
+        spk[e] = e < P ? make_float2(__ldg(g.pKf + e) * (k == j ? 0.5f : 1.f), __ldg(g.pBf + e)) : make_float2(0.f, 0.f);
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float* w = sw[wid];
+    unsigned char* mine = sgf + off.warp0 + wid * off.per_warp;
+    constexpr int NB = SLOTS > 5 ? 32 : 16;
+    float4* sv = reinterpret_cast<float4*>(mine);                                   // [cells][NB] vx, vy, vz, |G|
+    float4* sc = reinterpret_cast<float4*>(mine + GROWTH_F_CELLS * NB * 16);        // [cells][2] the cells' constants
+    float2* sts = reinterpret_cast<float2*>(mine + GROWTH_F_CELLS * (NB + 2) * 16); // [cells][NB] stopping time, t/t_L
+    float* srd = reinterpret_cast<float*>(sts + GROWTH_F_CELLS * NB);               // [cells][NB] densities
+    float2* w = reinterpret_cast<float2*>(srd + GROWTH_F_CELLS * NB);               // pair rates of two cells
     float* u = p.u_next;
+    const float* __restrict__ uc = p.u_cur;
+    const int pl = (int)p.plane;
     const unsigned FULL = 0xffffffffu;
+    const double dt = *p.dt;
     const bool ambi = (g.mode & SHARK_GROWTH_AMBIPOLAR) && p.chg_gamma_d;
+    const bool disk = p.setup == SHARK_SETUP_DISK_POLAR;
     const bool on = lane < N;
     const int b = on ? lane : 0;
     const bool thr_on = g.kernel == 0 && g.eps_thr > 0.0;
@@ -576,106 +624,189 @@ static __device__ __noinline__ unsigned grow_block_warps(const KParams<float>& p
     const float fctl = g.dtctl > 0.0 ? (float)(g.dtctl / dt) : 0.f, dtctl = (float)g.dtctl;
     const float stick = (float)g.sticking, cflg = (float)g.cfl;
     const float eps_thr = (float)g.eps_thr, rmin = (float)g.dust_ratio_min, smallr = (float)p.smallr;
-    // stopping times for the pair velocities (FP32): t_k = C_k / F_cell with the tabulated 1/C_k
-    // (dustyTurb F = c_s rho, polar disk F = rho/hs c_s: the setups with growth)
-    const float invc = p.dinvts_f[b];
     const GrowthRunF rf = growth_run_consts_f(g);
     const float4 row0 = growth_row_f(g, 0);        // the one temperature row (dustyTurb)
+    const int nchunk_x = (p.ng + p.nx + GROWTH_F_CELLS - 1) / GROWTH_F_CELLS;   // from column 0: whole sectors
+    const int nchunk = nchunk_x * (p.ndim == 2 ? p.ny : 1);
+    constexpr int BINS = 32 / GROWTH_F_CELLS;      // bins read at a time
+    const int c = lane % GROWTH_F_CELLS, bs = lane / GROWTH_F_CELLS;
     unsigned st = 0;
-    for (int c = 0; c < 32; ++c) {
-        const int gx = gx_block + wid * 32 + c;
-        if (gx >= p.ng + p.nx) break;
-        const float rho_old = p.u_cur[uidx(p, 0, gy, gx)];
-        const float qrho_old = rho_old > smallr ? rho_old : smallr;
-        float rd = u[uidx(p, 5 + b, gy, gx)];
-        const float F = p.setup == SHARK_SETUP_DUSTYTURB ? p.cs[gx] * qrho_old : qrho_old / (float)p.hsd[gx] * p.cs[gx];
-        const float ts = 1.f / (invc * F);
-        const float r0 = p.u_cur[uidx(p, 5 + b, gy, gx)];
-        const float vx = p.u_cur[uidx(p, 5 + N + b, gy, gx)] / r0;
-        const float vy = p.u_cur[uidx(p, 5 + 2 * N + b, gy, gx)] / r0;
-        const float vz = p.u_cur[uidx(p, 5 + 3 * N + b, gy, gx)] / r0;
-        const long long cidx = (long long)gy * p.pitch + gx;
-        float gm = 0.f, eta_a = 0.f;
-        if (ambi) {
-            const float ga = p.chg_gamma_d[(long long)b * p.plane + cidx];
-            gm = fabsf(ga) * rsqrtf(1.f + ga * ga);
-            eta_a = p.chg_eta[2 * p.plane + cidx];
+    // drho_b/dt of this lane's bin: the four partial sums of rows t mod 4, for one cell (rates at
+    // we[2 q]) or both
+    auto gather = [&](const float* we) -> float {
+        float a[4] = {0.f, 0.f, 0.f, 0.f}, d;
+        int r = 0;
+        if (!staged) {
+            d = 0.f;
+            for (; r < L; ++r) d += __ldg(g.gc + r * 32 + lane) * we[2 * __ldg(g.gq + r * 32 + lane)];
+            return d;
         }
-        const float hs = p.setup == SHARK_SETUP_DISK_POLAR ? (float)p.hsd[gx] : 1.f;
-        const float rho_gas = u[uidx(p, 0, gy, gx)];
-        const GrowthCellF cc = growth_cell_consts_f(g, rf, g.t_per_col ? growth_row_f(g, gx) : row0, qrho_old, hs, eta_a);
-        const float ihs = 1.f / hs;
-        float kp[GROWTH_PAIR_SLOTS];
-#pragma unroll
-        for (int i = 0; i < GROWTH_PAIR_SLOTS; ++i) {
-            kp[i] = 0.f;
-            if (32 * i >= P) continue;                      // uniform over the warp
-            const int q = lane + 32 * i;
-            const bool has = q < P;
-            const int pr = spair[q];
-            const int k = pr >> 8, j = pr & 255;
-            const float tk = __shfl_sync(FULL, ts, k), tj = __shfl_sync(FULL, ts, j);
-            const float dx = __shfl_sync(FULL, vx, k) - __shfl_sync(FULL, vx, j);
-            const float dy = __shfl_sync(FULL, vy, k) - __shfl_sync(FULL, vy, j);
-            const float dz = __shfl_sync(FULL, vz, k) - __shfl_sync(FULL, vz, j);
-            const float dg = __shfl_sync(FULL, gm, k) - __shfl_sync(FULL, gm, j);
-            if (!has) continue;
-            float dv = 1.f;
-            if (g.kernel == 0) dv = growth_dv_f(g, rf, cc, tk, tj, cc.T * __ldg(g.pBf + q), dx, dy, dz, dg, ambi);
-            kp[i] = __ldg(g.pKf + q) * dv * ihs * (k == j ? 0.5f : 1.f);
+        for (; r + 4 <= L; r += 4) {
+            const float4 cg = *reinterpret_cast<const float4*>(sgc + 32 * r + 4 * lane);
+            const uint2 ix = *reinterpret_cast<const uint2*>(sgi + 16 * r + 2 * lane);
+            a[0] = fmaf(cg.x, we[2 * (ix.x & 0xffffu)], a[0]);
+            a[1] = fmaf(cg.y, we[2 * (ix.x >> 16)], a[1]);
+            a[2] = fmaf(cg.z, we[2 * (ix.y & 0xffffu)], a[2]);
+            a[3] = fmaf(cg.w, we[2 * (ix.y >> 16)], a[3]);
         }
-        const float thr = eps_thr * rho_gas, fl = rho_gas * rmin;
-        float rem = 1.f;                                    // part of dt still to integrate
-        int niter = 0;
-        while (rem > 0.f && niter < grw::MAX_SUB) {
-            niter = niter + 1;
+        d = a[0];
+        for (; r < L; ++r) {
+            const unsigned iw = sgi[64 * (r >> 2) + 2 * lane + ((r >> 1) & 1)];
+            d = fmaf(sgc[128 * (r >> 2) + 4 * lane + (r & 3)], we[2 * ((r & 1) ? (iw >> 16) : (iw & 0xffffu))], d);
+        }
+        return (d + a[1]) + (a[2] + a[3]);
+    };
+    auto gather2 = [&](float& d0, float& d1) {
+        if (!staged) {
+            d0 = gather(reinterpret_cast<const float*>(w));
+            d1 = gather(reinterpret_cast<const float*>(w) + 1);
+            return;
+        }
+        float2 a[4];
 #pragma unroll
-            for (int i = 0; i < GROWTH_PAIR_SLOTS; ++i) {
-                if (32 * i >= P) continue;
-                const int q = lane + 32 * i;
-                const int pr = spair[q];
-                const float rk = __shfl_sync(FULL, rd, pr >> 8), rj = __shfl_sync(FULL, rd, pr & 255);
-                float pc = kp[i] * rk * rj;
-                if (thr_on && (rk < thr || rj < thr)) pc = 0.f;
-                if (q < P) w[q] = pc * stick;
+        for (int h = 0; h < 4; ++h) a[h] = make_float2(0.f, 0.f);
+        int r = 0;
+#pragma unroll 2
+        for (; r + 4 <= L; r += 4) {
+            const float4 cg = *reinterpret_cast<const float4*>(sgc + 32 * r + 4 * lane);
+            const uint2 ix = *reinterpret_cast<const uint2*>(sgi + 16 * r + 2 * lane);
+            a[0] = __ffma2_rn(make_float2(cg.x, cg.x), w[ix.x & 0xffffu], a[0]);
+            a[1] = __ffma2_rn(make_float2(cg.y, cg.y), w[ix.x >> 16], a[1]);
+            a[2] = __ffma2_rn(make_float2(cg.z, cg.z), w[ix.y & 0xffffu], a[2]);
+            a[3] = __ffma2_rn(make_float2(cg.w, cg.w), w[ix.y >> 16], a[3]);
+        }
+        float2 d = a[0];
+        for (; r < L; ++r) {
+            const float cg = sgc[128 * (r >> 2) + 4 * lane + (r & 3)];
+            const unsigned iw = sgi[64 * (r >> 2) + 2 * lane + ((r >> 1) & 1)];
+            d = __ffma2_rn(make_float2(cg, cg), w[(r & 1) ? (iw >> 16) : (iw & 0xffffu)], d);
+        }
+        d0 = (d.x + a[1].x) + (a[2].x + a[3].x);
+        d1 = (d.y + a[1].y) + (a[2].y + a[3].y);
+    };
+    // one sub-step of this lane's bin; rem: the part of dt still to integrate
+    auto advance = [&](float d, float& rd, float& rem, float fl) {
+        // non-negative floats order like their bit patterns read as unsigned integers
+        const float cand0 = (on && d != 0.f) ? fmaxf(rd / fabsf(d) * cflg, 0.f) : 1e30f;
+        const float cand = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(cand0)));
+        const float dtg0 = fctl > 0.f ? dtctl : cand;
+        const float frac = fctl > 0.f ? fctl : cand * idtf;
+        float dtg;
+        if (frac >= rem) { dtg = rem * dtf; rem = 0.f; }
+        else { dtg = dtg0; rem = rem - frac; }
+        rd = fmaxf(rd + d * dtg, fl);
+    };
+    for (int ch = blockIdx.x * GROWTH_F_WARPS + wid; ch < nchunk; ch += gridDim.x * GROWTH_F_WARPS) {
+        const int iy = ch / nchunk_x, x0 = (ch - iy * nchunk_x) * GROWTH_F_CELLS;
+        const int gy = p.ndim == 2 ? iy + p.ng : 0;
+        const int first = max(p.ng - x0, 0), last = min(p.ng + p.nx - x0, GROWTH_F_CELLS);   // cells of the chunk
+        {
+            const int gx = x0 + min(max(c, first), last - 1), cc = gy * p.pitch + gx;
+            const float rho_old = uc[cc];
+            const float qrho_old = rho_old > smallr ? rho_old : smallr;
+            const float rho_gas = u[cc];
+            // stopping times for the pair velocities (FP32): t_k = C_k / F_cell with the tabulated 1/C_k
+            // (dustyTurb F = c_s rho, polar disk F = rho/hs c_s: the setups with growth)
+            const float F = p.setup == SHARK_SETUP_DUSTYTURB ? p.cs[gx] * qrho_old : qrho_old / (float)p.hsd[gx] * p.cs[gx];
+            const float hs = disk ? (float)p.hsd[gx] : 1.f;
+            const float eta_a = ambi ? p.chg_eta[2 * p.plane + cc] : 0.f;
+            const GrowthCellF cf = growth_cell_consts_f(g, rf, g.t_per_col ? growth_row_f(g, gx) : row0, qrho_old, hs, eta_a);
+            if (bs == 0) {
+                sc[2 * c] = make_float4(cf.T, cf.cs_v, cf.t_L, cf.t_eta);
+                sc[2 * c + 1] = make_float4(cf.rm, cf.vambi, hs, rho_gas);
+            }
+#pragma unroll 4
+            for (int b0 = 0; b0 < N; b0 += BINS) {
+                const int k = b0 + bs;
+                if (k >= N) continue;
+                const float ts = 1.f / (p.dinvts_f[k] * F);
+                const float r0 = uc[cc + (5 + k) * pl];
+                const float vx = uc[cc + (5 + N + k) * pl] / r0;
+                const float vy = uc[cc + (5 + 2 * N + k) * pl] / r0;
+                const float vz = uc[cc + (5 + 3 * N + k) * pl] / r0;
+                float gm = 0.f;
+                if (ambi) {
+                    const float ga = p.chg_gamma_d[(long long)k * p.plane + cc];
+                    gm = fabsf(ga) * rsqrtf(1.f + ga * ga);
+                }
+                sv[c * NB + k] = make_float4(vx, vy, vz, gm);
+                sts[c * NB + k] = make_float2(ts, ts / cf.t_L);
+                srd[c * NB + k] = u[cc + (5 + k) * pl];
+            }
+        }
+        __syncwarp();
+        for (int i = first & ~1; i < last; i += 2) {   // two cells at a time (one of them may lie outside)
+            const float4 *v0 = sv + i * NB, *v1 = v0 + NB;
+            const float2 *t0 = sts + i * NB, *t1 = t0 + NB;
+            GrowthCellF cf[2];
+            float ihs[2], fl[2], thr[2], rd[2], rdt[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float4 c0 = sc[2 * (i + e)], c1 = sc[2 * (i + e) + 1];
+                cf[e] = GrowthCellF{c0.x, c0.y, c0.z, c0.w, c1.x, c1.y};
+                ihs[e] = 1.f / c1.z;
+                fl[e] = c1.w * rmin;
+                thr[e] = thr_on ? eps_thr * c1.w : -1.f;
+                rd[e] = srd[(i + e) * NB + b];
+                rdt[e] = rd[e] < thr[e] ? 0.f : rd[e];   // a bin below the threshold takes no part
+            }
+            float kp0[SLOTS], kp1[SLOTS];
+#pragma unroll 1
+            for (int s = 0; s < slots; ++s) {
+                const int q = lane + 32 * s;
+                const unsigned pr = spair[q];
+                const int k = pr >> 16, j = pr & 0xffffu;
+                const float2 pk = spk[q];
+                float d0 = 1.f, d1 = 1.f;
+                if (g.kernel == 0) {
+                    const float2 tk = t0[k], tj = t0[j];
+                    const float4 vk = v0[k], vj = v0[j];
+                    d0 = growth_dv_f(g, rf, cf[0], tk.x, tj.x, tk.y, tj.y, pk.y, vk.x - vj.x, vk.y - vj.y, vk.z - vj.z, vk.w - vj.w, ambi);
+                    const float2 uk = t1[k], uj = t1[j];
+                    const float4 wk = v1[k], wj = v1[j];
+                    d1 = growth_dv_f(g, rf, cf[1], uk.x, uj.x, uk.y, uj.y, pk.y, wk.x - wj.x, wk.y - wj.y, wk.z - wj.z, wk.w - wj.w, ambi);
+                }
+                kp0[s] = d0 = pk.x * d0 * ihs[0];
+                kp1[s] = d1 = pk.x * d1 * ihs[1];
+                w[q] = make_float2(d0 * __shfl_sync(FULL, rdt[0], k) * __shfl_sync(FULL, rdt[0], j) * stick,
+                                   d1 * __shfl_sync(FULL, rdt[1], k) * __shfl_sync(FULL, rdt[1], j) * stick);
             }
             __syncwarp();
-            float d = 0.f;
-            if (staged) {
-                // four partial sums: the gather's products are independent, its FMA chain is not
-                float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
-                int t = 0;
-                for (; t + 4 <= L; t += 4) {
-                    const float4 c = *reinterpret_cast<const float4*>(sgc + 32 * t + 4 * lane);
-                    const uint2 ix = *reinterpret_cast<const uint2*>(sgi + 16 * t + 2 * lane);
-                    a0 = __ffma2_rn(make_float2(c.x, c.y), make_float2(w[ix.x & 0xffffu], w[ix.x >> 16]), a0);
-                    a1 = __ffma2_rn(make_float2(c.z, c.w), make_float2(w[ix.y & 0xffffu], w[ix.y >> 16]), a1);
+            // the first sub-step of both
+            float d[2];
+            gather2(d[0], d[1]);
+            float rem[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) { rem[e] = 1.f; advance(d[e], rd[e], rem[e], fl[e]); }
+            // the cells that need more, by themselves
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float* kp = e ? kp1 : kp0;
+                float* we = reinterpret_cast<float*>(w) + e;
+                for (int niter = 1; rem[e] > 0.f && niter < grw::MAX_SUB; ++niter) {
+                    rdt[e] = rd[e] < thr[e] ? 0.f : rd[e];
+                    __syncwarp();                                   // the rates are read; the next ones may take their place
+#pragma unroll 1
+                    for (int s = 0; s < slots; ++s) {
+                        const int q = lane + 32 * s;
+                        const unsigned pr = spair[q];
+                        we[2 * q] = kp[s] * __shfl_sync(FULL, rdt[e], pr >> 16) * __shfl_sync(FULL, rdt[e], pr & 0xffffu) * stick;
+                    }
+                    __syncwarp();
+                    advance(gather(we), rd[e], rem[e], fl[e]);
                 }
-                d = a0.x;
-                for (; t < L; ++t) {
-                    const float c = sgc[128 * (t >> 2) + 4 * lane + (t & 3)];
-                    const unsigned iw = sgi[64 * (t >> 2) + 2 * lane + ((t >> 1) & 1)];
-                    d = fmaf(c, w[(t & 1) ? (iw >> 16) : (iw & 0xffffu)], d);
-                }
-                d = (d + a0.y) + (a1.x + a1.y);
-            } else {
-                for (int t = 0; t < L; ++t) d += __ldg(g.gc + t * 32 + lane) * w[__ldg(g.gq + t * 32 + lane)];
+                if (on) srd[(i + e) * NB + b] = rd[e];
+                if (rem[e] > 0.f && i + e >= first && i + e < last) st |= (unsigned)SHARK_STATUS_GROWTH;
             }
             __syncwarp();
-            // non-negative floats order like their bit patterns read as unsigned integers
-            const float c0 = (on && d != 0.f) ? fmaxf(rd / fabsf(d) * cflg, 0.f) : 1e30f;
-            const float cand = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(c0)));
-            const float dtg0 = fctl > 0.f ? dtctl : cand;
-            const float frac = fctl > 0.f ? fctl : cand * idtf;
-            float dtg;
-            if (frac >= rem) { dtg = rem * dtf; rem = 0.f; }
-            else { dtg = dtg0; rem = rem - frac; }
-            rd = fmaxf(rd + d * dtg, fl);
         }
-        if (on) u[uidx(p, 5 + b, gy, gx)] = rd;
-        if (rem > 0.f) st |= (unsigned)SHARK_STATUS_GROWTH;
+        if (c >= first && c < last) {
+            const int cc = gy * p.pitch + x0 + c;
+            for (int k = bs; k < N; k += BINS) u[cc + (5 + k) * pl] = srd[c * NB + k];
+        }
+        __syncwarp();
     }
-    return st;
+    if (st && lane == 0) atomicOr(p.status, st);
 }
 
 // Dust growth of the FP64 path without fragmentation (dust_growth.f90:3-256) on the post-drag state
@@ -1136,13 +1267,14 @@ __global__ void __launch_bounds__(GROW ? 256 : K2M_THREADS,
 k_finalize_mixed(KParams<float> p) {
     constexpr int NMAX = NS > 0 ? NS : 1;
     const int N = NS >= 0 ? NS : p.ndust;
-    const bool drag = MODE == 0 && N > 0 && (p.flags & SHARK_FLAG_DRAG);
+    const bool drag = (MODE == 0 || MODE == 2) && N > 0 && (p.flags & SHARK_FLAG_DRAG);
     // constant stopping times (SI): the FP64 coefficients of this step were computed once by
     // k_prepare_step; other setups compute them per cell below
     const bool const_ts = p.setup == SHARK_SETUP_SI;
     const float* __restrict__ cr = p.coef;
     const float* __restrict__ cw = p.coef + SHARK_MAX_DUST;
-    if (MODE == 0) stamp_start(p.stamps);
+    constexpr bool DRAG = MODE == 0 || MODE == 2, REST = MODE == 0 || MODE == 3;
+    if (DRAG) stamp_start(p.stamps);
     const double dt = *p.dt;
     const int gx = blockIdx.x * blockDim.x + threadIdx.x + p.ng;
     const int gy = (p.ndim == 2) ? blockIdx.y + p.ng : 0;
@@ -1171,9 +1303,9 @@ k_finalize_mixed(KParams<float> p) {
     bool cfl_done = false;
     float vmax_d = 0.f, vv_last = 0.f, fmx2_d = 0.f;
     const float xc = act ? p.xpos[gx] - p.f_half_box_l : 0.f;
-    // part 1: drag, floor, drag heating; part 2: kick, setup_inloop, CFL.  With growth in between
-    // (a block-wide phase) the two parts are separate; otherwise they form one block of code.
-    const bool heats = MODE == 0 && N > 0 && (p.flags & SHARK_FLAG_BACK_REACTION) && p.iso < 1;
+    // part 1: drag, floor, drag heating; part 2: kick, setup_inloop, CFL.  With growth in between they
+    // are two launches (MODES 2 and 3), or with fragmentation have it between them.
+    const bool heats = DRAG && N > 0 && (p.flags & SHARK_FLAG_BACK_REACTION) && p.iso < 1;
     const bool direct = !const_ts && p.setup != SHARK_SETUP_DUSTYTURB && p.setup != SHARK_SETUP_DISK_POLAR &&
                         p.setup != SHARK_SETUP_DISK_CART;
     auto part1 = [&]() {
@@ -1320,12 +1452,12 @@ k_finalize_mixed(KParams<float> p) {
         }
     };
     auto part2 = [&]() {
-        if (MODE == 0 && p.ou_nm > 0) {                                    // turbulence kick (solve.f90:129-146)
+        if (REST && p.ou_nm > 0) {                                    // turbulence kick (solve.f90:129-146)
             turb_kick_cell<float>(p, u, gx, gy, dt);
             px = u[cc + (1) * pl];
             py = u[cc + (2) * pl];
         }
-        if (MODE == 0 && p.setup == SHARK_SETUP_SI && !(p.flags & SHARK_FLAG_FORCE_KICK)) {
+        if (REST && p.setup == SHARK_SETUP_SI && !(p.flags & SHARK_FLAG_FORCE_KICK)) {
             // setup_inloop: Crank-Nicolson rotation (SI/setup.f90:299-332)
             in_regs = false;
             const float om = p.f_si_om, qsh = p.f_si_q;
@@ -1348,7 +1480,7 @@ k_finalize_mixed(KParams<float> p) {
                 u[ixx] = d * (vx * (1.f - O2) - 2.f * uz * Ohmdt + AA * Ohmdt) * inv;
             }
         }
-        if (MODE == 0 && ((p.setup == SHARK_SETUP_DISK_POLAR && disk_inloop_cell<float, float>(p, u, gx, gy, dt)) ||
+        if (REST && ((p.setup == SHARK_SETUP_DISK_POLAR && disk_inloop_cell<float, float>(p, u, gx, gy, dt)) ||
                           (p.setup == SHARK_SETUP_DISK_CART && cdisk_inloop_cell<float>(p, u, gx, gy)))) {
             in_regs = false;
             rho = u[cc + (0) * pl];
@@ -1430,23 +1562,15 @@ k_finalize_mixed(KParams<float> p) {
         if (!isfinite(vx) || !isfinite(vy) || !isfinite(vz)) st |= SHARK_STATUS_NAN;
         if (!(dtc > 0.f) || !isfinite(dtc)) { st |= SHARK_STATUS_DT_UNDERFLOW; dtc = 2e38f; }
     };
-    if constexpr (GROW && MODE == 0) {   // dust_growth (solve.f90:113) between the two parts
-        if (act) part1();
-        if (p.gw.mode & SHARK_GROWTH_FRAGMENTATION) {
-            if (act) st |= grow_in_finalize(p, u, gx, gy, dt);
-        } else {
-            __syncthreads();             // the block's cells after the drag
-            st |= grow_block_warps(p, blockIdx.x * blockDim.x + p.ng, gy, dt);
-            __syncthreads();
-        }
-        if (act) part2();
-    } else if (act) {
+    if (act) {
         part1();
-        part2();
+        if (GROW && MODE == 0) st |= grow_in_finalize(p, u, gx, gy, dt);   // dust_growth with fragmentation
+        if (MODE != 2) part2();
     }
+    if (MODE == 2) return;           // k_growth_f and MODE 3 follow
     block_reduce_dt_f(dtc, st, p.dt_next, p.status);
-    if (MODE == 0 && gx < p.ng + p.nx) fill_ghost_images(p, p.u_next, gx, gy);
-    if (MODE == 0) stamp_end(p.stamps, GROW);
+    if (REST && gx < p.ng + p.nx) fill_ghost_images(p, p.u_next, gx, gy);
+    if (REST) stamp_end(p.stamps, GROW);
 }
 
 // Per-step preparation, one small block before the flux kernels: reset the next-dt slot and,
