@@ -9,8 +9,8 @@
 //   T    = per temperature row (one row, or one per column for the disk), with the T-only
 //          constants sigmav_ie, vi, tau_k, alpha_k tabulated on the host
 //   zeta = chg_x, attenuated by exp(-Sigma unit_d unit_l/chg_sigma_att) for the disk.
-// R = double follows the CPU oracle operation by operation (nvcc --fmad=false); R = float
-// (mixed precision) runs the cold part of the iteration in FP32 and finishes it in FP64.  Outputs: psi_old (FP64, the warm start of the
+// R = double runs in FP64; R = float (mixed precision) runs the cold part of the iteration in FP32
+// and finishes it in FP64.  Outputs: psi_old (FP64, the warm start of the
 // next call), zd (N planes), ni, ne, and with SHARK_CHARGE_RESISTIVITIES eta_o/H/a and gamma_d,
 // plus the per-call histogram of Newton iteration counts.
 #pragma once
@@ -35,17 +35,20 @@ struct ChargeParams {
     int use_seed;                // 0 none, 1 seed where psi_old == 0, 2 seed always
     const double* hs;            // [nx_max] column-to-midplane factor (nullptr: 1)
     const double* trow;          // [rows][8]: T, sigmav_ie, vi, cs_T, c_el, c_ions, sigmav_el, sigmav_ions
-    const double* tau;           // [rows][N]
-    const double* alpha;         // [rows][N]
-    const double* l2;            // [N] grain radius^2 (cm^2)
-    const double* mkum;          // [N] grain mass (g)
-    const double* ak;            // [N] sqrt(pi gamma/8) rhograin_cgs l_k (stopping-time numerator)
-    const double* rtau;          // [rows][N] 1/tau_k        (mixed path)
-    const double* nfac;          // [N] unit_d / m_k (g)     (mixed path: n_k = rho_k / hs * nfac_k)
-    const double* rmk;           // [N] 1/m_k (g)            (mixed path)
-    const double* pl2;           // [N] pi l_k^2             (mixed path)
-    const float4* tf;            // [rows][N][2] (alpha, 1/tau, pi l^2/tau, tau), (unit_d/m, pi l^2, 1/m,
-                                 // sqrt(pi gamma/8) rhograin l) in FP32 (mixed path)
+    // per species and temperature row, element k * rows + row
+    const double* tau;
+    const double* alpha;
+    const double* ptau;          // pi l_k^2 / tau_k
+    const double* ntau;          // nfac_k tau_k
+    int rows;
+    // per species
+    const double* l2;            // grain radius^2 (cm^2)
+    const double* mkum;          // grain mass (g)
+    const double* nfac;          // unit_d / m_k (g): n_k = rho_k / hs * nfac_k
+    const double* npl;           // nfac_k pi l_k^2
+    const double* wk;            // sqrt(pi gamma/8) rhograin_cgs l_k / m_k: stopping time over mass, times rho_cgs cs
+    const float4* tf;            // (alpha, 1/tau, pi l^2/tau, tau) at (2 k) * rows + row and (unit_d/m, pi l^2, 1/m,
+                                 // sqrt(pi gamma/8) rhograin l) at (2 k + 1) * rows + row, FP32 (mixed path)
     double unH, ud, ul, x0, sig_att;
     double thetai, th2, th3, psi0, eps, B0, mu_ions;
     int nitermax;
@@ -67,74 +70,6 @@ constexpr double pi = 3.141592653589793238462643383279;
 constexpr double e_el = 4.8e-10, m_el = 9.109e-28, clight = 3e10, mH = 1.67e-24;
 }
 
-template <typename R>
-__device__ __forceinline__ R dexp(R x);
-template <> __device__ __forceinline__ double dexp<double>(double x) { return exp(x); }
-template <> __device__ __forceinline__ float dexp<float>(float x) { return expf(x); }
-template <typename R>
-__device__ __forceinline__ R dsqrt_(R x);
-template <> __device__ __forceinline__ double dsqrt_<double>(double x) { return sqrt(x); }
-template <> __device__ __forceinline__ float dsqrt_<float>(float x) { return sqrtf(x); }
-
-// One Newton iteration loop of ionisation.f90:79-135 in arithmetic C: iterates while
-// |f(psi)| > tol and niter < nitermax, updating psi, niter, lowT and conv (|f| of the last
-// evaluation).  `nk(k)` gives the grain number density of species k in C.  With stall = true the
-// loop also stops when an update leaves psi unchanged (no further progress in C).
-template <typename C, typename R, typename NK>
-__device__ __forceinline__ void charge_newton(const ChargeParams<R>& p, const double* tau, const double* alp, NK nk,
-                                              C nH, C x, C sigmav_ie, C vi, C tol, bool stall, C& psi, int& niter,
-                                              int& lowT, C& conv) {
-    const int N = p.ndust;
-    const C pi = C(chg::pi);
-    const C thetai = C(p.thetai), th2 = C(p.th2), th3 = C(p.th3), psi0 = C(p.psi0);
-    const C one = C(1), two = C(2);
-    const C xnH = x * nH;
-    while (conv > tol && niter < p.nitermax) {
-        const C eps_psi = (one - psi) / thetai * dexp<C>(-psi);
-        const C et = eps_psi * thetai;
-        const C et2 = et * et;
-        const C om = one - eps_psi;
-        const C D = (-eps_psi * (two - psi) / (one - psi));
-        C S1 = C(0), S2 = C(0), S3 = C(0), S4 = C(0), S5 = C(0), S6 = C(0);
-        C n_i = C(0);
-        for (int k = 0; k < N; ++k) {
-            const C n = nk(k), tk = C(tau[k]), ak = C(alp[k]), l2 = C(p.l2[k]);
-            const C den = one + et * ak + et2;
-            n_i = n_i + (-(psi * tk + (one - et2) / den) * n / om);
-            const C npl = n * pi * l2;
-            S1 = S1 + npl * ((one - psi) + (two / tk) * (et2 + et) / den);
-            S2 = S2 + n * (-(et2 * et2) + (C(4) * th2 - th3 * ak) * (eps_psi * eps_psi) +
-                           (two * thetai * ak - C(4) * th2) * eps_psi + one - thetai * ak) / (den * den);
-            S3 = S3 + n * tk;
-            S4 = S4 + npl / (tk * den);
-            S5 = S5 + npl * (two * eps_psi * th2 + thetai * ak) / (tk * (den * den));
-            S6 = S6 + npl;
-        }
-        const C fpsi = sigmav_ie * eps_psi * (n_i * n_i) / (xnH) + n_i * vi / (xnH) * (S1) - one;
-        const C dni = -one / (om * om) * (D) * (S2) - (psi / om * (D) + one) * S3 / om;
-        const C dfdpsi = sigmav_ie * n_i / (xnH) * (n_i * (D) + two * eps_psi * dni) +
-                         two * n_i * vi / (xnH) * (et2 + et) *
-                             ((dni / n_i + (D) * (two * et + one) / (eps_psi * (one + et))) * (S4) + ((D) * S5)) +
-                         n_i * vi / (xnH) * (dni / n_i * (one - psi) - one) * (S6);
-        const C prev = psi;
-        psi = psi - fpsi / dfdpsi;
-        if (psi < psi0) {
-            psi = psi0 * C(0.9999999);
-            lowT = 1;
-        } else if (psi > C(0)) {
-            psi = C(-1e-5);
-        }
-        conv = fabs(fpsi);
-        niter = niter + 1;
-        if (psi == prev) {
-            if (stall) break;   // FP32 phase: no further progress in FP32
-            // an unchanged psi with the residual above the tolerance repeats itself until
-            // nitermax (e.g. the psi0 clamp): go there directly, same final state
-            if (conv > tol) niter = p.nitermax;
-        }
-    }
-}
-
 // Compensated FP32 sum (Kahan): s + c carries the sum of the added terms to ~1 ulp.
 __device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
     const float y = x - c;
@@ -143,130 +78,229 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
     s = t;
 }
 
-// FP64 phase of the mixed path: the iteration of charge_newton with the residual f accurate to
-// ~1e-8.  Its species sums split into psi-independent parts, formed once per cell in FP64,
+// The Newton iteration of ionisation.f90:79-135 with its species sums in psi-independent parts, formed
+// once per cell,
 //   T1 = sum n_k tau_k,  T3 = sum n_k pi l_k^2,
-// and psi-dependent corrections of a few per cent, formed per iteration in compensated FP32,
-//   T2 = sum n_k r_k,  T4 = sum n_k pi l_k^2 r_k / tau_k,   r_k = 1/(1 + et alpha_k + et^2):
-//   n_i = -(psi T1 + (1 - et^2) T2)/(1 - eps),   S1 = (1 - psi) T3 + 2 (et^2 + et) T4.
-// The derivative's species sums are FP32 (Newton needs f' to a few digits).  n_k = rho_k/hs
-// unit_d/m_k; the FP32 sums run on rho_k unit_d/m_k and take 1/hs afterwards.  The stopping test
-// |f| < chg_eps is the reference's.  `uk` points at species 0 of the cell, `tf` at the cell's row.
+// and four sums per iteration over r_k = 1/(1 + et alpha_k + et^2), et = eps theta:
+//   T2 = sum n_k r_k,  T4 = sum n_k pi l_k^2 r_k / tau_k,
+//   S2 = sum n_k (A + B alpha_k) r_k^2,  S5 = sum n_k pi l_k^2 / tau_k (C + theta alpha_k) r_k^2,
+//   n_i = -(psi T1 + (1 - et^2) T2)/(1 - eps),   S1 = (1 - psi) T3 + 2 (et^2 + et) T4;
+// they are the reference's sums with the factors a cell's species share taken out.  The sums run on
+// rho_k unit_d / m_k and take 1/hs afterwards.
+
+// Quotients of the iteration's scalars: FP64 on reciprocals to an ulp, plain FP32 divisions.
+__device__ __forceinline__ double recip(double b) { return rcp64_any(b); }
+__device__ __forceinline__ float recip(float b) { return 1.0f / b; }
+
+// f(psi) in arithmetic C and its derivative in arithmetic E from the iteration's sums, 1/hs in all of
+// them, and the update of psi.  Newton needs f' to a few digits only: the mixed path forms it in FP32,
+// as it does the sums S2 and S5 in it.  Returns f at the psi it came with.
+template <typename C, typename E>
+__device__ __forceinline__ C charge_update(C T1, C T2, C T3, C T4, E S2, E S5, C eps_psi, C thetai, C rxnH, C sigmav_ie,
+                                           C vi, C psi0, C& psi, int& lowT) {
+    const C one = C(1), two = C(2);
+    const C et = eps_psi * thetai, et2 = et * et, et21 = et2 + et, rom = recip(one - eps_psi);
+    const C n_i = -(psi * T1 + (one - et2) * T2) * rom;
+    const C S1 = (one - psi) * T3 + two * et21 * T4;
+    const C nv = n_i * vi * rxnH, ns = sigmav_ie * n_i * rxnH;
+    const C f = ns * eps_psi * n_i + nv * S1 - one;
+    const E e1 = E(1), e2 = E(2), p = E(psi), ep = E(eps_psi), t = E(et), ro = E(rom), ni = E(n_i), nve = E(nv), nse = E(ns);
+    const E D = -ep * (e2 - p) * recip(e1 - p);
+    const E dni = -(ro * ro) * D * S2 - (p * ro * D + e1) * E(T1) * ro;
+    const E q = dni * recip(ni);
+    const E df = nse * (ni * D + e2 * ep * dni) +
+                 e2 * nve * E(et21) * ((q + D * (e2 * t + e1) * recip(ep * (e1 + t))) * E(T4) + D * S5) +
+                 nve * (q * (e1 - p) - e1) * E(T3);
+    psi = psi - C(E(f) * recip(df));
+    if (psi < psi0) {
+        psi = psi0 * C(0.9999999);
+        lowT = 1;
+    } else if (psi > C(0)) {
+        psi = C(-1e-5);
+    }
+    return f;
+}
+
+// FP32 iterations of the mixed path from a cold or network start, until |f| <= tol or psi stops moving.
+// The residual is steep (|df/dpsi| ~ 1e2-1e3 at the root), so an FP32 psi pins f only to ~1e-4.
 template <typename R>
-__device__ __forceinline__ void charge_newton_mix(const ChargeParams<R>& p, const float4* tf, const R* uk,
-                                                  double T1, double T3, double ihs, double nH, double x,
-                                                  double sigmav_ie, double vi, double& psi, int& niter, int& lowT,
-                                                  double& conv) {
-    const int N = p.ndust;
-    const double thetai = p.thetai, psi0 = p.psi0;
-    const float thf = (float)p.thetai, th2f = (float)p.th2, th3f = (float)p.th3;
-    const double rxnH = 1.0 / (x * nH);
-    while (conv > p.eps && niter < p.nitermax) {
-        const double eps_psi = (1.0 - psi) / thetai * exp(-psi);
-        const double et = eps_psi * thetai;
-        const double et2 = et * et, et21 = et2 + et, om = 1.0 - eps_psi, rom = 1.0 / om;
-        const double D = (-eps_psi * (2.0 - psi) / (1.0 - psi));
-        const float ef = (float)eps_psi, etf = (float)et, et2f = (float)et2;
-        const float c2a = -(et2f * et2f), c2b = ef * ef, c5 = 2.f * ef * th2f;
-        float T2 = 0.f, k2 = 0.f, T4 = 0.f, k4 = 0.f, S2 = 0.f, S5 = 0.f;
+__device__ __forceinline__ void charge_newton_f(const ChargeParams<R>& p, const float4* tf, const R* uk, float T1, float T3,
+                                                float ihs, float nH, float x, float sigmav_ie, float vi, float tol,
+                                                float& psi, int& niter, int& lowT) {
+    const int N = p.ndust, rows = p.rows;
+    const float th = (float)p.thetai, th2 = (float)p.th2, th3 = (float)p.th3, psi0 = (float)p.psi0;
+    const float rxnH = 1.0f / (x * nH);
+    float conv = 1e4f;
+    while (conv > tol && niter < p.nitermax) {
+        const float eps = (1.0f - psi) / th * expf(-psi), et = eps * th, et2 = et * et;
+        const float A = -(et2 * et2) + 4.f * th2 * (eps * eps) - 4.f * th2 * eps + 1.f, B = -th3 * (eps * eps) + 2.f * th * eps - th;
+        const float c5 = 2.f * eps * th2;
+        float T2 = 0.f, T4 = 0.f, S2 = 0.f, S5 = 0.f;
         for (int k = 0; k < N; ++k) {
-            const float4 a = tf[2 * k], b = tf[2 * k + 1];   // (alpha, 1/tau, pi l^2/tau, tau), (unit_d/m, ...)
-            const float nf = (float)uk[(long long)k * p.plane] * b.x;
-            const float r = 1.f / (1.f + etf * a.x + et2f);
-            const float nr = nf * r;
-            kahan_add(T2, k2, nr);
-            kahan_add(T4, k4, nr * a.z);
-            const float f2 = (c2a + (4.f * th2f - th3f * a.x) * c2b + (2.f * thf * a.x - 4.f * th2f) * ef + 1.f - thf * a.x) * r;
-            S2 = S2 + nr * f2;
-            S5 = S5 + nr * a.z * (c5 + thf * a.x) * r;
+            const float4 a = tf[2 * k * rows];
+            const float nf = (float)uk[(long long)k * p.plane] * tf[(2 * k + 1) * rows].x;
+            const float r = 1.f / (1.f + et * a.x + et2);
+            const float nr = nf * r, w = nr * a.z;
+            T2 += nr;
+            T4 += w;
+            S2 += nr * r * (A + B * a.x);
+            S5 += w * r * (c5 + th * a.x);
         }
-        const double T2d = ihs * (double)T2, T4d = ihs * (double)T4;
-        const double n_i = -(psi * T1 + (1.0 - et2) * T2d) * rom;
-        const double S1 = (1.0 - psi) * T3 + 2.0 * et21 * T4d;
-        const double fpsi = sigmav_ie * eps_psi * (n_i * n_i) * rxnH + n_i * vi * rxnH * S1 - 1.0;
-        const double S2d = ihs * (double)S2, S4d = T4d, S5d = ihs * (double)S5;
-        const double dni = -(rom * rom) * D * S2d - (psi * rom * D + 1.0) * T1 * rom;
-        const double dfdpsi = sigmav_ie * n_i * rxnH * (n_i * D + 2.0 * eps_psi * dni) +
-                              2.0 * n_i * vi * rxnH * et21 *
-                                  ((dni / n_i + D * (2.0 * et + 1.0) / (eps_psi * (1.0 + et))) * S4d + D * S5d) +
-                              n_i * vi * rxnH * (dni / n_i * (1.0 - psi) - 1.0) * T3;
-        const double prev = psi;
-        psi = psi - fpsi / dfdpsi;
-        if (psi < psi0) {
-            psi = psi0 * 0.9999999;
-            lowT = 1;
-        } else if (psi > 0.0) {
-            psi = -1e-5;
-        }
-        conv = fabs(fpsi);
+        const float prev = psi;
+        conv = fabsf(charge_update<float, float>(T1, ihs * T2, T3, ihs * T4, ihs * S2, ihs * S5, eps, th, rxnH, sigmav_ie, vi, psi0, psi, lowT));
         niter = niter + 1;
+        if (psi == prev) break;
+    }
+}
+
+// FP64 iterations to the reference's stopping test |f| < chg_eps.  FP64 path: the four sums in FP64.
+// Mixed path: T2 and T4, corrections of a few per cent, in compensated FP32 (f accurate to ~1e-8),
+// the derivative in FP32.
+template <typename R>
+__device__ __forceinline__ void charge_newton_d(const ChargeParams<R>& p, int row, const R* uk, double T1, double T3, double ihs,
+                                                double nH, double x, double sigmav_ie, double vi, double& psi, int& niter,
+                                                int& lowT, double& conv) {
+    const int N = p.ndust, rows = p.rows;
+    const double th = p.thetai, th2 = p.th2, th3 = p.th3, psi0 = p.psi0;
+    const double rth = rcp64(th), rxnH = rcp64_any(x * nH);
+    const R ihsr = R(ihs);
+    while (conv > p.eps && niter < p.nitermax) {
+        const double eps = (1.0 - psi) * rth * exp(-psi), et = eps * th, et2 = et * et;
+        double T2, T4;
+        R S2, S5;
+        if constexpr (sizeof(R) == 8) {
+            const double *al = p.alpha + row, *pt = p.ptau + row;
+            const double e2 = eps * eps, et21 = 1.0 + et2;
+            const double A = fma(4.0 * th2, e2 - eps, fma(-et2, et2, 1.0)), B = fma(-th3, e2, fma(2.0 * th, eps, -th));
+            const double C = 2.0 * eps * th2;
+            T2 = T4 = S2 = S5 = 0.0;
+            for (int k = 0; k < N; ++k) {
+                const double a = al[(size_t)k * rows], nf = uk[(long long)k * p.plane] * p.nfac[k];
+                const double r = rcp64(fma(et, a, et21));
+                const double nr = nf * r, w = nr * pt[(size_t)k * rows];
+                T2 += nr;
+                T4 += w;
+                S2 = fma(nr * r, fma(B, a, A), S2);
+                S5 = fma(w * r, fma(th, a, C), S5);
+            }
+        } else {
+            const float4* tf = p.tf + row;
+            const float ef = (float)eps, etf = (float)et, et2f = (float)et2, thf = (float)th, th2f = (float)th2, th3f = (float)th3;
+            const float c2a = -(et2f * et2f), c2b = ef * ef, c5 = 2.f * ef * th2f;
+            float t2 = 0.f, k2 = 0.f, t4 = 0.f, k4 = 0.f, s2 = 0.f, s5 = 0.f;
+            for (int k = 0; k < N; ++k) {
+                const float4 a = tf[2 * k * rows];
+                const float nf = (float)uk[(long long)k * p.plane] * tf[(2 * k + 1) * rows].x;
+                const float r = 1.f / (1.f + etf * a.x + et2f);
+                const float nr = nf * r;
+                kahan_add(t2, k2, nr);
+                kahan_add(t4, k4, nr * a.z);
+                const float f2 = (c2a + (4.f * th2f - th3f * a.x) * c2b + (2.f * thf * a.x - 4.f * th2f) * ef + 1.f - thf * a.x) * r;
+                s2 = s2 + nr * f2;
+                s5 = s5 + nr * a.z * (c5 + thf * a.x) * r;
+            }
+            T2 = widen(t2); T4 = widen(t4); S2 = s2; S5 = s5;
+        }
+        const double prev = psi;
+        conv = abs64(charge_update<double, R>(T1, ihs * T2, T3, ihs * T4, ihsr * S2, ihsr * S5, eps, th, rxnH, sigmav_ie, vi, psi0, psi, lowT));
+        niter = niter + 1;
+        // an unchanged psi with the residual above the tolerance repeats itself until nitermax
+        // (e.g. the psi0 clamp): go there directly, same final state
         if (psi == prev && conv > p.eps) niter = p.nitermax;
     }
 }
 
-// Outputs of the mixed path (ionisation.f90:137-206): Z_k, n_i, n_e, psi_old and, with the
-// resistivities, eta_o/H/a and gamma_d.  The per-species terms are FP32 (the outputs are stored
-// in FP32) with compensated sums; the cell-level electron and ion terms are FP64.
+// Outputs (ionisation.f90:137-206): Z_k, n_i, n_e, psi_old and, with the resistivities, eta_o/H/a and
+// gamma_d.  FP64 path: FP64 throughout.  Mixed path: the per-species terms are FP32 (the outputs are
+// stored in FP32) with compensated sums; the cell-level electron and ion terms are FP64.
 template <typename R>
-__device__ __forceinline__ void charge_outputs_mix(const ChargeParams<R>& p, const float4* tf, long long c, double ihs,
-                                                   double rho, double nH, double x, double sigmav_ie, const double* tr,
-                                                   double psi, double eps_psi, int lowT) {
-    const int N = p.ndust;
+__device__ __forceinline__ void charge_outputs(const ChargeParams<R>& p, int row, long long c, double ihs, double rho, double nH,
+                                               double x, double sigmav_ie, const double* tr, double psi, double eps_psi, int lowT) {
+    const int N = p.ndust, rows = p.rows;
     const R* uk = p.u + 5 * p.plane + c;
-    const float psif = (float)psi, e2t = (float)((eps_psi * eps_psi) * p.th2), et1 = (float)(eps_psi * p.thetai);
-    float zs = 0.f, kz = 0.f;
-    for (int k = 0; k < N; ++k) {
-        const float4 a = tf[2 * k], b = tf[2 * k + 1];
-        const float z = psif * a.w + (1.f - e2t) / (1.f + et1 * a.x + e2t);
-        p.zd[(long long)k * p.plane + c] = R(z);
-        kahan_add(zs, kz, z * ((float)uk[(long long)k * p.plane] * b.x));
+    const double e = chg::e_el, cl = chg::clight, mel = chg::m_el, mi = p.mu_ions * chg::mH;
+    const double B = p.B0 * sqrt(nH / 1e4);
+    const double irc = rcp64_any(rho * p.ud * tr[3]);   // t_sd = sqrt(pi gamma/8) rhograin l / (rho_cgs cs_T)
+    const double eBc = e * B / cl;
+    double zsum, so = 0.0, sp = 0.0, sh = 0.0;          // sums without 1/hs
+    if constexpr (sizeof(R) == 8) {
+        const double *ta = p.tau + row, *al = p.alpha + row;
+        const double e2t = (eps_psi * eps_psi) * p.th2, et1 = eps_psi * p.thetai, ome = 1.0 - e2t, ope = 1.0 + e2t;
+        const double wB = eBc * irc;
+        zsum = 0.0;
+        for (int k = 0; k < N; ++k) {
+            const double den = fma(et1, al[(size_t)k * rows], ope);
+            const double z = fma(psi, ta[(size_t)k * rows], ome * rcp64(den));
+            p.zd[(long long)k * p.plane + c] = z;
+            const double nz = uk[(long long)k * p.plane] * p.nfac[k] * z;
+            zsum += nz;
+            if (!p.res) continue;
+            const double W = p.wk[k];
+            const double sd = nz * z * W, wt = z * W * wB;
+            const double q = abs_less(wt, 1e150) ? rcp64(fma(wt, wt, 1.0)) : 0.0;
+            so += sd;
+            sp = fma(sd, q, sp);
+            sh = fma(sd, wt * q, sh);
+            p.gamma_d[(long long)k * p.plane + c] = wt;
+        }
+        const double e2i = (e * e) * irc;
+        so *= e2i; sp *= e2i; sh *= e2i;
+    } else {
+        const float4* tf = p.tf + row;
+        const float psif = (float)psi, e2t = (float)((eps_psi * eps_psi) * p.th2), et1 = (float)(eps_psi * p.thetai);
+        const float ircf = (float)irc, eBcf = (float)eBc, ef = (float)e;
+        float zs = 0.f, kz = 0.f, fo = 0.f, ko = 0.f, fp = 0.f, kp = 0.f, fh = 0.f, kh = 0.f;
+        for (int k = 0; k < N; ++k) {
+            const float4 a = tf[2 * k * rows], b = tf[(2 * k + 1) * rows];
+            const float z = psif * a.w + (1.f - e2t) / (1.f + et1 * a.x + e2t);
+            const float nf = (float)uk[(long long)k * p.plane] * b.x;
+            p.zd[(long long)k * p.plane + c] = R(z);
+            kahan_add(zs, kz, z * nf);
+            if (!p.res) continue;
+            const float t_sd = b.w * ircf;
+            const float ze = z * ef;
+            const float sd = nf * b.z * (ze * ze) * t_sd;
+            const float omd = z * eBcf * b.z;
+            const float wt = omd * t_sd;
+            const float q = 1.f / (1.f + wt * wt);
+            const float h = fabsf(wt) > 1e18f ? 1.f / wt : wt * q;   // wt / (1 + wt^2) without overflow
+            kahan_add(fo, ko, sd);
+            kahan_add(fp, kp, sd * q);
+            kahan_add(fh, kh, sd * h);
+            p.gamma_d[(long long)k * p.plane + c] = R(wt);
+        }
+        zsum = zs; so = fo; sp = fp; sh = fh;
     }
-    double nsum = -(ihs * (double)zs) / (1.0 - eps_psi);
+    double nsum = -(ihs * zsum) * rcp64_any(1.0 - eps_psi);
     if (lowT > 0 && N > 0) nsum = sqrt(eps_psi * x * nH / sigmav_ie);
     p.ni[c] = R(nsum);
     p.ne[c] = R(eps_psi * nsum);
     p.psi_old[c] = lowT > 0 ? p.psi0 : psi;
     if (!p.res) return;
-    const double e = chg::e_el, cl = chg::clight, mel = chg::m_el, mi = p.mu_ions * chg::mH;
-    const double B = p.B0 * sqrt(nH / 1e4);
-    const double rnH = 1.0 / nH;
+    const double rnH = rcp64_any(nH);
     const double t_sel = tr[4] * rnH, t_sions = tr[5] * rnH;
-    const double irc = 1.0 / (rho * p.ud * tr[3]);      // t_sd = sqrt(pi gamma/8) rhograin l / (rho_cgs cs_T)
-    const double sig_el = (eps_psi * nsum) * (e * e) * t_sel / mel;
-    const double sig_i = (nsum) * (e * e) * t_sions / mi;
-    const double om_el = -e * B / cl / mel;
-    const double om_i = e * B / cl / mi;
-    const float ircf = (float)irc, eBc = (float)(e * B / cl), ef = (float)e;
-    float so = 0.f, ko = 0.f, sp = 0.f, kp = 0.f, sh = 0.f, kh = 0.f;
-    for (int k = 0; k < N; ++k) {
-        const float4 a = tf[2 * k], b = tf[2 * k + 1];
-        const float z = psif * a.w + (1.f - e2t) / (1.f + et1 * a.x + e2t);
-        const float t_sd = b.w * ircf;
-        const float ze = z * ef;
-        const float sd = ((float)uk[(long long)k * p.plane] * b.x) * b.z * (ze * ze) * t_sd;   // times 1/hs below
-        const float omd = z * eBc * b.z;
-        const float wt = omd * t_sd;
-        const float q = 1.f / (1.f + wt * wt);
-        const float h = fabsf(wt) > 1e18f ? 1.f / wt : wt * q;   // wt / (1 + wt^2) without overflow
-        kahan_add(so, ko, sd);
-        kahan_add(sp, kp, sd * q);
-        kahan_add(sh, kh, sd * h);
-        p.gamma_d[(long long)k * p.plane + c] = R(wt);
-    }
-    const double wi = om_i * t_sions, we = om_el * t_sel;
-    const double sigma_o = ihs * (double)so + sig_i + sig_el;
-    const double sigma_p = sig_i / (1.0 + wi * wi) + sig_el / (1.0 + we * we) + ihs * (double)sp;
-    const double sigma_h = -sig_i * (wi) / (1.0 + wi * wi) - sig_el * (we) / (1.0 + we * we) - ihs * (double)sh;
-    p.eta[c] = R(1.0 / sigma_o);
-    p.eta[p.plane + c] = R(sigma_h / (sigma_p * 2.0 + sigma_h * sigma_h));
-    p.eta[2 * p.plane + c] = R(sigma_p / (sigma_p * sigma_p + sigma_h * sigma_h) - 1.0 / sigma_o);
+    const double sig_el = (eps_psi * nsum) * ((e * e) / mel) * t_sel;
+    const double sig_i = (nsum) * ((e * e) / mi) * t_sions;
+    const double we = -eBc / mel * t_sel, wi = eBc / mi * t_sions;
+    const double qe = recip(1.0 + we * we), qi = recip(1.0 + wi * wi);
+    const double sigma_o = ihs * so + sig_i + sig_el;
+    const double sigma_p = sig_i * qi + sig_el * qe + ihs * sp;
+    const double sigma_h = -sig_i * wi * qi - sig_el * we * qe - ihs * sh;
+    const double ro = recip(sigma_o);
+    p.eta[c] = R(ro);
+    p.eta[p.plane + c] = R(sigma_h * recip(sigma_p * 2.0 + sigma_h * sigma_h));
+    p.eta[2 * p.plane + c] = R(sigma_p * recip(sigma_p * sigma_p + sigma_h * sigma_h) - ro);
 }
 
-// K5.  R = double: the reference loop in FP64 (parity path).  R = float (mixed precision): from a
-// cold or network start, FP32 Newton steps until |f| < 1e-3 or psi stops moving in FP32, then FP64
-// steps to the reference tolerance chg_eps; a warm start (psi_old, FP64) goes to FP64 directly.
-// The residual is steep (|df/dpsi| ~ 1e2-1e3 at the root), so an FP32 psi pins f only to ~1e-4:
-// the last digits need FP64.  The iteration count is the sum of both phases.
+// K5.  A cell starts from psi_old (FP64, the last call's psi), cold from psi0 or the network's seed;
+// the mixed path begins a cold or seeded cell with FP32 iterations.  The iteration count is the sum
+// of both phases.  Bound by the FP64 pipe: per iteration FP64 spends 17 instructions for a species
+// (some 160 as the reference's expressions, whose shared factors and invariants it re-formed) and
+// some 75 for the cell; the mixed path some 45 for the cell (its derivative is FP32) and two a
+// species for T1 and T3.
+// Temperature tables are laid out species by species, so that a warp's columns read them together.
+// Cold start, 384^2 x 32: FP64 24.4 -> 4.0 ms, mixed 1.54 -> 0.25; warm, driven box 768^2 x 32 mixed 1.00 -> 0.62 ms a step, polar disk
+// 512 x 1024 x 16 0.675 -> 0.43, 128 x 256 x 16 FP64 0.68 -> 0.15.
 template <typename R>
 __global__ void __launch_bounds__(128) k_charge(ChargeParams<R> p) {
     const int N = p.ndust;
@@ -282,18 +316,14 @@ __global__ void __launch_bounds__(128) k_charge(ChargeParams<R> p) {
         const long long c = (long long)iy * p.pitch + ix;
         const int row = p.t_per_col ? ix : 0;
         const double* tr = p.trow + (size_t)row * 8;
-        const double* tau = p.tau + (size_t)row * N;
-        const double* alp = p.alpha + (size_t)row * N;
-        // cell inputs in FP64 (the FP64 path reproduces the oracle's operation order)
         const double hs = p.hs ? p.hs[ix] : 1.0;
         const double u0 = (double)p.u[c];
         const double rho = u0 / hs;
         const double nH = rho * p.unH;
         double x = p.x0;
         if (p.sig_att > 0.0) x = p.x0 * exp(-(u0 * p.ud * p.ul) / p.sig_att);
-        auto nk64 = [&](int k) -> double { return ((double)p.u[(long long)(5 + k) * p.plane + c] / hs) * p.ud / p.mkum[k]; };
         const double sigmav_ie = tr[1], vi = tr[2];
-        const double thetai = p.thetai, th2 = p.th2, psi0 = p.psi0;
+        const double psi0 = p.psi0;
         double psi = psi0, conv = 1e4;
         int niter = 0, lowT = 0;
         const double pold = p.psi_old[c];
@@ -304,74 +334,28 @@ __global__ void __launch_bounds__(128) k_charge(ChargeParams<R> p) {
             if (sd < 0.0f) { psi = (double)sd; cold = true; }
         }
         const double ihs = 1.0 / hs;
+        const R* uk = p.u + 5 * p.plane + c;
+        double T1 = 0.0, T3 = 0.0;                 // psi-independent sums
+        {
+            const double* nt = p.ntau + row;
+            for (int k = 0; k < N; ++k) {
+                const double u = widen(uk[(long long)k * p.plane]);
+                T1 = fma(u, nt[(size_t)k * p.rows], T1);
+                T3 = fma(u, p.npl[k], T3);
+            }
+            T1 *= ihs;
+            T3 *= ihs;
+        }
         if (sizeof(R) == 4 && cold) {
-            float psif = (float)psi, convf = 1e4f;
-            auto nk32 = [&](int k) -> float { return (float)((double)p.u[(long long)(5 + k) * p.plane + c] * ihs * p.nfac[k]); };
-            charge_newton<float>(p, tau, alp, nk32, (float)nH, (float)x, (float)sigmav_ie, (float)vi,
-                                 fmaxf((float)p.eps, 1e-3f), true, psif, niter, lowT, convf);
+            float psif = (float)psi;
+            charge_newton_f(p, p.tf + row, uk, (float)T1, (float)T3, (float)ihs, (float)nH, (float)x, (float)sigmav_ie, (float)vi,
+                            fmaxf((float)p.eps, 1e-3f), psif, niter, lowT);
             psi = (double)psif;
-            conv = 1e4;   // the FP64 phase re-evaluates the residual
         }
-        if constexpr (sizeof(R) == 4) {
-            double T1 = 0.0, T3 = 0.0;                 // psi-independent sums of the mixed iteration
-            for (int k = 0; k < N; ++k) {
-                const double n = (double)p.u[(long long)(5 + k) * p.plane + c] * ihs * p.nfac[k];
-                T1 = T1 + n * tau[k];
-                T3 = T3 + n * p.pl2[k];
-            }
-            charge_newton_mix(p, p.tf + (size_t)row * N * 2, p.u + 5 * p.plane + c, T1, T3, ihs, nH, x, sigmav_ie, vi,
-                              psi, niter, lowT, conv);
-        } else
-            charge_newton<double>(p, tau, alp, nk64, nH, x, sigmav_ie, vi, p.eps, false, psi, niter, lowT, conv);
-        double eps_psi = (1.0 - psi) / thetai * exp(-psi);
+        charge_newton_d(p, row, uk, T1, T3, ihs, nH, x, sigmav_ie, vi, psi, niter, lowT, conv);
+        double eps_psi = (1.0 - psi) / p.thetai * exp(-psi);
         if (lowT > 0) eps_psi = 0.99999;
-        if constexpr (sizeof(R) == 4)
-            charge_outputs_mix(p, p.tf + (size_t)row * N * 2, c, ihs, rho, nH, x, sigmav_ie, tr, psi, eps_psi, lowT);
-        else {
-            double nsum = 0.0;
-            for (int k = 0; k < N; ++k) {
-                const double tk = tau[k], ak = alp[k];
-                const double z = psi * tk + (1.0 - (eps_psi * eps_psi) * th2) / (1.0 + eps_psi * thetai * ak + (eps_psi * eps_psi) * th2);
-                p.zd[(long long)k * p.plane + c] = R(z);
-                nsum = nsum - z * nk64(k) / (1.0 - eps_psi);
-            }
-            if (lowT > 0 && N > 0) nsum = sqrt(eps_psi * x * nH / sigmav_ie);
-            p.ni[c] = R(nsum);
-            p.ne[c] = R(eps_psi * nsum);
-            p.psi_old[c] = lowT > 0 ? p.psi0 : psi;
-            if (p.res) {
-                // resistivities (ionisation.f90:163-206)
-                const double e = chg::e_el, cl = chg::clight, mel = chg::m_el, mi = p.mu_ions * chg::mH;
-                const double B = p.B0 * sqrt(nH / 1e4);
-                const double cs_T = tr[3];
-                const double t_sel = tr[4] / nH, t_sions = tr[5] / nH;
-                const double rho_cgs = rho * p.ud;
-                const double sig_el = (eps_psi * nsum) * (e * e) * t_sel / mel;
-                const double sig_i = (nsum) * (e * e) * t_sions / mi;
-                const double om_el = -e * B / cl / mel;
-                const double om_i = e * B / cl / mi;
-                double so = 0.0, sp = 0.0, sh = 0.0;
-                for (int k = 0; k < N; ++k) {
-                    const double tk = tau[k], ak = alp[k];
-                    const double z = psi * tk + (1.0 - (eps_psi * eps_psi) * th2) / (1.0 + eps_psi * thetai * ak + (eps_psi * eps_psi) * th2);
-                    const double t_sd = p.ak[k] / (rho_cgs * cs_T);
-                    const double sd = nk64(k) * ((z * e) * (z * e)) * t_sd / p.mkum[k];
-                    const double omd = z * e * B / cl / p.mkum[k];
-                    const double wt = omd * t_sd;
-                    so = so + sd;
-                    sp = sp + sd / (1.0 + wt * wt);
-                    sh = sh + sd * wt / (1.0 + wt * wt);
-                    p.gamma_d[(long long)k * p.plane + c] = R(t_sd * omd);
-                }
-                const double wi = om_i * t_sions, we = om_el * t_sel;
-                const double sigma_o = so + sig_i + sig_el;
-                const double sigma_p = sig_i / (1.0 + wi * wi) + sig_el / (1.0 + we * we) + sp;
-                const double sigma_h = -sig_i * (wi) / (1.0 + wi * wi) - sig_el * (we) / (1.0 + we * we) - sh;
-                p.eta[c] = R(1.0 / sigma_o);
-                p.eta[p.plane + c] = R(sigma_h / (sigma_p * 2.0 + sigma_h * sigma_h));
-                p.eta[2 * p.plane + c] = R(sigma_p / (sigma_p * sigma_p + sigma_h * sigma_h) - 1.0 / sigma_o);
-            }
-        }
+        charge_outputs(p, row, c, ihs, rho, nH, x, sigmav_ie, tr, psi, eps_psi, lowT);
         p.iters[c] = niter;
         atomicAdd(&s_hist[niter < CHARGE_HIST - 1 ? niter : CHARGE_HIST - 1], 1u);
         if (conv > p.eps) atomicAdd(&s_hist[CHARGE_HIST], 1u);

@@ -542,17 +542,18 @@ void build_charge_tables(const shark_gpu_config& c, const Columns& col, int nx_m
     const int rows = disk ? nx_max : 1;
     off[0] = 0;                               // hs
     off[1] = off[0] + nx_max;                 // trow
-    off[2] = off[1] + (size_t)rows * 8;       // tau
+    off[2] = off[1] + (size_t)rows * 8;       // tau    (from here to ntau: species by species, a row each)
     off[3] = off[2] + (size_t)rows * N;       // alpha
-    off[4] = off[3] + (size_t)rows * N;       // l2
-    off[5] = off[4] + N;                      // mkum
-    off[6] = off[5] + N;                      // ak
-    off[7] = off[6] + N;                      // rtau: 1/tau (mixed path)
-    off[8] = off[7] + (size_t)rows * N;       // nfac: unit_d / m_k (g), grain number per unit of rho_k
-    off[9] = off[8] + N;                      // rmk: 1/m_k (g)
-    off[10] = off[9] + N;                     // pl2: pi l_k^2
+    off[4] = off[3] + (size_t)rows * N;       // ptau: pi l_k^2 / tau_k
+    off[5] = off[4] + (size_t)rows * N;       // ntau: nfac_k tau_k
+    off[6] = off[5] + (size_t)rows * N;       // l2
+    off[7] = off[6] + N;                      // mkum
+    off[8] = off[7] + N;                      // nfac: unit_d / m_k (g), grain number per unit of rho_k
+    off[9] = off[8] + N;                      // npl: nfac_k pi l_k^2
+    off[10] = off[9] + N;                     // wk: sqrt(pi gamma/8) rhograin l_k / m_k
     h.assign(off[10] + N, 0.0);
     for (int ix = 0; ix < nx_max; ++ix) h[off[0] + ix] = disk ? col.hs[ix] : 1.0;
+    const double f43 = (double)(4.0f / 3.0f);   // Fortran 4./3. is a default-REAL quotient
     const double mu = c.chg_mu_ions;
     const double as_He_ions = (double)1.14f, as_He_el = (double)1.16f;   // REAL*4 literals
     for (int r = 0; r < rows; ++r) {
@@ -575,23 +576,25 @@ void build_charge_tables(const shark_gpu_config& c, const Columns& col, int nx_m
         tr[4] = 1.0 / as_He_el * ((kMel + 2.0 * kMH) / (2.0 * kMH)) / tr[6];
         tr[5] = 1.0 / as_He_ions * ((mu * kMH + 2.0 * kMH) / (2.0 * kMH)) / tr[7];
         for (int k = 0; k < N; ++k) {
-            const double lk = c.dust_size[k] * ul;
+            const size_t e = (size_t)k * rows + r;
+            const double sk = c.dust_size[k], lk = sk * ul;
+            const double m = (f43 * kPi * c.rhograin * (sk * sk * sk)) * um;
             const double tau = lk * kKB * T / (kEl * kEl);
-            h[off[2] + (size_t)r * N + k] = tau;
-            h[off[3] + (size_t)r * N + k] = std::sqrt(8.0 / (kPi * tau));
-            h[off[7] + (size_t)r * N + k] = 1.0 / tau;
+            h[off[2] + e] = tau;
+            h[off[3] + e] = std::sqrt(8.0 / (kPi * tau));
+            h[off[4] + e] = kPi * (lk * lk) / tau;
+            h[off[5] + e] = ud / m * tau;
         }
     }
-    const double f43 = (double)(4.0f / 3.0f);   // Fortran 4./3. is a default-REAL quotient
     for (int k = 0; k < N; ++k) {
         const double sk = c.dust_size[k], lk = sk * ul;
-        h[off[4] + k] = lk * lk;
-        h[off[5] + k] = (f43 * kPi * c.rhograin * (sk * sk * sk)) * um;
-        h[off[6] + k] = std::sqrt(kPi * c.gamma / 8.0) * (c.rhograin * ud) * (lk);
-        h[off[8] + k] = ud / h[off[5] + k];
-        h[off[9] + k] = 1.0 / h[off[5] + k];
-        h[off[10] + k] = kPi * h[off[4] + k];
+        h[off[6] + k] = lk * lk;
+        h[off[7] + k] = (f43 * kPi * c.rhograin * (sk * sk * sk)) * um;
+        h[off[8] + k] = ud / h[off[7] + k];
+        h[off[9] + k] = h[off[8] + k] * (kPi * h[off[6] + k]);
+        h[off[10] + k] = std::sqrt(kPi * c.gamma / 8.0) * (c.rhograin * ud) * lk / h[off[7] + k];
     }
+    cv.rows = rows;
     cv.t_per_col = disk ? 1 : 0;
     cv.analytical = (c.chg_mode & SHARK_CHARGE_ANALYTICAL) ? 1 : 0;
     cv.smallr = c.smallr;
@@ -1267,27 +1270,27 @@ int32_t shark_gpu_init(const shark_gpu_config* cfg, shark_gpu_ctx** out) {
         INIT_TRY(cudaMalloc(&c->chg_tables, h.size() * sizeof(double)));
         INIT_TRY(cudaMemcpy(c->chg_tables, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
         v.chg.hs = c->chg_tables + off[0]; v.chg.trow = c->chg_tables + off[1]; v.chg.tau = c->chg_tables + off[2];
-        v.chg.alpha = c->chg_tables + off[3]; v.chg.l2 = c->chg_tables + off[4]; v.chg.mkum = c->chg_tables + off[5];
-        v.chg.ak = c->chg_tables + off[6];
-        v.chg.rtau = c->chg_tables + off[7]; v.chg.nfac = c->chg_tables + off[8];
-        v.chg.rmk = c->chg_tables + off[9]; v.chg.pl2 = c->chg_tables + off[10];
+        v.chg.alpha = c->chg_tables + off[3]; v.chg.ptau = c->chg_tables + off[4]; v.chg.ntau = c->chg_tables + off[5];
+        v.chg.l2 = c->chg_tables + off[6]; v.chg.mkum = c->chg_tables + off[7]; v.chg.nfac = c->chg_tables + off[8];
+        v.chg.npl = c->chg_tables + off[9]; v.chg.wk = c->chg_tables + off[10];
         {
-            // FP32 copy for the mixed path, per temperature row and species: (alpha, 1/tau,
-            // pi l^2/tau, tau), (unit_d/m, pi l^2, 1/m, sqrt(pi gamma/8) rhograin l)
-            const int N = cfg->ndust, rows = v.chg.t_per_col ? v.nx_max : 1;
+            // FP32 copy for the mixed path: (alpha, 1/tau, pi l^2/tau, tau) at (2 k) * rows + row and
+            // (unit_d/m, pi l^2, 1/m, sqrt(pi gamma/8) rhograin l) at (2 k + 1) * rows + row
+            const int N = cfg->ndust, rows = v.chg.rows;
             std::vector<float> tf((size_t)rows * N * 8);
             for (int r = 0; r < rows; ++r)
                 for (int k = 0; k < N; ++k) {
-                    float* e = &tf[((size_t)r * N + k) * 8];
-                    const double tau = h[off[2] + (size_t)r * N + k];
-                    e[0] = (float)h[off[3] + (size_t)r * N + k];
-                    e[1] = (float)h[off[7] + (size_t)r * N + k];
-                    e[2] = (float)(h[off[10] + k] / tau);
-                    e[3] = (float)tau;
-                    e[4] = (float)h[off[8] + k];
-                    e[5] = (float)h[off[10] + k];
-                    e[6] = (float)h[off[9] + k];
-                    e[7] = (float)h[off[6] + k];
+                    float* e = &tf[((size_t)2 * k * rows + r) * 4];
+                    float* f = &tf[((size_t)(2 * k + 1) * rows + r) * 4];
+                    const size_t t = (size_t)k * rows + r;
+                    e[0] = (float)h[off[3] + t];
+                    e[1] = (float)(1.0 / h[off[2] + t]);
+                    e[2] = (float)h[off[4] + t];
+                    e[3] = (float)h[off[2] + t];
+                    f[0] = (float)h[off[8] + k];
+                    f[1] = (float)(kPi * h[off[6] + k]);
+                    f[2] = (float)(1.0 / h[off[7] + k]);
+                    f[3] = (float)(h[off[10] + k] * h[off[7] + k]);
                 }
             INIT_TRY(cudaMalloc(&c->chg_tf, tf.size() * sizeof(float)));
             INIT_TRY(cudaMemcpy(c->chg_tf, tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice));
