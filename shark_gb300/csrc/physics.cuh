@@ -59,21 +59,22 @@ __device__ __forceinline__ float limit_mc_f(float l, float r) {
 // FP64 forms of the limiters, bit for bit those of slope_limiters.f90's operations with fewer FP64
 // instructions:
 // compares and sign choices on the bit patterns, 1.5 min(|l|, |r|) for the smaller of the two
-// products (rounding keeps their order), one division by half the sum for 2 l r / (l + r).
+// products (rounding keeps their order), one division by half the sum for 2 l r / (l + r).  What is
+// not a number comes out as those operations leave it.
 __device__ __forceinline__ double limit_minmod_d(double l, double r) {
     const double s = abs_less(r, l) ? r : l;
-    return signs_differ(l, r) ? 0.0 : s;
+    return is_nan(l) || is_nan(r) ? l : signs_differ(l, r) ? 0.0 : s;
 }
 __device__ __forceinline__ double limit_vl_d(double l, double r) {
-    const double b = 0.5 * (l + r);
-    const double s = div64(l * r, b, rcp64(b));
-    return no_common_sign(l, r) ? 0.0 : s;
+    const double b = 0.5 * (l + r), a = l * r;
+    const double s = div64(a, b, rcp64(b));
+    return is_zero(a) || is_neg(a) ? 0.0 : s;
 }
 __device__ __forceinline__ double limit_mc_d(double l, double r) {
     const double c = 0.5 * (l + r);
     const double m = 1.5 * abs64(abs_less(r, l) ? r : l);
     const double s = abs_less(m, c) ? m : c;
-    return no_common_sign(l, r) ? 0.0 : with_sign(s, c);
+    return is_nan(c) ? c : no_common_sign(l, r) ? 0.0 : with_sign(s, c);
 }
 
 // Compile-time limiter choice (0 = first order) for kernels specialised per configuration.
@@ -196,7 +197,7 @@ __device__ __forceinline__ GasFlux<double> gas_hll_d(double gamma, double y1, do
                                                      double csl, double csr) {
     const double El = gas_energy_d(gamma - 1.0, y1, rl, ul, vl, wl, Pl), Er = gas_energy_d(gamma - 1.0, y1, rr, ur, vr, wr, Pr);
     const double ml = rl * ul, mr = rr * ur, cm = max64(csl, csr);
-    const double Sl = min64(min64(ul, ur) - cm, 0.0), Sr = max64(max64(ul, ur) + cm, 0.0);
+    const double Sl = min64_0(min64(ul, ur) - cm), Sr = max64_0(max64(ul, ur) + cm);
     const double ss = Sr * Sl, b = Sr - Sl, y = rcp64(b);
     GasFlux<double> f;
     f.rho = div64(Sr * ml - Sl * mr + ss * (rr - rl), b, y);
@@ -213,7 +214,7 @@ __device__ __forceinline__ GasFlux<double> gas_hllc_d(double gamma, double y1, d
                                                       double Pl, double rr, double ur, double vr, double wr, double Pr,
                                                       double csl, double csr) {
     const double cm = max64(csl, csr);
-    const double Sl = min64(min64(ul, ur) - cm, 0.0), Sr = max64(max64(ul, ur) + cm, 0.0);
+    const double Sl = min64_0(min64(ul, ur) - cm), Sr = max64_0(max64(ul, ur) + cm);
     const double hl = rl * (ul - Sl), hr = rr * (Sr - ur);
     const double b = hr + hl, y = rcp64(b);
     const double us = div64(hr * ur + hl * ul + (Pl - Pr), b, y);
@@ -242,16 +243,15 @@ __device__ __forceinline__ DustFlux<double> dust_hb_d(double rl, double ul, doub
                                                       double vr, double wr) {
     const bool takeL = is_pos(ul) && !is_zero(ur), takeR = is_neg(ur) && !is_zero(ul);
     const double rho = takeL ? rl : rr, u = takeL ? ul : ur, v = takeL ? vl : vr, w = takeL ? wl : wr;
-    const double m = rho * u;
-    DustFlux<double> f{m, rho * sq(u), m * v, m * w};
+    const bool any = takeL || takeR;
+    const double m = any ? rho * u : 0.0;
+    DustFlux<double> f{m, any ? rho * sq(u) : 0.0, m * v, m * w};
     if (takeL && takeR) {   // converging: the right side's flux on top
         const double mr = rr * ur;
         f.rho = f.rho + mr;
         f.mn = f.mn + rr * sq(ur);
         f.mt = f.mt + mr * vr;
         f.mz = f.mz + mr * wr;
-    } else if (!takeL && !takeR) {
-        f = {0.0, 0.0, 0.0, 0.0};
     }
     return f;
 }
@@ -267,7 +267,7 @@ __device__ __forceinline__ DustFlux<double> dust_llf_d(double rl, double ul, dou
 }
 __device__ __forceinline__ DustFlux<double> dust_hll_d(double rl, double ul, double vl, double wl, double rr, double ur,
                                                        double vr, double wr) {
-    const double Sl = min64(min64(ul, ur), 0.0), Sr = max64(max64(ul, ur), 0.0), b = Sr - Sl;
+    const double Sl = min64_0(min64(ul, ur)), Sr = max64_0(max64(ul, ur)), b = Sr - Sl;
     DustFlux<double> f{0.0, 0.0, 0.0, 0.0};
     if (!is_zero(b)) {
         const double y = rcp64(b), ss = Sr * Sl, ml = rl * ul, mr = rr * ur;
@@ -281,7 +281,7 @@ __device__ __forceinline__ DustFlux<double> dust_hll_d(double rl, double ul, dou
 __device__ __forceinline__ DustFlux<double> dust_hllc_d(double rl, double ul, double vl, double wl, double rr, double ur,
                                                         double vr, double wr, double csl, double csr) {
     const double cm = max64(csl, csr);
-    const double Sl = min64(min64(ul, ur) - cm, 0.0), Sr = max64(max64(ul, ur) + cm, 0.0);
+    const double Sl = min64_0(min64(ul, ur) - cm), Sr = max64_0(max64(ul, ur) + cm);
     const double hl = rl * (ul - Sl), hr = rr * (Sr - ur);
     const double b = hr + hl, y = rcp64(b);
     const double us = div64(hr * ur + hl * ul, b, y);

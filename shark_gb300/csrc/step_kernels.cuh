@@ -1036,7 +1036,7 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
                     u[ix_] = R(by_a((double)u[ix_]) + by_rhon(w * pnx) * rd);
                     u[iy_] = R(by_a((double)u[iy_]) + by_rhon(w * pny) * rd);
                     u[iz_] = R(by_a((double)u[iz_]) + by_rhon(w * pnz) * rd);
-                    if (less_num(rd, fl)) u[ir] = R(fl);
+                    if (is_less(rd, fl)) u[ir] = R(fl);
                 }
                 if (br) {
                     px = by_rhon(pnx) * rho;
@@ -1139,30 +1139,30 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
             const double vdy = by_rd((double)u[uidx(p, 5 + 2 * N + k, gy, gx)]);
             const double vdz = by_rd((double)u[uidx(p, 5 + 3 * N + k, gy, gx)]);
             vv = abs64(vdx) + abs64(vdy) + abs64(vdz);
-            vmax = less_num(vv, vmax) ? vmax : vv;
+            vmax = is_less(vv, vmax) ? vmax : vv;
             if (fk_si) {
                 const double f1 = tide - om2 * vdz;
                 const double f3 = om2 * vdx;
                 const double fm = f1 * f1 + f3 * f3;
-                fmax_d = less_num(fm, fmax_d) ? fmax_d : fm;
+                fmax_d = is_less(fm, fmax_d) ? fmax_d : fm;
             }
-            if (!is_pos_num(rd)) st |= SHARK_STATUS_NEG_DENSITY;
+            if (!is_pos(rd)) st |= SHARK_STATUS_NEG_DENSITY;
             if (!is_finite(vdx) || !is_finite(vdy) || !is_finite(vdz)) st |= SHARK_STATUS_NAN;
         }
         if (fk_si) fmax_d = sqrt(fmax_d);
         const double cd = cfl * dxx;
         // plain divisions where a wave speed may be zero or its square underflow
         const double c1 = cd / abs64(vmax);
-        dtc = less_num(2e44, c1) ? 2e44 : c1;
+        dtc = is_less(2e44, c1) ? 2e44 : c1;
         if (fk && !is_zero(vv)) {
             double fratio = fmax_d * dxx / (vv * vv);
             fratio = max64_pos(fratio, 1e-3);
             const double c2 = Over<double>(fratio)(cd / vv * (sqrt(1.0 + 2.0 * cfl * fratio) - 1.0));
-            dtc = less_num(dtc, c2) ? dtc : c2;
+            dtc = is_less(dtc, c2) ? dtc : c2;
         }
-        if (!is_pos_num(rho)) st |= SHARK_STATUS_NEG_DENSITY;
+        if (!is_pos(rho)) st |= SHARK_STATUS_NEG_DENSITY;
         if (!is_finite(vx) || !is_finite(vy) || !is_finite(vz) || !is_finite(rho)) st |= SHARK_STATUS_NAN;
-        if (!is_pos_num(dtc) || !is_finite(dtc)) { st |= SHARK_STATUS_DT_UNDERFLOW; dtc = 2e44; }
+        if (!is_pos(dtc) || !is_finite(dtc)) { st |= SHARK_STATUS_DT_UNDERFLOW; dtc = 2e44; }
     }
     if (MODE == 2) return;
     block_reduce_dt(dtc, st, p.dt_next, p.status);

@@ -31,3 +31,17 @@ def test_isothermal_forced_box(n, ndust, slope, solver, solverdust):
     assert st == 0
     np.testing.assert_allclose(dtg, dto, rtol=1e-14, atol=0)
     assert rel_l1(cfg, ug, uo).max() <= FP64_TOL
+
+
+@pytest.mark.parametrize("n,ndust", [(9, 1), (31, 3)])
+@pytest.mark.parametrize("slope,solver,solverdust", [(1, 2, 0), (2, 1, 2), (3, 0, 1), (1, 0, 2), (3, 2, 0)])
+def test_not_a_number_spreads_as_in_the_oracle(n, ndust, slope, solver, solverdust):
+    # an odd box has the star's softened offsets 0/0 in its middle cell; what is not a number takes
+    # the cells of its stencil that the operations take it to, and no others (one step: the cells that
+    # are not numbers count differently in the two time steps)
+    cfg, u0 = setups.disk_cart(n=n, ndust=ndust, slope_type=slope)
+    cfg.solver, cfg.solverdust = solver, solverdust
+    assert not np.isfinite(u0).all()
+    dto, dtg, uo, ug, st = run_pair(cfg, u0, 1)
+    assert st != 0
+    np.testing.assert_array_equal(np.isfinite(ug), np.isfinite(uo))
