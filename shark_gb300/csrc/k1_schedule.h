@@ -37,7 +37,10 @@ constexpr int K1_STRIP_UX = 60;
 //   phases x (rows per piece + K1_PIECE_ROWS) x the class's weight per row (gas 6 isothermal or
 //   8 adiabatic, dust 4),
 //   K1_PIECE_ROWS standing for a piece's halo rows and its ring refill, pieces of at most
-//   K1_MAX_ROWS rows unless that needs more phases and of at least K1_MIN_ROWS rows.  On the SI box
+//   K1_MAX_ROWS rows unless that needs more phases and of at least K1_MIN_ROWS rows: a box too
+//   small for the wave is as long as one warp's march, so its pieces are as short as can be (2
+//   against 16 rows: SI 128^2 x 8 0.0236 -> 0.0123 ms, 256^2 x 8 0.0248 -> 0.0171, KH 500 x 301 x 4
+//   0.0437 -> 0.0211; 4 rows 0.0128, 0.0170, 0.0235).  On the SI box
 //   (1024^2, 8 species: 32-row strips are 2.13 waves) this is 14 dust pieces of 73 rows and 23 gas
 //   pieces of 44.5 rows per column block, 2430 warps (K1 0.1085 -> 0.1020 ms).
 // Rows reach the strips through a per-warp ring of TMA stages in dynamic shared memory (K1_R rows
@@ -52,7 +55,7 @@ struct K1Work {
 };
 // weights per row: isothermal gas, adiabatic gas (it carries the pressure and the energy), dust
 // species (measured best of 5-9 on the SI box, of 6 and 8 on the adiabatic dusty KH box)
-constexpr int K1_WG_ISO = 6, K1_WG_ADI = 8, K1_WD = 4, K1_PIECE_ROWS = 4, K1_MIN_ROWS = 16, K1_MAX_ROWS = 128,
+constexpr int K1_WG_ISO = 6, K1_WG_ADI = 8, K1_WD = 4, K1_PIECE_ROWS = 4, K1_MIN_ROWS = 2, K1_MAX_ROWS = 128,
               K1_WAVES = 8;
 
 // `warps`: the warps of one wave (SMs x resident blocks x warps per block); `iso`: the gas is
