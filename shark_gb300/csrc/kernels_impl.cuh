@@ -316,23 +316,16 @@ static cudaError_t strip_launch(const DeviceView& v, KParams<R> p) {
 
 // K3: FARGO remap of p.u_next into `dst` (polar disk with FARGO only)
 template <typename R>
-static cudaError_t fargo_launch(const KParams<R>& p, R* dst, cudaStream_t st) {
-    const size_t smem = Fargo<R>::smem_bytes(p.ny);
-    dim3 grid((p.nx + Fargo<R>::W - 1) / Fargo<R>::W, p.nvar, 1);
-    cudaError_t e = cudaSuccess;
+static cudaError_t fargo_launch(const KParams<R>& p, FargoShift<R>* tab, R* dst, cudaStream_t st) {
+    k_fargo_shift<R><<<(p.nx + 63) / 64, 64, 0, st>>>(p, tab);
+    const int rows = FARGO_ROWS * FARGO_WARPS;
+    const dim3 grid((p.nx + 31) / 32, (p.ny + rows - 1) / rows, p.nvar), block(32, FARGO_WARPS);
     switch (p.slope_type) {
-#define SHARK_FARGO_CASE(ST)                                                                       \
-    case ST:                                                                                      \
-        e = cudaFuncSetAttribute(k_fargo<R, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        if (e == cudaSuccess) k_fargo<R, ST><<<grid, Fargo<R>::THREADS, smem, st>>>(p, p.u_next, dst);  \
-        break;
-        SHARK_FARGO_CASE(0)
-        SHARK_FARGO_CASE(1)
-        SHARK_FARGO_CASE(2)
-        default: SHARK_FARGO_CASE(3)
-#undef SHARK_FARGO_CASE
+        case 0: k_fargo<R, 0><<<grid, block, 0, st>>>(p, tab, p.u_next, dst); break;
+        case 1: k_fargo<R, 1><<<grid, block, 0, st>>>(p, tab, p.u_next, dst); break;
+        case 2: k_fargo<R, 2><<<grid, block, 0, st>>>(p, tab, p.u_next, dst); break;
+        default: k_fargo<R, 3><<<grid, block, 0, st>>>(p, tab, p.u_next, dst);
     }
-    if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
 
@@ -357,7 +350,7 @@ cudaError_t launch_step(const DeviceView& v, int slot) {
     if (e != cudaSuccess) return e;
     if (v.nbuf == 3) {   // fargo_scheme after source_terms (solve.f90:105), into the third buffer
         R* dst = (R*)v.u[(v.cur + 2) % 3];
-        if ((e = fargo_launch<R>(p, dst, v.stream)) != cudaSuccess) return e;
+        if ((e = fargo_launch<R>(p, (FargoShift<R>*)v.fargo, dst, v.stream)) != cudaSuccess) return e;
         p.u_next = dst;
     }
     if (v.time_kernels) cudaEventRecord(v.ev[2], v.stream);

@@ -53,6 +53,12 @@ struct StepPost {
     long long step;
 };
 
+// Longest FARGO ring taken: what one block's shared memory holds as rows of 64 bytes.
+constexpr int FARGO_MAX_NY = 200 * 1024 / 64;
+// One column's FARGO shift in a step: the first output row's lower donor row and the weights of the
+// donors' values and slopes.
+template <typename R> struct FargoShift { R w0, w1, c1, c2; int off; };
+
 // Device-side view of a context, shared by both precisions.  Metric arrays come in two copies:
 // `m` in the state precision (flux/update) and `md` in FP64 (drag, courant).
 struct DeviceView {
@@ -70,6 +76,7 @@ struct DeviceView {
                                 // disk relaxation time (0 outside r_relax), hs = sqrt(2 pi) H,
                                 // vk the FARGO orbital velocity
     const double* dK;           // per-species constants (device)
+    void* fargo;                // FargoShift per column (with FARGO)
     const double* dtstop;
     const double* dsize;
     const double* dstokes;

@@ -83,6 +83,7 @@ struct shark_gpu_ctx {
     bool have_uinit = false;
     void* metrics = nullptr;         // 13 arrays x nx_max in state precision
     double* metrics_d = nullptr;     // 9 arrays x nx_max FP64
+    void* fargo = nullptr;           // DeviceView::fargo
     double* species = nullptr;       // dK | dtstop | dsize | dstokes | dinvts (5 x SHARK_MAX_DUST)
     double* dt_slots = nullptr;      // [2]
     unsigned int* status = nullptr;
@@ -491,9 +492,8 @@ int32_t validate(const shark_gpu_config* c) {
         // the orbital velocity is defined by the disk setups only (allocate_init.f90:109-111)
         if (c->setup != SHARK_SETUP_DISK_POLAR)
             return fail(SHARK_ERR_UNSUPPORTED, "FARGO needs the polar disk setup");
-        const size_t ring = (size_t)c->ny * (c->precision == SHARK_PREC_MIXED ? 16 * 4 : 8 * 8);
-        if (ring > 200 * 1024)
-            return fail(SHARK_ERR_UNSUPPORTED, "FARGO ring of %d cells exceeds one CTA's shared memory", c->ny);
+        if (c->ny > shark::FARGO_MAX_NY)
+            return fail(SHARK_ERR_UNSUPPORTED, "FARGO ring of %d cells exceeds the limit of %d", c->ny, shark::FARGO_MAX_NY);
     }
     if (c->setup == SHARK_SETUP_SI && c->ndust > 0 && !(f & SHARK_FLAG_DRAG) && (f & SHARK_FLAG_FORCE_KICK))
         return fail(SHARK_ERR_UNSUPPORTED, "SI explicit drag forces (drag=.false.) are not built");
@@ -862,6 +862,7 @@ int32_t release(shark_gpu_ctx* c) {
     if (c->status) cudaFree(c->status);
     if (c->coef) cudaFree(c->coef);
     if (c->post) cudaFreeHost(c->post);
+    if (c->fargo) cudaFree(c->fargo);
     if (c->stamps) cudaFree(c->stamps);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
@@ -1227,6 +1228,8 @@ int32_t shark_gpu_init(const shark_gpu_config* cfg, shark_gpu_ctx** out) {
         INIT_TRY(cudaMemcpy(c->metrics_d, hd.data(), hd.size() * sizeof(double), cudaMemcpyHostToDevice));
         for (int a = 0; a < 9; ++a) v.md[a] = c->metrics_d + a * ncol;
     }
+    if (cfg->flags & SHARK_FLAG_FARGO) INIT_TRY(cudaMalloc(&c->fargo, ncol * sizeof(shark::FargoShift<double>)));
+    v.fargo = c->fargo;
     INIT_TRY(cudaMalloc(&c->species, 5 * SHARK_MAX_DUST * sizeof(double)));
     float invf[SHARK_MAX_DUST] = {0};   // FP32 copy of 1/C_k for the mixed path's coefficients
     {
