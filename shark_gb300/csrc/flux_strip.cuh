@@ -20,8 +20,7 @@
 namespace shark {
 
 constexpr int STRIP_UX = 28;     // columns updated per warp
-constexpr int STRIP_H = 32;      // rows updated per warp on the mixed path (strip_heights on the FP64 path)
-constexpr int STRIP_WARPS = 4;   // warps per CTA (along y) on the mixed path, one on the FP64 path
+constexpr int STRIP_F_GAS = 16, STRIP_F_DUST = 20;   // resident warps an SM on the mixed path (128 and 96 registers)
 
 template <typename R>
 __device__ __forceinline__ R shfl_up1(R v) { return __shfl_up_sync(0xffffffffu, v, 1); }
@@ -484,15 +483,14 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
 }
 
 // Gas and dust run as separate kernels so the dust warps (N of every N+1) are not held to the
-// register footprint of the 5-variable gas path with its HLLC solver.  FP64: 10 dust warps an SM
-// (192 registers); 12 at 168 registers measured the same (the FP64 pipe is the bound).
+// register footprint of the 5-variable gas path with its HLLC solver.  One strip a block, so that a
+// strip's end makes room for the next at once.  FP64: 10 dust warps an SM (192 registers); 12 at 168
+// registers measured the same (the FP64 pipe is the bound).  Mixed: 16 gas warps an SM in place of 12
+// (147 registers) took the adiabatic 1000^2 gas from 47 to 42 us.
 template <typename R, bool IS_GAS, int ST, int SOLV>
-__global__ void __launch_bounds__(std::is_same<R, float>::value ? 32 * STRIP_WARPS : 32,
-                                  std::is_same<R, float>::value ? (IS_GAS ? 1 : 5) : (IS_GAS ? 8 : 10))
+__global__ void __launch_bounds__(32, std::is_same<R, float>::value ? (IS_GAS ? STRIP_F_GAS : STRIP_F_DUST) : (IS_GAS ? 8 : 10))
 k_flux_strip(KParams<R> p) {
-    const int warp = threadIdx.x >> 5;
-    const int bx = blockIdx.x;
-    const int by = blockIdx.y * (blockDim.x >> 5) + warp;
+    const int bx = blockIdx.x, by = blockIdx.y;
     const int s = IS_GAS ? 0 : blockIdx.z + 1;
     flux_strip<R, IS_GAS, ST, SOLV>(p, s, bx, by);
 }

@@ -23,6 +23,7 @@
 namespace shark {
 
 constexpr int STRIP2_UX = K1_STRIP_UX;   // columns updated per warp
+constexpr int K1_WARPS = 4;               // warps per block
 
 __device__ __forceinline__ float2 bc2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
@@ -329,7 +330,7 @@ struct K1Maps {
 
 constexpr int K1_R = K1_TMA_ROWS, K1_NST = K1_TMA_STAGES;
 using K1Ring = RingSize<K1_R, K1_NST, 5>;
-constexpr int K1_SMEM = STRIP_WARPS * (K1Ring::ring_bytes + K1Ring::bar_bytes);
+constexpr int K1_SMEM = K1_WARPS * (K1Ring::ring_bytes + K1Ring::bar_bytes);
 
 // The pieces of warp i of a class (K1Class): k1_piece (k1_schedule.h) for every phase with such a
 // block; calls strip(block, first row, last row) (active-row numbering from 0) until one fails.
@@ -348,15 +349,15 @@ template <int NV> using K1Rows = TmaRows<NV, K1_R, K1_NST>;
 // ISO: the gas is isothermal (p.iso == 1); compiled apart so that each instance inlines one gas
 // strip (both in one kernel spill registers).
 template <int ST, int GSOLV, bool ISO>
-__global__ void __launch_bounds__(32 * STRIP_WARPS, SHARK_K1_MINBLOCKS)
+__global__ void __launch_bounds__(32 * K1_WARPS, SHARK_K1_MINBLOCKS)
     k_flux_strip_mixed(const __grid_constant__ K1Maps maps, const __grid_constant__ KParams<float> p, K1Work wk) {
     extern __shared__ __align__(128) unsigned char k1_smem[];
     const int warp = threadIdx.x >> 5;
-    const int w = blockIdx.x * STRIP_WARPS + warp;
+    const int w = blockIdx.x * K1_WARPS + warp;
     if (w >= wk.g.n + wk.d.n) return;   // whole warps; the kernel has no block-wide barrier
     RingArgs ra;
     ra.ring = reinterpret_cast<float*>(k1_smem + warp * K1Ring::ring_bytes);
-    ra.bar = reinterpret_cast<uint64_t*>(k1_smem + STRIP_WARPS * K1Ring::ring_bytes + warp * K1Ring::bar_bytes);
+    ra.bar = reinterpret_cast<uint64_t*>(k1_smem + K1_WARPS * K1Ring::ring_bytes + warp * K1Ring::bar_bytes);
     const int ng = p.ng;
     if (w < wk.g.n) {
         ra.map = &maps.gas;

@@ -199,13 +199,9 @@ static cudaError_t line_launch(const KParams<R>& p, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Warps (strips, along y) per block of the column march.
-template <typename R>
-constexpr int strip_warps() { return std::is_same<R, float>::value ? STRIP_WARPS : 1; }
-
 template <typename R, bool IS_GAS, int ST, int SOLV>
 static void strip_kernel(const KParams<R>& p, dim3 grid, cudaStream_t st) {
-    k_flux_strip<R, IS_GAS, ST, SOLV><<<grid, 32 * strip_warps<R>(), 0, st>>>(p);
+    k_flux_strip<R, IS_GAS, ST, SOLV><<<grid, 32, 0, st>>>(p);
 }
 
 template <typename R, bool IS_GAS, int ST>
@@ -245,7 +241,7 @@ static void strip_dispatch(const KParams<R>& p, dim3 grid, cudaStream_t st) {
 struct StripHeights {
     int gas, dust;
 };
-inline StripHeights strip_heights(int nbx, int ny, int ndust, int nsm) {
+inline StripHeights strip_heights_d(int nbx, int ny, int ndust, int nsm) {
     constexpr double GAS_ROWS = 1.6;
     StripHeights best{ny, ny};
     double least = 0.0;
@@ -261,22 +257,42 @@ inline StripHeights strip_heights(int nbx, int ny, int ndust, int nsm) {
     return best;
 }
 
+// The same on the mixed path, which a row's latency bounds where warps are few (a row takes one warp
+// alone 1.4 us, four of a partition 2.2 us) and the issue of instructions where they are many: the
+// shortest strips whose warps are all resident at once, so that small boxes fill the GPU, and at
+// most 32 rows, which waste little on halo rows.  A row of gas takes longer than one of dust: gas
+// strips of a quarter of the dust's rows end with them.  Against 32-row strips in blocks of four
+// warps (us): adiabatic gas 1000^2 56 -> 42, 450^2 50 -> 18, 200^2 50 -> 13; Cartesian disk of 4
+// species 512^2 61 -> 35, 128^2 54 -> 13; polar disk of 16 species 512 x 1024 246 -> 232,
+// 128 x 256 58 -> 33.
+inline StripHeights strip_heights_f(int nbx, int ny, int ndust, int nsm) {
+    constexpr int MAX_H = 32;
+    const int least = ndust > 0 ? 4 : 2;
+    auto gas = [&](int h) { return ndust > 0 ? std::max(2, h / 4) : h; };
+    for (int h = least; h < MAX_H; ++h) {
+        const double wg = (double)nbx * ((ny + gas(h) - 1) / gas(h)), wd = (double)nbx * ndust * ((ny + h - 1) / h);
+        if (wg / STRIP_F_GAS + wd / STRIP_F_DUST <= nsm) return {gas(h), h};
+    }
+    return {gas(MAX_H), MAX_H};
+}
+
 // 2D K1: the dust species on the main stream and the gas concurrently on the side stream
 // (forked and joined with events), so the small gas grid does not run alone.
 template <typename R>
 static cudaError_t strip_launch(const DeviceView& v, KParams<R> p) {
     const int nbx = (p.nx + STRIP_UX - 1) / STRIP_UX;
-    const StripHeights h = std::is_same<R, float>::value ? StripHeights{STRIP_H, STRIP_H} : strip_heights(nbx, p.ny, p.ndust, v.nsm);
+    const StripHeights h = std::is_same<R, float>::value ? strip_heights_f(nbx, p.ny, p.ndust, v.nsm)
+                                                                 : strip_heights_d(nbx, p.ny, p.ndust, v.nsm);
     auto strips = [&](int rows) {   // the grid's y for strips of that many rows
         p.strip_h = rows;
-        return (unsigned)(((p.ny + rows - 1) / rows + strip_warps<R>() - 1) / strip_warps<R>());
+        return (unsigned)((p.ny + rows - 1) / rows);
     };
     if constexpr (std::is_same<R, float>::value) {
         if (p.ndust > 0 && p.geom != 2 && p.solverdust == 0 && p.ng % 2 == 0 && v.uniform && !v.cdisk.on) {
             // mixed path, uniform Cartesian grid, Huang & Bai dust: gas and dust strips in one
             // launch (K1Work: one persistent wave, or one piece per warp when the pieces fill many waves)
             const K1Work wk = k1_work(p.nx, p.ny, p.ndust, v.k1_warps, p.iso == 1);
-            const dim3 g1((unsigned)((wk.g.n + wk.d.n + STRIP_WARPS - 1) / STRIP_WARPS), 1, 1), b1(32 * STRIP_WARPS, 1, 1);
+            const dim3 g1((unsigned)((wk.g.n + wk.d.n + K1_WARPS - 1) / K1_WARPS), 1, 1), b1(32 * K1_WARPS, 1, 1);
             const int gs = p.solver == 0 ? 0 : p.solver == 1 ? 1 : 2;
             K1Maps maps;
             maps.gas = v.k1_gas[v.cur];
@@ -520,13 +536,13 @@ template <typename R>
 int k1_resident_warps(int nsm) {
     if constexpr (std::is_same<R, float>::value) {
         int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_flux_strip_mixed<3, 2, true>, 32 * STRIP_WARPS, K1_SMEM) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_flux_strip_mixed<3, 2, true>, 32 * K1_WARPS, K1_SMEM) !=
                 cudaSuccess ||
             nb < 1) {
             cudaGetLastError();
             nb = 1;
         }
-        return nsm * nb * STRIP_WARPS;
+        return nsm * nb * K1_WARPS;
     } else {
         return 0;
     }
