@@ -362,13 +362,13 @@ __device__ __forceinline__ void block_reduce_dt_f(float dtc, unsigned int st, un
 template <typename R>
 __device__ __forceinline__ double cs_start(const KParams<R>& p, int gx, int gy) {
     if (p.iso == 1) return p.ccsd ? p.ccsd[(long long)gy * p.pitch + gx] : p.csd[gx];
-    const double rho = (double)p.u_cur[uidx(p, 0, gy, gx)];
+    const double rho = widen(p.u_cur[uidx(p, 0, gy, gx)]);
     const Over<double> by_rho(rho);
-    const double vx = by_rho((double)p.u_cur[uidx(p, 1, gy, gx)]), vy = by_rho((double)p.u_cur[uidx(p, 2, gy, gx)]);
-    const double vz = by_rho((double)p.u_cur[uidx(p, 3, gy, gx)]);
+    const double vx = by_rho(widen(p.u_cur[uidx(p, 1, gy, gx)])), vy = by_rho(widen(p.u_cur[uidx(p, 2, gy, gx)]));
+    const double vz = by_rho(widen(p.u_cur[uidx(p, 3, gy, gx)]));
     const double hr = 0.5 * rho;
     const double ekin = hr * (vx * vx) + hr * (vy * vy) + hr * (vz * vz);
-    double P = (p.gamma - 1.0) * ((double)p.u_cur[uidx(p, 4, gy, gx)] - ekin);
+    double P = (p.gamma - 1.0) * (widen(p.u_cur[uidx(p, 4, gy, gx)]) - ekin);
     P = max64_pos(P, p.smallp);
     const Over<double> by_q(max64_pos(rho, p.smallr));
     return sqrt(by_q(p.gamma * P));
@@ -1184,8 +1184,8 @@ __device__ __forceinline__ void drag_coeffs(double a, float& r, float& w) {
 }
 
 // a_k = dt/t_k of the mixed path where the per-cell stopping time factors as t_k = C_k / F_cell
-// (dustyTurb C_k = St_0,k L rho_0, F = c_s rho; the disks' Epstein F = rho/hs c_s, Epstein of an
-// adiabatic gas F = rho c_s): dt F_cell times the tabulated 1/C_k.  The dusty wave's t_k = rho_k/K_k
+// (dustyTurb C_k = St_0,k L rho_0, F = c_s rho; the disks' Epstein F = rho/hs c_s, Epstein F = rho c_s of an
+// isothermal gas): dt F_cell times the tabulated 1/C_k.  The dusty wave's t_k = rho_k/K_k
 // divides per species.
 __device__ __forceinline__ double drag_cell_factor(const KParams<float>& p, double dt, double qrho_old, int gx, int gy) {
     if (p.setup == SHARK_SETUP_DUSTYTURB) return dt * (p.csd[gx] * qrho_old);
@@ -1194,44 +1194,54 @@ __device__ __forceinline__ double drag_cell_factor(const KParams<float>& p, doub
         return dt * (qrho_old / p.chsd[e] * p.ccsd[e]);
     }
     if (p.setup == SHARK_SETUP_DISK_POLAR) return dt * (qrho_old / p.hsd[gx] * p.csd[gx]);
-    return dt * (qrho_old * cs_start(p, gx, gy));
+    return dt * (qrho_old * p.csd[gx]);
 }
 
 // Drag coefficients and drag heating (source_terms.f90:88-97) of one cell in FP64 for the setups
 // whose sound speed or stopping times need the state at the start of the step.  Bound by the FP64
-// pipe: the cell's sound speed is formed once and 1/t_k = F_cell / C_k multiplied out, for the
-// coefficients and the heating alike (adiabatic KH box 500 x 301 x 4: K2 0.289 -> 0.076 ms).
+// pipe, so the forms take few of its instructions: F_cell = rho cs = sqrt(gamma P rho) once a cell,
+// 1/t_k = F_cell / C_k multiplied out, v.(v - v_k) as (p.p/rho - p.p_k/rho_k)/rho with one quotient a
+// species, p.p/rho shared with the kinetic energy, conversions to and from floats as integer
+// instructions (adiabatic KH box 500 x 301 x 4: K2 0.076 -> 0.050 ms).
 struct DragCell {
     const KParams<float>& p;
     int cc;
-    double dt, dtF, heat, vx, vy, vz;   // heat: sum of dt v.(v - v_k)/t_k
+    double dt, dtF, w, heat, px, py, pz;   // w = p.p/rho, heat: sum of rho dt v.(v - v_k)/t_k
+    Over<double> by_rho;
     bool wave, heats;
     __device__ __forceinline__ DragCell(const KParams<float>& p_, double dt_, double qrho_old, int gx, int gy, bool heats_,
                                         bool used = true)
-        : p(p_), cc(gy * p_.pitch + gx), dt(dt_), dtF(0.0), heat(0.0), vx(0.0), vy(0.0), vz(0.0),
-          wave(p_.setup == SHARK_SETUP_DUSTYWAVE), heats(heats_) {
-        if (used && !wave) dtF = drag_cell_factor(p, dt, qrho_old, gx, gy);
-        if (heats) {
-            const Over<double> by_rho((double)p.u_cur[cc]);
-            vx = by_rho((double)p.u_cur[cc + p.plane]);
-            vy = by_rho((double)p.u_cur[cc + 2 * p.plane]);
-            vz = by_rho((double)p.u_cur[cc + 3 * p.plane]);
+        : p(p_), cc(gy * p_.pitch + gx), dt(dt_), dtF(0.0), w(0.0), heat(0.0), px(0.0), py(0.0), pz(0.0),
+          by_rho(widen(p_.u_cur[gy * p_.pitch + gx])), wave(p_.setup == SHARK_SETUP_DUSTYWAVE), heats(heats_) {
+        const bool adi = used && !wave && p.iso != 1;
+        if (adi || heats) {
+            px = widen(p.u_cur[cc + p.plane]);
+            py = widen(p.u_cur[cc + 2 * p.plane]);
+            pz = widen(p.u_cur[cc + 3 * p.plane]);
+            w = by_rho(px * px + py * py + pz * pz);
+        }
+        if (adi) {
+            const double P = max64_pos((p.gamma - 1.0) * (widen(p.u_cur[cc + 4 * p.plane]) - 0.5 * w), p.smallp);
+            dtF = dt * sqrt(p.gamma * P * qrho_old);
+        } else if (used && !wave) {
+            dtF = drag_cell_factor(p, dt, qrho_old, gx, gy);
         }
     }
-    // a_k = dt/t_k of species k, its heating added
-    __device__ __forceinline__ double operator()(int k) {
-        const int N = p.ndust;
-        const double rd = (wave || heats) ? (double)p.u_cur[cc + (5 + k) * p.plane] : 1.0;
-        const Over<double> by_rd(rd);
+    // species k's density and momenta at the start of the step, where they are needed
+    __device__ __forceinline__ float4 load(int k) const {
+        if (!wave && !heats) return make_float4(1.f, 0.f, 0.f, 0.f);
+        const float* __restrict__ u = p.u_cur + cc + (5 + k) * p.plane;
+        const long long s = p.ndust * p.plane;
+        return make_float4(u[0], u[s], u[2 * s], u[3 * s]);
+    }
+    // a_k = dt/t_k of species k, its heating added; o = load(k)
+    __device__ __forceinline__ double operator()(int k, float4 o) {
+        const Over<double> by_rd(widen(o.x));
         const double a = wave ? by_rd(dt * p.dK[k]) : dtF * p.dinvts[k];
-        if (heats) {
-            const double ux = by_rd((double)p.u_cur[cc + (5 + N + k) * p.plane]);
-            const double uy = by_rd((double)p.u_cur[cc + (5 + 2 * N + k) * p.plane]);
-            const double uz = by_rd((double)p.u_cur[cc + (5 + 3 * N + k) * p.plane]);
-            heat += a * (vx * (vx - ux) + vy * (vy - uy) + vz * (vz - uz));
-        }
+        if (heats) heat += a * (w - by_rd(px * widen(o.y) + py * widen(o.z) + pz * widen(o.w)));
         return a;
     }
+    __device__ __forceinline__ double gain() const { return by_rho(heat); }
 };
 
 // The same coefficients in FP32 from a = dt F_cell / C_k formed in FP32 (dt F_cell once per cell
@@ -1246,10 +1256,10 @@ __device__ __forceinline__ void drag_coeffs_f(float a, float& r, float& w) {
 
 __device__ __forceinline__ void drag_coeffs_mix(double a, float& r, float& w) {
     const double d = 1.0 + a;
-    if (d < 1e30) {
+    if (__double2hiint(d) < 0x46200000) {   // below 6e29, within FP32 range
         const double q = rcp_refined(d);
-        r = (float)q;
-        w = (float)(a * q);
+        r = narrow(q);
+        w = narrow(a * q);
     } else {
         drag_coeffs(a, r, w);
     }
@@ -1332,12 +1342,18 @@ k_finalize_mixed(KParams<float> p) {
                     for (int k = 0; k < NS; ++k) { rk[k] = cr[k]; wk[k] = cw[k]; }
                 } else {
                     const float rho_old = ucur[cc + (0) * pl];
-                    const double qrho_old = (double)fmaxf(rho_old, p.f_smallr);
+                    const double qrho_old = widen(fmaxf(rho_old, p.f_smallr));
                     if (direct) {
                         DragCell dc(p, dt, qrho_old, gx, gy, heats);
 #pragma unroll
-                        for (int k = 0; k < NS; ++k) drag_coeffs_mix(dc(k), rk[k], wk[k]);
-                        gain = dc.heat;
+                        for (int k0 = 0; k0 < NS; k0 += 4) {   // four species' loads in flight together
+                            float4 o[4];
+#pragma unroll
+                            for (int i = 0; i < 4 && k0 + i < NS; ++i) o[i] = dc.load(k0 + i);
+#pragma unroll
+                            for (int i = 0; i < 4 && k0 + i < NS; ++i) drag_coeffs_mix(dc(k0 + i, o[i]), rk[k0 + i], wk[k0 + i]);
+                        }
+                        gain = dc.gain();
                         heated = heats;
                     } else {
                         const float Fcf = (float)drag_cell_factor(p, dt, qrho_old, gx, gy);
@@ -1404,7 +1420,7 @@ k_finalize_mixed(KParams<float> p) {
             for (int k = 0; k < N; ++k) {
                 float r, w;
                 if (const_ts) { r = cr[k]; w = cw[k]; }
-                else if (direct) drag_coeffs_mix(dc(k), r, w);
+                else if (direct) drag_coeffs_mix(dc(k, dc.load(k)), r, w);
                 else drag_coeffs_f(Fcf * p.dinvts_f[k], r, w);
                 if (NS > 0) { rk[k < NMAX ? k : 0] = r; wk[k < NMAX ? k : 0] = w; }
                 else if (!const_ts) rw_local[k] = make_float2(r, w);
@@ -1413,7 +1429,7 @@ k_finalize_mixed(KParams<float> p) {
                 pnz += w * u[cc + (5 + 3 * N + k) * pl];
                 rhon += w * u[cc + (5 + k) * pl];
             }
-            gain = dc.heat;
+            gain = dc.gain();
             heated = direct && heats;
             const float irhon = 1.0f / rhon;
             const float vbx = pnx * irhon, vby = pny * irhon, vbz = pnz * irhon;
@@ -1448,7 +1464,7 @@ k_finalize_mixed(KParams<float> p) {
                 const double rho_old = (double)ucur[cc];
                 gain = drag_heating(p, TStop<float>(p, max64_pos(rho_old, p.smallr), gx, gy), gx, gy, dt);
             }
-            u[ie] = (float)((double)u[ie] + gain);
+            u[ie] = narrow(widen(u[ie]) + gain);
         }
     };
     auto part2 = [&]() {
