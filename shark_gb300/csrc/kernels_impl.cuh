@@ -39,6 +39,7 @@ static KParams<R> make_params(const DeviceView& v) {
     p.ou_nm = v.ou_nm;
     p.ou = v.ou;
     p.ou_modes = v.ou_modes;
+    p.ou_f = v.ou_f;
     p.box_l_y = c.box_l_y;
     p.chg_eta = (const R*)v.chg.eta;
     p.chg_gamma_d = (const R*)v.chg.gamma_d;
@@ -360,7 +361,8 @@ cudaError_t launch_step(const DeviceView& v, int slot) {
                                                       v.stamps);
     if (v.chg.on && (e = launch_charge<R>(v)) != cudaSuccess) return e;   // charge: solve.f90:36-42
     if (v.ou_nm > 0)   // this step's forcing coefficients, from the dt on the device
-        k_ou_update<<<1, 2 * v.ou_nm, 0, v.stream>>>(v.ou, v.ou_nm, p.dt, v.ou_sigma, v.ou_tcorr, v.ou_seed, v.step, v.stamps);
+        k_ou_update<<<1, 2 * v.ou_nm, 0, v.stream>>>(v.ou, v.ou_modes, v.ou_f, v.ou_nm, p.dt, v.ou_sigma, v.ou_tcorr, v.ou_seed, v.step,
+                                                     v.stamps);
     if (v.time_kernels) cudaEventRecord(v.ev[1], v.stream);
     e = (v.ndim == 2) ? strip_launch<R>(v, p) : line_launch<R>(p, v.stream);
     if (e != cudaSuccess) return e;

@@ -101,6 +101,7 @@ struct DeviceView {
     int ou_nm;
     double* ou;                 // [2 nm] coefficients (a_m, b_m)
     const double* ou_modes;     // [3 nm] k_x', k_y', |k'|
+    float* ou_f;                // [6 nm] KParams::ou_f (mixed path)
     double ou_sigma, ou_tcorr;
     unsigned long long ou_seed;
     long long step;             // 1-based number of the step being launched

@@ -106,7 +106,7 @@ struct shark_gpu_ctx {
     float* chg_seed = nullptr;       // network start points (plane layout)
     int32_t* chg_iters = nullptr;    // Newton iterations per cell (plane layout)
     double* grw_d = nullptr;         // dust growth tables (FP64)
-    double* ou_d = nullptr;          // forcing: modes [3 nm] | coefficients [2 nm]
+    double* ou_d = nullptr;          // forcing: floats [6 nm] | modes [3 nm] | coefficients [2 nm]
     std::vector<double> ou_init;     // initial coefficients (stationary law, seeded)
     std::vector<double> out_x, out_y;   // output positions of the active cells (x / radius, y)
     int32_t* grw_i = nullptr;        // dust growth target bins | net-transfer bins
@@ -1323,17 +1323,19 @@ int32_t shark_gpu_init(const shark_gpu_config* cfg, shark_gpu_ctx** out) {
     v.ou_nm = 0;
     v.ou = nullptr;
     v.ou_modes = nullptr;
+    v.ou_f = nullptr;
     if (cfg->setup == SHARK_SETUP_DUSTYTURB && cfg->turb_mach > 0.0) {
         std::vector<double> modes;
         double sigma;
         build_forcing(*cfg, modes, c->ou_init, sigma);
         const int nm = (int)modes.size() / 3;
-        INIT_TRY(cudaMalloc(&c->ou_d, (size_t)5 * nm * sizeof(double)));
-        INIT_TRY(cudaMemcpy(c->ou_d, modes.data(), modes.size() * sizeof(double), cudaMemcpyHostToDevice));
-        INIT_TRY(cudaMemcpy(c->ou_d + 3 * nm, c->ou_init.data(), c->ou_init.size() * sizeof(double), cudaMemcpyHostToDevice));
+        INIT_TRY(cudaMalloc(&c->ou_d, (size_t)8 * nm * sizeof(double)));
+        INIT_TRY(cudaMemcpy(c->ou_d + 3 * nm, modes.data(), modes.size() * sizeof(double), cudaMemcpyHostToDevice));
+        INIT_TRY(cudaMemcpy(c->ou_d + 6 * nm, c->ou_init.data(), c->ou_init.size() * sizeof(double), cudaMemcpyHostToDevice));
         v.ou_nm = nm;
-        v.ou_modes = c->ou_d;
-        v.ou = c->ou_d + 3 * nm;
+        v.ou_f = is_mixed(c) ? reinterpret_cast<float*>(c->ou_d) : nullptr;
+        v.ou_modes = c->ou_d + 3 * nm;
+        v.ou = c->ou_d + 6 * nm;
         v.ou_sigma = sigma;
         v.ou_tcorr = cfg->turb_tcorr;
         v.ou_seed = (unsigned long long)cfg->turb_seed;

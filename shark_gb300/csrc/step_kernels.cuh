@@ -47,6 +47,7 @@ struct KParams {
     GrowthDev gw;                      // dust growth tables and constants
     int ou_nm;                         // dustyTurb forcing modes (0: no forcing)
     const double* ou;                  // [2 nm] this step's coefficients
+    const float* ou_f;                 // the mixed path's table of this step: k_x', k_y', k_y'/k, k_x'/k of the modes, then the coefficients
     const double* ou_modes;            // [3 nm]
     double box_l_y;
     const R* chg_eta;                  // charging outputs: eta (3 planes), gamma_d (N planes)
@@ -958,21 +959,31 @@ static __global__ void __launch_bounds__(GROWTH_D_THREADS) k_growth_d(KParams<do
 
 // Driven-turbulence kick of the dustyTurb box (turb.f90:227-324 in 2D): the gas momentum gains
 // rho a dt with the solenoidal Ornstein-Uhlenbeck acceleration of this step at the cell centre.
-// C = double follows the oracle's operations; C = float is the mixed-precision form.
+// C = double follows the oracle's operations; C = float is the mixed-precision form, whose mode
+// table k_ou_update leaves in floats (converted by every cell, it was 70 instructions of the FP64
+// pipe for 14 modes, three times the sines' time).
 template <typename C, typename R>
 __device__ __forceinline__ void turb_kick_cell(const KParams<R>& p, R* u, int gx, int gy, double dt) {
     const C x = C(p.xposd[gx]);
-    const C y = C(((double)(float)(gy - p.ng) + 0.5) * p.box_l_y / (double)(float)p.ny);
+    const C y = C(Over<double>((double)(float)p.ny)(((double)(float)(gy - p.ng) + 0.5) * p.box_l_y));
     C ax = C(0), ay = C(0);
     for (int m = 0; m < p.ou_nm; ++m) {
-        const C kxp = C(p.ou_modes[3 * m]), kyp = C(p.ou_modes[3 * m + 1]), kk = C(p.ou_modes[3 * m + 2]);
-        const C ph = kxp * x + kyp * y;
-        C sn, cs;
-        if constexpr (sizeof(C) == 8) sincos(ph, &sn, &cs);
-        else sincosf(ph, &sn, &cs);
-        const C w = C(p.ou[2 * m]) * cs + C(p.ou[2 * m + 1]) * sn;
-        ax = ax + kyp / kk * w;
-        ay = ay - kxp / kk * w;
+        if constexpr (sizeof(C) == 8) {
+            const C kxp = p.ou_modes[3 * m], kyp = p.ou_modes[3 * m + 1], kk = p.ou_modes[3 * m + 2];
+            C sn, cs;
+            sincos(kxp * x + kyp * y, &sn, &cs);
+            const C w = p.ou[2 * m] * cs + p.ou[2 * m + 1] * sn;
+            ax = ax + kyp / kk * w;
+            ay = ay - kxp / kk * w;
+        } else {
+            const float4 k = reinterpret_cast<const float4*>(p.ou_f)[m];
+            const float2 c = reinterpret_cast<const float2*>(p.ou_f + 4 * p.ou_nm)[m];
+            C sn, cs;
+            sincosf(k.x * x + k.y * y, &sn, &cs);
+            const C w = c.x * cs + c.y * sn;
+            ax = ax + k.z * w;
+            ay = ay - k.w * w;
+        }
     }
     const C rho = C(u[uidx(p, 0, gy, gx)]);
     u[uidx(p, 1, gy, gx)] = R(C(u[uidx(p, 1, gy, gx)]) + rho * ax * C(dt));
@@ -1408,54 +1419,80 @@ k_finalize_mixed(KParams<float> p) {
                 in_regs = true;
             }
         } else if (drag) {
-            float rk[NMAX], wk[NMAX];
             float rhon = rho, pnx = px, pny = py, pnz = pz;
             const float rho_old = ucur[cc + (0) * pl];
             const double qrho_old = (double)fmaxf(rho_old, p.f_smallr);
             const float Fcf = (const_ts || direct) ? 0.f : (float)drag_cell_factor(p, dt, qrho_old, gx, gy);
             DragCell dc(p, dt, qrho_old, gx, gy, direct && heats, direct);
-            // run-time species count: the cell's coefficients are kept (thread-local memory) for
-            // the update loop instead of being formed a second time
-            float2 rw_local[NS < 0 ? SHARK_MAX_DUST : 1];
-            for (int k = 0; k < N; ++k) {
-                float r, w;
-                if (const_ts) { r = cr[k]; w = cw[k]; }
-                else if (direct) drag_coeffs_mix(dc(k, dc.load(k)), r, w);
-                else drag_coeffs_f(Fcf * p.dinvts_f[k], r, w);
-                if (NS > 0) { rk[k < NMAX ? k : 0] = r; wk[k < NMAX ? k : 0] = w; }
-                else if (!const_ts) rw_local[k] = make_float2(r, w);
-                pnx += w * u[cc + (5 + N + k) * pl];
-                pny += w * u[cc + (5 + 2 * N + k) * pl];
-                pnz += w * u[cc + (5 + 3 * N + k) * pl];
-                rhon += w * u[cc + (5 + k) * pl];
+            // Run-time species count: two passes over the cell's species, CH species' loads in flight
+            // together (a species at a time, each waited for its loads behind the one before's
+            // stores: 590 k cells of 32 species 0.27 -> 0.13 ms).  Coefficients that cost FP64 work are
+            // kept (thread-local memory) for the second pass, the others formed again.
+            constexpr int CH = 4;
+            float2 rw_local[SHARK_MAX_DUST];
+            for (int k0 = 0; k0 < N; k0 += CH) {
+                float d[CH], x[CH], y[CH], z[CH];
+                float4 o[CH];
+#pragma unroll
+                for (int i = 0; i < CH; ++i) {
+                    const int k = k0 + i;
+                    if (k >= N) break;
+                    d[i] = u[cc + (5 + k) * pl];
+                    x[i] = u[cc + (5 + N + k) * pl];
+                    y[i] = u[cc + (5 + 2 * N + k) * pl];
+                    z[i] = u[cc + (5 + 3 * N + k) * pl];
+                    if (direct) o[i] = dc.load(k);
+                }
+#pragma unroll
+                for (int i = 0; i < CH; ++i) {
+                    const int k = k0 + i;
+                    if (k >= N) break;
+                    float r, w;
+                    if (const_ts) { w = cw[k]; }
+                    else if (direct) { drag_coeffs_mix(dc(k, o[i]), r, w); rw_local[k] = make_float2(r, w); }
+                    else drag_coeffs_f(Fcf * p.dinvts_f[k], r, w);
+                    pnx += w * x[i];
+                    pny += w * y[i];
+                    pnz += w * z[i];
+                    rhon += w * d[i];
+                }
             }
             gain = dc.gain();
             heated = direct && heats;
             const float irhon = 1.0f / rhon;
             const float vbx = pnx * irhon, vby = pny * irhon, vbz = pnz * irhon;
-            for (int k = 0; k < N; ++k) {
-                float r, w;
-                if (NS > 0) { r = rk[k < NMAX ? k : 0]; w = wk[k < NMAX ? k : 0]; }
-                else if (const_ts) { r = cr[k]; w = cw[k]; }
-                else { r = rw_local[k].x; w = rw_local[k].y; }
-                const float rd = u[cc + (5 + k) * pl];
-                const long long ixx = uidx(p, 5 + N + k, gy, gx), iyy = uidx(p, 5 + 2 * N + k, gy, gx),
-                                izz = uidx(p, 5 + 3 * N + k, gy, gx);
-                const float wr = w * rd;
-                u[ixx] = u[ixx] * r + wr * vbx;
-                u[iyy] = u[iyy] * r + wr * vby;
-                u[izz] = u[izz] * r + wr * vbz;
+            const float fl = rho * p.f_dust_ratio_min;   // floor (dust_drag.f90:63-73)
+            for (int k0 = 0; k0 < N; k0 += CH) {
+                float d[CH], x[CH], y[CH], z[CH];
+#pragma unroll
+                for (int i = 0; i < CH; ++i) {
+                    const int k = k0 + i;
+                    if (k >= N) break;
+                    d[i] = u[cc + (5 + k) * pl];
+                    x[i] = u[cc + (5 + N + k) * pl];
+                    y[i] = u[cc + (5 + 2 * N + k) * pl];
+                    z[i] = u[cc + (5 + 3 * N + k) * pl];
+                }
+#pragma unroll
+                for (int i = 0; i < CH; ++i) {
+                    const int k = k0 + i;
+                    if (k >= N) break;
+                    float r, w;
+                    if (const_ts) { r = cr[k]; w = cw[k]; }
+                    else if (direct) { r = rw_local[k].x; w = rw_local[k].y; }
+                    else drag_coeffs_f(Fcf * p.dinvts_f[k], r, w);
+                    const float wr = w * d[i];
+                    u[cc + (5 + N + k) * pl] = fmaf(wr, vbx, __fmul_rn(x[i], r));
+                    u[cc + (5 + 2 * N + k) * pl] = fmaf(wr, vby, __fmul_rn(y[i], r));
+                    u[cc + (5 + 3 * N + k) * pl] = fmaf(wr, vbz, __fmul_rn(z[i], r));
+                    if (fl > d[i]) u[cc + (5 + k) * pl] = fl;
+                }
             }
             if (p.flags & SHARK_FLAG_BACK_REACTION) {
                 px = vbx * rho; py = vby * rho; pz = vbz * rho;
                 u[cc + (1) * pl] = px;
                 u[cc + (2) * pl] = py;
                 u[cc + (3) * pl] = pz;
-            }
-            const float fl = rho * p.f_dust_ratio_min;   // floor (dust_drag.f90:63-73)
-            for (int k = 0; k < N; ++k) {
-                const long long ir = uidx(p, 5 + k, gy, gx);
-                if (fl > u[ir]) u[ir] = fl;
             }
         }
         if (heats) {   // drag heating; without the drag, or with a setup's own stopping times, by itself
@@ -1602,8 +1639,9 @@ __device__ __forceinline__ double hash_uniform_d(unsigned long long seed, unsign
 
 // Ornstein-Uhlenbeck update of the forcing coefficients for step `step` (one thread each):
 // c <- f c + sigma sqrt(1 - f^2) xi with f = exp(-dt/tcorr) and a Box-Muller normal deviate.
-static __global__ void k_ou_update(double* ou, int nm, const double* dt, double sigma, double tcorr,
-                                   unsigned long long seed, long long step, unsigned long long* stamps) {
+// ou_f (mixed path): the modes' table in floats, KParams::ou_f.
+static __global__ void k_ou_update(double* ou, const double* modes, float* ou_f, int nm, const double* dt, double sigma,
+                                   double tcorr, unsigned long long seed, long long step, unsigned long long* stamps) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q == 0) stamps[1] = clock_ns();
     if (q >= 2 * nm) return;
@@ -1613,6 +1651,13 @@ static __global__ void k_ou_update(double* ou, int nm, const double* dt, double 
     const double u1 = hash_uniform_d(seed, 2 * cnt), u2 = hash_uniform_d(seed, 2 * cnt + 1);
     const double xi = sqrt(-2.0 * log(1.0 - u1)) * cos(2.0 * 3.141592653589793238462643383279 * u2);
     ou[q] = f * ou[q] + sg * xi;
+    if (ou_f) {
+        ou_f[4 * nm + q] = (float)ou[q];
+        if (q < nm) {
+            const float kx = (float)modes[3 * q], ky = (float)modes[3 * q + 1], kk = (float)modes[3 * q + 2];
+            reinterpret_cast<float4*>(ou_f)[q] = make_float4(kx, ky, ky / kk, kx / kk);
+        }
+    }
 }
 
 // It also posts the step's dt, the status word so far and then the step's number to pinned host
