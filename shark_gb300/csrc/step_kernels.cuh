@@ -121,6 +121,24 @@ __device__ __forceinline__ int svar(int s, int c, int N) {
     return s == 0 ? c : 5 + c * N + (s - 1);
 }
 
+// Values of `n` variables of one cell at a time, all loads in flight before the first store: a store
+// may alias the next load for all the compiler knows, so a loop that copies variable by variable
+// waits for memory once a variable.
+constexpr int COPY_BATCH = 8;
+template <typename R, typename L, typename S>
+__device__ __forceinline__ void in_batches(int n, L load, S store) {
+    constexpr int B = COPY_BATCH;
+    for (int v0 = 0; v0 < n; v0 += B) {
+        R val[B];
+#pragma unroll
+        for (int i = 0; i < B; ++i)
+            if (v0 + i < n) val[i] = load(v0 + i);
+#pragma unroll
+        for (int i = 0; i < B; ++i)
+            if (v0 + i < n) store(v0 + i, val[i]);
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
 // Boundaries: one thread per ghost cell.  Periodic and shear-periodic fills are done in a single
 // pass with the source at (wrap(ix), wrap(iy)); this equals the reference's two passes (y rows for
@@ -169,7 +187,7 @@ __global__ void k_boundaries(KParams<R> p, R* u) {
         // active cell of its row, phi image included, with the radial velocities clipped so that
         // nothing flows in (the reference's row-less u_prim(first_active) read as the row's cell)
         const int rx = ix < ng ? ng : (ix >= ng + nx ? ng + nx - 1 : ix);
-        for (int v = 0; v < p.nvar; ++v) u[uidx(p, v, iy, ix)] = u[uidx(p, v, sy, rx)];
+        in_batches<R>(p.nvar, [&](int v) { return u[uidx(p, v, sy, rx)]; }, [&](int v, R val) { u[uidx(p, v, iy, ix)] = val; });
         if (xg) {
             for (int k = -1; k < N; ++k) {
                 const long long i = uidx(p, k < 0 ? 1 : 5 + N + k, iy, ix);
@@ -179,15 +197,16 @@ __global__ void k_boundaries(KParams<R> p, R* u) {
         }
         return;
     }
-    for (int v = 0; v < p.nvar; ++v) u[uidx(p, v, iy, ix)] = u[uidx(p, v, sy, sx)];
+    in_batches<R>(p.nvar, [&](int v) { return u[uidx(p, v, sy, sx)]; }, [&](int v, R val) { u[uidx(p, v, iy, ix)] = val; });
     if (p.setup == SHARK_SETUP_SI && xg) {
         // shear: vz momentum -/+ rho * q * Omega * L (SI/boundaries.f90:60-74)
         const R sgn = ix < ng ? R(-1) : R(1);
         const R qsh = R(p.si_q), om = R(p.si_om), L = R(p.box_l);
-        u[uidx(p, 3, iy, ix)] = u[uidx(p, 3, sy, sx)] + sgn * (u[uidx(p, 0, sy, sx)] * qsh * om * L);
-        for (int k = 0; k < N; ++k)
-            u[uidx(p, 5 + 3 * N + k, iy, ix)] =
-                u[uidx(p, 5 + 3 * N + k, sy, sx)] + sgn * (u[uidx(p, 5 + k, sy, sx)] * qsh * om * L);
+        auto shear = [&](int k) {   // gas, then the species
+            const long long z = uidx(p, k == 0 ? 3 : 4 + 3 * N + k, sy, sx), r = uidx(p, k == 0 ? 0 : 4 + k, sy, sx);
+            return u[z] + sgn * (u[r] * qsh * om * L);
+        };
+        in_batches<R>(N + 1, shear, [&](int k, R val) { u[uidx(p, k == 0 ? 3 : 4 + 3 * N + k, iy, ix)] = val; });
     }
     (void)yg;
 }
@@ -207,91 +226,99 @@ namespace shark {
 // its floor and heating, and the rest, as two launches with k_growth_d between them (FP64).
 // ---------------------------------------------------------------------------------------------
 
-// Producer-side boundary fill: an active cell within nghost of a periodic or shear-periodic edge
-// writes its own ghost images (with the SI shear of the vz momenta for x images) from its final
-// values.  This is apply_boundaries of the next step (SI/boundaries.f90, boundary_types.f90:149-186,
-// SOD/boundaries.f90 periodic directions) done by the producer; fixed SOD ghosts never change after
-// the upload and are skipped.  Reads back this thread's own just-written values.
+// Producer-side boundary fill: the block with an active cell within nghost of a periodic or
+// shear-periodic edge writes that cell's ghost images (with the SI shear of the vz momenta for x
+// images) from its final values.  This is apply_boundaries of the next step (SI/boundaries.f90,
+// boundary_types.f90:149-186, SOD/boundaries.f90 periodic directions) done by the producer; fixed SOD
+// ghosts never change after the upload and are skipped.  Called by every thread of a block after a
+// barrier behind the cells' last writes.  The images of a row's ends are shared out among the block's
+// threads, a value each: left to the two threads of the edge cells they were nvar waits for memory,
+// in two of eight blocks of a 1024-column row (K2 in us, SI 128^2 x 8 14.7 -> 11.4, 1024^2 x 8 79 -> 66, Cartesian disk
+// 512^2 x 4 38 -> 29).
 template <typename R>
 __device__ __forceinline__ void fill_ghost_images(const KParams<R>& p, R* u, int gx, int gy) {
-    const int ng = p.ng, nx = p.nx, ny = p.ny;
+    const int ng = p.ng, nx = p.nx, ny = p.ny, N = p.ndust;
+    const int x0 = gx - threadIdx.x, x1 = min(x0 + (int)blockDim.x, ng + nx);   // the block's columns [x0, x1)
+    const bool lft = x0 == ng, rgt = x1 == ng + nx;
+    const int items = ng * p.nvar;   // of one end of the row: variable v = it / ng, column c = it % ng
     if (p.setup == SHARK_SETUP_DISK_CART) {
         // zero_gradients as written (boundary_types.f90:48-100) from the second call on: every
         // ghost takes the state of cell (first_active, 1), which no step changes (k_cdisk_ghosts
         // does the first call).  The active cells on the edge write the ghosts next to them.
-        const bool l = gx == ng, r = gx == ng + nx - 1, b = gy == ng, t = gy == ng + ny - 1;
-        if (!(l || r || b || t)) return;
-        for (int v = 0; v < p.nvar; ++v) {
-            const R val = p.cgs[v];
-            for (int g = 0; g < ng; ++g) {
-                if (b) u[uidx(p, v, g, gx)] = val;
-                if (t) u[uidx(p, v, ng + ny + g, gx)] = val;
-                if (l) u[uidx(p, v, gy, g)] = val;
-                if (r) u[uidx(p, v, gy, ng + nx + g)] = val;
-                for (int h = 0; h < ng; ++h) {   // corners, by the corner cells
-                    if (l && b) u[uidx(p, v, g, h)] = val;
-                    if (r && b) u[uidx(p, v, g, ng + nx + h)] = val;
-                    if (l && t) u[uidx(p, v, ng + ny + g, h)] = val;
-                    if (r && t) u[uidx(p, v, ng + ny + g, ng + nx + h)] = val;
-                }
-            }
-        }
-        return;
-    }
-    if (p.setup == SHARK_SETUP_DISK_POLAR) {
-        // disk_polar/boundaries.f90:1-70 by the producer: phi images of the rows next to the
-        // periodic seam; the first/last active column also writes its radial ghosts (and their
-        // phi images) with the radial velocities clipped to outflow
-        const int ty = gy < 2 * ng ? gy + ny : (gy >= ny ? gy - ny : -1);
-        const bool left = gx == ng, right = gx == ng + nx - 1;
-        if (ty < 0 && !left && !right) return;
-        const int N = p.ndust;
-        for (int v = 0; v < p.nvar; ++v) {
-            const R val = u[uidx(p, v, gy, gx)];
-            if (ty >= 0) u[uidx(p, v, ty, gx)] = val;
-            if (left || right) {
-                R xv = val;
-                if (v == 1 || (v >= 5 + N && v < 5 + 2 * N))
-                    xv = left ? (val > R(0) ? val : R(0)) : (val < R(0) ? val : R(0));
+        const bool b = gy == ng, t = gy == ng + ny - 1;
+        if (!(lft || rgt || b || t)) return;
+        if ((b || t) && gx < x1) {
+            in_batches<R>(p.nvar, [&](int v) { return p.cgs[v]; }, [&](int v, R val) {
                 for (int g = 0; g < ng; ++g) {
-                    const int col = left ? g : ng + nx + g;
-                    u[uidx(p, v, gy, col)] = xv;
-                    if (ty >= 0) u[uidx(p, v, ty, col)] = xv;
+                    if (b) u[uidx(p, v, g, gx)] = val;
+                    if (t) u[uidx(p, v, ng + ny + g, gx)] = val;
                 }
+            });
+        }
+        if (!(lft || rgt)) return;
+        for (int it = threadIdx.x; it < items; it += blockDim.x) {
+            const int v = it / ng, c = it - v * ng;
+            const R val = p.cgs[v];
+            if (lft) u[uidx(p, v, gy, c)] = val;
+            if (rgt) u[uidx(p, v, gy, ng + nx + c)] = val;
+            for (int g = 0; g < ng; ++g) {   // corners
+                if (lft && b) u[uidx(p, v, g, c)] = val;
+                if (rgt && b) u[uidx(p, v, g, ng + nx + c)] = val;
+                if (lft && t) u[uidx(p, v, ng + ny + g, c)] = val;
+                if (rgt && t) u[uidx(p, v, ng + ny + g, ng + nx + c)] = val;
             }
         }
         return;
     }
-    const bool xper = !(p.setup == SHARK_SETUP_SOD && p.sod_dir == 0);
+    const bool polar = p.setup == SHARK_SETUP_DISK_POLAR;
+    const bool xper = !polar && !(p.setup == SHARK_SETUP_SOD && p.sod_dir == 0);
     const bool yper = p.ndim == 2 && !(p.setup == SHARK_SETUP_SOD && p.sod_dir == 1);
-    int tx = -1, ty = -1;
-    if (xper) {
-        if (gx < 2 * ng) tx = gx + nx;            // source of a right ghost
-        else if (gx >= nx) tx = gx - nx;          // source of a left ghost
-    }
+    int ty = -1;   // this row's image across the periodic seam
     if (yper) {
         if (gy < 2 * ng) ty = gy + ny;
         else if (gy >= ny) ty = gy - ny;
     }
-    if (tx < 0 && ty < 0) return;
-    const bool shear = p.setup == SHARK_SETUP_SI;
-    const R sgn = (tx >= 0 && tx > gx) ? R(1) : R(-1);   // right ghost: + rho q Omega L
-    const R qoL = prm<R>(p.si_q, p.f_si_q), om = prm<R>(p.si_om, p.f_si_om), L = prm<R>(p.box_l, p.f_box_l);
-    const int N = p.ndust;
-    for (int v = 0; v < p.nvar; ++v) {
-        R val = u[uidx(p, v, gy, gx)];
-        if (ty >= 0) u[uidx(p, v, ty, gx)] = val;               // y image (no shear)
-        if (tx >= 0) {
-            R xv = val;
-            if (shear) {
-                int vr = -1;
-                if (v == 3) vr = 0;
-                else if (v >= 5 + 3 * N) vr = v - 3 * N;         // vz momentum of dust species -> its density
-                if (vr >= 0) xv = val + sgn * (u[uidx(p, vr, gy, gx)] * qoL * om * L);
+    if (ty >= 0 && gx < x1) {   // y images (no shear)
+        const int src = gy * p.pitch + gx, dst = ty * p.pitch + gx, pl = (int)p.plane;
+        in_batches<R>(p.nvar, [&](int v) { return u[src + v * pl]; }, [&](int v, R val) { u[dst + v * pl] = val; });
+    }
+    if (polar) {
+        // disk_polar/boundaries.f90:1-70 by the producer: the first (last) active column's cell in its
+        // row's radial ghosts (and their phi images) with the radial velocities clipped to outflow
+        if (!(lft || rgt)) return;
+        for (int it = threadIdx.x; it < items; it += blockDim.x) {
+            const int v = it / ng, c = it - v * ng;
+            const bool vr = v == 1 || (v >= 5 + N && v < 5 + 2 * N);
+            if (lft) {
+                R val = u[uidx(p, v, gy, ng)];
+                if (vr) val = val > R(0) ? val : R(0);
+                u[uidx(p, v, gy, c)] = val;
+                if (ty >= 0) u[uidx(p, v, ty, c)] = val;
             }
-            u[uidx(p, v, gy, tx)] = xv;                             // x image
-            if (ty >= 0) u[uidx(p, v, ty, tx)] = xv;                // corner image
+            if (rgt) {
+                R val = u[uidx(p, v, gy, ng + nx - 1)];
+                if (vr) val = val < R(0) ? val : R(0);
+                u[uidx(p, v, gy, ng + nx + c)] = val;
+                if (ty >= 0) u[uidx(p, v, ty, ng + nx + c)] = val;
+            }
         }
+        return;
+    }
+    // sources of the right ghosts: columns [ng, 2 ng); of the left ghosts: the others from column nx on
+    if (!xper || !(x0 < 2 * ng || x1 > nx)) return;
+    const bool shear = p.setup == SHARK_SETUP_SI;
+    const R qoL = prm<R>(p.si_q, p.f_si_q), om = prm<R>(p.si_om, p.f_si_om), L = prm<R>(p.box_l, p.f_box_l);
+    for (int it = threadIdx.x; it < 2 * items; it += blockDim.x) {
+        const bool left = it >= items;   // a left ghost
+        const int i = left ? it - items : it, v = i / ng, c = i - v * ng;
+        const int sx = left ? nx + c : ng + c, tx = left ? c : ng + nx + c;
+        if (sx < x0 || sx >= x1 || (left && sx < 2 * ng)) continue;
+        R val = u[uidx(p, v, gy, sx)];
+        // vz momenta of the gas and the species: -/+ rho q Omega L (right ghost: +)
+        if (shear && (v == 3 || v >= 5 + 3 * N))
+            val = val + R(left ? -1 : 1) * (u[uidx(p, v == 3 ? 0 : v - 3 * N, gy, sx)] * qoL * om * L);
+        u[uidx(p, v, gy, tx)] = val;                            // x image
+        if (ty >= 0) u[uidx(p, v, ty, tx)] = val;               // corner image
     }
 }
 
@@ -442,28 +469,40 @@ template <typename R, typename C>
 __device__ __forceinline__ bool disk_inloop_cell(const KParams<R>& p, R* u, int gx, int gy, double dt) {
     const int N = p.ndust;
     if (gx == p.ng) {
-        for (int v = 0; v < p.nvar; ++v) u[uidx(p, v, gy, gx)] = p.u_init[uidx(p, v, gy, gx)];
+        in_batches<R>(p.nvar, [&](int v) { return p.u_init[uidx(p, v, gy, gx)]; }, [&](int v, R val) { u[uidx(p, v, gy, gx)] = val; });
         return true;
     }
     const double trel = p.treld[gx];
     if (!(trel > 0.0)) return false;
     const C e = C(exp(-dt / trel));
-    for (int s = 0; s <= N; ++s) {
-        const int ir = svar(s, 0, N), ivx = svar(s, 1, N), ivy = svar(s, 2, N);
-        const C rho_init = C(p.u_init[uidx(p, ir, gy, gx)]);
-        const Over<C> by_init(rho_init);
-        const C vx_init = by_init(C(p.u_init[uidx(p, ivx, gy, gx)]));
-        const C vy_init = by_init(C(p.u_init[uidx(p, ivy, gy, gx)]));
-        const C rho_old = C(u[uidx(p, ir, gy, gx)]);
-        const Over<C> by_old(rho_old);
-        const C vx_old = by_old(C(u[uidx(p, ivx, gy, gx)]));
-        const C vy_old = by_old(C(u[uidx(p, ivy, gy, gx)]));
-        const C rho_new = (rho_init) * (C(1) - e) + rho_old * e;
-        const C vx_new = (vx_init) * (C(1) - e) + vx_old * e;
-        const C vy_new = (vy_init) * (C(1) - e) + vy_old * e;
-        u[uidx(p, ir, gy, gx)] = R(rho_new);
-        u[uidx(p, ivx, gy, gx)] = R(rho_new * vx_new);
-        u[uidx(p, ivy, gy, gx)] = R(rho_new * vy_new);
+    constexpr int CH = 4;   // species whose loads are in flight together
+    for (int s0 = 0; s0 <= N; s0 += CH) {
+        R q[CH][6];
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            if (s0 + i > N) break;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const long long e = uidx(p, svar(s0 + i, c, N), gy, gx);
+                q[i][c] = p.u_init[e];
+                q[i][3 + c] = u[e];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const int s = s0 + i;
+            if (s > N) break;
+            const C rho_init = C(q[i][0]), rho_old = C(q[i][3]);
+            const Over<C> by_init(rho_init), by_old(rho_old);
+            const C vx_init = by_init(C(q[i][1])), vy_init = by_init(C(q[i][2]));
+            const C vx_old = by_old(C(q[i][4])), vy_old = by_old(C(q[i][5]));
+            const C rho_new = (rho_init) * (C(1) - e) + rho_old * e;
+            const C vx_new = (vx_init) * (C(1) - e) + vx_old * e;
+            const C vy_new = (vy_init) * (C(1) - e) + vy_old * e;
+            u[uidx(p, svar(s, 0, N), gy, gx)] = R(rho_new);
+            u[uidx(p, svar(s, 1, N), gy, gx)] = R(rho_new * vx_new);
+            u[uidx(p, svar(s, 2, N), gy, gx)] = R(rho_new * vy_new);
+        }
     }
     return true;
 }
@@ -1035,19 +1074,31 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
                 }
                 const Over<double> by_rhon(rhon);
                 const double fl = rho * p.dust_ratio_min;   // regularisation floor (dust_drag.f90:63-73)
-                for (int k = 0; k < N; ++k) {
-                    double a;
-                    if (NS > 0) a = alpha[k < NMAX ? k : 0];
-                    else a = Over<double>(tstop(k))(dt);    // run-time species count
-                    const Over<double> by_a(1.0 + a);
-                    const double w = by_a(a);
-                    const long long ir = uidx(p, 5 + k, gy, gx), ix_ = uidx(p, 5 + N + k, gy, gx),
-                                    iy_ = uidx(p, 5 + 2 * N + k, gy, gx), iz_ = uidx(p, 5 + 3 * N + k, gy, gx);
-                    const double rd = (double)u[ir];
-                    u[ix_] = R(by_a((double)u[ix_]) + by_rhon(w * pnx) * rd);
-                    u[iy_] = R(by_a((double)u[iy_]) + by_rhon(w * pny) * rd);
-                    u[iz_] = R(by_a((double)u[iz_]) + by_rhon(w * pnz) * rd);
-                    if (is_less(rd, fl)) u[ir] = R(fl);
+                constexpr int CH = 4;   // species whose loads are in flight together
+#pragma unroll
+                for (int k0 = 0; k0 < (NS > 0 ? NS : N); k0 += CH) {
+                    double d[CH], m[CH][3];
+#pragma unroll
+                    for (int i = 0; i < CH; ++i) {
+                        if (k0 + i >= N) break;
+                        d[i] = (double)u[uidx(p, 5 + k0 + i, gy, gx)];
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) m[i][c] = (double)u[uidx(p, 5 + (c + 1) * N + k0 + i, gy, gx)];
+                    }
+#pragma unroll
+                    for (int i = 0; i < CH; ++i) {
+                        const int k = k0 + i;
+                        if (k >= N) break;
+                        double a;
+                        if (NS > 0) a = alpha[k < NMAX ? k : 0];
+                        else a = Over<double>(tstop(k))(dt);    // run-time species count
+                        const Over<double> by_a(1.0 + a);
+                        const double w = by_a(a);
+                        u[uidx(p, 5 + N + k, gy, gx)] = R(by_a(m[i][0]) + by_rhon(w * pnx) * d[i]);
+                        u[uidx(p, 5 + 2 * N + k, gy, gx)] = R(by_a(m[i][1]) + by_rhon(w * pny) * d[i]);
+                        u[uidx(p, 5 + 3 * N + k, gy, gx)] = R(by_a(m[i][2]) + by_rhon(w * pnz) * d[i]);
+                        if (is_less(d[i], fl)) u[uidx(p, 5 + k, gy, gx)] = R(fl);
+                    }
                 }
                 if (br) {
                     px = by_rhon(pnx) * rho;
@@ -1177,7 +1228,7 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
     }
     if (MODE == 2) return;
     block_reduce_dt(dtc, st, p.dt_next, p.status);
-    if (REST && gx < p.ng + p.nx) fill_ghost_images(p, p.u_next, gx, gy);
+    if (REST) fill_ghost_images(p, p.u_next, gx, gy);
     if (REST) stamp_end(p.stamps, GROW);
 }
 
@@ -1622,7 +1673,7 @@ k_finalize_mixed(KParams<float> p) {
     }
     if (MODE == 2) return;           // k_growth_f and MODE 3 follow
     block_reduce_dt_f(dtc, st, p.dt_next, p.status);
-    if (REST && gx < p.ng + p.nx) fill_ghost_images(p, p.u_next, gx, gy);
+    if (REST) fill_ghost_images(p, p.u_next, gx, gy);
     if (REST) stamp_end(p.stamps, GROW);
 }
 
