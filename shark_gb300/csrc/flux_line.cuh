@@ -294,6 +294,7 @@ __device__ __forceinline__ void flux_line(const KParams<R>& p, int s) {
 
 template <typename R, int ST>
 __global__ void __launch_bounds__(32) k_flux_line(KParams<R> p) {
+    chain_begin();
     if (blockIdx.y == 0) flux_line<R, true, ST>(p, 0);
     else flux_line<R, false, ST>(p, blockIdx.y);
 }

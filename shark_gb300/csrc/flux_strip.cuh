@@ -490,6 +490,7 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
 template <typename R, bool IS_GAS, int ST, int SOLV>
 __global__ void __launch_bounds__(32, std::is_same<R, float>::value ? (IS_GAS ? STRIP_F_GAS : STRIP_F_DUST) : (IS_GAS ? 8 : 10))
 k_flux_strip(KParams<R> p) {
+    chain_begin();
     const int bx = blockIdx.x, by = blockIdx.y;
     const int s = IS_GAS ? 0 : blockIdx.z + 1;
     flux_strip<R, IS_GAS, ST, SOLV>(p, s, bx, by);

@@ -354,6 +354,7 @@ __global__ void __launch_bounds__(32 * K1_WARPS, SHARK_K1_MINBLOCKS)
     extern __shared__ __align__(128) unsigned char k1_smem[];
     const int warp = threadIdx.x >> 5;
     const int w = blockIdx.x * K1_WARPS + warp;
+    chain_begin();
     if (w >= wk.g.n + wk.d.n) return;   // whole warps; the kernel has no block-wide barrier
     RingArgs ra;
     ra.ring = reinterpret_cast<float*>(k1_smem + warp * K1Ring::ring_bytes);

@@ -74,21 +74,38 @@ static KParams<R> make_params(const DeviceView& v) {
     return p;
 }
 
+// Launch of a step's kernel; `chained`, it comes in while its predecessor in the stream drains and waits
+// there (chain_begin), which takes the launch latency out of the step: steps of a few tens of us are
+// three such kernels (us a step: Sod FP64 1000 25.8 -> 20.1, SI 128^2 x 8 24 -> 18.4, KH 500 x 301 x 4 68
+// -> 62, blast wave 1000^2 62 -> 56, dusty wave FP64 2048 x 4 42 -> 36).  Not for kernels next to a fork
+// or join of streams or without chain_begin, nor where events time the kernels.
+template <typename... P>
+static void launch_chained(bool chained, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, P... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <typename R, int NS, int MODE, bool GROW = false>
-static void finalize_launch(const KParams<R>& p, dim3 grid, cudaStream_t st) {
+static void finalize_launch(const KParams<R>& p, dim3 grid, cudaStream_t st, bool chained) {
     if constexpr (std::is_same<R, float>::value) {
         if constexpr (GROW) {
-            k_finalize_mixed<NS, MODE, GROW><<<grid, 256, 0, st>>>(p);
+            launch_chained(chained, k_finalize_mixed<NS, MODE, GROW>, grid, dim3(256), 0, st, p);
         } else {
             dim3 g = grid;
             g.x = (p.nx + K2M_THREADS - 1) / K2M_THREADS;
-            k_finalize_mixed<NS, MODE, GROW><<<g, K2M_THREADS, 0, st>>>(p);
+            launch_chained(chained, k_finalize_mixed<NS, MODE, GROW>, g, dim3(K2M_THREADS), 0, st, p);
         }
     }
     else {
         dim3 g = grid;
         g.x = (p.nx + K2D_THREADS - 1) / K2D_THREADS;
-        k_finalize<R, NS, MODE, GROW><<<g, K2D_THREADS, 0, st>>>(p);
+        launch_chained(chained, k_finalize<R, NS, MODE, GROW>, g, dim3(K2D_THREADS), 0, st, p);
     }
 }
 
@@ -113,31 +130,31 @@ static void growth_kernel_f(const KParams<float>& p, int nsm, cudaStream_t st) {
 }
 
 template <typename R, int MODE>
-static void finalize_dispatch(const KParams<R>& p, dim3 grid, int nsm, cudaStream_t st) {
+static void finalize_dispatch(const KParams<R>& p, dim3 grid, int nsm, cudaStream_t st, bool chained) {
     if (MODE == 0 && p.gw.on) {   // dust growth: run-time species count
         if (!(p.gw.mode & SHARK_GROWTH_FRAGMENTATION)) {
             // the drag, the growth kernel, the rest of K2
-            finalize_launch<R, -1, 2>(p, grid, st);
+            finalize_launch<R, -1, 2>(p, grid, st, chained);
             if constexpr (std::is_same<R, double>::value) {
                 if (growth_lanes(p.ndust) == 8) growth_kernel_d<8>(p, st);
                 else growth_kernel_d<16>(p, st);
             } else {
                 growth_kernel_f(p, nsm, st);
             }
-            finalize_launch<R, -1, 3>(p, grid, st);
+            finalize_launch<R, -1, 3>(p, grid, st, false);
             return;
         }
-        finalize_launch<R, -1, MODE, true>(p, grid, st);   // growth within K2
+        finalize_launch<R, -1, MODE, true>(p, grid, st, chained);   // growth within K2
         return;
     }
     switch (p.ndust) {
-        case 0: finalize_launch<R, 0, MODE>(p, grid, st); break;
-        case 1: finalize_launch<R, 1, MODE>(p, grid, st); break;
-        case 2: finalize_launch<R, 2, MODE>(p, grid, st); break;
-        case 4: finalize_launch<R, 4, MODE>(p, grid, st); break;
-        case 8: finalize_launch<R, 8, MODE>(p, grid, st); break;
-        case 16: finalize_launch<R, 16, MODE>(p, grid, st); break;
-        default: finalize_launch<R, -1, MODE>(p, grid, st); break;
+        case 0: finalize_launch<R, 0, MODE>(p, grid, st, chained); break;
+        case 1: finalize_launch<R, 1, MODE>(p, grid, st, chained); break;
+        case 2: finalize_launch<R, 2, MODE>(p, grid, st, chained); break;
+        case 4: finalize_launch<R, 4, MODE>(p, grid, st, chained); break;
+        case 8: finalize_launch<R, 8, MODE>(p, grid, st, chained); break;
+        case 16: finalize_launch<R, 16, MODE>(p, grid, st, chained); break;
+        default: finalize_launch<R, -1, MODE>(p, grid, st, chained); break;
     }
 }
 
@@ -189,44 +206,44 @@ cudaError_t launch_boundaries(const DeviceView& v) {
 
 // 1D K1: gas and dust in one launch.
 template <typename R>
-static cudaError_t line_launch(const KParams<R>& p, cudaStream_t st) {
+static cudaError_t line_launch(const KParams<R>& p, cudaStream_t st, bool chained) {
     const dim3 grid((p.nx + LINE_UX - 1) / LINE_UX, p.ndust + 1, 1);
     switch (p.slope_type) {
-        case 0: k_flux_line<R, 0><<<grid, 32, 0, st>>>(p); break;
-        case 1: k_flux_line<R, 1><<<grid, 32, 0, st>>>(p); break;
-        case 2: k_flux_line<R, 2><<<grid, 32, 0, st>>>(p); break;
-        default: k_flux_line<R, 3><<<grid, 32, 0, st>>>(p); break;
+        case 0: launch_chained(chained, k_flux_line<R, 0>, grid, dim3(32), 0, st, p); break;
+        case 1: launch_chained(chained, k_flux_line<R, 1>, grid, dim3(32), 0, st, p); break;
+        case 2: launch_chained(chained, k_flux_line<R, 2>, grid, dim3(32), 0, st, p); break;
+        default: launch_chained(chained, k_flux_line<R, 3>, grid, dim3(32), 0, st, p); break;
     }
     return cudaGetLastError();
 }
 
 template <typename R, bool IS_GAS, int ST, int SOLV>
-static void strip_kernel(const KParams<R>& p, dim3 grid, cudaStream_t st) {
-    k_flux_strip<R, IS_GAS, ST, SOLV><<<grid, 32, 0, st>>>(p);
+static void strip_kernel(const KParams<R>& p, dim3 grid, cudaStream_t st, bool chained) {
+    launch_chained(chained, k_flux_strip<R, IS_GAS, ST, SOLV>, grid, dim3(32), 0, st, p);
 }
 
 template <typename R, bool IS_GAS, int ST>
-static void strip_by_solver(const KParams<R>& p, dim3 grid, cudaStream_t st) {
+static void strip_by_solver(const KParams<R>& p, dim3 grid, cudaStream_t st, bool chained) {
     if constexpr (!IS_GAS) {
         if (p.solverdust == 3) {   // HLLC dust (solver_hllc_dust)
-            strip_kernel<R, false, ST, 3>(p, grid, st);
+            strip_kernel<R, false, ST, 3>(p, grid, st, chained);
             return;
         }
     }
     switch (IS_GAS ? p.solver : p.solverdust) {
-        case 0: strip_kernel<R, IS_GAS, ST, 0>(p, grid, st); break;
-        case 1: strip_kernel<R, IS_GAS, ST, 1>(p, grid, st); break;
-        default: strip_kernel<R, IS_GAS, ST, 2>(p, grid, st); break;
+        case 0: strip_kernel<R, IS_GAS, ST, 0>(p, grid, st, chained); break;
+        case 1: strip_kernel<R, IS_GAS, ST, 1>(p, grid, st, chained); break;
+        default: strip_kernel<R, IS_GAS, ST, 2>(p, grid, st, chained); break;
     }
 }
 
 template <typename R, bool IS_GAS>
-static void strip_dispatch(const KParams<R>& p, dim3 grid, cudaStream_t st) {
+static void strip_dispatch(const KParams<R>& p, dim3 grid, cudaStream_t st, bool chained) {
     switch (p.slope_type) {
-        case 0: strip_by_solver<R, IS_GAS, 0>(p, grid, st); break;
-        case 1: strip_by_solver<R, IS_GAS, 1>(p, grid, st); break;
-        case 2: strip_by_solver<R, IS_GAS, 2>(p, grid, st); break;
-        default: strip_by_solver<R, IS_GAS, 3>(p, grid, st); break;
+        case 0: strip_by_solver<R, IS_GAS, 0>(p, grid, st, chained); break;
+        case 1: strip_by_solver<R, IS_GAS, 1>(p, grid, st, chained); break;
+        case 2: strip_by_solver<R, IS_GAS, 2>(p, grid, st, chained); break;
+        default: strip_by_solver<R, IS_GAS, 3>(p, grid, st, chained); break;
     }
 }
 
@@ -277,10 +294,18 @@ inline StripHeights strip_heights_f(int nbx, int ny, int ndust, int nsm) {
     return {gas(MAX_H), MAX_H};
 }
 
+// 2D K1 in one launch of the two-column march, or with gas and dust strips on two streams
+template <typename R>
+static bool strip_fused(const DeviceView& v, const KParams<R>& p) {
+    return std::is_same<R, float>::value && p.ndust > 0 && p.geom != 2 && p.solverdust == 0 && p.ng % 2 == 0 && v.uniform && !v.cdisk.on;
+}
+template <typename R>
+static bool strip_forks(const DeviceView& v, const KParams<R>& p) { return v.ndim == 2 && p.ndust > 0 && !strip_fused<R>(v, p); }
+
 // 2D K1: the dust species on the main stream and the gas concurrently on the side stream
 // (forked and joined with events), so the small gas grid does not run alone.
 template <typename R>
-static cudaError_t strip_launch(const DeviceView& v, KParams<R> p) {
+static cudaError_t strip_launch(const DeviceView& v, KParams<R> p, bool chained) {
     const int nbx = (p.nx + STRIP_UX - 1) / STRIP_UX;
     const StripHeights h = std::is_same<R, float>::value ? strip_heights_f(nbx, p.ny, p.ndust, v.nsm)
                                                                  : strip_heights_d(nbx, p.ny, p.ndust, v.nsm);
@@ -289,7 +314,7 @@ static cudaError_t strip_launch(const DeviceView& v, KParams<R> p) {
         return (unsigned)((p.ny + rows - 1) / rows);
     };
     if constexpr (std::is_same<R, float>::value) {
-        if (p.ndust > 0 && p.geom != 2 && p.solverdust == 0 && p.ng % 2 == 0 && v.uniform && !v.cdisk.on) {
+        if (strip_fused<R>(v, p)) {
             // mixed path, uniform Cartesian grid, Huang & Bai dust: gas and dust strips in one
             // launch (K1Work: one persistent wave, or one piece per warp when the pieces fill many waves)
             const K1Work wk = k1_work(p.nx, p.ny, p.ndust, v.k1_warps, p.iso == 1);
@@ -301,15 +326,15 @@ static cudaError_t strip_launch(const DeviceView& v, KParams<R> p) {
             switch ((p.slope_type * 3 + gs) * 2 + (p.iso == 1 ? 1 : 0)) {
 #define SHARK_K1M(ST, GS)                                                                                \
     case (ST * 3 + GS) * 2:                                                                              \
-        k_flux_strip_mixed<ST, GS, false><<<g1, b1, K1_SMEM, v.stream>>>(maps, p, wk); break;            \
+        launch_chained(chained, k_flux_strip_mixed<ST, GS, false>, g1, b1, K1_SMEM, v.stream, maps, p, wk); break;            \
     case (ST * 3 + GS) * 2 + 1:                                                                          \
-        k_flux_strip_mixed<ST, GS, true><<<g1, b1, K1_SMEM, v.stream>>>(maps, p, wk); break;
+        launch_chained(chained, k_flux_strip_mixed<ST, GS, true>, g1, b1, K1_SMEM, v.stream, maps, p, wk); break;
                 SHARK_K1M(0, 0) SHARK_K1M(0, 1) SHARK_K1M(0, 2)
                 SHARK_K1M(1, 0) SHARK_K1M(1, 1) SHARK_K1M(1, 2)
                 SHARK_K1M(2, 0) SHARK_K1M(2, 1) SHARK_K1M(2, 2)
                 SHARK_K1M(3, 0) SHARK_K1M(3, 1)
-                case (3 * 3 + 2) * 2: k_flux_strip_mixed<3, 2, false><<<g1, b1, K1_SMEM, v.stream>>>(maps, p, wk); break;
-                default: k_flux_strip_mixed<3, 2, true><<<g1, b1, K1_SMEM, v.stream>>>(maps, p, wk); break;
+                case (3 * 3 + 2) * 2: launch_chained(chained, k_flux_strip_mixed<3, 2, false>, g1, b1, K1_SMEM, v.stream, maps, p, wk); break;
+                default: launch_chained(chained, k_flux_strip_mixed<3, 2, true>, g1, b1, K1_SMEM, v.stream, maps, p, wk); break;
 #undef SHARK_K1M
             }
             return cudaGetLastError();
@@ -319,14 +344,14 @@ static cudaError_t strip_launch(const DeviceView& v, KParams<R> p) {
         cudaEventRecord(v.fork, v.stream);
         cudaStreamWaitEvent(v.stream2, v.fork, 0);
         const dim3 gg(nbx, strips(h.gas), 1);
-        strip_dispatch<R, true>(p, gg, v.stream2);
+        strip_dispatch<R, true>(p, gg, v.stream2, false);
         cudaEventRecord(v.join, v.stream2);
         const dim3 gd(nbx, strips(h.dust), p.ndust);
-        strip_dispatch<R, false>(p, gd, v.stream);
+        strip_dispatch<R, false>(p, gd, v.stream, false);
         cudaStreamWaitEvent(v.stream, v.join, 0);
     } else {
         const dim3 gg(nbx, strips(h.gas), 1);
-        strip_dispatch<R, true>(p, gg, v.stream);
+        strip_dispatch<R, true>(p, gg, v.stream, chained);
     }
     return cudaGetLastError();
 }
@@ -355,16 +380,17 @@ cudaError_t launch_step(const DeviceView& v, int slot) {
     // ghost cells of the current state were written by the previous step's k_finalize (or by
     // launch_boundaries after an upload)
     if (v.time_kernels) cudaEventRecord(v.ev[0], v.stream);
-    k_prepare_step<<<1, SHARK_MAX_DUST, 0, v.stream>>>(p.dt_next, p.dt, p.dtstop, p.ndust,
-                                                      (p.setup == SHARK_SETUP_SI && std::is_same<R, float>::value) ? 1 : 0,
-                                                      p.coef, v.dt_log, v.post, v.status, v.post_step,
-                                                      v.stamps);
+    const bool chained = !v.time_kernels;
+    const int const_ts = p.setup == SHARK_SETUP_SI && std::is_same<R, float>::value;
+    launch_chained(chained, k_prepare_step, dim3(1), dim3(SHARK_MAX_DUST), 0, v.stream, p.dt_next, p.dt, p.dtstop, p.ndust, const_ts,
+                   p.coef, v.dt_log, v.post, (const unsigned int*)v.status, v.post_step, v.stamps);
     if (v.chg.on && (e = launch_charge<R>(v)) != cudaSuccess) return e;   // charge: solve.f90:36-42
     if (v.ou_nm > 0)   // this step's forcing coefficients, from the dt on the device
         k_ou_update<<<1, 2 * v.ou_nm, 0, v.stream>>>(v.ou, v.ou_modes, v.ou_f, v.ou_nm, p.dt, v.ou_sigma, v.ou_tcorr, v.ou_seed, v.step,
                                                      v.stamps);
     if (v.time_kernels) cudaEventRecord(v.ev[1], v.stream);
-    e = (v.ndim == 2) ? strip_launch<R>(v, p) : line_launch<R>(p, v.stream);
+    const bool flux_chained = chained && !v.chg.on && v.ou_nm == 0;   // right behind k_prepare_step
+    e = (v.ndim == 2) ? strip_launch<R>(v, p, flux_chained) : line_launch<R>(p, v.stream, flux_chained);
     if (e != cudaSuccess) return e;
     if (v.nbuf == 3) {   // fargo_scheme after source_terms (solve.f90:105), into the third buffer
         R* dst = (R*)v.u[(v.cur + 2) % 3];
@@ -373,7 +399,7 @@ cudaError_t launch_step(const DeviceView& v, int slot) {
     }
     if (v.time_kernels) cudaEventRecord(v.ev[2], v.stream);
     dim3 g2((v.nx + 255) / 256, v.ndim == 2 ? v.ny : 1, 1);
-    finalize_dispatch<R, 0>(p, g2, v.nsm, v.stream);
+    finalize_dispatch<R, 0>(p, g2, v.nsm, v.stream, chained && !strip_forks<R>(v, p) && v.nbuf == 2);
     if (v.time_kernels) cudaEventRecord(v.ev[3], v.stream);
     return cudaGetLastError();
 }
@@ -388,7 +414,7 @@ cudaError_t launch_courant(const DeviceView& v, int slot) {
     p.dt_next = reinterpret_cast<unsigned long long*>(v.dt_slots + slot);
     k_prepare_step<<<1, 32, 0, v.stream>>>(p.dt_next, p.dt, p.dtstop, 0, 0, p.coef, nullptr, nullptr, nullptr, 0, v.stamps);
     dim3 g2((v.nx + 255) / 256, v.ndim == 2 ? v.ny : 1, 1);
-    finalize_dispatch<R, 1>(p, g2, v.nsm, v.stream);
+    finalize_dispatch<R, 1>(p, g2, v.nsm, v.stream, false);
     return cudaGetLastError();
 }
 

@@ -97,6 +97,17 @@ __device__ __forceinline__ void stamp_end(unsigned long long* stamps, bool every
     if (threadIdx.x == 0 && (every_block || blockIdx.y == gridDim.y - 1)) atomicMax(stamps + 3, clock_ns());
 }
 
+// Start of a kernel that may be launched before its predecessor in the stream has ended (launch_chained
+// in kernels_impl.cuh): wait for the predecessor, then let the successor's blocks come in as this grid's
+// make room.  In that order what a kernel reads ahead of its wait (loads through restricted pointers
+// may be moved there) was written by grids that had ended before the predecessor's wait returned: the
+// current state, by the step before, and tables.  The state that the predecessor writes, the dt and the
+// coefficients go through plain pointers, behind the wait.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // A scalar parameter in the kernel's precision: the double itself, or its float copy.
 template <typename R>
 __device__ __forceinline__ R prm(double d, float f) {
@@ -1045,6 +1056,7 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
     const int gy = (p.ndim == 2) ? blockIdx.y + p.ng : 0;
     double dtc = 2e44;
     unsigned int st = 0;
+    chain_begin();
     if (DRAG) stamp_start(p.stamps);
     if (gx < p.ng + p.nx) {
         R* u = p.u_next;
@@ -1343,9 +1355,10 @@ k_finalize_mixed(KParams<float> p) {
     // constant stopping times (SI): the FP64 coefficients of this step were computed once by
     // k_prepare_step; other setups compute them per cell below
     const bool const_ts = p.setup == SHARK_SETUP_SI;
-    const float* __restrict__ cr = p.coef;
-    const float* __restrict__ cw = p.coef + SHARK_MAX_DUST;
+    const float* cr = p.coef;
+    const float* cw = p.coef + SHARK_MAX_DUST;
     constexpr bool DRAG = MODE == 0 || MODE == 2, REST = MODE == 0 || MODE == 3;
+    chain_begin();
     if (DRAG) stamp_start(p.stamps);
     const double dt = *p.dt;
     const int gx = blockIdx.x * blockDim.x + threadIdx.x + p.ng;
@@ -1717,6 +1730,7 @@ static __global__ void k_prepare_step(unsigned long long* dt_next, const double*
                                       int const_ts, float* coef, double* dt_log, StepPost* post, const unsigned int* status,
                                       long long step, unsigned long long* stamps) {
     const int k = threadIdx.x;
+    chain_begin();
     if (k == 1) {
         stamps[0] = stamps[1] = clock_ns();
         stamps[3] = 0;
