@@ -381,7 +381,7 @@ cudaError_t launch_step(const DeviceView& v, int slot) {
     // launch_boundaries after an upload)
     if (v.time_kernels) cudaEventRecord(v.ev[0], v.stream);
     const bool chained = !v.time_kernels;
-    const int const_ts = p.setup == SHARK_SETUP_SI && std::is_same<R, float>::value;
+    const int const_ts = p.setup != SHARK_SETUP_SI ? 0 : std::is_same<R, float>::value ? 1 : 2;
     launch_chained(chained, k_prepare_step, dim3(1), dim3(SHARK_MAX_DUST), 0, v.stream, p.dt_next, p.dt, p.dtstop, p.ndust, const_ts,
                    p.coef, v.dt_log, v.post, (const unsigned int*)v.status, v.post_step, v.stamps);
     if (v.chg.on && (e = launch_charge<R>(v)) != cudaSuccess) return e;   // charge: solve.f90:36-42

@@ -25,7 +25,10 @@ constexpr int K1_TMA_STAGES = SHARK_K1_TMA_STAGES;
 // Floats of the buffer `coef`: the per-step drag coefficients 1/(1+a_k), a_k/(1+a_k) of the
 // species, the step's dt as float, then (from SHARK_COEF_INVTS, written once) 1/C_k as float.
 constexpr int SHARK_COEF_INVTS = 2 * SHARK_MAX_DUST + 4;
-constexpr int SHARK_COEF_FLOATS = SHARK_COEF_INVTS + SHARK_MAX_DUST;
+// From SHARK_COEF_D (FP64 path): w_k, 1 + a_k and its reciprocal as doubles, SHARK_MAX_DUST of each.
+constexpr int SHARK_COEF_D = SHARK_COEF_INVTS + SHARK_MAX_DUST;
+constexpr int SHARK_COEF_FLOATS = SHARK_COEF_D + 6 * SHARK_MAX_DUST;
+static_assert(SHARK_COEF_D % 2 == 0, "doubles");
 
 // Charging (K5) tables, outputs and constants; see charge.cuh.
 struct ChargeView {

@@ -1071,18 +1071,25 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
             // update in solve.f90:34-35)
             const double rho_old = (double)p.u_cur[uidx(p, 0, gy, gx)];
             const TStop<R> tstop(p, max64_pos(rho_old, p.smallr), gx, gy);
-            if (drag) {
-                // dust_drag(1.0) (src/dust/dust_drag.f90:2-75), FP64 arithmetic
+            // dust_drag(1.0) (src/dust/dust_drag.f90:2-75), FP64 arithmetic; constant stopping times (SI box)
+            // take the step's coefficients from k_prepare_step (SI 256^2 x 8: K2 0.102 -> 0.088 ms)
+            auto drag_update = [&](auto constant) {
+                constexpr bool const_ts = decltype(constant)::value;
+                const double* cd = reinterpret_cast<const double*>(p.coef + SHARK_COEF_D);
                 double alpha[NMAX];
                 double rhon = rho, pnx = px, pny = py, pnz = pz;
                 for (int k = 0; k < N; ++k) {
-                    const double a = Over<double>(tstop(k))(dt);
-                    const double w = Over<double>(1.0 + a)(a);
+                    double w;
+                    if constexpr (const_ts) w = cd[k];
+                    else {
+                        const double a = Over<double>(tstop(k))(dt);
+                        w = Over<double>(1.0 + a)(a);
+                        if (NS > 0) alpha[k < NMAX ? k : 0] = a;
+                    }
                     pnx = pnx + w * (double)u[uidx(p, 5 + N + k, gy, gx)];
                     pny = pny + w * (double)u[uidx(p, 5 + 2 * N + k, gy, gx)];
                     pnz = pnz + w * (double)u[uidx(p, 5 + 3 * N + k, gy, gx)];
                     rhon = rhon + w * (double)u[uidx(p, 5 + k, gy, gx)];
-                    if (NS > 0) alpha[k < NMAX ? k : 0] = a;
                 }
                 const Over<double> by_rhon(rhon);
                 const double fl = rho * p.dust_ratio_min;   // regularisation floor (dust_drag.f90:63-73)
@@ -1101,11 +1108,13 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
                     for (int i = 0; i < CH; ++i) {
                         const int k = k0 + i;
                         if (k >= N) break;
-                        double a;
-                        if (NS > 0) a = alpha[k < NMAX ? k : 0];
-                        else a = Over<double>(tstop(k))(dt);    // run-time species count
-                        const Over<double> by_a(1.0 + a);
-                        const double w = by_a(a);
+                        double a = 0.0;
+                        if constexpr (!const_ts) {
+                            if (NS > 0) a = alpha[k < NMAX ? k : 0];
+                            else a = Over<double>(tstop(k))(dt);    // run-time species count
+                        }
+                        const Over<double> by_a = const_ts ? Over<double>(cd[SHARK_MAX_DUST + k], cd[2 * SHARK_MAX_DUST + k]) : Over<double>(1.0 + a);
+                        const double w = const_ts ? cd[k] : by_a(a);
                         u[uidx(p, 5 + N + k, gy, gx)] = R(by_a(m[i][0]) + by_rhon(w * pnx) * d[i]);
                         u[uidx(p, 5 + 2 * N + k, gy, gx)] = R(by_a(m[i][1]) + by_rhon(w * pny) * d[i]);
                         u[uidx(p, 5 + 3 * N + k, gy, gx)] = R(by_a(m[i][2]) + by_rhon(w * pnz) * d[i]);
@@ -1120,7 +1129,9 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
                     u[uidx(p, 2, gy, gx)] = R(py);
                     u[uidx(p, 3, gy, gx)] = R(pz);
                 }
-            }
+            };
+            if (drag && p.setup == SHARK_SETUP_SI) drag_update(std::true_type{});
+            else if (drag) drag_update(std::false_type{});
             if (heat) {   // drag heating, part of S_U (source_terms.f90:88-97)
                 const long long ie = uidx(p, 4, gy, gx);
                 u[ie] = R((double)u[ie] + drag_heating(p, tstop, gx, gy, dt));
@@ -1692,7 +1703,8 @@ k_finalize_mixed(KParams<float> p) {
 
 // Per-step preparation, one small block before the flux kernels: reset the next-dt slot and,
 // when the stopping times are per-species constants (SI box), compute the stiff drag
-// coefficients 1/(1+a_k) and a_k/(1+a_k), a_k = dt/t_k, once in FP64 (dust_drag.f90:29-46).
+// coefficients 1/(1+a_k) and a_k/(1+a_k), a_k = dt/t_k, once in FP64 (dust_drag.f90:29-46): const_ts
+// 1 as floats, 2 as K2's FP64 form takes them.
 __device__ __forceinline__ double hash_uniform_d(unsigned long long seed, unsigned long long counter) {
     unsigned long long z = seed * 0x9E3779B97F4A7C15ull + counter + 0x632BE59BD9B4E019ull;
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -1746,11 +1758,19 @@ static __global__ void k_prepare_step(unsigned long long* dt_next, const double*
         __threadfence_system();
         *(volatile long long*)&post->step = step;
     }
-    if (const_ts && k < ndust) {
+    if (const_ts == 1 && k < ndust) {
         float r, w;
         drag_coeffs(1.0 * (*dt) / dtstop[k], r, w);
         coef[k] = r;
         coef[SHARK_MAX_DUST + k] = w;
+    }
+    if (const_ts == 2 && k < ndust) {
+        const double a = Over<double>(dtstop[k])(*dt);
+        const Over<double> by_a(1.0 + a);
+        double* cd = reinterpret_cast<double*>(coef + SHARK_COEF_D);
+        cd[k] = by_a(a);
+        cd[SHARK_MAX_DUST + k] = by_a.b;
+        cd[2 * SHARK_MAX_DUST + k] = by_a.y;
     }
 }
 
