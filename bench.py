@@ -87,14 +87,16 @@ def describe(args, cfg):
 
 def launches_per_step(cfg):
     """Kernels of one mixed-precision step: k_prepare_step, charging, forcing update, K1 (one launch
-    on Cartesian grids with the Huang & Bai dust solver, gas and dust launches otherwise), FARGO, K2."""
+    on Cartesian grids with the Huang & Bai dust solver, gas and dust launches otherwise), FARGO (shifts and
+    remap), K2 (with growth: the drag, the growth, the rest)."""
     from shark_gb300 import config as K
     n = 2
     n += 1 if cfg.flags & K.FLAG_CHARGING else 0
     n += 1 if getattr(cfg, "turb_mach", 0.0) > 0.0 else 0
     cart_hb = cfg.geom != 2 and cfg.solverdust == 0 and cfg.ndust > 0
     n += 1 if (cart_hb or cfg.ndust == 0) else 2
-    n += 1 if cfg.flags & K.FLAG_FARGO else 0
+    n += 2 if cfg.flags & K.FLAG_FARGO else 0
+    n += 2 if cfg.flags & K.FLAG_GROWTH and not cfg.grw_mode & K.GROWTH_FRAGMENTATION else 0
     return n
 
 
@@ -362,7 +364,7 @@ def run_gpu(args):
     el = time.perf_counter() - t0
     barrier()
     e2e_value = replica_rate(zs_step, e2e_steps, world, max_over_ranks(el, world, "cuda"))
-    # resident variant: what the Fortran driver does (solve + 8-byte dt readback per step)
+    # resident variant: what the Fortran driver does (solve + the wait for the dt post per step)
     t0 = time.perf_counter()
     for _ in range(e2e_steps):
         gm.solve()
@@ -419,7 +421,7 @@ def run_gpu(args):
                 "steps": e2e_steps,
                 "note": "per step: shark_gpu_upload from pinned host FP64 u_prim, shark_gpu_step, shark_gpu_download",
                 "resident_value": zs_step * e2e_steps / el_res,
-                "resident_note": "state kept on the device, per step shark_gpu_step with its 12-byte dt/status readback"},
+                "resident_note": "state kept on the device, per step shark_gpu_step with its dt/status post"},
         "cpu_baseline": cpu,
         "gpu_launches": launches_per_step(cfg_m) * args.steps,
         "gpu_launches_note": launches_note(cfg_m),
@@ -454,7 +456,9 @@ def launches_note(cfg):
     else:
         parts.append("k_flux_strip (gas, side stream) + k_flux_strip (dust)")
     if cfg.flags & K.FLAG_FARGO:
-        parts.append("k_fargo")
+        parts.append("k_fargo_shift, k_fargo")
+    if cfg.flags & K.FLAG_GROWTH and not cfg.grw_mode & K.GROWTH_FRAGMENTATION:
+        parts.append("k_finalize_mixed (drag), k_growth_f")
     parts.append("k_finalize_mixed")
     return "per step: " + ", ".join(parts)
 
@@ -525,7 +529,7 @@ def alu_roofline_turb(cfg, kernel_ms):
     fp32_peak, fp64_peak = vals["fp32_peak_tflops_at_2070mhz"], vals["fp64_peak_tflops_at_2070mhz"]
     g32 = vals["k_finalize_mixed_growth_fp32_flop_per_cell"] * cells / growth_s / 1e12
     c64 = vals["k_charge_fp64_flop_per_cell"] * cells / charge_s / 1e12
-    return {"growth": {"kernel": "k_finalize_mixed (drag + growth + CFL)", "bound": "fp32 issue latency",
+    return {"growth": {"kernel": "k_finalize_mixed (drag), k_growth_f, k_finalize_mixed (rest)", "bound": "fp32 issue",
                        "achieved": g32, "peak": fp32_peak, "unit": "TFLOP/s", "frac": g32 / fp32_peak},
             "charging": {"kernel": "k_charge (+ OU forcing update)", "bound": "fp64 pipe",
                          "achieved": c64, "peak": fp64_peak, "unit": "TFLOP/s", "frac": c64 / fp64_peak},

@@ -2,8 +2,8 @@
 //
 // Owns the device-resident state of one run and sequences the kernels of one `solve`
 // (src/solver/solve.f90:10-181).  The conserved state never leaves the GPU between steps; the
-// only per-step device->host traffic is the 8-byte dt (plus the 4-byte status word) that the
-// Fortran driver needs for `time = time + dt` (src/shark.f90:107).
+// only per-step device->host traffic is the post of dt, status and step number in pinned memory that
+// the Fortran driver needs for `time = time + dt` (src/shark.f90:107).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>

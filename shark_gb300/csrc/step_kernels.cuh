@@ -1043,7 +1043,7 @@ __device__ __forceinline__ void turb_kick_cell(const KParams<R>& p, R* u, int gx
 // Bound by the FP64 pipe (64 clocks of an SM partition for a warp's instruction): quotients share
 // reciprocals, compares and finiteness checks run on the bits, one square root takes the largest of
 // the force limiter's sums; all exact.  SI boxes of 8 species: 1024^2 2.36 -> 1.38 ms, 256^2 0.183 ->
-// 0.116 ms; dusty wave of 2048 x 4 0.075 -> 0.026 ms.  Blocks of 128: the warps of one or two
+// 0.088 ms; dusty wave of 2048 x 4 0.075 -> 0.026 ms.  Blocks of 128: the warps of one or two
 // thousand cells then each have a partition of their own.
 constexpr int K2D_THREADS = 128;
 
