@@ -13,9 +13,9 @@
 // columns: neighbouring columns' shifts differ by few cells, so its loads fall on few rows.
 // What a column shares (whole cells, weights) a kernel of one thread per column forms first, in FP64
 // in both precisions: the two divisions and the remainder cost more than the remap of a column.
-// 512 x 1024, 16 species, mixed: 0.254 -> 0.060 ms; 128 x 256, FP64: 0.081 -> 0.053 ms (before: whole rings staged
-// in shared memory by blocks of 64-byte row segments, two limited slopes an output, the shifts
-// formed by every block).
+// 512 x 1024, 16 species, mixed: 0.254 -> 0.060 ms; 128 x 256, FP64: 0.081 -> 0.053 ms (before: whole
+// rings staged in shared memory by blocks of 64-byte row segments, two limited slopes an output, the
+// shifts formed by every block).
 //
 // Restated with the defects of the reference fixed (the oracle does the same):
 //   `one` is 1 and `eps` FP64 (an undeclared uninitialised REAL and an implicit REAL*4 there);

@@ -47,7 +47,8 @@ struct KParams {
     GrowthDev gw;                      // dust growth tables and constants
     int ou_nm;                         // dustyTurb forcing modes (0: no forcing)
     const double* ou;                  // [2 nm] this step's coefficients
-    const float* ou_f;                 // the mixed path's table of this step: k_x', k_y', k_y'/k, k_x'/k of the modes, then the coefficients
+    const float* ou_f;                 // mixed path, this step: k_x', k_y', k_y'/k, k_x'/k of the modes,
+                                       // then the coefficients
     const double* ou_modes;            // [3 nm]
     double box_l_y;
     const R* chg_eta;                  // charging outputs: eta (3 planes), gamma_d (N planes)
@@ -1113,7 +1114,8 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
                             if (NS > 0) a = alpha[k < NMAX ? k : 0];
                             else a = Over<double>(tstop(k))(dt);    // run-time species count
                         }
-                        const Over<double> by_a = const_ts ? Over<double>(cd[SHARK_MAX_DUST + k], cd[2 * SHARK_MAX_DUST + k]) : Over<double>(1.0 + a);
+                        const Over<double> by_a = const_ts ? Over<double>(cd[SHARK_MAX_DUST + k], cd[2 * SHARK_MAX_DUST + k])
+                                                           : Over<double>(1.0 + a);
                         const double w = const_ts ? cd[k] : by_a(a);
                         u[uidx(p, 5 + N + k, gy, gx)] = R(by_a(m[i][0]) + by_rhon(w * pnx) * d[i]);
                         u[uidx(p, 5 + 2 * N + k, gy, gx)] = R(by_a(m[i][1]) + by_rhon(w * pny) * d[i]);

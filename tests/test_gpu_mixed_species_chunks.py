@@ -1,5 +1,6 @@
 """Mixed-precision K2 with a run-time species count: its passes take four species at a time.  Counts
-around whole chunks, with each kind of drag coefficient (one set a step, per cell) against the oracle, at the mixed path's tolerance on the same setups."""
+around whole chunks, with each kind of drag coefficient (one set a step, per cell) against the oracle,
+at the mixed path's tolerance on the same setups."""
 import numpy as np
 import pytest
 
