@@ -1359,10 +1359,12 @@ constexpr int K2M_THREADS = 128;
 
 // Blocks per SM: 8 species at 5 blocks of 128 threads (96 registers), measured best of 4-6; a gas
 // alone at 10 (48 registers), whose few loads a thread need many warps (1000^2 21.6 -> 19.5 us against 6,
-// 20.0 at 8, 19.7 at 12).
+// 20.0 at 8, 19.7 at 12).  1 and 2 species at 8 (64 registers) against 6:
+// KH 500 x 301 x 1 28.5 -> 22.5, SI 1024^2 x 2 34.1 -> 31.4; 4 species stay at 6, where 8 gain on the
+// adiabatic box (46.8 -> 44.6) and lose on the isothermal one (40.8 -> 45.1).
 template <int NS, int MODE, bool GROW = false>
 __global__ void __launch_bounds__(GROW ? 256 : K2M_THREADS,
-                                  GROW ? ((NS >= 8) ? 2 : 3) : (NS == 0 ? 10 : NS == 8 ? 5 : ((NS > 8) ? 2 : 3) * (256 / K2M_THREADS)))
+                                  GROW ? ((NS >= 8) ? 2 : 3) : (NS == 0 ? 10 : NS == 1 || NS == 2 ? 8 : NS == 8 ? 5 : ((NS > 8) ? 2 : 3) * (256 / K2M_THREADS)))
 k_finalize_mixed(KParams<float> p) {
     constexpr int NMAX = NS > 0 ? NS : 1;
     const int N = NS >= 0 ? NS : p.ndust;
