@@ -108,7 +108,7 @@ __device__ __forceinline__ GasFlux<float> gas_hll_fast(float inv_g1, float rho_l
 }
 
 // Compile-time solver choice (solve_wrapper, godunov.f90:768-833) for specialised kernels.
-template <int SOLVER, typename R>
+template <int SOLVER, int WHERE, typename R>
 __device__ __forceinline__ GasFlux<R> gas_flux_t(R gamma, R inv_g1, R rl, R ul, R vl, R wl, R pl, R rr, R ur, R vr,
                                                  R wr, R pr, R csl, R csr) {
     if constexpr (std::is_same<R, float>::value) {
@@ -116,21 +116,21 @@ __device__ __forceinline__ GasFlux<R> gas_flux_t(R gamma, R inv_g1, R rl, R ul, 
         else if constexpr (SOLVER == 1) return gas_hll_fast(inv_g1, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
         else return gas_llf(gamma, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
     } else {
-        if constexpr (SOLVER == 2) return gas_hllc_d(gamma, inv_g1, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
-        else if constexpr (SOLVER == 1) return gas_hll_d(gamma, inv_g1, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
+        if constexpr (SOLVER == 2) return gas_hllc_d<WHERE>(gamma, inv_g1, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
+        else if constexpr (SOLVER == 1) return gas_hll_d<WHERE>(gamma, inv_g1, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
         else return gas_llf_d(gamma, inv_g1, rl, ul, vl, wl, pl, rr, ur, vr, wr, pr, csl, csr);
     }
 }
 
 // csl, csr: the gas sound speeds of the face (used by the HLLC dust solver only).
-template <int SOLVERDUST, typename R>
+template <int SOLVERDUST, int WHERE, typename R>
 __device__ __forceinline__ DustFlux<R> dust_flux_t(R rl, R ul, R vl, R wl, R rr, R ur, R vr, R wr, R csl, R csr) {
     if constexpr (SOLVERDUST == 0 && std::is_same<R, float>::value) return dust_hb_f(rl, ul, vl, wl, rr, ur, vr, wr);
     else if constexpr (std::is_same<R, double>::value) {
         if constexpr (SOLVERDUST == 0) return dust_hb_d(rl, ul, vl, wl, rr, ur, vr, wr);
         else if constexpr (SOLVERDUST == 1) return dust_llf_d(rl, ul, vl, wl, rr, ur, vr, wr);
-        else if constexpr (SOLVERDUST == 2) return dust_hll_d(rl, ul, vl, wl, rr, ur, vr, wr);
-        else return dust_hllc_d(rl, ul, vl, wl, rr, ur, vr, wr, csl, csr);
+        else if constexpr (SOLVERDUST == 2) return dust_hll_d<WHERE>(rl, ul, vl, wl, rr, ur, vr, wr);
+        else return dust_hllc_d<WHERE>(rl, ul, vl, wl, rr, ur, vr, wr, csl, csr);
     }
     else if constexpr (SOLVERDUST == 1) return dust_llf(rl, ul, vl, wl, rr, ur, vr, wr);
     else if constexpr (SOLVERDUST == 2) return dust_hll(rl, ul, vl, wl, rr, ur, vr, wr);
@@ -139,9 +139,10 @@ __device__ __forceinline__ DustFlux<R> dust_flux_t(R rl, R ul, R vl, R wl, R rr,
 
 constexpr int LINE_UX = 28;   // columns updated per warp
 
-// One species of one strip.  ST: slope limiter (0..3).
-template <typename R, bool IS_GAS, int ST>
-__device__ __forceinline__ void flux_line(const KParams<R>& p, int s) {
+// One species of one strip.  ST: slope limiter (0..3).  WHERE = TRIED (FP64): false where a denominator of
+// the strip lies outside div64_const's range; what it stored is then to be written over.
+template <typename R, bool IS_GAS, int ST, int WHERE>
+__device__ __forceinline__ bool flux_line(const KParams<R>& p, int s) {
     constexpr bool FAST = std::is_same<R, float>::value;
     constexpr int NV = IS_GAS ? 5 : 4;
     const int N = p.ndust, lane = threadIdx.x & 31;
@@ -156,7 +157,8 @@ __device__ __forceinline__ void flux_line(const KParams<R>& p, int s) {
     R uu[NV], q[NV], cs = p.cs[gxc];
 #pragma unroll
     for (int k = 0; k < NV; ++k) uu[k] = p.u_cur[svar(s, k, N) * p.plane + gxc];
-    const Over<R> by_rho(uu[0]);
+    const Over<R, WHERE> by_rho(uu[0]);
+    bool inside = by_rho.inside();
     q[0] = uu[0];
     if constexpr (FAST) {
         const R ir = R(1) / uu[0];
@@ -177,7 +179,7 @@ __device__ __forceinline__ void flux_line(const KParams<R>& p, int s) {
             } else {
                 const R hr = half * uu[0];
                 q[4] = max64_pos((gamma - R(1)) * (uu[4] - (hr * sq(q[1]) + hr * sq(q[2]) + hr * sq(q[3]))), smallP);
-                cs = sqrt(Over<R>(q[0])(gamma * q[4]));
+                cs = sqrt(Over<R, WHERE>(q[0])(gamma * q[4]));
             }
         }
     }
@@ -185,7 +187,7 @@ __device__ __forceinline__ void flux_line(const KParams<R>& p, int s) {
     const R dx1 = p.dx1[gxc];
     const R bl = half * (dx1 + p.dx1[gxl]), br = half * (p.dx1[gxr] + dx1);   // 2 d / (dx + dx') = d / ((dx + dx') / 2)
     const R sfl = p.sfx[gxc], sfr = p.sfx[gxr];
-    const Over<R> by_l(bl), by_r(br);
+    const Over<R, CONSTANT> by_l(bl), by_r(br);
     R dq[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
@@ -215,7 +217,11 @@ __device__ __forceinline__ void flux_line(const KParams<R>& p, int s) {
         if (iso) { q[4] = q[0] * sq(cs); dq[4] = dq[0] * sq(cs); }
         R dp_r;
         if constexpr (FAST) dp_r = dq[4] * (R(1) / q[0]);
-        else dp_r = Over<R>(q[0])(dq[4]);
+        else {
+            const Over<R, WHERE> by_q(q[0]);
+            dp_r = by_q(dq[4]);
+            inside = inside && by_q.inside();
+        }
         b[1] = u + hdt * (-u * dq[1] - dp_r);
         b[4] = q[4] + hdt * (-u * dq[4] - dq[1] * gamma * q[4]);
     } else {
@@ -247,25 +253,32 @@ __device__ __forceinline__ void flux_line(const KParams<R>& p, int s) {
         R csl = up(cs), csr = cs;
         if (!iso) {
             if constexpr (FAST) { csl = sqrt(gamma * ql[4] / ql[0]); csr = sqrt(gamma * qp[4] / qp[0]); }
-            else { csl = sqrt(Over<R>(ql[0])(gamma * ql[4])); csr = sqrt(Over<R>(qp[0])(gamma * qp[4])); }
+            else {
+                const Over<R, WHERE> by_ql(ql[0]), by_qp(qp[0]);
+                csl = sqrt(by_ql(gamma * ql[4]));
+                csr = sqrt(by_qp(gamma * qp[4]));
+                inside = inside && by_ql.inside() && by_qp.inside();
+            }
         }
         R g1;   // 1/(gamma - 1)
         if constexpr (FAST) g1 = p.f_inv_g1;
         else g1 = rcp64(gamma - R(1));
         GasFlux<R> g;
-        if (p.solver == 2) g = gas_flux_t<2>(gamma, g1, ql[0], ql[1], ql[2], ql[3], ql[4], qp[0], qp[1], qp[2], qp[3], qp[4], csl, csr);
-        else if (p.solver == 1) g = gas_flux_t<1>(gamma, g1, ql[0], ql[1], ql[2], ql[3], ql[4], qp[0], qp[1], qp[2], qp[3], qp[4], csl, csr);
-        else g = gas_flux_t<0>(gamma, g1, ql[0], ql[1], ql[2], ql[3], ql[4], qp[0], qp[1], qp[2], qp[3], qp[4], csl, csr);
+        if (p.solver == 2) g = gas_flux_t<2, WHERE>(gamma, g1, ql[0], ql[1], ql[2], ql[3], ql[4], qp[0], qp[1], qp[2], qp[3], qp[4], csl, csr);
+        else if (p.solver == 1) g = gas_flux_t<1, WHERE>(gamma, g1, ql[0], ql[1], ql[2], ql[3], ql[4], qp[0], qp[1], qp[2], qp[3], qp[4], csl, csr);
+        else g = gas_flux_t<0, WHERE>(gamma, g1, ql[0], ql[1], ql[2], ql[3], ql[4], qp[0], qp[1], qp[2], qp[3], qp[4], csl, csr);
         fl[0] = g.rho; fl[1] = g.mn; fl[2] = g.mt; fl[3] = g.mz; fl[4] = g.e;
+        inside = inside && g.inside;
     } else {
         // the HLLC dust solver's gas sound speeds (isothermal gas: per column, godunov.f90:675-677)
         const R csl = up(cs);
         DustFlux<R> d;
-        if (p.solverdust == 0) d = dust_flux_t<0>(ql[0], ql[1], ql[2], ql[3], qp[0], qp[1], qp[2], qp[3], csl, cs);
-        else if (p.solverdust == 1) d = dust_flux_t<1>(ql[0], ql[1], ql[2], ql[3], qp[0], qp[1], qp[2], qp[3], csl, cs);
-        else if (p.solverdust == 2) d = dust_flux_t<2>(ql[0], ql[1], ql[2], ql[3], qp[0], qp[1], qp[2], qp[3], csl, cs);
-        else d = dust_flux_t<3>(ql[0], ql[1], ql[2], ql[3], qp[0], qp[1], qp[2], qp[3], csl, cs);
+        if (p.solverdust == 0) d = dust_flux_t<0, WHERE>(ql[0], ql[1], ql[2], ql[3], qp[0], qp[1], qp[2], qp[3], csl, cs);
+        else if (p.solverdust == 1) d = dust_flux_t<1, WHERE>(ql[0], ql[1], ql[2], ql[3], qp[0], qp[1], qp[2], qp[3], csl, cs);
+        else if (p.solverdust == 2) d = dust_flux_t<2, WHERE>(ql[0], ql[1], ql[2], ql[3], qp[0], qp[1], qp[2], qp[3], csl, cs);
+        else d = dust_flux_t<3, WHERE>(ql[0], ql[1], ql[2], ql[3], qp[0], qp[1], qp[2], qp[3], csl, cs);
         fl[0] = d.rho; fl[1] = d.mn; fl[2] = d.mt; fl[3] = d.mz;
+        inside = inside && d.inside;
     }
     // kick(1.0) (force_kicks.f90:2-41), then the flux difference
     if (fk) {
@@ -282,7 +295,7 @@ __device__ __forceinline__ void flux_line(const KParams<R>& p, int s) {
         if constexpr (IS_GAS) uu[4] = uu[4] + (kinetic() - eo);
     }
     const R s1 = p.surf1[gxc], vol = p.vol[gxc];
-    const Over<R> by_vol(vol);
+    const Over<R, CONSTANT> by_vol(vol);
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         const R a = fl[k] * s1, ar = dn(a);   // the right face is the right neighbour's left one
@@ -290,13 +303,22 @@ __device__ __forceinline__ void flux_line(const KParams<R>& p, int s) {
         else uu[k] = uu[k] + by_vol(a - ar) * dt;
         if (lane >= 2 && lane <= 29 && gx < p.ng + p.nx) p.u_next[svar(s, k, N) * p.plane + gx] = uu[k];
     }
+    return FAST || WHERE != TRIED || __all_sync(0xffffffffu, inside);
 }
 
+// The strip with a denominator outside the range, out of line: the kernel keeps to the registers (72) and
+// the code of the other form.
+template <typename R, bool IS_GAS, int ST>
+static __device__ __noinline__ void flux_line_wide(const KParams<R>& p, int s) { flux_line<R, IS_GAS, ST, ANYWHERE>(p, s); }
+
 template <typename R, int ST>
-__global__ void __launch_bounds__(32) k_flux_line(KParams<R> p) {
+__global__ void __launch_bounds__(32, 28) k_flux_line(const __grid_constant__ KParams<R> p) {
     chain_begin();
-    if (blockIdx.y == 0) flux_line<R, true, ST>(p, 0);
-    else flux_line<R, false, ST>(p, blockIdx.y);
+    if (blockIdx.y == 0) {
+        if (!flux_line<R, true, ST, TRIED>(p, 0)) flux_line_wide<R, true, ST>(p, 0);
+    } else {
+        if (!flux_line<R, false, ST, TRIED>(p, blockIdx.y)) flux_line_wide<R, false, ST>(p, blockIdx.y);
+    }
 }
 
 }  // namespace shark

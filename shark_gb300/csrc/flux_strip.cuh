@@ -65,7 +65,7 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
     // scaling by 1/2 is exact, so half * a * b rounds as a * (half * b) does
     const R hdt = half * dt, hdx = half * dxl, hdy = half * dyl;
     // FP64: the halved denominators of the x slopes (2 d / (dx + dx') = d / ((dx + dx') / 2) exactly;
-    // along y the half is dx2 itself), and the reciprocals of the grid's denominators for div64
+    // along y the half is dx2 itself), and the reciprocals of the grid's denominators
     const bool even_x = __all_sync(0xffffffffu, dx1l == dx1 && dx1r == dx1);
     R bxl = R(0), bxr = R(0), yxl = R(0), yxr = R(0), yy = R(0), yr = R(0), yvol = R(0), yg1 = R(0), ff1 = R(0), ff2 = R(0);
     if constexpr (!FAST) {
@@ -81,22 +81,22 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
             ff1 = p.fgrav[gxc];
         }
     }
-    auto over_vol = [&](R x) -> R { if constexpr (FAST) return x * rvol; else return div64(x, vol, yvol); };
+    auto over_vol = [&](R x) -> R { if constexpr (FAST) return x * rvol; else return div64_const(x, vol, yvol); };
     // slopes at one row from the differences to both neighbours
     auto slope_x = [&](R dl, R dr) -> R {
         if constexpr (FAST) return slope_limit_t<ST>(dl * sfl, dr * sfr);
         else {
             // minmod takes one of the two quotients and division keeps their order
-            if (ST == 1 && even_x) return div64(limit_minmod_d(dl, dr), bxl, yxl);
-            return slope_limit_t<ST>(div64(dl, bxl, yxl), div64(dr, bxr, yxr));
+            if (ST == 1 && even_x) return div64_const(limit_minmod_d(dl, dr), bxl, yxl);
+            return slope_limit_t<ST>(div64_const(dl, bxl, yxl), div64_const(dr, bxr, yxr));
         }
     };
     auto slope_y = [&](R dl, R dr) -> R {
         if constexpr (FAST) return slope_limit_t<ST>(dl * sfy, dr * sfy);
         else {
-            const R s = ST == 1 ? div64(limit_minmod_d(dl, dr), dx2, yy)
-                                : slope_limit_t<ST>(div64(dl, dx2, yy), div64(dr, dx2, yy));
-            return polar ? div64(s, radc, yr) : s;
+            const R s = ST == 1 ? div64_const(limit_minmod_d(dl, dr), dx2, yy)
+                                : slope_limit_t<ST>(div64_const(dl, dx2, yy), div64_const(dr, dx2, yy));
+            return polar ? div64_const(s, radc, yr) : s;
         }
     };
 
@@ -232,7 +232,7 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                 }
             }
         }
-        auto over_r = [&](R x) -> R { if constexpr (FAST) return x * irp; else return div64(x, radc, yr); };
+        auto over_r = [&](R x) -> R { if constexpr (FAST) return x * irp; else return div64_const(x, radc, yr); };
         R qmx[NV], qpx[NV], qmy[NV], qpy[NV];
         R sr0 = -u * drx - v * dry - (dux + dvy) * r_rho;
         if (IS_GAS) {
@@ -311,12 +311,12 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                 R csl, csr;
                 if (iso) { csl = shfl_up1(c1); csr = c1; }
                 else { csl = face_cs(ql[4], ql[0]); csr = face_cs(qpx[4], qpx[0]); }
-                const GasFlux<R> g = gas_flux_t<SOLV>(gamma, FAST ? inv_g1 : yg1, ql[0], ql[1], ql[2], ql[3], ql[4],
+                const GasFlux<R> g = gas_flux_t<SOLV, ANYWHERE>(gamma, FAST ? inv_g1 : yg1, ql[0], ql[1], ql[2], ql[3], ql[4],
                                               qpx[0], qpx[1], qpx[2], qpx[3], qpx[4], csl, csr);
                 fxl[0] = g.rho; fxl[1] = g.mn; fxl[2] = g.mt; fxl[3] = g.mz; fxl[4] = g.e;
             } else {
                 // gas sound speeds of the face for the HLLC dust solver (isothermal: per column)
-                const DustFlux<R> d = dust_flux_t<SOLV>(ql[0], ql[1], ql[2], ql[3], qpx[0], qpx[1], qpx[2], qpx[3],
+                const DustFlux<R> d = dust_flux_t<SOLV, ANYWHERE>(ql[0], ql[1], ql[2], ql[3], qpx[0], qpx[1], qpx[2], qpx[3],
                                                         shfl_up1(cs_col), cs_col);
                 fxl[0] = d.rho; fxl[1] = d.mn; fxl[2] = d.mt; fxl[3] = d.mz;
             }
@@ -338,11 +338,11 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                 if (iso) { csl = c_prev; csr = c1; }
                 else { csl = face_cs(qmy_prev[4], qmy_prev[0]); csr = face_cs(qpy[4], qpy[0]); }
                 // idim = 2: normal velocity vy, transverse vx (allocate_init.f90:249-252)
-                const GasFlux<R> g = gas_flux_t<SOLV>(gamma, FAST ? inv_g1 : yg1, qmy_prev[0], qmy_prev[2], qmy_prev[1], qmy_prev[3], qmy_prev[4],
+                const GasFlux<R> g = gas_flux_t<SOLV, ANYWHERE>(gamma, FAST ? inv_g1 : yg1, qmy_prev[0], qmy_prev[2], qmy_prev[1], qmy_prev[3], qmy_prev[4],
                                               qpy[0], qpy[2], qpy[1], qpy[3], qpy[4], csl, csr);
                 gb[0] = g.rho; gb[2] = g.mn; gb[1] = g.mt; gb[3] = g.mz; gb[4] = g.e;
             } else {
-                const DustFlux<R> d = dust_flux_t<SOLV>(qmy_prev[0], qmy_prev[2], qmy_prev[1], qmy_prev[3],
+                const DustFlux<R> d = dust_flux_t<SOLV, ANYWHERE>(qmy_prev[0], qmy_prev[2], qmy_prev[1], qmy_prev[3],
                                                 qpy[0], qpy[2], qpy[1], qpy[3], cs_col, cs_col);
                 gb[0] = d.rho; gb[2] = d.mn; gb[1] = d.mt; gb[3] = d.mz;
             }

@@ -67,7 +67,7 @@ __device__ __forceinline__ double limit_minmod_d(double l, double r) {
 }
 __device__ __forceinline__ double limit_vl_d(double l, double r) {
     const double b = 0.5 * (l + r), a = l * r;
-    const double s = div64(a, b, rcp64(b));
+    const double s = div64_const(a, b, rcp64(b));   // a is zero where b is below the normal range
     return is_zero(a) || is_neg(a) ? 0.0 : s;
 }
 __device__ __forceinline__ double limit_mc_d(double l, double r) {
@@ -90,8 +90,9 @@ __device__ __forceinline__ R slope_limit_t(R l, R r) {
     else return limit_mc_d(l, r);
 }
 
-template <typename R> struct GasFlux { R rho, mn, mt, mz, e; };
-template <typename R> struct DustFlux { R rho, mn, mt, mz; };
+// inside (FP64 solvers, WHERE = TRIED): the solver's denominators lay inside div64_const's range.
+template <typename R> struct GasFlux { R rho, mn, mt, mz, e; bool inside = true; };
+template <typename R> struct DustFlux { R rho, mn, mt, mz; bool inside = true; };
 
 // solver_llf (src/solver/solvers.f90:4-155), non-MHD
 template <typename R>
@@ -175,7 +176,7 @@ __device__ __forceinline__ DustFlux<R> dust_hll(R rho_lft, R u_lft, R v_lft, R w
 // on the bit patterns, and the HLLC's energy and star state for the sampled side only.  y1 = rcp64 of gamma - 1.
 __device__ __forceinline__ double gas_energy_d(double g1, double y1, double rho, double u, double v, double w, double P) {
     const double hr = 0.5 * rho;
-    return div64(P, g1, y1) + hr * sq(u) + hr * sq(v) + hr * sq(w);
+    return div64_const(P, g1, y1) + hr * sq(u) + hr * sq(v) + hr * sq(w);
 }
 __device__ __forceinline__ GasFlux<double> gas_llf_d(double gamma, double y1, double rl, double ul, double vl, double wl,
                                                      double Pl, double rr, double ur, double vr, double wr, double Pr,
@@ -192,46 +193,54 @@ __device__ __forceinline__ GasFlux<double> gas_llf_d(double gamma, double y1, do
     return f;
 }
 // solver_hll (src/solver/solvers.f90:157-306), non-MHD
+template <int WHERE>
 __device__ __forceinline__ GasFlux<double> gas_hll_d(double gamma, double y1, double rl, double ul, double vl, double wl,
                                                      double Pl, double rr, double ur, double vr, double wr, double Pr,
                                                      double csl, double csr) {
     const double El = gas_energy_d(gamma - 1.0, y1, rl, ul, vl, wl, Pl), Er = gas_energy_d(gamma - 1.0, y1, rr, ur, vr, wr, Pr);
     const double ml = rl * ul, mr = rr * ur, cm = max64(csl, csr);
     const double Sl = min64_0(min64(ul, ur) - cm), Sr = max64_0(max64(ul, ur) + cm);
-    const double ss = Sr * Sl, b = Sr - Sl, y = rcp64(b);
+    const double ss = Sr * Sl;
+    const Over<double, WHERE> by_b(Sr - Sl);
     GasFlux<double> f;
-    f.rho = div64(Sr * ml - Sl * mr + ss * (rr - rl), b, y);
-    f.mn = div64(Sr * (rl * sq(ul) + Pl) - Sl * (rr * sq(ur) + Pr) + ss * (mr - ml), b, y);
-    f.mt = div64(Sr * (ml * vl) - Sl * (mr * vr) + ss * (rr * vr - rl * vl), b, y);
-    f.mz = div64(Sr * (ml * wl) - Sl * (mr * wr) + ss * (rr * wr - rl * wl), b, y);
-    f.e = div64(Sr * ((El + Pl) * ul) - Sl * ((Er + Pr) * ur) + ss * (Er - El), b, y);
+    f.inside = by_b.inside();
+    f.rho = by_b(Sr * ml - Sl * mr + ss * (rr - rl));
+    f.mn = by_b(Sr * (rl * sq(ul) + Pl) - Sl * (rr * sq(ur) + Pr) + ss * (mr - ml));
+    f.mt = by_b(Sr * (ml * vl) - Sl * (mr * vr) + ss * (rr * vr - rl * vl));
+    f.mz = by_b(Sr * (ml * wl) - Sl * (mr * wr) + ss * (rr * wr - rl * wl));
+    f.e = by_b(Sr * ((El + Pl) * ul) - Sl * ((Er + Pr) * ur) + ss * (Er - El));
     return f;
 }
 // solver_hllc (src/solver/solvers.f90:308-500): RAMSES-style HLLC with the wave speeds clipped to
 // include 0 (:435-436), Lagrangian star state (:450-463), sampling at x/t = 0 (:466-486) and the
 // passive transverse momenta upwinded on the sign of u* (:491-497).
+template <int WHERE>
 __device__ __forceinline__ GasFlux<double> gas_hllc_d(double gamma, double y1, double rl, double ul, double vl, double wl,
                                                       double Pl, double rr, double ur, double vr, double wr, double Pr,
                                                       double csl, double csr) {
     const double cm = max64(csl, csr);
     const double Sl = min64_0(min64(ul, ur) - cm), Sr = max64_0(max64(ul, ur) + cm);
     const double hl = rl * (ul - Sl), hr = rr * (Sr - ur);
-    const double b = hr + hl, y = rcp64(b);
-    const double us = div64(hr * ur + hl * ul + (Pl - Pr), b, y);
-    const double Ps = div64(hr * Pl + hl * Pr + hl * hr * (ul - ur), b, y);
+    const Over<double, WHERE> by_b(hr + hl);
+    const double us = by_b(hr * ur + hl * ul + (Pl - Pr));
+    const double Ps = by_b(hr * Pl + hl * Pr + hl * hr * (ul - ur));
+    bool inside = by_b.inside();
     const bool left = is_pos(us);
     const double S = left ? Sl : Sr, rho = left ? rl : rr, u = left ? ul : ur, v = left ? vl : vr, w = left ? wl : wr;
     const double P = left ? Pl : Pr;
     const double E = gas_energy_d(gamma - 1.0, y1, rho, u, v, w, P);
     double ro = rho, uo = u, Po = P, eo = E;
     if (left || is_pos(Sr)) {   // Sl is at most 0, so the left state itself is never sampled
-        const double d = S - u, c = S - us, yc = rcp64(c);
-        ro = div64(rho * d, c, yc);
+        const double d = S - u;
+        const Over<double, WHERE> by_c(S - us);
+        ro = by_c(rho * d);
         uo = us;
         Po = Ps;
-        eo = div64(d * E - P * u + Ps * us, c, yc);
+        eo = by_c(d * E - P * u + Ps * us);
+        inside = inside && by_c.inside();
     }
     GasFlux<double> f;
+    f.inside = inside;
     f.rho = ro * uo;
     f.mn = f.rho * uo + Po;
     f.e = (eo + Po) * uo;
@@ -265,37 +274,44 @@ __device__ __forceinline__ DustFlux<double> dust_llf_d(double rl, double ul, dou
     f.mz = 0.5 * (ml * wl + mr * wr) - hl * (rr * wr - rl * wl);
     return f;
 }
+template <int WHERE>
 __device__ __forceinline__ DustFlux<double> dust_hll_d(double rl, double ul, double vl, double wl, double rr, double ur,
                                                        double vr, double wr) {
     const double Sl = min64_0(min64(ul, ur)), Sr = max64_0(max64(ul, ur)), b = Sr - Sl;
     DustFlux<double> f{0.0, 0.0, 0.0, 0.0};
     if (!is_zero(b)) {
-        const double y = rcp64(b), ss = Sr * Sl, ml = rl * ul, mr = rr * ur;
-        f.rho = div64(Sr * ml - Sl * mr + ss * (rr - rl), b, y);
-        f.mn = div64(Sr * (rl * sq(ul)) - Sl * (rr * sq(ur)) + ss * (mr - ml), b, y);
-        f.mt = div64(Sr * (ml * vl) - Sl * (mr * vr) + ss * (rr * vr - rl * vl), b, y);
-        f.mz = div64(Sr * (ml * wl) - Sl * (mr * wr) + ss * (rr * wr - rl * wl), b, y);
+        const Over<double, WHERE> by_b(b);
+        const double ss = Sr * Sl, ml = rl * ul, mr = rr * ur;
+        f.inside = by_b.inside();
+        f.rho = by_b(Sr * ml - Sl * mr + ss * (rr - rl));
+        f.mn = by_b(Sr * (rl * sq(ul)) - Sl * (rr * sq(ur)) + ss * (mr - ml));
+        f.mt = by_b(Sr * (ml * vl) - Sl * (mr * vr) + ss * (rr * vr - rl * vl));
+        f.mz = by_b(Sr * (ml * wl) - Sl * (mr * wr) + ss * (rr * wr - rl * wl));
     }
     return f;
 }
+template <int WHERE>
 __device__ __forceinline__ DustFlux<double> dust_hllc_d(double rl, double ul, double vl, double wl, double rr, double ur,
                                                         double vr, double wr, double csl, double csr) {
     const double cm = max64(csl, csr);
     const double Sl = min64_0(min64(ul, ur) - cm), Sr = max64_0(max64(ul, ur) + cm);
     const double hl = rl * (ul - Sl), hr = rr * (Sr - ur);
-    const double b = hr + hl, y = rcp64(b);
-    const double us = div64(hr * ur + hl * ul, b, y);
-    const double Ps = div64(hl * hr * (ul - ur), b, y);
+    const Over<double, WHERE> by_b(hr + hl);
+    const double us = by_b(hr * ur + hl * ul);
+    const double Ps = by_b(hl * hr * (ul - ur));
+    bool inside = by_b.inside();
     const bool left = is_pos(us);
     const double S = left ? Sl : Sr, rho = left ? rl : rr, u = left ? ul : ur, v = left ? vl : vr, w = left ? wl : wr;
     double ro = rho, uo = u, Po = 0.0;
     if (left || is_pos(Sr)) {
-        const double c = S - us;
-        ro = div64(rho * (S - u), c, rcp64(c));
+        const Over<double, WHERE> by_c(S - us);
+        ro = by_c(rho * (S - u));
         uo = us;
         Po = Ps;
+        inside = inside && by_c.inside();
     }
     DustFlux<double> f;
+    f.inside = inside;
     f.rho = ro * uo;
     f.mn = f.rho * uo + Po;
     f.mt = f.rho * v;

@@ -397,32 +397,35 @@ __device__ __forceinline__ void block_reduce_dt_f(float dtc, unsigned int st, un
     }
 }
 
+// Where a denominator formed from the state lies: from floats it cannot leave the range of div64_const.
+template <typename R> constexpr int STATE_RANGE = std::is_same<R, float>::value ? CONSTANT : ANYWHERE;
+
 // Sound speed of the cell at the start of the step: the isothermal column value, or ctoprim's
 // sqrt(gamma P / max(rho, smallr)) of the adiabatic state (solve.f90:205-233).
 template <typename R>
 __device__ __forceinline__ double cs_start(const KParams<R>& p, int gx, int gy) {
     if (p.iso == 1) return p.ccsd ? p.ccsd[(long long)gy * p.pitch + gx] : p.csd[gx];
     const double rho = widen(p.u_cur[uidx(p, 0, gy, gx)]);
-    const Over<double> by_rho(rho);
+    const Over<double, STATE_RANGE<R>> by_rho(rho);
     const double vx = by_rho(widen(p.u_cur[uidx(p, 1, gy, gx)])), vy = by_rho(widen(p.u_cur[uidx(p, 2, gy, gx)]));
     const double vz = by_rho(widen(p.u_cur[uidx(p, 3, gy, gx)]));
     const double hr = 0.5 * rho;
     const double ekin = hr * (vx * vx) + hr * (vy * vy) + hr * (vz * vz);
     double P = (p.gamma - 1.0) * (widen(p.u_cur[uidx(p, 4, gy, gx)]) - ekin);
     P = max64_pos(P, p.smallp);
-    const Over<double> by_q(max64_pos(rho, p.smallr));
+    const Over<double, STATE_RANGE<R>> by_q(max64_pos(rho, p.smallr));
     return sqrt(by_q(p.gamma * P));
 }
 
 // Stopping times of a cell's species from the state at the start of the step (compute_tstop runs
 // before the update, solve.f90:34-35); qrho_old = max(rho_old, smallr).  What the species share (the
 // sound speed, the reciprocals) is formed once per cell.
-template <typename R>
+template <typename R, int WHERE = STATE_RANGE<R>>
 struct TStop {
     const KParams<R>& p;
     long long cell;
     double c0;
-    Over<double> by_q, by_d;   // qrho_old; the sound speed (dustyTurb) or Epstein's rho cs
+    Over<double, WHERE> by_q, by_d;   // qrho_old; the sound speed (dustyTurb) or Epstein's rho cs
     __device__ __forceinline__ TStop(const KParams<R>& p_, double qrho_old, int gx, int gy)
         : p(p_), cell((long long)gy * p_.pitch + gx), c0(0.0),
           by_q(p_.setup == SHARK_SETUP_DUSTYWAVE || p_.setup == SHARK_SETUP_DUSTYTURB ? qrho_old : 1.0),
@@ -435,18 +438,19 @@ struct TStop {
         if (p.setup == SHARK_SETUP_SI || p.setup == SHARK_SETUP_DUSTYWAVE) return 1.0;
         if (p.setup == SHARK_SETUP_DUSTYTURB) return p.csd[gx];
         if (p.setup == SHARK_SETUP_DISK_POLAR)   // Epstein on the midplane density Sigma/(sqrt(2 pi) H)
-            return Over<double>(p.hsd[gx])(qrho_old) * p.csd[gx];
+            return Over<double, CONSTANT>(p.hsd[gx])(qrho_old) * p.csd[gx];
         if (p.setup == SHARK_SETUP_DISK_CART) {  // disk/setup.f90 compute_tstop: Sigma/sqrt(2 pi H)
             const long long e = (long long)gy * p.pitch + gx;
-            return Over<double>(p.chsd[e])(qrho_old) * p.ccsd[e];
+            return Over<double, CONSTANT>(p.chsd[e])(qrho_old) * p.ccsd[e];
         }
         // Epstein (SOD/setup.f90:179-185) with the cell's sound speed
         return qrho_old * cs_start(p, gx, gy);
     }
+    __device__ __forceinline__ bool inside() const { return by_q.inside() && by_d.inside(); }
     __device__ __forceinline__ double operator()(int k) const {
         if (p.setup == SHARK_SETUP_SI) return p.dtstop[k];                       // SI/setup.f90:389-397
         if (p.setup == SHARK_SETUP_DUSTYWAVE)                                    // DUSTYWAVE/setup.f90:217
-            return by_q(Over<double>(p.dK[k])((double)p.u_cur[(5 + k) * p.plane + cell] * by_q.b));
+            return by_q(Over<double, CONSTANT>(p.dK[k])((double)p.u_cur[(5 + k) * p.plane + cell] * by_q.b));
         if (p.setup == SHARK_SETUP_DUSTYTURB)                                    // dustyTurb/setup.f90:456
             return by_q(by_d(p.dstokes[k] * p.box_l * c0));
         return by_d(c0 * p.dsize[k]);
@@ -455,16 +459,20 @@ struct TStop {
 
 // Drag heating of an adiabatic gas with back reaction (source_terms.f90:88-97): the energy
 // gains sum_k dt v.(v - v_k)/t_k with the velocities and stopping times at the start of the step.
-template <typename R>
-__device__ __forceinline__ double drag_heating(const KParams<R>& p, const TStop<R>& tstop, int gx, int gy, double dt) {
+// WHERE = TRIED: `inside` becomes false where a denominator lies outside div64_const's range.
+template <typename R, int WHERE>
+__device__ __forceinline__ double drag_heating(const KParams<R>& p, const TStop<R, WHERE>& tstop, int gx, int gy, double dt,
+                                               bool& inside) {
     const int N = p.ndust;
     const double rho = (double)p.u_cur[uidx(p, 0, gy, gx)];
-    const Over<double> by_rho(rho);
+    const Over<double, WHERE> by_rho(rho);
+    inside = tstop.inside() && by_rho.inside();
     const double vx = by_rho((double)p.u_cur[uidx(p, 1, gy, gx)]), vy = by_rho((double)p.u_cur[uidx(p, 2, gy, gx)]);
     const double vz = by_rho((double)p.u_cur[uidx(p, 3, gy, gx)]);
     double S = 0.0;
     for (int k = 0; k < N; ++k) {
-        const Over<double> by_ts(tstop(k)), by_rd((double)p.u_cur[uidx(p, 5 + k, gy, gx)]);
+        const Over<double, WHERE> by_ts(tstop(k)), by_rd((double)p.u_cur[uidx(p, 5 + k, gy, gx)]);
+        inside = inside && by_ts.inside() && by_rd.inside();
         const double vdx = by_rd((double)p.u_cur[uidx(p, 5 + N + k, gy, gx)]);
         const double vdy = by_rd((double)p.u_cur[uidx(p, 5 + 2 * N + k, gy, gx)]);
         const double vdz = by_rd((double)p.u_cur[uidx(p, 5 + 3 * N + k, gy, gx)]);
@@ -937,7 +945,7 @@ static __global__ void __launch_bounds__(GROWTH_D_THREADS) k_growth_d(KParams<do
         const int pr = g.pair[q], k = pr >> 8, j = pr & 255, kj = k * N + j;
         double a = 1.0;
         if (g.kernel == 0) {
-            const double pD = g.pD[kj], X = div64(div64(cB * g.pS[kj], pD, rcp64(pD)), g.uv2, yuv2);
+            const double pD = g.pD[kj], X = div64_const(div64_const(cB * g.pS[kj], pD, rcp64(pD)), g.uv2, yuv2);
             a = g.pA[kj] * growth_dv_pair_d(g, c, ts[k], ts[j], S[k], S[j], W[k], W[j], I[k], I[j], X, vx[k] - vx[j],
                                             vy[k] - vy[j], vz[k] - vz[j], G[k] - G[j], ambi);
         } else if (g.kernel == 2) {
@@ -959,8 +967,8 @@ static __global__ void __launch_bounds__(GROWTH_D_THREADS) k_growth_d(KParams<do
             const int pr = g.pair[q], k = pr >> 8, j = pr & 255;
             const double rk = rd[k], rj = rd[j];
             double d = (g.kernel == 1 ? rk : ka[i] * rk) * rj;
-            d = div64(div64(d, smk[k], symk[k]), smk[j], symk[j]);
-            if (hs_on) d = div64(d, hs, yhs);
+            d = div64_const(div64_const(d, smk[k], symk[k]), smk[j], symk[j]);
+            if (hs_on) d = div64_const(d, hs, yhs);
             if (k == j) d = 0.5 * d;
             if (thr_on && (is_less(rk, thr) || is_less(rj, thr))) d = 0.0;
             w[q] = d;
@@ -1016,7 +1024,7 @@ static __global__ void __launch_bounds__(GROWTH_D_THREADS) k_growth_d(KParams<do
 template <typename C, typename R>
 __device__ __forceinline__ void turb_kick_cell(const KParams<R>& p, R* u, int gx, int gy, double dt) {
     const C x = C(p.xposd[gx]);
-    const C y = C(Over<double>((double)(float)p.ny)(((double)(float)(gy - p.ng) + 0.5) * p.box_l_y));
+    const C y = C(Over<double, CONSTANT>((double)(float)p.ny)(((double)(float)(gy - p.ng) + 0.5) * p.box_l_y));
     C ax = C(0), ay = C(0);
     for (int m = 0; m < p.ou_nm; ++m) {
         if constexpr (sizeof(C) == 8) {
@@ -1041,6 +1049,196 @@ __device__ __forceinline__ void turb_kick_cell(const KParams<R>& p, R* u, int gx
     u[uidx(p, 2, gy, gx)] = R(C(u[uidx(p, 2, gy, gx)]) + rho * ay * C(dt));
 }
 
+// dust_drag(1.0) (src/dust/dust_drag.f90:2-75) of a cell, FP64 arithmetic; the stopping times are those of
+// the state at the start of the step (compute_tstop runs before the update in solve.f90:34-35).
+// CONST_TS: constant stopping times (SI box) take the step's coefficients from k_prepare_step (SI 256^2 x 8:
+// K2 0.102 -> 0.088 ms).  WHERE = TRIED: false, and nothing stored, where a denominator lies outside
+// div64_const's range.
+template <typename R, int NS, bool CONST_TS, int WHERE>
+__device__ __forceinline__ bool drag_cell_d(const KParams<R>& p, R* u, const TStop<R, WHERE>& tstop, int gx, int gy, double dt,
+                                            double rho, double& px, double& py, double& pz) {
+    constexpr int NMAX = NS > 0 ? NS : 1;
+    const int N = NS >= 0 ? NS : p.ndust;
+    bool inside = tstop.inside();
+    const double* cd = reinterpret_cast<const double*>(p.coef + SHARK_COEF_D);
+    double alpha[NMAX];
+    double rhon = rho, pnx = px, pny = py, pnz = pz;
+    for (int k = 0; k < N; ++k) {
+        double w;
+        if constexpr (CONST_TS) w = cd[k];
+        else {
+            const Over<double, WHERE> by_ts(tstop(k));
+            const double a = by_ts(dt);
+            const Over<double, WHERE> by_a(1.0 + a);
+            w = by_a(a);
+            inside = inside && by_ts.inside() && by_a.inside();
+            if (NS > 0) alpha[k < NMAX ? k : 0] = a;
+        }
+        pnx = pnx + w * (double)u[uidx(p, 5 + N + k, gy, gx)];
+        pny = pny + w * (double)u[uidx(p, 5 + 2 * N + k, gy, gx)];
+        pnz = pnz + w * (double)u[uidx(p, 5 + 3 * N + k, gy, gx)];
+        rhon = rhon + w * (double)u[uidx(p, 5 + k, gy, gx)];
+    }
+    const Over<double, WHERE> by_rhon(rhon);
+    if (WHERE == TRIED) {
+        if constexpr (CONST_TS)
+            for (int k = 0; k < N; ++k) inside = inside && is_plain(cd[2 * SHARK_MAX_DUST + k]);
+        if (!inside || !by_rhon.inside()) return false;
+    }
+    const double fl = rho * p.dust_ratio_min;   // regularisation floor (dust_drag.f90:63-73)
+    constexpr int CH = 4;   // species whose loads are in flight together
+#pragma unroll
+    for (int k0 = 0; k0 < (NS > 0 ? NS : N); k0 += CH) {
+        double d[CH], m[CH][3];
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            if (k0 + i >= N) break;
+            d[i] = (double)u[uidx(p, 5 + k0 + i, gy, gx)];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) m[i][c] = (double)u[uidx(p, 5 + (c + 1) * N + k0 + i, gy, gx)];
+        }
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const int k = k0 + i;
+            if (k >= N) break;
+            double a = 0.0;
+            if constexpr (!CONST_TS) {
+                if (NS > 0) a = alpha[k < NMAX ? k : 0];
+                else a = Over<double, WHERE>(tstop(k))(dt);    // run-time species count
+            }
+            const Over<double, WHERE> by_a = CONST_TS ? Over<double, WHERE>(cd[SHARK_MAX_DUST + k], cd[2 * SHARK_MAX_DUST + k])
+                                                       : Over<double, WHERE>(1.0 + a);
+            const double w = CONST_TS ? cd[k] : by_a(a);
+            u[uidx(p, 5 + N + k, gy, gx)] = R(by_a(m[i][0]) + by_rhon(w * pnx) * d[i]);
+            u[uidx(p, 5 + 2 * N + k, gy, gx)] = R(by_a(m[i][1]) + by_rhon(w * pny) * d[i]);
+            u[uidx(p, 5 + 3 * N + k, gy, gx)] = R(by_a(m[i][2]) + by_rhon(w * pnz) * d[i]);
+            if (is_less(d[i], fl)) u[uidx(p, 5 + k, gy, gx)] = R(fl);
+        }
+    }
+    if (p.flags & SHARK_FLAG_BACK_REACTION) {
+        px = by_rhon(pnx) * rho;
+        py = by_rhon(pny) * rho;
+        pz = by_rhon(pnz) * rho;
+        u[uidx(p, 1, gy, gx)] = R(px);
+        u[uidx(p, 2, gy, gx)] = R(py);
+        u[uidx(p, 3, gy, gx)] = R(pz);
+    }
+    return true;
+}
+
+// courant on the final state of a cell (src/solver/courant.f90:11-124): the time step it allows and its
+// status bits.  WHERE = TRIED: `inside` is false where a denominator lies outside div64_const's range.
+struct CourantCell {
+    double dt;
+    unsigned bits;
+    bool inside;
+};
+template <typename R, int NS, int WHERE>
+__device__ __forceinline__ CourantCell courant_cell_d(const KParams<R>& p, const R* u, int gx, int gy, double rho, double px,
+                                                      double py, double pz) {
+    const int N = NS >= 0 ? NS : p.ndust;
+    double dtc;
+    unsigned bits = 0;
+    const double cfl = p.cfl;
+    const Over<double, WHERE> by_rho(rho);
+    bool inside = by_rho.inside();
+    const double vx = by_rho(px), vy = by_rho(py), vz = by_rho(pz);
+    double cs;
+    if (p.iso == 1) cs = p.ccsd ? p.ccsd[(long long)gy * p.pitch + gx] : p.csd[gx];
+    else {
+        const double qrho = max64_pos(rho, p.smallr);
+        const double E = (double)u[uidx(p, 4, gy, gx)];
+        const double hr = 0.5 * rho;
+        const double ekin = hr * (vx * vx) + hr * (vy * vy) + hr * (vz * vz);
+        const double P = max64_pos((p.gamma - 1.0) * (E - ekin), p.smallp);
+        const Over<double, WHERE> by_q(qrho);
+        cs = sqrt(by_q(p.gamma * P));
+        inside = inside && by_q.inside();
+        if (abs_bits(E) > 0x7ff0000000000000ull) bits |= SHARK_STATUS_NAN;
+    }
+    double dxx;
+    if (p.ndim == 1) dxx = p.dx1d[gx];
+    else if (p.geom == 2) dxx = min64(p.dx1d[gx], p.radcd[gx] * p.dx2d[gx]);
+    else dxx = min64(p.dx1d[gx], p.dx2d[gx]);
+    double vv = abs64(vx) + abs64(vy) + abs64(vz);
+    double vmax = cs + vv;
+    double fmax_d = 0.0;     // SI: the largest square of a force until its root is taken below
+    const bool fk = (p.flags & SHARK_FLAG_FORCE_KICK) != 0;
+    const bool fk_si = fk && p.setup == SHARK_SETUP_SI;
+    double tide = 0.0, om2 = 0.0;
+    if (fk_si) {
+        const double xc = p.xposd[gx] - 0.5 * p.box_l, om = p.si_om, qsh = p.si_q;
+        tide = 2.0 * qsh * (om * om) * xc;
+        om2 = 2.0 * om;
+        const double f1 = tide - om2 * vz - 2.0 * p.si_r0 * om * p.si_eta;
+        const double f3 = om2 * vx;
+        fmax_d = f1 * f1 + f3 * f3;
+    } else if (fk && p.setup == SHARK_SETUP_DISK_POLAR) {
+        // the same point-mass force acts on gas and every dust species
+        const double g = p.fgravd[gx];
+        fmax_d = sqrt(g * g);
+    } else if (fk && p.setup == SHARK_SETUP_DISK_CART) {   // the star's softened force, gas and dust
+        const long long e = (long long)gy * p.pitch + gx;
+        const double fx = (double)p.cfx[e], fy = (double)p.cfy[e];
+        fmax_d = sqrt(fx * fx + fy * fy);
+    }
+    for (int k = 0; k < N; ++k) {
+        const double rd = (double)u[uidx(p, 5 + k, gy, gx)];
+        const Over<double, WHERE> by_rd(rd);
+        inside = inside && by_rd.inside();
+        const double vdx = by_rd((double)u[uidx(p, 5 + N + k, gy, gx)]);
+        const double vdy = by_rd((double)u[uidx(p, 5 + 2 * N + k, gy, gx)]);
+        const double vdz = by_rd((double)u[uidx(p, 5 + 3 * N + k, gy, gx)]);
+        vv = abs64(vdx) + abs64(vdy) + abs64(vdz);
+        vmax = is_less(vv, vmax) ? vmax : vv;
+        if (fk_si) {
+            const double f1 = tide - om2 * vdz;
+            const double f3 = om2 * vdx;
+            const double fm = f1 * f1 + f3 * f3;
+            fmax_d = is_less(fm, fmax_d) ? fmax_d : fm;
+        }
+        if (!is_pos(rd)) bits |= SHARK_STATUS_NEG_DENSITY;
+        if (!is_finite(vdx) || !is_finite(vdy) || !is_finite(vdz)) bits |= SHARK_STATUS_NAN;
+    }
+    if (fk_si) fmax_d = sqrt(fmax_d);
+    const double cd = cfl * dxx;
+    // plain divisions where a wave speed may be zero or its square underflow
+    const double c1 = cd / abs64(vmax);
+    dtc = is_less(2e44, c1) ? 2e44 : c1;
+    if (fk && !is_zero(vv)) {
+        double fratio = fmax_d * dxx / (vv * vv);
+        fratio = max64_pos(fratio, 1e-3);
+        const Over<double, WHERE> by_f(fratio);
+        inside = inside && by_f.inside();
+        const double c2 = by_f(cd / vv * (sqrt(1.0 + 2.0 * cfl * fratio) - 1.0));
+        dtc = is_less(dtc, c2) ? dtc : c2;
+    }
+    if (!is_pos(rho)) bits |= SHARK_STATUS_NEG_DENSITY;
+    if (!is_finite(vx) || !is_finite(vy) || !is_finite(vz) || !is_finite(rho)) bits |= SHARK_STATUS_NAN;
+    if (!is_pos(dtc) || !is_finite(dtc)) { bits |= SHARK_STATUS_DT_UNDERFLOW; dtc = 2e44; }
+    return CourantCell{dtc, bits, inside};
+}
+
+// The same for a cell with a denominator outside the range: out of line, so that the kernels keep to the
+// registers and the code of the other form.
+template <typename R>
+static __device__ __noinline__ void drag_cell_wide(const KParams<R>& p, R* u, int gx, int gy, double dt, double qrho_old, double rho,
+                                                   double* m) {
+    const TStop<R> tstop(p, qrho_old, gx, gy);
+    if (p.setup == SHARK_SETUP_SI) drag_cell_d<R, -1, true, ANYWHERE>(p, u, tstop, gx, gy, dt, rho, m[0], m[1], m[2]);
+    else drag_cell_d<R, -1, false, ANYWHERE>(p, u, tstop, gx, gy, dt, rho, m[0], m[1], m[2]);
+}
+template <typename R>
+static __device__ __noinline__ double drag_heating_wide(const KParams<R>& p, double qrho_old, int gx, int gy, double dt) {
+    bool inside;
+    return drag_heating(p, TStop<R>(p, qrho_old, gx, gy), gx, gy, dt, inside);
+}
+template <typename R>
+static __device__ __noinline__ CourantCell courant_cell_wide(const KParams<R>& p, const R* u, int gx, int gy, double rho, double px,
+                                                             double py, double pz) {
+    return courant_cell_d<R, -1, ANYWHERE>(p, u, gx, gy, rho, px, py, pz);
+}
+
 // Bound by the FP64 pipe (64 clocks of an SM partition for a warp's instruction): quotients share
 // reciprocals, compares and finiteness checks run on the bits, one square root takes the largest of
 // the force limiter's sums; all exact.  SI boxes of 8 species: 1024^2 2.36 -> 1.38 ms, 256^2 0.183 ->
@@ -1048,9 +1246,12 @@ __device__ __forceinline__ void turb_kick_cell(const KParams<R>& p, R* u, int gx
 // thousand cells then each have a partition of their own.
 constexpr int K2D_THREADS = 128;
 
+// Blocks an SM: without the bound the compiler takes up to 238 registers to overlap the quotients, and the
+// fewer warps cost more (us, SI 256^2: 1 species 46 -> 32, 4 species 75 -> 57, 8 species 109 -> 89).
+constexpr int k2d_blocks(int NS) { return NS == 0 ? 6 : NS == 1 || NS == 2 ? 5 : 4; }
+
 template <typename R, int NS, int MODE, bool GROW = false>
-__global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
-    constexpr int NMAX = NS > 0 ? NS : 1;
+__global__ void __launch_bounds__(K2D_THREADS, k2d_blocks(NS)) k_finalize(const __grid_constant__ KParams<R> p) {
     constexpr bool DRAG = MODE == 0 || MODE == 2, REST = MODE == 0 || MODE == 3;
     const int N = NS >= 0 ? NS : p.ndust;
     const int gx = blockIdx.x * blockDim.x + threadIdx.x + p.ng;
@@ -1071,72 +1272,24 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
             // stopping times from the state at the start of the step (compute_tstop runs before the
             // update in solve.f90:34-35)
             const double rho_old = (double)p.u_cur[uidx(p, 0, gy, gx)];
-            const TStop<R> tstop(p, max64_pos(rho_old, p.smallr), gx, gy);
-            // dust_drag(1.0) (src/dust/dust_drag.f90:2-75), FP64 arithmetic; constant stopping times (SI box)
-            // take the step's coefficients from k_prepare_step (SI 256^2 x 8: K2 0.102 -> 0.088 ms)
-            auto drag_update = [&](auto constant) {
-                constexpr bool const_ts = decltype(constant)::value;
-                const double* cd = reinterpret_cast<const double*>(p.coef + SHARK_COEF_D);
-                double alpha[NMAX];
-                double rhon = rho, pnx = px, pny = py, pnz = pz;
-                for (int k = 0; k < N; ++k) {
-                    double w;
-                    if constexpr (const_ts) w = cd[k];
-                    else {
-                        const double a = Over<double>(tstop(k))(dt);
-                        w = Over<double>(1.0 + a)(a);
-                        if (NS > 0) alpha[k < NMAX ? k : 0] = a;
-                    }
-                    pnx = pnx + w * (double)u[uidx(p, 5 + N + k, gy, gx)];
-                    pny = pny + w * (double)u[uidx(p, 5 + 2 * N + k, gy, gx)];
-                    pnz = pnz + w * (double)u[uidx(p, 5 + 3 * N + k, gy, gx)];
-                    rhon = rhon + w * (double)u[uidx(p, 5 + k, gy, gx)];
+            const double qrho_old = max64_pos(rho_old, p.smallr);
+            const TStop<R, TRIED> tstop(p, qrho_old, gx, gy);
+            if (drag) {
+                bool done;
+                if (p.setup == SHARK_SETUP_SI) done = drag_cell_d<R, NS, true, TRIED>(p, u, tstop, gx, gy, dt, rho, px, py, pz);
+                else done = drag_cell_d<R, NS, false, TRIED>(p, u, tstop, gx, gy, dt, rho, px, py, pz);
+                if (!done) {
+                    double m[3] = {px, py, pz};
+                    drag_cell_wide(p, u, gx, gy, dt, qrho_old, rho, m);
+                    px = m[0]; py = m[1]; pz = m[2];
                 }
-                const Over<double> by_rhon(rhon);
-                const double fl = rho * p.dust_ratio_min;   // regularisation floor (dust_drag.f90:63-73)
-                constexpr int CH = 4;   // species whose loads are in flight together
-#pragma unroll
-                for (int k0 = 0; k0 < (NS > 0 ? NS : N); k0 += CH) {
-                    double d[CH], m[CH][3];
-#pragma unroll
-                    for (int i = 0; i < CH; ++i) {
-                        if (k0 + i >= N) break;
-                        d[i] = (double)u[uidx(p, 5 + k0 + i, gy, gx)];
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) m[i][c] = (double)u[uidx(p, 5 + (c + 1) * N + k0 + i, gy, gx)];
-                    }
-#pragma unroll
-                    for (int i = 0; i < CH; ++i) {
-                        const int k = k0 + i;
-                        if (k >= N) break;
-                        double a = 0.0;
-                        if constexpr (!const_ts) {
-                            if (NS > 0) a = alpha[k < NMAX ? k : 0];
-                            else a = Over<double>(tstop(k))(dt);    // run-time species count
-                        }
-                        const Over<double> by_a = const_ts ? Over<double>(cd[SHARK_MAX_DUST + k], cd[2 * SHARK_MAX_DUST + k])
-                                                           : Over<double>(1.0 + a);
-                        const double w = const_ts ? cd[k] : by_a(a);
-                        u[uidx(p, 5 + N + k, gy, gx)] = R(by_a(m[i][0]) + by_rhon(w * pnx) * d[i]);
-                        u[uidx(p, 5 + 2 * N + k, gy, gx)] = R(by_a(m[i][1]) + by_rhon(w * pny) * d[i]);
-                        u[uidx(p, 5 + 3 * N + k, gy, gx)] = R(by_a(m[i][2]) + by_rhon(w * pnz) * d[i]);
-                        if (is_less(d[i], fl)) u[uidx(p, 5 + k, gy, gx)] = R(fl);
-                    }
-                }
-                if (br) {
-                    px = by_rhon(pnx) * rho;
-                    py = by_rhon(pny) * rho;
-                    pz = by_rhon(pnz) * rho;
-                    u[uidx(p, 1, gy, gx)] = R(px);
-                    u[uidx(p, 2, gy, gx)] = R(py);
-                    u[uidx(p, 3, gy, gx)] = R(pz);
-                }
-            };
-            if (drag && p.setup == SHARK_SETUP_SI) drag_update(std::true_type{});
-            else if (drag) drag_update(std::false_type{});
+            }
             if (heat) {   // drag heating, part of S_U (source_terms.f90:88-97)
                 const long long ie = uidx(p, 4, gy, gx);
-                u[ie] = R((double)u[ie] + drag_heating(p, tstop, gx, gy, dt));
+                bool inside = true;
+                double gain = drag_heating(p, tstop, gx, gy, dt, inside);
+                if (!inside) gain = drag_heating_wide(p, qrho_old, gx, gy, dt);
+                u[ie] = R((double)u[ie] + gain);
             }
         }
         if (GROW && MODE == 0) st |= grow_in_finalize(p, u, gx, gy, dt);   // dust_growth (solve.f90:113)
@@ -1178,78 +1331,10 @@ __global__ void __launch_bounds__(K2D_THREADS) k_finalize(KParams<R> p) {
             pz = (double)u[uidx(p, 3, gy, gx)];
         }
         if (MODE == 2) return;   // k_growth_d and MODE 3 follow
-        // ---- courant on the final state (src/solver/courant.f90:11-124) -----------------------
-        const double cfl = p.cfl;
-        const Over<double> by_rho(rho);
-        const double vx = by_rho(px), vy = by_rho(py), vz = by_rho(pz);
-        double cs;
-        if (p.iso == 1) cs = p.ccsd ? p.ccsd[(long long)gy * p.pitch + gx] : p.csd[gx];
-        else {
-            const double qrho = max64_pos(rho, p.smallr);
-            const double E = (double)u[uidx(p, 4, gy, gx)];
-            const double hr = 0.5 * rho;
-            const double ekin = hr * (vx * vx) + hr * (vy * vy) + hr * (vz * vz);
-            const double P = max64_pos((p.gamma - 1.0) * (E - ekin), p.smallp);
-            cs = sqrt(Over<double>(qrho)(p.gamma * P));
-            if (abs_bits(E) > 0x7ff0000000000000ull) st |= SHARK_STATUS_NAN;
-        }
-        double dxx;
-        if (p.ndim == 1) dxx = p.dx1d[gx];
-        else if (p.geom == 2) dxx = min64(p.dx1d[gx], p.radcd[gx] * p.dx2d[gx]);
-        else dxx = min64(p.dx1d[gx], p.dx2d[gx]);
-        double vv = abs64(vx) + abs64(vy) + abs64(vz);
-        double vmax = cs + vv;
-        double fmax_d = 0.0;     // SI: the largest square of a force until its root is taken below
-        const bool fk = (p.flags & SHARK_FLAG_FORCE_KICK) != 0;
-        const bool fk_si = fk && p.setup == SHARK_SETUP_SI;
-        double tide = 0.0, om2 = 0.0;
-        if (fk_si) {
-            const double xc = p.xposd[gx] - 0.5 * p.box_l, om = p.si_om, qsh = p.si_q;
-            tide = 2.0 * qsh * (om * om) * xc;
-            om2 = 2.0 * om;
-            const double f1 = tide - om2 * vz - 2.0 * p.si_r0 * om * p.si_eta;
-            const double f3 = om2 * vx;
-            fmax_d = f1 * f1 + f3 * f3;
-        } else if (fk && p.setup == SHARK_SETUP_DISK_POLAR) {
-            // the same point-mass force acts on gas and every dust species
-            const double g = p.fgravd[gx];
-            fmax_d = sqrt(g * g);
-        } else if (fk && p.setup == SHARK_SETUP_DISK_CART) {   // the star's softened force, gas and dust
-            const long long e = (long long)gy * p.pitch + gx;
-            const double fx = (double)p.cfx[e], fy = (double)p.cfy[e];
-            fmax_d = sqrt(fx * fx + fy * fy);
-        }
-        for (int k = 0; k < N; ++k) {
-            const double rd = (double)u[uidx(p, 5 + k, gy, gx)];
-            const Over<double> by_rd(rd);
-            const double vdx = by_rd((double)u[uidx(p, 5 + N + k, gy, gx)]);
-            const double vdy = by_rd((double)u[uidx(p, 5 + 2 * N + k, gy, gx)]);
-            const double vdz = by_rd((double)u[uidx(p, 5 + 3 * N + k, gy, gx)]);
-            vv = abs64(vdx) + abs64(vdy) + abs64(vdz);
-            vmax = is_less(vv, vmax) ? vmax : vv;
-            if (fk_si) {
-                const double f1 = tide - om2 * vdz;
-                const double f3 = om2 * vdx;
-                const double fm = f1 * f1 + f3 * f3;
-                fmax_d = is_less(fm, fmax_d) ? fmax_d : fm;
-            }
-            if (!is_pos(rd)) st |= SHARK_STATUS_NEG_DENSITY;
-            if (!is_finite(vdx) || !is_finite(vdy) || !is_finite(vdz)) st |= SHARK_STATUS_NAN;
-        }
-        if (fk_si) fmax_d = sqrt(fmax_d);
-        const double cd = cfl * dxx;
-        // plain divisions where a wave speed may be zero or its square underflow
-        const double c1 = cd / abs64(vmax);
-        dtc = is_less(2e44, c1) ? 2e44 : c1;
-        if (fk && !is_zero(vv)) {
-            double fratio = fmax_d * dxx / (vv * vv);
-            fratio = max64_pos(fratio, 1e-3);
-            const double c2 = Over<double>(fratio)(cd / vv * (sqrt(1.0 + 2.0 * cfl * fratio) - 1.0));
-            dtc = is_less(dtc, c2) ? dtc : c2;
-        }
-        if (!is_pos(rho)) st |= SHARK_STATUS_NEG_DENSITY;
-        if (!is_finite(vx) || !is_finite(vy) || !is_finite(vz) || !is_finite(rho)) st |= SHARK_STATUS_NAN;
-        if (!is_pos(dtc) || !is_finite(dtc)) { st |= SHARK_STATUS_DT_UNDERFLOW; dtc = 2e44; }
+        CourantCell c = courant_cell_d<R, NS, TRIED>(p, u, gx, gy, rho, px, py, pz);
+        if (!c.inside) c = courant_cell_wide(p, u, gx, gy, rho, px, py, pz);
+        dtc = c.dt;
+        st |= c.bits;
     }
     if (MODE == 2) return;
     block_reduce_dt(dtc, st, p.dt_next, p.status);
@@ -1294,7 +1379,7 @@ struct DragCell {
     const KParams<float>& p;
     int cc;
     double dt, dtF, w, heat, px, py, pz;   // w = p.p/rho, heat: sum of rho dt v.(v - v_k)/t_k
-    Over<double> by_rho;
+    Over<double, CONSTANT> by_rho;
     bool wave, heats;
     __device__ __forceinline__ DragCell(const KParams<float>& p_, double dt_, double qrho_old, int gx, int gy, bool heats_,
                                         bool used = true)
@@ -1323,7 +1408,7 @@ struct DragCell {
     }
     // a_k = dt/t_k of species k, its heating added; o = load(k)
     __device__ __forceinline__ double operator()(int k, float4 o) {
-        const Over<double> by_rd(widen(o.x));
+        const Over<double, CONSTANT> by_rd(widen(o.x));
         const double a = wave ? by_rd(dt * p.dK[k]) : dtF * p.dinvts[k];
         if (heats) heat += a * (w - by_rd(px * widen(o.y) + py * widen(o.z) + pz * widen(o.w)));
         return a;
@@ -1580,7 +1665,8 @@ k_finalize_mixed(KParams<float> p) {
             const long long ie = uidx(p, 4, gy, gx);
             if (!heated) {
                 const double rho_old = (double)ucur[cc];
-                gain = drag_heating(p, TStop<float>(p, max64_pos(rho_old, p.smallr), gx, gy), gx, gy, dt);
+                bool inside;
+                gain = drag_heating(p, TStop<float>(p, max64_pos(rho_old, p.smallr), gx, gy), gx, gy, dt, inside);
             }
             u[ie] = narrow(widen(u[ie]) + gain);
         }
