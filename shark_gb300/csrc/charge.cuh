@@ -165,7 +165,9 @@ __device__ __forceinline__ void charge_newton_d(const ChargeParams<R>& p, int ro
     const double rth = rcp64(th), rxnH = rcp64_any(x * nH);
     const R ihsr = R(ihs);
     while (conv > p.eps && niter < p.nitermax) {
-        const double eps = (1.0 - psi) * rth * exp(-psi), et = eps * th, et2 = et * et;
+        // eps is the reference's quotient to the bit: where the column shields the ions psi goes to -0 (1e-20 at
+        // 4e3 g/cm2), et to 1, and the root lies where 1 - et^2 is exactly zero
+        const double eps = div64_const(1.0 - psi, th, rth) * exp(-psi), et = eps * th, et2 = et * et;
         double T2, T4;
         R S2, S5;
         if constexpr (sizeof(R) == 8) {
