@@ -92,11 +92,10 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
 __device__ __forceinline__ double recip(double b) { return rcp64_any(b); }
 __device__ __forceinline__ float recip(float b) { return 1.0f / b; }
 
-// f(psi) in arithmetic C and its derivative in arithmetic E from the iteration's sums, 1/hs in all of
-// them, and the update of psi.  Newton needs f' to a few digits only: the mixed path forms it in FP32,
-// as it does the sums S2 and S5 in it.  Returns f at the psi it came with.
-template <typename C, typename E>
-__device__ __forceinline__ C charge_update(C T1, C T2, C T3, C T4, E S2, E S5, C eps_psi, C thetai, C rxnH, C sigmav_ie,
+// f(psi) and its derivative from the iteration's sums, 1/hs in all of them, and the update of psi.
+// Returns f at the psi it came with.
+template <typename C>
+__device__ __forceinline__ C charge_update(C T1, C T2, C T3, C T4, C S2, C S5, C eps_psi, C thetai, C rxnH, C sigmav_ie,
                                            C vi, C psi0, C& psi, int& lowT) {
     const C one = C(1), two = C(2);
     const C et = eps_psi * thetai, et2 = et * et, et21 = et2 + et, rom = recip(one - eps_psi);
@@ -104,14 +103,13 @@ __device__ __forceinline__ C charge_update(C T1, C T2, C T3, C T4, E S2, E S5, C
     const C S1 = (one - psi) * T3 + two * et21 * T4;
     const C nv = n_i * vi * rxnH, ns = sigmav_ie * n_i * rxnH;
     const C f = ns * eps_psi * n_i + nv * S1 - one;
-    const E e1 = E(1), e2 = E(2), p = E(psi), ep = E(eps_psi), t = E(et), ro = E(rom), ni = E(n_i), nve = E(nv), nse = E(ns);
-    const E D = -ep * (e2 - p) * recip(e1 - p);
-    const E dni = -(ro * ro) * D * S2 - (p * ro * D + e1) * E(T1) * ro;
-    const E q = dni * recip(ni);
-    const E df = nse * (ni * D + e2 * ep * dni) +
-                 e2 * nve * E(et21) * ((q + D * (e2 * t + e1) * recip(ep * (e1 + t))) * E(T4) + D * S5) +
-                 nve * (q * (e1 - p) - e1) * E(T3);
-    psi = psi - C(E(f) * recip(df));
+    const C D = -eps_psi * (two - psi) * recip(one - psi);
+    const C dni = -(rom * rom) * D * S2 - (psi * rom * D + one) * T1 * rom;
+    const C q = dni * recip(n_i);
+    const C df = ns * (n_i * D + two * eps_psi * dni) +
+                 two * nv * et21 * ((q + D * (two * et + one) * recip(eps_psi * (one + et))) * T4 + D * S5) +
+                 nv * (q * (one - psi) - one) * T3;
+    psi = psi - f * recip(df);
     if (psi < psi0) {
         psi = psi0 * C(0.9999999);
         lowT = 1;
@@ -147,15 +145,15 @@ __device__ __forceinline__ void charge_newton_f(const ChargeParams<R>& p, const 
             S5 += w * r * (c5 + th * a.x);
         }
         const float prev = psi;
-        conv = fabsf(charge_update<float, float>(T1, ihs * T2, T3, ihs * T4, ihs * S2, ihs * S5, eps, th, rxnH, sigmav_ie, vi, psi0, psi, lowT));
+        conv = fabsf(charge_update<float>(T1, ihs * T2, T3, ihs * T4, ihs * S2, ihs * S5, eps, th, rxnH, sigmav_ie, vi, psi0, psi, lowT));
         niter = niter + 1;
         if (psi == prev) break;
     }
 }
 
 // FP64 iterations to the reference's stopping test |f| < chg_eps.  FP64 path: the four sums in FP64.
-// Mixed path: T2 and T4, corrections of a few per cent, in compensated FP32 (f accurate to ~1e-8),
-// the derivative in FP32.
+// Mixed path: T2 and T4, corrections of a few per cent, in compensated FP32 (f accurate to ~1e-8), and
+// the derivative's sums S2 and S5 in FP32 (Newton needs f' to a few digits).
 template <typename R>
 __device__ __forceinline__ void charge_newton_d(const ChargeParams<R>& p, int row, const R* uk, double T1, double T3, double ihs,
                                                 double nH, double x, double sigmav_ie, double vi, double& psi, int& niter,
@@ -163,13 +161,11 @@ __device__ __forceinline__ void charge_newton_d(const ChargeParams<R>& p, int ro
     const int N = p.ndust, rows = p.rows;
     const double th = p.thetai, th2 = p.th2, th3 = p.th3, psi0 = p.psi0;
     const double rth = rcp64(th), rxnH = rcp64_any(x * nH);
-    const R ihsr = R(ihs);
     while (conv > p.eps && niter < p.nitermax) {
         // eps is the reference's quotient to the bit: where the column shields the ions psi goes to -0 (1e-20 at
         // 4e3 g/cm2), et to 1, and the root lies where 1 - et^2 is exactly zero
         const double eps = div64_const(1.0 - psi, th, rth) * exp(-psi), et = eps * th, et2 = et * et;
-        double T2, T4;
-        R S2, S5;
+        double T2, T4, S2, S5;
         if constexpr (sizeof(R) == 8) {
             const double *al = p.alpha + row, *pt = p.ptau + row;
             const double e2 = eps * eps, et21 = 1.0 + et2;
@@ -201,10 +197,10 @@ __device__ __forceinline__ void charge_newton_d(const ChargeParams<R>& p, int ro
                 s2 = s2 + nr * f2;
                 s5 = s5 + nr * a.z * (c5 + thf * a.x) * r;
             }
-            T2 = widen(t2); T4 = widen(t4); S2 = s2; S5 = s5;
+            T2 = widen(t2); T4 = widen(t4); S2 = widen(s2); S5 = widen(s5);
         }
         const double prev = psi;
-        conv = abs64(charge_update<double, R>(T1, ihs * T2, T3, ihs * T4, ihsr * S2, ihsr * S5, eps, th, rxnH, sigmav_ie, vi, psi0, psi, lowT));
+        conv = abs64(charge_update<double>(T1, ihs * T2, T3, ihs * T4, ihs * S2, ihs * S5, eps, th, rxnH, sigmav_ie, vi, psi0, psi, lowT));
         niter = niter + 1;
         // an unchanged psi with the residual above the tolerance repeats itself until nitermax
         // (e.g. the psi0 clamp): go there directly, same final state
@@ -298,11 +294,12 @@ __device__ __forceinline__ void charge_outputs(const ChargeParams<R>& p, int row
 // the mixed path begins a cold or seeded cell with FP32 iterations.  The iteration count is the sum
 // of both phases.  Bound by the FP64 pipe: per iteration FP64 spends 17 instructions for a species
 // (some 160 as the reference's expressions, whose shared factors and invariants it re-formed) and
-// some 75 for the cell; the mixed path some 45 for the cell (its derivative is FP32) and two a
-// species for T1 and T3.
+// some 75 for the cell, the mixed path those 75 and two a species for T1 and T3.  (With the derivative's
+// scalars in FP32 the mixed path took 45, driven box 0.59 and polar disk 0.42 ms, and lost cells whose
+// scalars leave FP32's range: shielded columns, test_gpu_charge_shielded.py.)
 // Temperature tables are laid out species by species, so that a warp's columns read them together.
-// Cold start, 384^2 x 32: FP64 24.4 -> 4.0 ms, mixed 1.54 -> 0.25; warm, driven box 768^2 x 32 mixed 1.00 -> 0.62 ms a step, polar disk
-// 512 x 1024 x 16 0.675 -> 0.43, 128 x 256 x 16 FP64 0.68 -> 0.15.
+// Cold start, 384^2 x 32: FP64 24.4 -> 4.0 ms, mixed 1.54 -> 0.25; warm, driven box 768^2 x 32 mixed 1.00 ->
+// 0.71 ms a step, polar disk 512 x 1024 x 16 0.675 -> 0.49, 128 x 256 x 16 FP64 0.68 -> 0.15.
 template <typename R>
 __global__ void __launch_bounds__(128) k_charge(ChargeParams<R> p) {
     const int N = p.ndust;
