@@ -61,7 +61,7 @@ struct ChargeParams {
     const float* seed;           // [plane] network start points (nullptr: none)
     int32_t* iters;              // [plane] Newton iterations of the last call
     unsigned long long* hist;    // [CHARGE_HIST + 2]: histogram, non-converged cells, total iterations
-    unsigned long long* stamps;  // [1]: device clock at the end of the charging (the latest block's)
+    unsigned long long* stamps;  // [1]: device clock at the end of a step's charging (the latest block's); null outside a step
     unsigned int* status;        // the step's status word: SHARK_STATUS_NEWTON if a cell did not converge
 };
 
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(128) k_charge(ChargeParams<R> p) {
         if (s_hist[b]) atomicAdd(&p.hist[b], (unsigned long long)s_hist[b]);
     if (threadIdx.x == 0 && s_iter) atomicAdd(&p.hist[CHARGE_HIST + 1], s_iter);
     if (threadIdx.x == 0 && s_hist[CHARGE_HIST] && p.status) atomicOr(p.status, (unsigned)SHARK_STATUS_NEWTON);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && p.stamps) {
         unsigned long long now;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
         atomicMax(p.stamps + 1, now);
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(128) k_charge_fujii(ChargeParams<R> p, double 
         if (s_hist[b]) atomicAdd(&p.hist[b], (unsigned long long)s_hist[b]);
     if (threadIdx.x == 0 && s_iter) atomicAdd(&p.hist[CHARGE_HIST + 1], s_iter);
     if (threadIdx.x == 0 && s_hist[CHARGE_HIST] && p.status) atomicOr(p.status, (unsigned)SHARK_STATUS_NEWTON);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && p.stamps) {
         unsigned long long now;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
         atomicMax(p.stamps + 1, now);

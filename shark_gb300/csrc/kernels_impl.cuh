@@ -384,7 +384,7 @@ cudaError_t launch_step(const DeviceView& v, int slot) {
     const int const_ts = p.setup != SHARK_SETUP_SI ? 0 : std::is_same<R, float>::value ? 1 : 2;
     launch_chained(chained, k_prepare_step, dim3(1), dim3(SHARK_MAX_DUST), 0, v.stream, p.dt_next, p.dt, p.dtstop, p.ndust, const_ts,
                    p.coef, v.dt_log, v.post, (const unsigned int*)v.status, v.post_step, v.stamps);
-    if (v.chg.on && (e = launch_charge<R>(v)) != cudaSuccess) return e;   // charge: solve.f90:36-42
+    if (v.chg.on && (e = launch_charge<R>(v, true)) != cudaSuccess) return e;   // charge: solve.f90:36-42
     if (v.ou_nm > 0)   // this step's forcing coefficients, from the dt on the device
         k_ou_update<<<1, 2 * v.ou_nm, 0, v.stream>>>(v.ou, v.ou_modes, v.ou_f, v.ou_nm, p.dt, v.ou_sigma, v.ou_tcorr, v.ou_seed, v.step,
                                                      v.stamps);
@@ -468,14 +468,15 @@ static ChargeParams<R> charge_params(const DeviceView& v) {
     q.psi_old = c.psi_old; q.zd = (R*)c.zd; q.ni = (R*)c.ni; q.ne = (R*)c.ne; q.eta = (R*)c.eta;
     q.gamma_d = (R*)c.gamma_d; q.seed = c.seed; q.hist = c.hist; q.iters = c.iters;
     q.status = v.status;
-    q.stamps = v.stamps;
+    q.stamps = nullptr;
     return q;
 }
 
 template <typename R>
-cudaError_t launch_charge(const DeviceView& v) {
+cudaError_t launch_charge(const DeviceView& v, bool in_step) {
     const ChargeView& c = v.chg;
     ChargeParams<R> q = charge_params<R>(v);
+    if (in_step) q.stamps = v.stamps;
     cudaError_t e = cudaMemsetAsync(c.hist, 0, (CHARGE_HIST + 2) * sizeof(unsigned long long), v.stream);
     if (e != cudaSuccess) return e;
     const long long n = (long long)v.nx_max * v.ny_max;
@@ -585,7 +586,7 @@ int k1_resident_warps(int nsm) {
     template cudaError_t launch_to_fortran<R>(const DeviceView&, const void*, double*);            \
     template cudaError_t launch_ctoprim<R>(const DeviceView&, double*, double*);                   \
     template cudaError_t launch_totals<R>(const DeviceView&, double*, int, double*);               \
-    template cudaError_t launch_charge<R>(const DeviceView&);                                      \
+    template cudaError_t launch_charge<R>(const DeviceView&, bool);                                      \
     template cudaError_t launch_charge_features<R>(const DeviceView&, float*);                     \
     template cudaError_t launch_charge_collect<R>(const DeviceView&, const float*, float*, unsigned long long*, long long); \
     template cudaError_t launch_planes_to_fortran<R>(const DeviceView&, const void*, int, double*);                  \

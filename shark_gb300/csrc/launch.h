@@ -153,8 +153,9 @@ template <typename R> cudaError_t launch_from_fortran(const DeviceView& v, const
 template <typename R> cudaError_t launch_to_fortran(const DeviceView& v, const void* src, double* dst_dev);
 template <typename R> cudaError_t launch_ctoprim(const DeviceView& v, double* q_dev, double* cs_dev);
 template <typename R> cudaError_t launch_totals(const DeviceView& v, double* part_dev, int nblocks, double* out_dev);
-// charging (K5) on the current state; resets the iteration histogram first
-template <typename R> cudaError_t launch_charge(const DeviceView& v);
+// charging (K5) on the current state; resets the iteration histogram first.  in_step: it leaves its end
+// in the step's stamps
+template <typename R> cudaError_t launch_charge(const DeviceView& v, bool in_step);
 // network features of every cell of the current state ([plane][SHARK_MLP_NFEAT] floats)
 template <typename R> cudaError_t launch_charge_features(const DeviceView& v, float* feat);
 // append (features, t) of the cells the last charging call converged to a training buffer

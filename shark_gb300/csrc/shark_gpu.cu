@@ -1927,7 +1927,7 @@ int32_t shark_gpu_charge(shark_gpu_ctx* c) {
     if (!c->uploaded) return fail(SHARK_ERR_STATE, "charge before upload");
     int32_t rc = seed_charges(c);
     if (rc) return rc;
-    cudaError_t e = is_mixed(c) ? shark::launch_charge<float>(c->v) : shark::launch_charge<double>(c->v);
+    cudaError_t e = is_mixed(c) ? shark::launch_charge<float>(c->v, false) : shark::launch_charge<double>(c->v, false);
     if (e != cudaSuccess) return fail(SHARK_ERR_CUDA, "charge: %s", cudaGetErrorString(e));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->chg_cold = false;
@@ -1985,7 +1985,7 @@ int32_t shark_gpu_mlp_collect(shark_gpu_ctx* c, int64_t capacity, int64_t* count
     shark::ChargeView& cv = c->v.chg;
     cv.use_seed = 0;
     cv.seed = nullptr;
-    cudaError_t e = is_mixed(c) ? shark::launch_charge<float>(c->v) : shark::launch_charge<double>(c->v);
+    cudaError_t e = is_mixed(c) ? shark::launch_charge<float>(c->v, false) : shark::launch_charge<double>(c->v, false);
     if (e != cudaSuccess) return fail(SHARK_ERR_CUDA, "charge: %s", cudaGetErrorString(e));
     c->chg_cold = false;
     if ((rc = features(c))) return rc;
