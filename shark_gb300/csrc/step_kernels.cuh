@@ -88,14 +88,13 @@ __device__ __forceinline__ unsigned long long clock_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// K2's start (its first block) and end (the latest of its blocks, of its last row of blocks without
-// growth): one store and one reduction that nothing waits for, in place of two timing events a step
-// (some 2 us each).
+// K2's start (its first block) and end (the latest of its blocks): a store, and a reduction a block that
+// nothing waits for, in place of two timing events a step (some 2 us each).
 __device__ __forceinline__ void stamp_start(unsigned long long* stamps) {
     if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) stamps[2] = clock_ns();
 }
-__device__ __forceinline__ void stamp_end(unsigned long long* stamps, bool every_block) {
-    if (threadIdx.x == 0 && (every_block || blockIdx.y == gridDim.y - 1)) atomicMax(stamps + 3, clock_ns());
+__device__ __forceinline__ void stamp_end(unsigned long long* stamps) {
+    if (threadIdx.x == 0) atomicMax(stamps + 3, clock_ns());
 }
 
 // Start of a kernel that may be launched before its predecessor in the stream has ended (launch_chained
@@ -1339,7 +1338,7 @@ __global__ void __launch_bounds__(K2D_THREADS, k2d_blocks(NS)) k_finalize(const 
     if (MODE == 2) return;
     block_reduce_dt(dtc, st, p.dt_next, p.status);
     if (REST) fill_ghost_images(p, p.u_next, gx, gy);
-    if (REST) stamp_end(p.stamps, GROW);
+    if (REST) stamp_end(p.stamps);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1790,7 +1789,7 @@ k_finalize_mixed(KParams<float> p) {
     if (MODE == 2) return;           // k_growth_f and MODE 3 follow
     block_reduce_dt_f(dtc, st, p.dt_next, p.status);
     if (REST) fill_ghost_images(p, p.u_next, gx, gy);
-    if (REST) stamp_end(p.stamps, GROW);
+    if (REST) stamp_end(p.stamps);
 }
 
 // Per-step preparation, one small block before the flux kernels: reset the next-dt slot and,
@@ -1811,7 +1810,6 @@ __device__ __forceinline__ double hash_uniform_d(unsigned long long seed, unsign
 static __global__ void k_ou_update(double* ou, const double* modes, float* ou_f, int nm, const double* dt, double sigma,
                                    double tcorr, unsigned long long seed, long long step, unsigned long long* stamps) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q == 0) stamps[1] = clock_ns();
     if (q >= 2 * nm) return;
     const double f = exp(-(*dt) / tcorr);
     const double sg = sigma * sqrt(1.0 - f * f);
@@ -1826,6 +1824,7 @@ static __global__ void k_ou_update(double* ou, const double* modes, float* ou_f,
             reinterpret_cast<float4*>(ou_f)[q] = make_float4(kx, ky, ky / kk, kx / kk);
         }
     }
+    if (q == 0) stamps[1] = clock_ns();
 }
 
 // It also posts the step's dt, the status word so far and then the step's number to pinned host
