@@ -116,21 +116,34 @@ static void growth_kernel_d(const KParams<double>& p, cudaStream_t st) {
     const long long nact = (long long)p.nx * (p.ndim == 2 ? p.ny : 1);
     k_growth_d<GL><<<(unsigned)((nact + cells - 1) / cells), GROWTH_D_THREADS, smem, st>>>(p);
 }
-// one wave of blocks, each through chunks of cells
-static void growth_kernel_f(const KParams<float>& p, int nsm, cudaStream_t st) {
-    const GrowthSmemF smem(p.ndust, p.gw.npair, p.gw.gL);
-    const void* kernel = p.ndust <= 16 ? (const void*)k_growth_f<5> : (const void*)k_growth_f<GROWTH_PAIR_SLOTS>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem.total);
-    int resident = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, 32 * GROWTH_F_WARPS, smem.total);
-    const long long chunks = (long long)((p.ng + p.nx + GROWTH_F_CELLS - 1) / GROWTH_F_CELLS) * (p.ndim == 2 ? p.ny : 1);
-    const unsigned blocks = (unsigned)std::min<long long>((long long)nsm * std::max(resident, 1), (chunks + GROWTH_F_WARPS - 1) / GROWTH_F_WARPS);
-    if (p.ndust <= 16) k_growth_f<5><<<blocks, 32 * GROWTH_F_WARPS, smem.total, st>>>(p);
-    else k_growth_f<GROWTH_PAIR_SLOTS><<<blocks, 32 * GROWTH_F_WARPS, smem.total, st>>>(p);
+// k_growth_f: one wave of blocks, each through chunks of cells.  The kernel's shared memory limit is one
+// for the process, so every context sets the most that any may need: a limit of the context's own
+// could fall between another thread's setting and its launch.
+template <typename R>
+cudaError_t plan_growth(DeviceView& v) {
+    if (!std::is_same<R, float>::value || !v.gw.on || (v.gw.mode & SHARK_GROWTH_FRAGMENTATION)) return cudaSuccess;
+    const GrowthSmemF smem(v.ndust, v.gw.npair, v.gw.gL);
+    const bool few = v.ndust <= 16;
+    const void* kernel = few ? (const void*)k_growth_f<5> : (const void*)k_growth_f<GROWTH_PAIR_SLOTS>;
+    const GrowthSmemF most = few ? GrowthSmemF(16, 136, GROWTH_SMEM_ROWS) : GrowthSmemF(GROWTH_MAX_DUST, GROWTH_MAX_PAIRS, GROWTH_SMEM_ROWS);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most.total);
+    int resident = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, 32 * GROWTH_F_WARPS, smem.total);
+    if (e != cudaSuccess) return e;
+    if (resident < 1) return cudaErrorLaunchOutOfResources;
+    const long long chunks = (long long)((v.ng + v.nx + GROWTH_F_CELLS - 1) / GROWTH_F_CELLS) * (v.ndim == 2 ? v.ny : 1);
+    v.growth_blocks = (unsigned)std::min<long long>((long long)v.nsm * resident, (chunks + GROWTH_F_WARPS - 1) / GROWTH_F_WARPS);
+    v.growth_smem = smem.total;
+    return cudaSuccess;
+}
+static void growth_kernel_f(const DeviceView& v, const KParams<float>& p) {
+    if (p.ndust <= 16) k_growth_f<5><<<v.growth_blocks, 32 * GROWTH_F_WARPS, v.growth_smem, v.stream>>>(p);
+    else k_growth_f<GROWTH_PAIR_SLOTS><<<v.growth_blocks, 32 * GROWTH_F_WARPS, v.growth_smem, v.stream>>>(p);
 }
 
 template <typename R, int MODE>
-static void finalize_dispatch(const KParams<R>& p, dim3 grid, int nsm, cudaStream_t st, bool chained) {
+static void finalize_dispatch(const DeviceView& v, const KParams<R>& p, dim3 grid, bool chained) {
+    const cudaStream_t st = v.stream;
     if (MODE == 0 && p.gw.on) {   // dust growth: run-time species count
         if (!(p.gw.mode & SHARK_GROWTH_FRAGMENTATION)) {
             // the drag, the growth kernel, the rest of K2
@@ -139,7 +152,7 @@ static void finalize_dispatch(const KParams<R>& p, dim3 grid, int nsm, cudaStrea
                 if (growth_lanes(p.ndust) == 8) growth_kernel_d<8>(p, st);
                 else growth_kernel_d<16>(p, st);
             } else {
-                growth_kernel_f(p, nsm, st);
+                growth_kernel_f(v, p);
             }
             finalize_launch<R, -1, 3>(p, grid, st, false);
             return;
@@ -399,7 +412,7 @@ cudaError_t launch_step(const DeviceView& v, int slot) {
     }
     if (v.time_kernels) cudaEventRecord(v.ev[2], v.stream);
     dim3 g2((v.nx + 255) / 256, v.ndim == 2 ? v.ny : 1, 1);
-    finalize_dispatch<R, 0>(p, g2, v.nsm, v.stream, chained && !strip_forks<R>(v, p) && v.nbuf == 2);
+    finalize_dispatch<R, 0>(v, p, g2, chained && !strip_forks<R>(v, p) && v.nbuf == 2);
     if (v.time_kernels) cudaEventRecord(v.ev[3], v.stream);
     return cudaGetLastError();
 }
@@ -414,7 +427,7 @@ cudaError_t launch_courant(const DeviceView& v, int slot) {
     p.dt_next = reinterpret_cast<unsigned long long*>(v.dt_slots + slot);
     k_prepare_step<<<1, 32, 0, v.stream>>>(p.dt_next, p.dt, p.dtstop, 0, 0, p.coef, nullptr, nullptr, nullptr, 0, v.stamps);
     dim3 g2((v.nx + 255) / 256, v.ndim == 2 ? v.ny : 1, 1);
-    finalize_dispatch<R, 1>(p, g2, v.nsm, v.stream, false);
+    finalize_dispatch<R, 1>(v, p, g2, false);
     return cudaGetLastError();
 }
 
@@ -579,6 +592,7 @@ int k1_resident_warps(int nsm) {
 
 #define SHARK_INSTANTIATE(R)                                                                       \
     template int k1_resident_warps<R>(int);                                                        \
+    template cudaError_t plan_growth<R>(DeviceView&);                                              \
     template cudaError_t launch_step<R>(const DeviceView&, int);                                   \
     template cudaError_t launch_courant<R>(const DeviceView&, int);                                \
     template cudaError_t launch_boundaries<R>(const DeviceView&);                                  \

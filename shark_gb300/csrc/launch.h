@@ -113,6 +113,8 @@ struct DeviceView {
     CUtensorMap k1_gas[3], k1_dust[3];
     int k1_warps;               // warps of one wave of the mixed 2D K1: SMs x resident blocks x warps per block
     int nsm;                    // SMs of the device
+    unsigned growth_blocks;     // k_growth_f's launch (mixed growth without fragmentation, plan_growth)
+    int growth_smem;
     bool uniform;               // Cartesian grid with the same dx1, dx2, surf1, surf2, vol in every column
     bool cs_uniform;            // the same isothermal sound speed in every column
     // reference gas density of the mixed fused flux kernel: the mean active density of the first
@@ -140,6 +142,8 @@ int32_t set_error(int32_t code, const char* msg);
 // orbital remap moves that into u[(cur+2) % 3], where the finalize kernel completes the step.
 inline int next_cur(const DeviceView& v) { return v.nbuf == 3 ? (v.cur + 2) % 3 : 1 - v.cur; }
 
+// the growth kernel's launch shape, once at the context's start
+template <typename R> cudaError_t plan_growth(DeviceView& v);
 // one full step on view.u[view.cur] -> view.u[next_cur(view)]; dt read from slot `slot`, next dt
 // written to slot 1-slot.  Returns a cudaError_t.
 template <typename R> cudaError_t launch_step(const DeviceView& v, int slot);

@@ -1405,6 +1405,7 @@ int32_t shark_gpu_init(const shark_gpu_config* cfg, shark_gpu_ctx** out) {
     INIT_TRY(cudaMalloc(&c->tot_out, 4 * (v.ndust + 1) * sizeof(double)));
     for (auto& e : v.ev) e = nullptr;
     v.time_kernels = false;
+    INIT_TRY(is_mixed(c) ? shark::plan_growth<float>(v) : shark::plan_growth<double>(v));
     INIT_TRY(cudaStreamSynchronize(c->stream));
 #undef INIT_TRY
     *out = c;
