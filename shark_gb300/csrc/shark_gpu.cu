@@ -1234,14 +1234,17 @@ int32_t shark_gpu_init(const shark_gpu_config* cfg, shark_gpu_ctx** out) {
     float invf[SHARK_MAX_DUST] = {0};   // FP32 copy of 1/C_k for the mixed path's coefficients
     {
         // 1/C_k of the stopping times t_k = C_k / F_cell that K2's mixed path multiplies out:
-        // dustyTurb C_k = St_0,k L rho_0 (F = c_s rho), polar disk (Epstein on the midplane density)
-        // C_k = sqrt(pi gamma/8) rho_grain s_k (F = rho/hs c_s)
+        // dustyTurb C_k = St_0,k L rho_0 (F = c_s rho), Epstein C_k = sqrt(pi gamma/8) rho_grain s_k (the disks'
+        // F = rho/hs c_s, else F = rho c_s).  A grain of no size stops at once: dt/t_k is infinite, as where
+        // it is divided, and the step's status tells of it.
+        const bool sized = cfg->setup == SHARK_SETUP_DISK_POLAR || cfg->setup == SHARK_SETUP_DISK_CART ||
+                           cfg->setup == SHARK_SETUP_DUSTYTURB;   // validated: C_k = 0 only without the drag
         double inv[SHARK_MAX_DUST] = {0};
         for (int k = 0; k < cfg->ndust; ++k) {
             const double C = cfg->setup == SHARK_SETUP_DUSTYTURB
                                  ? cfg->dust_stokes[k] * cfg->box_l * cfg->turb_rho0
                                  : std::sqrt(kPi * cfg->gamma / 8.0) * cfg->rhograin * cfg->dust_size[k];
-            inv[k] = C != 0.0 ? 1.0 / C : 0.0;
+            inv[k] = C != 0.0 || !sized ? 1.0 / C : 0.0;
             invf[k] = (float)inv[k];
         }
         INIT_TRY(cudaMemcpy(c->species + 4 * SHARK_MAX_DUST, inv, SHARK_MAX_DUST * sizeof(double), cudaMemcpyHostToDevice));
