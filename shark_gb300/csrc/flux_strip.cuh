@@ -139,7 +139,8 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                 q[0] = qrho;
             } else {
                 const R y = rcp64(rho);
-                vx = div64(px, rho, y); vy = div64(py, rho, y); vz = div64(pz, rho, y);
+                vx = px; vy = py; vz = pz;
+                Over<R>(rho, y).all(vx, vy, vz);
                 q[0] = max64_pos(rho, smallR);
                 if (iso) {
                     c = cs_at(row);
@@ -158,8 +159,8 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                 const R ir = R(1) / us[0];
                 q[1] = us[1] * ir; q[2] = us[2] * ir; q[3] = us[3] * ir;
             } else {
-                const R y = rcp64(us[0]);
-                q[1] = div64(us[1], us[0], y); q[2] = div64(us[2], us[0], y); q[3] = div64(us[3], us[0], y);
+                q[1] = us[1]; q[2] = us[2]; q[3] = us[3];
+                Over<R>(us[0]).all(q[1], q[2], q[3]);
             }
         }
     };
@@ -244,7 +245,7 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
             }
             R dpx_r, dpy_r;
             if constexpr (FAST) { const R ir = R(1) / r_rho; dpx_r = dpx * ir; dpy_r = dpy * ir; }
-            else { const R y = rcp64(r_rho); dpx_r = div64(dpx, r_rho, y); dpy_r = div64(dpy, r_rho, y); }
+            else { dpx_r = dpx; dpy_r = dpy; Over<R>(r_rho).all(dpx_r, dpy_r); }
             R su0 = -u * dux - v * duy - dpx_r;
             R sv0 = -u * dvx - v * dvy - dpy_r;
             R sw0 = -u * dwx - v * dwy;
@@ -436,8 +437,8 @@ __device__ void flux_strip(const KParams<R>& p, int s, int bx, int by) {
                     } else {
                         // a component without a force keeps its momentum and its energy
                         const R y = rcp64(rho), rdt = rho * dt;
-                        const R e1 = div64(half * sq(uu[1]), rho, y), e2 = div64(half * sq(uu[2]), rho, y),
-                                e3 = div64(half * sq(uu[3]), rho, y);
+                        R e1 = half * sq(uu[1]), e2 = half * sq(uu[2]), e3 = half * sq(uu[3]);
+                        Over<R>(rho, y).all(e1, e2, e3);
                         eo = e1 + e2 + e3;
                         uu[1] = uu[1] + rdt * f1;
                         R n2 = e2, n3 = e3;

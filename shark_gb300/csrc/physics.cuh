@@ -57,7 +57,8 @@ __device__ __forceinline__ float limit_mc_f(float l, float r) {
 }
 
 // FP64 forms of the limiters, bit for bit those of slope_limiters.f90's operations with fewer FP64
-// instructions:
+// instructions (but where the product of the slopes underflows, below 1e-162 each: its sign decides here,
+// there the zero that it rounds to):
 // compares and sign choices on the bit patterns, 1.5 min(|l|, |r|) for the smaller of the two
 // products (rounding keeps their order), one division by half the sum for 2 l r / (l + r).  What is
 // not a number comes out as those operations leave it.
@@ -172,8 +173,9 @@ __device__ __forceinline__ DustFlux<R> dust_hll(R rho_lft, R u_lft, R v_lft, R w
     return f;
 }
 
-// FP64 forms of the solvers, rounding as the reference's operations do with fewer FP64 instructions: one reciprocal for the quotients of a denominator, minima, maxima and case choices
-// on the bit patterns, and the HLLC's energy and star state for the sampled side only.  y1 = rcp64 of gamma - 1.
+// FP64 forms of the solvers, rounding as the reference's operations do with fewer FP64 instructions: one
+// reciprocal for the quotients of a denominator, minima, maxima and case choices on the bit patterns, and
+// the HLLC's energy and star state for the sampled side only.  y1 = rcp64 of gamma - 1.
 __device__ __forceinline__ double gas_energy_d(double g1, double y1, double rho, double u, double v, double w, double P) {
     const double hr = 0.5 * rho;
     return div64_const(P, g1, y1) + hr * sq(u) + hr * sq(v) + hr * sq(w);
@@ -204,11 +206,12 @@ __device__ __forceinline__ GasFlux<double> gas_hll_d(double gamma, double y1, do
     const Over<double, WHERE> by_b(Sr - Sl);
     GasFlux<double> f;
     f.inside = by_b.inside();
-    f.rho = by_b(Sr * ml - Sl * mr + ss * (rr - rl));
-    f.mn = by_b(Sr * (rl * sq(ul) + Pl) - Sl * (rr * sq(ur) + Pr) + ss * (mr - ml));
-    f.mt = by_b(Sr * (ml * vl) - Sl * (mr * vr) + ss * (rr * vr - rl * vl));
-    f.mz = by_b(Sr * (ml * wl) - Sl * (mr * wr) + ss * (rr * wr - rl * wl));
-    f.e = by_b(Sr * ((El + Pl) * ul) - Sl * ((Er + Pr) * ur) + ss * (Er - El));
+    f.rho = Sr * ml - Sl * mr + ss * (rr - rl);
+    f.mn = Sr * (rl * sq(ul) + Pl) - Sl * (rr * sq(ur) + Pr) + ss * (mr - ml);
+    f.mt = Sr * (ml * vl) - Sl * (mr * vr) + ss * (rr * vr - rl * vl);
+    f.mz = Sr * (ml * wl) - Sl * (mr * wr) + ss * (rr * wr - rl * wl);
+    f.e = Sr * ((El + Pl) * ul) - Sl * ((Er + Pr) * ur) + ss * (Er - El);
+    by_b.all(f.rho, f.mn, f.mt, f.mz, f.e);
     return f;
 }
 // solver_hllc (src/solver/solvers.f90:308-500): RAMSES-style HLLC with the wave speeds clipped to
@@ -222,8 +225,8 @@ __device__ __forceinline__ GasFlux<double> gas_hllc_d(double gamma, double y1, d
     const double Sl = min64_0(min64(ul, ur) - cm), Sr = max64_0(max64(ul, ur) + cm);
     const double hl = rl * (ul - Sl), hr = rr * (Sr - ur);
     const Over<double, WHERE> by_b(hr + hl);
-    const double us = by_b(hr * ur + hl * ul + (Pl - Pr));
-    const double Ps = by_b(hr * Pl + hl * Pr + hl * hr * (ul - ur));
+    double us = hr * ur + hl * ul + (Pl - Pr), Ps = hr * Pl + hl * Pr + hl * hr * (ul - ur);
+    by_b.all(us, Ps);
     bool inside = by_b.inside();
     const bool left = is_pos(us);
     const double S = left ? Sl : Sr, rho = left ? rl : rr, u = left ? ul : ur, v = left ? vl : vr, w = left ? wl : wr;
@@ -233,10 +236,11 @@ __device__ __forceinline__ GasFlux<double> gas_hllc_d(double gamma, double y1, d
     if (left || is_pos(Sr)) {   // Sl is at most 0, so the left state itself is never sampled
         const double d = S - u;
         const Over<double, WHERE> by_c(S - us);
-        ro = by_c(rho * d);
+        ro = rho * d;
         uo = us;
         Po = Ps;
-        eo = by_c(d * E - P * u + Ps * us);
+        eo = d * E - P * u + Ps * us;
+        by_c.all(ro, eo);
         inside = inside && by_c.inside();
     }
     GasFlux<double> f;
@@ -283,10 +287,11 @@ __device__ __forceinline__ DustFlux<double> dust_hll_d(double rl, double ul, dou
         const Over<double, WHERE> by_b(b);
         const double ss = Sr * Sl, ml = rl * ul, mr = rr * ur;
         f.inside = by_b.inside();
-        f.rho = by_b(Sr * ml - Sl * mr + ss * (rr - rl));
-        f.mn = by_b(Sr * (rl * sq(ul)) - Sl * (rr * sq(ur)) + ss * (mr - ml));
-        f.mt = by_b(Sr * (ml * vl) - Sl * (mr * vr) + ss * (rr * vr - rl * vl));
-        f.mz = by_b(Sr * (ml * wl) - Sl * (mr * wr) + ss * (rr * wr - rl * wl));
+        f.rho = Sr * ml - Sl * mr + ss * (rr - rl);
+        f.mn = Sr * (rl * sq(ul)) - Sl * (rr * sq(ur)) + ss * (mr - ml);
+        f.mt = Sr * (ml * vl) - Sl * (mr * vr) + ss * (rr * vr - rl * vl);
+        f.mz = Sr * (ml * wl) - Sl * (mr * wr) + ss * (rr * wr - rl * wl);
+        by_b.all(f.rho, f.mn, f.mt, f.mz);
     }
     return f;
 }
@@ -297,8 +302,8 @@ __device__ __forceinline__ DustFlux<double> dust_hllc_d(double rl, double ul, do
     const double Sl = min64_0(min64(ul, ur) - cm), Sr = max64_0(max64(ul, ur) + cm);
     const double hl = rl * (ul - Sl), hr = rr * (Sr - ur);
     const Over<double, WHERE> by_b(hr + hl);
-    const double us = by_b(hr * ur + hl * ul);
-    const double Ps = by_b(hl * hr * (ul - ur));
+    double us = hr * ur + hl * ul, Ps = hl * hr * (ul - ur);
+    by_b.all(us, Ps);
     bool inside = by_b.inside();
     const bool left = is_pos(us);
     const double S = left ? Sl : Sr, rho = left ? rl : rr, u = left ? ul : ur, v = left ? vl : vr, w = left ? wl : wr;
