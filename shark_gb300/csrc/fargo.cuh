@@ -6,7 +6,8 @@
 // rotation of the ring, so it cannot run in place: the kernel reads the flux kernel's output and
 // writes a third state buffer.
 //
-// The remap moves each value once, so memory bounds it.  A thread owns one column of one conserved
+// The remap moves each value once, so memory bounds it (mixed, 4.2 TB/s); in FP64 the limiter's and the
+// remap's operations do (the FP64 pipe 81 % busy).  A thread owns one column of one conserved
 // variable and marches down FARGO_ROWS output rows with its window of donor cells in registers:
 // an output costs one load, one limited slope (the lower donor's is the next output's upper one) and
 // one store; the loads of FARGO_BATCH rows are in flight together.  A warp's 32 lanes are adjacent

@@ -252,7 +252,7 @@ __device__ __forceinline__ float growth_dv_f(const GrowthDev& g, const GrowthRun
 }
 
 // Mixed-precision form of the cell update with fragmentation, one thread per cell (without
-// fragmentation the warp-per-cell form in the mixed K2 runs instead): the same algorithm with the
+// fragmentation k_growth_f, a warp per cell, runs instead): the same algorithm with the
 // relative velocities, rates, mass bookkeeping and sub-steps in FP32 (the state is FP32 on this
 // path), the elapsed growth time in FP64.  Masses are counted in units of the smallest grain mass
 // and rates in grains of that mass, so the bookkeeping stays in FP32 range whatever the code units.

@@ -56,7 +56,8 @@ struct StepPost {
     long long step;
 };
 
-// Longest FARGO ring taken: what one block's shared memory holds as rows of 64 bytes.
+// Longest FARGO ring taken: a limit of the library's configurations.  (The remap's offsets within a ring
+// are below 2^31 elements as a plane's are.)
 constexpr int FARGO_MAX_NY = 200 * 1024 / 64;
 // One column's FARGO shift in a step: the first output row's lower donor row and the weights of the
 // donors' values and slopes.

@@ -530,8 +530,8 @@ double charge_psi0(double thetai) {
     return psi0;
 }
 
-// Host tables of the charging kernel: [hs | trow | tau | alpha | l2 | mkum | ak] and the
-// constants of the view.  Temperature rows: one per column for the polar disk (T from the
+// Host tables of the charging kernel: [hs | trow | tau | alpha | ptau | ntau | l2 | mkum | nfac | npl | wk]
+// and the constants of the view.  Temperature rows: one per column for the polar disk (T from the
 // isothermal cs through cs_eos), one row (T_cloud) for dustyTurb.
 void build_charge_tables(const shark_gpu_config& c, const Columns& col, int nx_max, std::vector<double>& h,
                          shark::ChargeView& cv, size_t off[11]) {

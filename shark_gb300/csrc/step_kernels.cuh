@@ -1,13 +1,16 @@
 // step_kernels.cuh -- the device kernels of one `solve` step (src/solver/solve.f90:10-181).
 //
 //   k_boundaries   apply_boundaries of the setup (ghost fill), before anything reads the halo
-//   k_flux         K1: per (tile, species): ctoprim on the halo tile, limited slopes, MUSCL-Hancock
-//                  predictor, Riemann fluxes (HLLC/HLL/LLF gas, Huang-Bai/LLF/HLL dust), force
-//                  kick, conservative update and the local source terms, in one pass through
-//                  shared memory.  No qm/qp/flux array ever reaches HBM.
-//   k_finalize     K2: per cell, all species: implicit multi-species drag (FP64 arithmetic),
-//                  dust floor, setup_inloop, status checks, and the CFL dt of the NEXT step
-//                  (courant on the final state: warp shuffle -> block -> one atomicMin).
+//   k_prepare_step the step's dt and status to the host, the next dt's slot, constant drag coefficients
+//   k_flux_*       K1: per species: ctoprim, limited slopes, MUSCL-Hancock predictor, Riemann fluxes
+//                  (HLLC/HLL/LLF gas, Huang-Bai/LLF/HLL/HLLC dust), force kick, conservative update
+//                  and the local source terms, a warp marching over its columns with the rows in
+//                  registers (flux_line.cuh in 1D, flux_strip*.cuh in 2D).  No qm/qp/flux array ever
+//                  reaches HBM.
+//   k_finalize*    K2: per cell, all species: implicit multi-species drag, dust floor, setup_inloop,
+//                  status checks, the CFL dt of the NEXT step (courant on the final state: warp
+//                  shuffle -> block -> one atomicMin) and the next step's ghost cells.
+//   k_growth_*     dust growth without fragmentation, between K2's drag and the rest of it
 //
 // Device state layout: variable-major planes, each plane ny_max rows of `pitch` elements
 // (pitch >= nx_max, rounded up to 32 elements so every row starts 128-byte aligned), ghost cells
@@ -234,7 +237,7 @@ namespace shark {
 // K2: drag + floor + inloop + status + next-step CFL dt, one thread per active cell.
 // NS > 0: compile-time species count (register arrays); NS < 0: run-time count.
 // MODE 0: full finalize; MODE 1: dt only (first step after an upload); MODES 2 and 3: the drag with
-// its floor and heating, and the rest, as two launches with k_growth_d between them (FP64).
+// its floor and heating, and the rest, as two launches with the growth kernel between them.
 // ---------------------------------------------------------------------------------------------
 
 // Producer-side boundary fill: the block with an active cell within nghost of a periodic or
@@ -598,7 +601,7 @@ __device__ __noinline__ unsigned grow_in_finalize(const KParams<R>& p, R* u, int
 //     and the part of dt still to integrate is kept as an FP32 fraction (the last sub-step takes all
 //     of it).  A cell that needs more sub-steps goes on by itself;
 //  3. the cells' densities are written back together.
-// Bound by instruction issue (71 % of the slots).  The loops over pairs are not unrolled: unrolled
+// Bound by instruction issue (74 % of the slots at 32 species, 76 % at 16).  The loops over pairs are not unrolled: unrolled
 // they overflowed the instruction cache (the largest stall).  As a phase of K2 with each cell's
 // inputs read by lane = bin and every turbulent case formed for every pair, K2 took 2.09 ms on the
 // disk 512 x 1024 x 16 and 5.20 ms on the driven box 768^2 x 32; unrolled per-cell warps 1.06 and
@@ -1437,8 +1440,8 @@ __device__ __forceinline__ void drag_coeffs_mix(double a, float& r, float& w) {
 }
 
 // Threads per block of the mixed K2 without growth: small blocks, so that the warps of a block
-// waiting at the dt reduction's barrier and the last wave hold fewer idle slots (the growth
-// variant keeps 256 threads: its block-cooperative phase is laid out for 8 warps).
+// waiting at the dt reduction's barrier and the last wave hold fewer idle slots.  The variant with
+// fragmenting growth within it takes 256: a cell's sub-cycle in one thread outweighs the reduction.
 constexpr int K2M_THREADS = 128;
 
 // Blocks per SM: 8 species at 5 blocks of 128 threads (96 registers), measured best of 4-6; a gas
@@ -1448,7 +1451,7 @@ constexpr int K2M_THREADS = 128;
 // adiabatic box (46.8 -> 44.6) and lose on the isothermal one (40.8 -> 45.1).
 template <int NS, int MODE, bool GROW = false>
 __global__ void __launch_bounds__(GROW ? 256 : K2M_THREADS,
-                                  GROW ? ((NS >= 8) ? 2 : 3) : (NS == 0 ? 10 : NS == 1 || NS == 2 ? 8 : NS == 8 ? 5 : ((NS > 8) ? 2 : 3) * (256 / K2M_THREADS)))
+                                  GROW ? 3 : (NS == 0 ? 10 : NS == 1 || NS == 2 ? 8 : NS == 8 ? 5 : ((NS > 8) ? 2 : 3) * (256 / K2M_THREADS)))
 k_finalize_mixed(KParams<float> p) {
     constexpr int NMAX = NS > 0 ? NS : 1;
     const int N = NS >= 0 ? NS : p.ndust;
