@@ -14,6 +14,7 @@ import numpy as np
 import pytest
 
 from shark_gb300 import build as B, config as K, setups
+from oracle.oracle import Oracle
 from tests.test_gpu_parity import active, run_pair
 
 pytestmark = pytest.mark.gpu
@@ -184,3 +185,28 @@ def test_dust_density_below_the_normal_range(solverdust):
     a, b = active(cfg, ug), active(cfg, uo)
     assert np.isfinite(a).all()
     np.testing.assert_allclose(a, b, rtol=1e-12, atol=1e-305)
+
+
+@pytest.mark.parametrize("setup", ["sod", "si"])
+def test_stopping_times_below_the_normal_range(setup):
+    """dt/t_k near the largest number: 1 + dt/t_k has a reciprocal below the normal range, the drag's
+    weight is 1 and the dust moves with the gas."""
+    if setup == "sod":
+        cfg, u0 = setups.sod(nx=64, ndust=2, rho_r=1.0, P_r=1.0)
+    else:
+        cfg, u0 = setups.si(n=16, ndust=2)
+    u = u0.reshape(cfg.nvar, -1)
+    u[7:9] += 0.01 * u[5:7]          # the dust's x velocities
+    o = Oracle(cfg)
+    o.set_u(u0)
+    ts = o.solve() / 8e307
+    for k in range(2):
+        if setup == "si":
+            cfg.dust_tstop[k] = ts
+        else:                         # t = sqrt(pi gamma / 8) rhograin s / (rho c_s) with rho = P = 1
+            cfg.dust_size[k] = ts * np.sqrt(cfg.gamma) / (np.sqrt(np.pi * cfg.gamma / 8.0) * cfg.rhograin)
+    dto, dtg, uo, ug, st = run_pair(cfg, u0, 1)
+    assert st == 0
+    np.testing.assert_allclose(dtg, dto, rtol=1e-14, atol=0)
+    assert np.isfinite(uo).all()
+    np.testing.assert_allclose(active(cfg, ug), active(cfg, uo), rtol=1e-12, atol=1e-15)
