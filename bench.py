@@ -411,7 +411,7 @@ def run_gpu(args):
         "timed_runs_ms": runs,
         "kernel_ms": {"pre_flux": kt[0], "flux_update": kt[1], "drag_dt_ghosts": kt[2], "step": kt[3]},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
-                     "frac": achieved / hbm, "traffic": traffic, "kernel": "k_flux (K1 fused flux/update)",
+                     "frac": achieved / hbm, "traffic": traffic, "kernel": "k_flux_strip_mixed (K1 fused flux/update)",
                      "peak_kind": peak_kind,
                      "algorithmic_bytes_per_launch": alg_bytes_k1,
                      "drag_kernel_bytes_per_cell": alg_bytes_k2 // ncell,
